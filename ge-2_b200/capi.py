@@ -123,6 +123,9 @@ def load_library():
                                                      C.c_int64, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.ge2_tournament_select.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int,
                                           C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.ge2_eval_workspace_bytes.restype = C.c_size_t
+    lib.ge2_eval_workspace_bytes.argtypes = [C.POINTER(EvalDesc)]
+    lib.ge2_eval_ranks.argtypes = [C.POINTER(EvalDesc), C.c_void_p]
     _lib = lib
     return lib
 
@@ -336,13 +339,10 @@ def eval_ranks(decoder, node_emb, edges, rel=None, inv_rel=None, dst_filter=None
     import torch
 
     lib = load_library()
-    lib.ge2_eval_workspace_bytes.restype = C.c_size_t
-    lib.ge2_eval_workspace_bytes.argtypes = [C.POINTER(EvalDesc)]
-    lib.ge2_eval_ranks.argtypes = [C.POINTER(EvalDesc), C.c_void_p]
     B, cols = edges.shape
     dev = node_emb.device
     d = EvalDesc()
-    d.decoder = {"DISTMULT": 0, "DOT": 0, "COMPLEX": 1}[decoder]
+    d.decoder = DECODER[decoder]
     d.has_relations = int(cols == 3 and rel is not None)
     d.use_inverse = int(d.has_relations and inv_rel is not None)
     d.D, d.B, d.num_nodes = node_emb.shape[1], B, node_emb.shape[0]
@@ -355,8 +355,8 @@ def eval_ranks(decoder, node_emb, edges, rel=None, inv_rel=None, dst_filter=None
     d.neg_ids, d.num_negs = ptr(neg_ids), (neg_ids.numel() if neg_ids is not None else 0)
     d.dst_filter, d.dst_filter_n = ptr(dst_filter), (dst_filter.shape[0] if dst_filter is not None else 0)
     d.src_filter, d.src_filter_n = ptr(src_filter), (src_filter.shape[0] if src_filter is not None else 0)
-    dst_ranks = torch.zeros(B, dtype=torch.int64, device=dev)
-    src_ranks = torch.zeros(B, dtype=torch.int64, device=dev) if d.use_inverse else None
+    dst_ranks = torch.empty(B, dtype=torch.int64, device=dev)  # every entry is written by the call
+    src_ranks = torch.empty(B, dtype=torch.int64, device=dev) if d.use_inverse else None
     d.dst_ranks, d.src_ranks = ptr(dst_ranks), ptr(src_ranks)
     d.status = ptr(status)
     ws = torch.empty(int(lib.ge2_eval_workspace_bytes(C.byref(d))), dtype=torch.uint8, device=dev)

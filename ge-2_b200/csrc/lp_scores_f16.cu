@@ -55,7 +55,7 @@
 #include <algorithm>
 
 #include "lp_internal.cuh"
-#include "tc_ptx.cuh"
+#include "tc_pipe.cuh"
 
 namespace ge2 {
 namespace {
@@ -69,8 +69,6 @@ constexpr int kThreads = 736;           // lse pass: 16 softmax warps + 4 combin
 constexpr int kThreadsB = 864;          // gradient pass: 16 softmax warps + 8 drain warps (16-19 and 23-26) + TMA warp + two MMA warps
 constexpr int kDrainWarps = 8;
 constexpr int kDrainWarp0 = kSoftmaxWarps, kTmaWarp = kDrainWarp0 + 4, kMmaWarp = kTmaWarp + 1, kGradWarp = kMmaWarp + 1;
-constexpr int kBlockBytes = 128 * 128;  // one 64-half column block of 128 rows
-constexpr int kMmaK = 16;               // k extent of one kind::f16 MMA (32 bytes)
 constexpr int kStages = 3;              // Y ring depth of the gradient pass (shared memory is full there: X, 3 Y, W, 16 staging slabs)
 constexpr int kStagesA = 5;             // Y ring depth of the lse pass (no W tiles: room for a deeper ring, which the load latency wants)
 constexpr int kMaxStages = kStagesA;
@@ -119,22 +117,6 @@ struct Layout {
     static_assert(kDynamicB <= 227 * 1024, "gradient pass exceeds the shared memory of an SM");
 };
 
-// Descriptors are built once per tile; a k-step only adds its byte offset (>> 4) to the start-address field, which cannot
-// carry out of the field because shared-memory addresses stay below 256 KB.
-// K-major operand: k-step `ks` (16 halves = 32 bytes) sits in column block ks/4 at byte (ks%4)*32; 8-row groups are 1024 bytes apart
-__device__ __forceinline__ uint64_t desc_kmajor_base(uint32_t tile) { return smem_desc_sw128(tile, 16, 1024); }
-__host__ __device__ constexpr uint64_t koff_kmajor(int ks) { return (uint64_t)(((ks >> 2) * kBlockBytes + (ks & 3) * 32) >> 4); }
-// MN-major operand: k-step `ks` is rows [16 ks, 16 ks + 16) = two 8-row groups of 1024 bytes; the 64-element MN blocks are
-// kBlockBytes apart
-__device__ __forceinline__ uint64_t desc_mnmajor_base(uint32_t tile) { return smem_desc_sw128(tile, kBlockBytes, 1024); }
-__host__ __device__ constexpr uint64_t koff_mnmajor(int ks) { return (uint64_t)((ks * 2048) >> 4); }
-
-// byte offset of the 16-byte chunk holding halves [col, col + 8) of row `row` in the swizzled block layout (col % 8 == 0)
-__device__ __forceinline__ uint32_t swz_chunk_offset(int row, int col) {
-    const int chunk = (col & 63) >> 3;
-    return (uint32_t)((col >> 6) * kBlockBytes + row * 128 + ((chunk ^ (row & 7)) << 4));
-}
-
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
@@ -145,22 +127,6 @@ __device__ __forceinline__ float exp2f_fast(float x) {  // one MUFU.EX2; 2^-inf 
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Bounded wait that also gives up as soon as another role has raised the abort flag.
-__device__ __forceinline__ bool pipe_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
-    for (uint32_t i = 0; i < (1u << 20); i++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (i > 64) __nanosleep(i > 4096 ? 256 : 32);  // long waits (a role idle for a whole block) must not eat issue slots
-        if ((i & 255u) == 255u && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    or_status(status, GE2_STATUS_PIPE_TIMEOUT);
-    return false;
-}
-
 // what a CTA needs to know about one unit of the lse pass
 struct UnitA {
     int item, tile, rb, zc;
@@ -211,14 +177,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int n_iter = ue - ub;
     constexpr int NB = LY::NB;
     auto wait = [&](int bar, uint32_t parity) { return pipe_wait(&bars[bar], parity, s_abort, d.status); };
-    auto warp_wait = [&](int bar, uint32_t parity) -> bool {  // one lane polls; then every lane observes the completed phase itself
-        if (__all_sync(0xffffffffu, mbar_try_wait(&bars[bar], parity) ? 1 : 0)) return true;  // usually complete already
-        int ok = 1;
-        if (lane == 0) ok = wait(bar, parity) ? 1 : 0;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (ok) ok = mbar_try_wait(&bars[bar], parity) ? 1 : 0;
-        return __all_sync(0xffffffffu, ok) != 0;
-    };
+    auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, d.status); };
     // TMA producer state: runs a few units before the block-wide barrier (their latency overlaps the allocation of tensor
     // memory), the rest afterwards
     int tma_it = 0, tma_sg = -1;
@@ -565,14 +524,7 @@ __global__ void __launch_bounds__(kThreadsB, 1)
     const int n_iter = ue - ub;
     constexpr int NB = LY::NB;
     auto wait = [&](int bar, uint32_t parity) { return pipe_wait(&bars[bar], parity, s_abort, d.status); };
-    auto warp_wait = [&](int bar, uint32_t parity) -> bool {
-        if (__all_sync(0xffffffffu, mbar_try_wait(&bars[bar], parity) ? 1 : 0)) return true;  // usually complete already
-        int ok = 1;
-        if (lane == 0) ok = wait(bar, parity) ? 1 : 0;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (ok) ok = mbar_try_wait(&bars[bar], parity) ? 1 : 0;
-        return __all_sync(0xffffffffu, ok) != 0;
-    };
+    auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, d.status); };
     constexpr int kBarDqFull = kBarAccFull, kBarDqEmpty = kBarAccEmpty;
     // Only real columns of dQ / dK leave the SM: D / 32 full slabs of 32 columns, then one narrow slab (its own tensor map,
     // dense rows of `tail` floats) for the remainder rounded up to 4.  Worker warp w drains slab w / 4 of its lane quarter.
@@ -930,59 +882,6 @@ __global__ void __launch_bounds__(kThreadsB, 1)
     }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point lookup: the library does not link libcuda, so it still
-// loads on a machine without a driver
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (fn == nullptr) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) return nullptr;
-        fn = (EncodeTiledFn)p;
-    }
-    return fn;
-}
-
-// [S*C matrices][rows][ld halves] viewed as a 3-D tensor; box = 64 halves x 128 rows of one matrix, 128-byte swizzle,
-// rows past the matrix end read as zero
-int make_map(CUtensorMap* map, __half* base, int ld, int rows, int mats) {
-    EncodeTiledFn fn = encode_fn();
-    if (fn == nullptr) return GE2_ERR_CUDA;
-    cuuint64_t dims[3] = {(cuuint64_t)ld, (cuuint64_t)rows, (cuuint64_t)mats};
-    cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)rows * ld * 2};
-    cuuint32_t box[3] = {64, 128, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        g_last_cuda_error = (int)r;
-        return GE2_ERR_CUDA;
-    }
-    return GE2_OK;
-}
-
-// dK / dQ [S*C][rows][ld floats] as a 3-D tensor for the stores: box = 32 floats x 32 rows with the 128-byte swizzle, or
-// (narrow slab) box_cols < 32 floats x 32 rows, dense
-int make_map_f32_slab(CUtensorMap* map, float* base, int ld, int rows, int mats, int box_cols = 32) {
-    EncodeTiledFn fn = encode_fn();
-    if (fn == nullptr) return GE2_ERR_CUDA;
-    cuuint64_t dims[3] = {(cuuint64_t)ld, (cuuint64_t)rows, (cuuint64_t)mats};
-    cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)rows * ld * 4};
-    cuuint32_t box[3] = {(cuuint32_t)box_cols, 32, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        g_last_cuda_error = (int)r;
-        return GE2_ERR_CUDA;
-    }
-    return GE2_OK;
-}
-
 int env_int(const char* name, int fallback) {
     const char* e = getenv(name);
     return e != nullptr ? atoi(e) : fallback;
@@ -993,26 +892,26 @@ int launch(const LpKernelArgs& a, cudaStream_t stream) {
     if (a.L.Qh == nullptr || a.L.Kh == nullptr || a.L.lse2s == nullptr || a.L.item_ctr == nullptr) return GE2_ERR_WORKSPACE;
     const int ZC = a.L.S * a.d.C;
     CUtensorMap tmQ, tmK;
-    int rc = make_map(&tmQ, a.L.Qh, DP, a.L.npc, ZC);
+    int rc = make_operand_map(&tmQ, a.L.Qh, false, DP, a.L.npc, ZC);
     if (rc != GE2_OK) return rc;
-    rc = make_map(&tmK, a.L.Kh, DP, a.d.N, ZC);
+    rc = make_operand_map(&tmK, a.L.Kh, false, DP, a.d.N, ZC);
     if (rc != GE2_OK) return rc;
     CUtensorMap tmDK;
-    rc = make_map_f32_slab(&tmDK, a.L.dK, DP, a.d.N, ZC);
+    rc = make_slab_map(&tmDK, a.L.dK, DP, a.d.N, ZC);
     if (rc != GE2_OK) return rc;
     CUtensorMap tmDKt = tmDK;  // narrow slab for the last D % 32 columns (rounded up to 4), when there are any
     const int tail_cols = ((a.d.D % 32) + 3) & ~3;
     if (tail_cols > 0 && tail_cols < 32) {
-        rc = make_map_f32_slab(&tmDKt, a.L.dK, DP, a.d.N, ZC, tail_cols);
+        rc = make_slab_map(&tmDKt, a.L.dK, DP, a.d.N, ZC, tail_cols);
         if (rc != GE2_OK) return rc;
     }
     // dQ [S*C chunks][rows per chunk][ld floats]: the same slab shapes
     CUtensorMap tmDQ, tmDQt;
-    rc = make_map_f32_slab(&tmDQ, a.L.dQ, DP, a.L.npc, ZC);
+    rc = make_slab_map(&tmDQ, a.L.dQ, DP, a.L.npc, ZC);
     if (rc != GE2_OK) return rc;
     tmDQt = tmDQ;
     if (tail_cols > 0 && tail_cols < 32) {
-        rc = make_map_f32_slab(&tmDQt, a.L.dQ, DP, a.L.npc, ZC, tail_cols);
+        rc = make_slab_map(&tmDQt, a.L.dQ, DP, a.L.npc, ZC, tail_cols);
         if (rc != GE2_OK) return rc;
     }
     Sched sc;

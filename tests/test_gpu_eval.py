@@ -88,3 +88,26 @@ def test_candidate_list_and_bad_ids(capi, cuda_device):
     ok[[3, 7]] = False
     exp_d, _ = O.eval_ranks("COMPLEX", table, rel, inv, edges)
     assert np.array_equal(got_d.cpu().numpy()[ok], exp_d[ok])
+
+
+@pytest.mark.parametrize("nodes,B,D,scale", [
+    (255, 127, 64, 1.0), (256, 128, 65, 1e-3), (257, 129, 128, 30.0),   # edges of the score tiles; odd, half and full row widths
+    (513, 1, 2, 1.0), (40, 300, 100, 1e-12), (5000, 40, 98, 1e6),       # few candidates, few queries, values far from one
+])
+def test_ranks_are_exact_at_tile_edges_and_on_ties(capi, cuda_device, nodes, B, D, scale):
+    """The counting pass compares scores computed on the tensor cores and evaluates only what those leave open: ranks must still be
+    those of the fp32 chains, ties included."""
+    rng = np.random.default_rng(nodes * 1000 + B)
+    table = (rng.standard_normal((nodes, D)) * scale).astype(np.float32)
+    table[nodes // 2] = table[0]                      # equal candidates
+    table[nodes - 1] = np.nextafter(table[0], np.float32(np.inf))  # and one that differs in the last bits
+    table[1] = 0.0                                    # every score equals its positive's
+    table[2] *= 1000.0                                # a row far larger than its neighbours
+    edges = rng.integers(0, nodes, (B, 2)).astype(np.int64)
+    edges[0] = (1, 0)
+    edges[-1] = (nodes - 1, 0)
+    filt = np.stack([rng.integers(0, B, 3 * B), rng.integers(0, nodes, 3 * B)], 1).astype(np.int64)
+    exp, _ = O.eval_ranks("DISTMULT", table, None, None, edges, filt, None)
+    t = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
+    got, none = capi.eval_ranks("DISTMULT", t(table), t(edges), dst_filter=t(filt))
+    assert none is None and np.array_equal(got.cpu().numpy(), exp)
