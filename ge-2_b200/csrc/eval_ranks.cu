@@ -322,7 +322,6 @@ __global__ void __launch_bounds__(kCountThreads, 1)
     griddep_wait();  // the query rows come from the kernel before this one
     const uint32_t tmem = *s_tmem;
 
-    const uint32_t leader = lane == 0 ? 1u : 0u;
     if (warp == kTmaWarp) {
         int slot = 0;
         uint32_t phase = 1;
@@ -333,8 +332,8 @@ __global__ void __launch_bounds__(kCountThreads, 1)
                 for (int k = 0; k < 2 * NB; k++) {  // second terms first
                     ok = ok && spin_wait(kQEmpty + slot, phase);
                     if (!ok) break;
-                    tma_load_3d_warp(leader, smem + SM::kRing + slot * kBlockBytes, &tmQ, (k % NB) * 64, qt * kTileQ, k < NB ? 1 : 0, &bars[kQFull + slot],
-                                     kBlockBytes);
+                    mbar_expect_tx_warp(&bars[kQFull + slot], kBlockBytes);
+                    tma_load_3d_warp(smem + SM::kRing + slot * kBlockBytes, &tmQ, (k % NB) * 64, qt * kTileQ, k < NB ? 1 : 0, &bars[kQFull + slot]);
                     if (++slot == SM::kSlots) slot = 0, phase ^= 1;
                 }
             }
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(kCountThreads, 1)
                 auto product = [&](uint32_t da, uint32_t db, int b, bool first) {
 #pragma unroll
                     for (int ks = 0; ks < 4; ks++)
-                        if (ks + 4 * b < KS) mma_f16_ss_warp(leader, acc, da + ks * 2, db + b * kCandStep + ks * 2, kIdesc, (first && ks == 0) ? 0u : 1u);
+                        if (ks + 4 * b < KS) mma_f16_ss_warp(acc, da + ks * 2, db + b * kCandStep + ks * 2, kIdesc, (first && ks == 0) ? 0u : 1u);
                 };
 #pragma unroll
                 for (int k = 0; k < 2 * NB; k++) {
@@ -374,12 +373,12 @@ __global__ void __launch_bounds__(kCountThreads, 1)
                         product(da, cl, k - NB, false);
                         product(da, ch, k - NB, false);
                     }
-                    mma_commit_warp(leader, &bars[kQEmpty + slot]);
-                    if (k == 2 * NB - 1) mma_commit_warp(leader, &bars[kAccFull + ab]);
+                    mma_commit_warp(&bars[kQEmpty + slot]);
+                    if (k == 2 * NB - 1) mma_commit_warp(&bars[kAccFull + ab]);
                     if (++slot == SM::kSlots) slot = 0, phase ^= 1;
                 }
             }
-            if (ok) mma_commit_warp(leader, &bars[kCEmpty + cb]);
+            if (ok) mma_commit_warp(&bars[kCEmpty + cb]);
         }
         // the last arrivals that the tensor pipe makes on barriers of this CTA have landed before it can exit
         if (ok && cc > 0) spin_wait(kCEmpty + (cc - 1) % SM::kCandBufs, ((cc - 1) / SM::kCandBufs) & 1);

@@ -54,7 +54,7 @@
 
 #include <algorithm>
 
-#include "lp_internal.cuh"
+#include "lp_sched.cuh"
 #include "tc_pipe.cuh"
 
 namespace ge2 {
@@ -72,7 +72,6 @@ constexpr int kDrainWarp0 = kSoftmaxWarps, kTmaWarp = kDrainWarp0 + 4, kMmaWarp 
 constexpr int kStages = 3;              // Y ring depth of the gradient pass (shared memory is full there: X, 3 Y, W, 16 staging slabs)
 constexpr int kStagesA = 5;             // Y ring depth of the lse pass (no W tiles: room for a deeper ring, which the load latency wants)
 constexpr int kMaxStages = kStagesA;
-constexpr int kMaxParts = 8;            // most CTAs that can share one row block in the lse pass; size of a row's partial list
 constexpr uint32_t kTmemCols = 512;
 constexpr float kMasked = -1e9f;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
@@ -84,15 +83,6 @@ enum Bar { kBarXFull = 0, kBarXEmpty, kBarYFull, kBarYEmpty = kBarYFull + kMaxSt
            kBarWFull = kBarSEmpty + 2, kBarWEmpty = kBarWFull + 2, kBarAccFull = kBarWEmpty + 2, kBarAccEmpty = kBarAccFull + 2,
            kBarXch = kBarAccEmpty + 2, kBarXchFree = kBarXch + 2, kBarDkFull = kBarXchFree + 2, kBarDkEmpty = kBarDkFull + 2,
            kNumBars = kBarDkEmpty + 2 };
-
-// How the units of a launch are dealt to its CTAs: CTA k takes units [k * units / grid, (k + 1) * units / grid).
-struct Sched {
-    int RB, T, ZC;       // row blocks per chunk, negative tiles per chunk, sides * chunks
-    int unitsA, gridA;   // lse pass: unit = (zc, row block, tile), numbered (zc * RB + rb) * T + tile
-    int unitsB, gridB;   // gradient pass: the same units (X = Q block, stream over the K tiles)
-};
-__host__ __device__ __forceinline__ int range_begin(int k, int units, int grid) { return (int)(((long long)k * units) / grid); }
-__host__ __device__ __forceinline__ int cta_of_unit(int u, int units, int grid) { return (int)((((long long)u + 1) * grid - 1) / units); }
 
 template <int DP>
 struct Layout {
@@ -127,33 +117,6 @@ __device__ __forceinline__ float exp2f_fast(float x) {  // one MUFU.EX2; 2^-inf 
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// what a CTA needs to know about one unit of the lse pass
-struct UnitA {
-    int item, tile, rb, zc;
-};
-__device__ __forceinline__ UnitA decode_a(int u, const Sched& sc) {
-    UnitA r;
-    r.item = u / sc.T;
-    r.tile = u - r.item * sc.T;
-    r.zc = r.item / sc.RB;
-    r.rb = r.item - r.zc * sc.RB;
-    return r;
-}
-// The loops walk their units with these instead of decoding every index (no divisions inside the pipelines).
-struct IterA {
-    int item, tile, rb, zc;
-    __device__ __forceinline__ IterA(int u, const Sched& sc) {
-        const UnitA un = decode_a(u, sc);
-        item = un.item, tile = un.tile, rb = un.rb, zc = un.zc;
-    }
-    __device__ __forceinline__ void next(const Sched& sc) {
-        if (++tile == sc.T) {
-            tile = 0;
-            item++;
-            if (++rb == sc.RB) rb = 0, zc++;
-        }
-    }
-};
 // =====================================================================================================================
 // launch 1: row logsumexp
 // =====================================================================================================================
@@ -176,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int ub = range_begin(blockIdx.x, sc.unitsA, gridDim.x), ue = range_begin(blockIdx.x + 1, sc.unitsA, gridDim.x);
     const int n_iter = ue - ub;
     constexpr int NB = LY::NB;
-    auto wait = [&](int bar, uint32_t parity) { return pipe_wait(&bars[bar], parity, s_abort, d.status); };
+    auto spin_wait = [&](int bar, uint32_t parity) { return warp_spin_wait(&bars[bar], parity, s_abort, d.status); };
     auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, d.status); };
     // TMA producer state: runs a few units before the block-wide barrier (their latency overlaps the allocation of tensor
     // memory), the rest afterwards
@@ -186,16 +149,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         const IterA& un = tma_un;
         if (it == 0 || un.tile == 0) {  // a new block: X may be overwritten once the score contractions of the last one are done
             tma_sg++;
-            if (!wait(kBarXEmpty, (tma_sg & 1) ^ 1)) return false;
-            mbar_expect_tx(&bars[kBarXFull], LY::kTileBytes);
+            if (!spin_wait(kBarXEmpty, (tma_sg & 1) ^ 1)) return false;
+            mbar_expect_tx_warp(&bars[kBarXFull], LY::kTileBytes);
 #pragma unroll
-            for (int b = 0; b < NB; b++) tma_load_3d(sX + b * kBlockBytes, &tmQ, b * 64, un.rb * BM, un.zc, &bars[kBarXFull]);
+            for (int b = 0; b < NB; b++) tma_load_3d_warp(sX + b * kBlockBytes, &tmQ, b * 64, un.rb * BM, un.zc, &bars[kBarXFull]);
         }
         const int st = it % kStagesA, use = it / kStagesA;
-        if (!wait(kBarYEmpty + st, (use & 1) ^ 1)) return false;
-        mbar_expect_tx(&bars[kBarYFull + st], LY::kTileBytes);
+        if (!spin_wait(kBarYEmpty + st, (use & 1) ^ 1)) return false;
+        mbar_expect_tx_warp(&bars[kBarYFull + st], LY::kTileBytes);
 #pragma unroll
-        for (int b = 0; b < NB; b++) tma_load_3d(sY + st * LY::kTileBytes + b * kBlockBytes, &tmK, b * 64, un.tile * BN, un.zc, &bars[kBarYFull + st]);
+        for (int b = 0; b < NB; b++)
+            tma_load_3d_warp(sY + st * LY::kTileBytes + b * kBlockBytes, &tmK, b * 64, un.tile * BN, un.zc, &bars[kBarYFull + st]);
         tma_un.next(sc);
         return true;
     };
@@ -216,6 +180,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         mbar_init_fence();
         prefetch_tensormap(&tmQ);
         prefetch_tensormap(&tmK);
+    }
+    if (warp == kTmaWarp) {
+        __syncwarp();
         griddep_wait();  // the operands come from the kernel before this one
         // early loads: the first two tiles, and only while no wait can depend on another role (first block)
         while (tma_it < n_iter && tma_it < 2 && (tma_it == 0 || tma_un.tile != 0)) {
@@ -235,34 +202,31 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;  // this warp's quarter of the 128 tensor-memory lanes
 
     if (warp == kTmaWarp) {
-        if (lane == 0) {
-            for (; tma_it < n_iter; tma_it++)
-                if (!produce(tma_it)) break;
-        }
+        for (; tma_it < n_iter; tma_it++)
+            if (!produce(tma_it)) break;
     } else if (warp == kMmaWarp) {
         // ================================ score contractions ================================
-        if (lane == 0) {
-            const uint32_t aX = smem_u32(sX), aY0 = smem_u32(sY);
-            constexpr uint32_t kIdescS = idesc_f16(BM, BN, 0, 0);
-            const uint64_t dXk = desc_kmajor_base(aX);
-            int sg = -1;
-            IterA un(ub, sc);
-            for (int it = 0; it < n_iter; it++, un.next(sc)) {
-                if (it == 0 || un.tile == 0) {
-                    sg++;
-                    if (!wait(kBarXFull, sg & 1)) break;
-                }
-                const int st = it % kStagesA, use = it / kStagesA, sb = it & 1, su = it >> 1;
-                if (!wait(kBarYFull + st, use & 1)) break;
-                if (!wait(kBarSEmpty + sb, (su & 1) ^ 1)) break;
-                tc_fence_after();
-                const uint64_t dYk = desc_kmajor_base(aY0 + st * LY::kTileBytes);
-#pragma unroll
-                for (int ks = 0; ks < DP / kMmaK; ks++) mma_f16_ss(tmem + sb * 128, dXk + koff_kmajor(ks), dYk + koff_kmajor(ks), kIdescS, ks > 0);
-                mma_commit(&bars[kBarSFull + sb]);
-                mma_commit(&bars[kBarYEmpty + st]);
-                if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit(&bars[kBarXEmpty]);
+        // (the whole warp walks the loop; the asynchronous instructions are lane 0's)
+        constexpr uint32_t kIdescS = idesc_f16(BM, BN, 0, 0);
+        const uint32_t dX = desc_lo_sw128(smem_u32(sX), 16), dY0 = desc_lo_sw128(smem_u32(sY), 16);
+        int sg = -1;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            if (it == 0 || un.tile == 0) {
+                sg++;
+                if (!spin_wait(kBarXFull, sg & 1)) break;
             }
+            const int st = it % kStagesA, use = it / kStagesA, sb = it & 1, su = it >> 1;
+            if (!spin_wait(kBarYFull + st, use & 1)) break;
+            if (!spin_wait(kBarSEmpty + sb, (su & 1) ^ 1)) break;
+            tc_fence_after();
+            const uint32_t dY = dY0 + st * (LY::kTileBytes >> 4);
+#pragma unroll
+            for (int ks = 0; ks < DP / kMmaK; ks++)
+                mma_f16_ss_warp(tmem + sb * 128, dX + (uint32_t)koff_kmajor(ks), dY + (uint32_t)koff_kmajor(ks), kIdescS, ks > 0);
+            mma_commit_warp(&bars[kBarSFull + sb]);
+            mma_commit_warp(&bars[kBarYEmpty + st]);
+            if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit_warp(&bars[kBarXEmpty]);
         }
     } else if (warp == kDrainWarp0) {
         // ================================ combine warp ================================
@@ -523,7 +487,7 @@ __global__ void __launch_bounds__(kThreadsB, 1)
     const int ub = range_begin(blockIdx.x, sc.unitsB, gridDim.x), ue = range_begin(blockIdx.x + 1, sc.unitsB, gridDim.x);
     const int n_iter = ue - ub;
     constexpr int NB = LY::NB;
-    auto wait = [&](int bar, uint32_t parity) { return pipe_wait(&bars[bar], parity, s_abort, d.status); };
+    auto spin_wait = [&](int bar, uint32_t parity) { return warp_spin_wait(&bars[bar], parity, s_abort, d.status); };
     auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, d.status); };
     constexpr int kBarDqFull = kBarAccFull, kBarDqEmpty = kBarAccEmpty;
     // Only real columns of dQ / dK leave the SM: D / 32 full slabs of 32 columns, then one narrow slab (its own tensor map,
@@ -540,16 +504,17 @@ __global__ void __launch_bounds__(kThreadsB, 1)
         const IterA& un = tma_un;
         if (it == 0 || un.tile == 0) {
             tma_sg++;
-            if (!wait(kBarXEmpty, (tma_sg & 1) ^ 1)) return false;
-            mbar_expect_tx(&bars[kBarXFull], LY::kTileBytes);
+            if (!spin_wait(kBarXEmpty, (tma_sg & 1) ^ 1)) return false;
+            mbar_expect_tx_warp(&bars[kBarXFull], LY::kTileBytes);
 #pragma unroll
-            for (int b = 0; b < NB; b++) tma_load_3d(sX + b * kBlockBytes, &tmQ, b * 64, un.rb * BM, un.zc, &bars[kBarXFull]);
+            for (int b = 0; b < NB; b++) tma_load_3d_warp(sX + b * kBlockBytes, &tmQ, b * 64, un.rb * BM, un.zc, &bars[kBarXFull]);
         }
         const int st = it % kStages, use = it / kStages;
-        if (!wait(kBarYEmpty + st, (use & 1) ^ 1)) return false;
-        mbar_expect_tx(&bars[kBarYFull + st], LY::kTileBytes);
+        if (!spin_wait(kBarYEmpty + st, (use & 1) ^ 1)) return false;
+        mbar_expect_tx_warp(&bars[kBarYFull + st], LY::kTileBytes);
 #pragma unroll
-        for (int b = 0; b < NB; b++) tma_load_3d(sY + st * LY::kTileBytes + b * kBlockBytes, &tmK, b * 64, un.tile * BN, un.zc, &bars[kBarYFull + st]);
+        for (int b = 0; b < NB; b++)
+            tma_load_3d_warp(sY + st * LY::kTileBytes + b * kBlockBytes, &tmK, b * 64, un.tile * BN, un.zc, &bars[kBarYFull + st]);
         tma_un.next(sc);
         return true;
     };
@@ -574,6 +539,9 @@ __global__ void __launch_bounds__(kThreadsB, 1)
         mbar_init_fence();
         prefetch_tensormap(&tmQ);
         prefetch_tensormap(&tmK);
+    }
+    if (warp == kTmaWarp) {
+        __syncwarp();
         griddep_wait();  // the operands come from the kernel before this one
         // early loads: the first two tiles, and only while no wait can depend on another role (first block)
         while (tma_it < n_iter && tma_it < 2 && (tma_it == 0 || tma_un.tile != 0)) {
@@ -596,75 +564,69 @@ __global__ void __launch_bounds__(kThreadsB, 1)
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
 
     if (warp == kTmaWarp) {
-        if (lane == 0) {
-            for (; tma_it < n_iter; tma_it++)
-                if (!produce(tma_it)) break;
-        }
+        for (; tma_it < n_iter; tma_it++)
+            if (!produce(tma_it)) break;
     } else if (warp == kMmaWarp) {
         // ================================ MMA issuer 1: score contractions S = Q K^T ================================
-        if (lane == 0) {
-            const uint32_t aX = smem_u32(sX), aY0 = smem_u32(sY);
-            constexpr uint32_t kIdescS = idesc_f16(BM, BN, 0, 0);
-            const uint64_t dXk = desc_kmajor_base(aX);
-            int sg = -1;
-            IterA un(ub, sc);
-            for (int it = 0; it < n_iter; it++, un.next(sc)) {
-                if (it == 0 || un.tile == 0) {
-                    sg++;
-                    if (!wait(kBarXFull, sg & 1)) break;
-                }
-                const int st = it % kStages, use = it / kStages;
-                if (!wait(kBarYFull + st, use & 1)) break;
-                if (!wait(kBarSEmpty, (it & 1) ^ 1)) break;  // every worker warp holds the previous tile's scores in registers
-                tc_fence_after();
-                const uint64_t dYk = desc_kmajor_base(aY0 + st * LY::kTileBytes);
-#pragma unroll
-                for (int ks = 0; ks < DP / kMmaK; ks++) mma_f16_ss(tS, dXk + koff_kmajor(ks), dYk + koff_kmajor(ks), kIdescS, ks > 0);
-                mma_commit(&bars[kBarSFull]);
+        // (the whole warp walks the loop; the asynchronous instructions are lane 0's)
+        constexpr uint32_t kIdescS = idesc_f16(BM, BN, 0, 0);
+        const uint32_t dX = desc_lo_sw128(smem_u32(sX), 16), dY0 = desc_lo_sw128(smem_u32(sY), 16);
+        int sg = -1;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            if (it == 0 || un.tile == 0) {
+                sg++;
+                if (!spin_wait(kBarXFull, sg & 1)) break;
             }
+            const int st = it % kStages, use = it / kStages;
+            if (!spin_wait(kBarYFull + st, use & 1)) break;
+            if (!spin_wait(kBarSEmpty, (it & 1) ^ 1)) break;  // every worker warp holds the previous tile's scores in registers
+            tc_fence_after();
+            const uint32_t dY = dY0 + st * (LY::kTileBytes >> 4);
+#pragma unroll
+            for (int ks = 0; ks < DP / kMmaK; ks++)
+                mma_f16_ss_warp(tS, dX + (uint32_t)koff_kmajor(ks), dY + (uint32_t)koff_kmajor(ks), kIdescS, ks > 0);
+            mma_commit_warp(&bars[kBarSFull]);
         }
     } else if (warp == kGradWarp) {
         // ================================ MMA issuer 2: dQ += W K, dK = W^T Q ================================
-        // A thread of its own, so that the score contraction of the next tile is issued while this one still waits for
+        // A warp of its own, so that the score contraction of the next tile is issued while this one still waits for
         // the W of the current tile.
-        if (lane == 0) {
-            const uint32_t aX = smem_u32(sX), aY0 = smem_u32(sY), aW0 = smem_u32(sW);
-            // the embedding dimension rounded up to the MMA k step, not to the 64-column block: D = 100 costs 7/8 of DP = 128
-            const int D16 = ((d.D + kMmaK - 1) / kMmaK) * kMmaK;
-            const uint32_t kIdescDQ = idesc_f16(BM, D16, 0, 1);
-            const uint32_t kIdescDK = idesc_f16(BN, D16, 1, 1);
-            const uint64_t dXm = desc_mnmajor_base(aX);
-            int sg = -1;
-            bool fresh = true;
-            IterA un(ub, sc);
-            for (int it = 0; it < n_iter; it++, un.next(sc)) {
-                if (it == 0 || un.tile == 0) {
-                    sg++;
-                    fresh = true;
-                    if (!wait(kBarDqEmpty, (sg & 1) ^ 1)) break;  // the drain of the previous block has read dQ
-                }
-                const int st = it % kStages, pb = it & 1;
-                // (no wait on X or the Y stage: W was made from scores that were made from them)
-                if (!wait(kBarWFull, it & 1)) break;
-                if (!wait(kBarDkEmpty + pb, ((it >> 1) & 1) ^ 1)) break;  // the tile before last has been drained out of this accumulator
-                tc_fence_after();
-                const uint32_t tdK = tdK0 + pb * 128;
-                const uint32_t aW = aW0;
-                const uint64_t dWk = desc_kmajor_base(aW), dWm = desc_mnmajor_base(aW), dYm = desc_mnmajor_base(aY0 + st * LY::kTileBytes);
+        // the embedding dimension rounded up to the MMA k step, not to the 64-column block: D = 100 costs 7/8 of DP = 128
+        const int D16 = ((d.D + kMmaK - 1) / kMmaK) * kMmaK;
+        const uint32_t kIdescDQ = idesc_f16(BM, D16, 0, 1);
+        const uint32_t kIdescDK = idesc_f16(BN, D16, 1, 1);
+        const uint32_t dXm = desc_lo_sw128(smem_u32(sX), kBlockBytes), dWk = desc_lo_sw128(smem_u32(sW), 16), dWm = desc_lo_sw128(smem_u32(sW), kBlockBytes),
+                       dY0 = desc_lo_sw128(smem_u32(sY), kBlockBytes);
+        int sg = -1;
+        bool fresh = true;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            if (it == 0 || un.tile == 0) {
+                sg++;
+                fresh = true;
+                if (!spin_wait(kBarDqEmpty, (sg & 1) ^ 1)) break;  // the drain of the previous block has read dQ
+            }
+            const int st = it % kStages, pb = it & 1;
+            // (no wait on X or the Y stage: W was made from scores that were made from them)
+            if (!spin_wait(kBarWFull, it & 1)) break;
+            if (!spin_wait(kBarDkEmpty + pb, ((it >> 1) & 1) ^ 1)) break;  // the tile before last has been drained out of this accumulator
+            tc_fence_after();
+            const uint32_t tdK = tdK0 + pb * 128;
+            const uint32_t dYm = dY0 + st * (LY::kTileBytes >> 4);
 #pragma unroll
-                for (int ks = 0; ks < BM / kMmaK; ks++)  // dK = W^T Q, k runs over the block's rows; first, so that its drain starts early
-                    mma_f16_ss(tdK, dWm + koff_mnmajor(ks), dXm + koff_mnmajor(ks), kIdescDK, ks > 0);
-                mma_commit(&bars[kBarDkFull + pb]);
+            for (int ks = 0; ks < BM / kMmaK; ks++)  // dK = W^T Q, k runs over the block's rows; first, so that its drain starts early
+                mma_f16_ss_warp(tdK, dWm + (uint32_t)koff_mnmajor(ks), dXm + (uint32_t)koff_mnmajor(ks), kIdescDK, ks > 0);
+            mma_commit_warp(&bars[kBarDkFull + pb]);
 #pragma unroll
-                for (int ks = 0; ks < BN / kMmaK; ks++)  // dQ += W K, k runs over the tile's negatives
-                    mma_f16_ss(tdQ, dWk + koff_kmajor(ks), dYm + koff_mnmajor(ks), kIdescDQ, (!fresh || ks > 0) ? 1u : 0u);
-                fresh = false;
-                mma_commit(&bars[kBarYEmpty + st]);
-                mma_commit(&bars[kBarWEmpty]);
-                if (it == n_iter - 1 || un.tile == sc.T - 1) {
-                    mma_commit(&bars[kBarDqFull]);
-                    mma_commit(&bars[kBarXEmpty]);  // Q is an operand of the score and the dK contractions; those of this block are all behind this point
-                }
+            for (int ks = 0; ks < BN / kMmaK; ks++)  // dQ += W K, k runs over the tile's negatives
+                mma_f16_ss_warp(tdQ, dWk + (uint32_t)koff_kmajor(ks), dYm + (uint32_t)koff_mnmajor(ks), kIdescDQ, (!fresh || ks > 0) ? 1u : 0u);
+            fresh = false;
+            mma_commit_warp(&bars[kBarYEmpty + st]);
+            mma_commit_warp(&bars[kBarWEmpty]);
+            if (it == n_iter - 1 || un.tile == sc.T - 1) {
+                mma_commit_warp(&bars[kBarDqFull]);
+                mma_commit_warp(&bars[kBarXEmpty]);  // Q is an operand of the score and the dK contractions; those of this block are all behind this point
             }
         }
     } else if (warp < kSoftmaxWarps) {
@@ -889,7 +851,7 @@ int env_int(const char* name, int fallback) {
 
 template <int DP>
 int launch(const LpKernelArgs& a, cudaStream_t stream) {
-    if (a.L.Qh == nullptr || a.L.Kh == nullptr || a.L.lse2s == nullptr || a.L.item_ctr == nullptr) return GE2_ERR_WORKSPACE;
+    if (a.L.Qh == nullptr || a.L.Kh == nullptr || a.L.lse2s == nullptr) return GE2_ERR_WORKSPACE;
     const int ZC = a.L.S * a.d.C;
     CUtensorMap tmQ, tmK;
     int rc = make_operand_map(&tmQ, a.L.Qh, false, DP, a.L.npc, ZC);

@@ -1,283 +1,632 @@
-// fp32 (CUDA-core FFMA) scores kernel of the link-prediction step: the 1e-4-parity path.
-//
-// One CTA = (side, chunk, 64-row block).  It keeps its 64 query rows in shared memory and streams the chunk's
-// negatives past them twice, 64 at a time:
-//   sweep 1: S = Q K^T per tile, mask, running (max, sum-exp) per row            -> lse (with the positive score folded in)
-//   sweep 2: S again, P = exp(S - lse); dQ += P K (registers, whole sweep); dK tile = P^T Q -> atomics into dK
-// The [rows x N] score matrix only ever exists as 64x64 tiles in registers / shared memory.
-// Stands in for the reference's bmm + logsumexp + cross_entropy + autograd chain
+// fp32 scores kernels of the link-prediction step (the 1e-4-parity path) on the tensor cores.
+// Stand in for the reference's bmm + logsumexp + cross_entropy + autograd chain
 // (cpp/src/nn/decoders/edge/comparators.cpp:128-138, cpp/src/nn/loss.cpp:46-63 of the reference project).
+//
+// Every fp32 operand is the exact sum of three bf16 values, x = xh + xm + xl (24 bits as 8 + 8 + 8, any exponent), and a product is
+// taken as xl yh + xh yl + xm ym + xm yh + xh ym + xh yh: what is left out is below 2^-24 of |x y|, the size of one fp32 rounding.
+// tcgen05.mma kind::f16 sums such products in fp32, but it truncates every addend and every sum (measured: products aligned to 25
+// fraction bits of the largest addend, the sum cut to 24 bits), where the CUDA cores round.  So no long sum is left to it:
+//   * the small products come first, when the accumulator is small; only the ceil(k / 16) steps of xh yh add to a full one;
+//   * dQ, a sum over all negatives, is summed per tile of 64 negatives only; the tiles are added in registers, rounded to nearest;
+//   * dK, a sum over all rows of a chunk, leaves every tile of 128 rows by fp32 atomic adds.
+// Exponentials and logarithms are CUDA's expf / logf.  Errors against float64 are those of the multiply-add kernel this replaced.
+//
+// Two persistent launches, as on the f16 path (lp_scores_f16.cu): a block X of 128 query rows stays in shared memory and tiles Y of 64
+// negatives stream past it,
+//   lp_lse32_kernel    S = X Y^T tile by tile, running (max, sum) per row                                             -> lse, loss
+//   lp_grad32_kernel   S again, P = exp(S - lse) split into W (three planes in shared memory), dQ += W Y, dK^T = X^T W
+// All operands sit in shared memory as planes of 64-column blocks in the 128-byte-swizzled layout that TMA writes; read along rows a
+// block is a K-major operand, along columns an MN-major one, so each serves both of its contractions.
+//
+// Bound by the contractions: 6 products a multiply-add, 4 contractions' worth of them (S twice, dQ, dK) = 24 x S B N D x 2 flops of bf16.
+// B = 10 000, 1 000 negatives, D = 100, two sides: 53 + 101 us (one kernel of fp32 multiply-adds: 776 us); 1 000 edges, D = 50: 13 + 21 us
+// (202 us).  Relative 2-norm error of the node gradient against float64 at B = 4 000, N = 1 000, D = 100: 5.3e-7 (4.2e-7), of the scores 1.5e-7
+// (1.6e-7).
 #include <math.h>
 
-#include "lp_internal.cuh"
+#include <algorithm>
+
+#include "lp_sched.cuh"
+#include "tc_pipe.cuh"
 
 namespace ge2 {
 namespace {
 
-constexpr int BM = 64;        // query rows per CTA
-constexpr int BN = 64;        // negatives per tile
-constexpr int kThreads = 256; // 16 x 16 threads, 4 x 4 scores each
+using namespace tc;
+
+constexpr int BM = 128, BN = 64;
+constexpr int kPlanes = 3;
 constexpr float kMasked = -1e9f;
+constexpr float kDeadRow = 1e30f;  // "lse" of a row past the end of its chunk: exp(anything - 1e30) = 0
+constexpr int kLseStages = 2;
+constexpr int kYSlots = 5;         // gradient pass: ring of Y planes; three belong to a tile, two are ahead
+
+// the six products, small ones first: plane of the first / second operand, two bits each
+constexpr uint32_t codes(int a, int b, int c, int d, int e, int f) { return (uint32_t)(a | b << 2 | c << 4 | d << 6 | e << 8 | f << 10); }
+constexpr uint32_t kFirst = codes(2, 0, 1, 1, 0, 0), kSecond = codes(0, 2, 1, 0, 1, 0);  // (l,h) (h,l) (m,m) (m,h) (h,m) (h,h)
+// the gradient pass takes Y planes in the order m, h, l of their arrival, and gives them back in the same order
+constexpr uint32_t kFirstS = codes(0, 1, 2, 1, 0, 0), kSecondS = codes(1, 1, 0, 0, 2, 0);   // S:  (h,m) (m,m) (l,h) (m,h) (h,l) (h,h)
+constexpr uint32_t kFirstDq = codes(0, 1, 0, 2, 1, 0), kSecondDq = codes(1, 1, 2, 0, 0, 0); // dQ: (h,m) (m,m) | (h,l) | (l,h) (m,h) (h,h)
+__device__ __forceinline__ int slot_of_plane(int plane) { return plane == 1 ? 0 : plane == 0 ? 1 : 2; }
 
 template <int DP>
-struct Smem {
-    float q[BM][DP + 4];
-    float k[BN][DP + 4];
-    float p[BM][BN + 4];
-    float lse[BM];
-    float loss[BM];  // per-row lse - pos, summed by one thread
-    int32_t mask[BN];
+struct Layout32 {
+    static constexpr int NB = DP / 64;
+    static constexpr int kXBlock = BM * 128, kYBlock = BN * 128;
+    static constexpr int kXPlane = NB * kXBlock, kYPlane = NB * kYBlock, kWPlane = BM * 128;
+    static constexpr int kX = 0, kY = kPlanes * kXPlane;
+    // logsumexp pass
+    static constexpr int kXch = kY + kLseStages * kPlanes * kYPlane;  // [2][128] (max, sum) of the right half of the columns
+    static constexpr int kMiscA = kXch + 2 * BM * 8;
+    static constexpr int kBytesA = (kMiscA + 512 + 1024) > 120 * 1024 ? (kMiscA + 512 + 1024) : 120 * 1024;  // one CTA an SM
+    // gradient pass
+    static constexpr int kW = kY + kYSlots * kYPlane;
+    static constexpr int kMiscB = kW + kPlanes * kWPlane;
+    static constexpr int kBytesB = (kMiscB + 512 + 1024) > 120 * 1024 ? (kMiscB + 512 + 1024) : 120 * 1024;
+    static_assert(kBytesA <= 227 * 1024 && kBytesB <= 227 * 1024, "exceeds the shared memory of an SM");
 };
 
-template <int DP>
-__device__ __forceinline__ void load_rows(float (*dst)[DP + 4], const float* __restrict__ src, int valid_rows, int tid) {
-    // 64 rows x DP floats, float4 granularity; rows >= valid_rows are zero-filled
-    constexpr int V = DP / 4;
-    for (int e = tid; e < 64 * V; e += kThreads) {
-        const int r = e / V, c = e - r * V;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < valid_rows) v = __ldg(reinterpret_cast<const float4*>(src + (int64_t)r * DP) + c);
-        *reinterpret_cast<float4*>(&dst[r][c * 4]) = v;
+// the filter words of 32 columns starting at n0 + base: lane l holds column l's; bit j of the result = column j is masked for row `brow`
+__device__ __forceinline__ uint32_t mask_bits(int32_t word, int wrow0, int brow) {
+    uint32_t mb = 0u;
+    unsigned ballot = __ballot_sync(0xffffffffu, (unsigned)(word - wrow0) < 32u);
+    while (ballot != 0) {
+        const int src = __ffs(ballot) - 1;
+        ballot &= ballot - 1;
+        if (__shfl_sync(0xffffffffu, word, src) == brow) mb |= 1u << src;
     }
+    return mb;
 }
 
-template <int DP>
-__device__ __forceinline__ void score_tile(const Smem<DP>& sm, int ty, int tx, float (&acc)[4][4]) {
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) acc[r][c] = 0.f;
-#pragma unroll 4
-    for (int d4 = 0; d4 < DP / 4; d4++) {
-        float4 a[4], b[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) a[r] = *reinterpret_cast<const float4*>(&sm.q[ty + 16 * r][d4 * 4]);
-#pragma unroll
-        for (int c = 0; c < 4; c++) b[c] = *reinterpret_cast<const float4*>(&sm.k[tx + 16 * c][d4 * 4]);
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                acc[r][c] = fmaf(a[r].x, b[c].x, acc[r][c]);
-                acc[r][c] = fmaf(a[r].y, b[c].y, acc[r][c]);
-                acc[r][c] = fmaf(a[r].z, b[c].z, acc[r][c]);
-                acc[r][c] = fmaf(a[r].w, b[c].w, acc[r][c]);
-            }
-    }
-}
+// =====================================================================================================================
+// launch 1: row logsumexp
+// =====================================================================================================================
+constexpr int kSoftWarps = 8;                                    // 4 row quarters x 2 halves of 32 columns
+constexpr int kTmaWarpA = 8, kMmaWarpA = 9, kClearWarpA = 10, kClearWarps = 3, kThreadsA = 416;
+enum BarA { kAXFull = 0, kAXEmpty, kAYFull, kAYEmpty = kAYFull + kLseStages, kASFull = kAYEmpty + kLseStages, kASEmpty = kASFull + 2, kAXch = kASEmpty + 2,
+            kAXchFree = kAXch + 2, kNumBarsA = kAXchFree + 2 };
 
 template <int DP>
-__global__ void __launch_bounds__(kThreads, 2) lp_scores_fp32_kernel(LpKernelArgs a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Smem<DP>& sm = *reinterpret_cast<Smem<DP>*>(smem_raw);
+__global__ void __launch_bounds__(kThreadsA, 1)
+    lp_lse32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, LpKernelArgs a, Sched sc) {
+    using LY = Layout32<DP>;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    float2* s_xch = reinterpret_cast<float2*>(smem + LY::kXch);
+    uint64_t* bars = (uint64_t*)(smem + LY::kMiscA);
+    uint32_t* s_tmem = (uint32_t*)(smem + LY::kMiscA + kNumBarsA * 8);
+    volatile int* s_abort = (volatile int*)(smem + LY::kMiscA + kNumBarsA * 8 + 4);
     const ge2_lp_desc& d = a.d;
     const LpLayout& L = a.L;
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int s = blockIdx.z, c = blockIdx.y;
-    const int row0 = blockIdx.x * BM;                 // first row of this block inside the chunk
-    const int valid_rows = min(BM, L.npc - row0);      // rows past the chunk end do not exist
-    const int64_t grow0 = (int64_t)s * L.Bp + (int64_t)c * L.npc + row0;  // row in the [S*Bp] arrays
-    const float* Kc = L.K + ((int64_t)s * L.CN + (int64_t)c * d.N) * DP;
-    const int32_t* maskc = L.mask + (int64_t)s * L.CN + (int64_t)c * d.N;
-    float* dKc = L.dK + ((int64_t)s * L.CN + (int64_t)c * d.N) * DP;
-    float* dump = s == 0 ? d.neg_scores : d.inv_neg_scores;  // optional [Bp, N] score dump
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ub = range_begin(blockIdx.x, sc.unitsA, gridDim.x), ue = range_begin(blockIdx.x + 1, sc.unitsA, gridDim.x);
+    const int n_iter = ue - ub;
+    auto spin_wait = [&](int bar, uint32_t parity) { return warp_spin_wait(&bars[bar], parity, s_abort, d.status); };
+    auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, d.status); };
 
-    load_rows<DP>(sm.q, L.Q + grow0 * DP, valid_rows, tid);
-    const int n_tiles = (d.N + BN - 1) / BN;
-
-    // ---- sweep 1: row-wise logsumexp over the negatives --------------------------------------------
-    float run_m[4], run_l[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        run_m[r] = -INFINITY;
-        run_l[r] = 0.f;
-    }
-    for (int t = 0; t < n_tiles; t++) {
-        const int n0 = t * BN;
-        const int valid_n = min(BN, d.N - n0);
-        __syncthreads();  // previous tile fully consumed (also orders the q load before first use)
-        load_rows<DP>(sm.k, Kc + (int64_t)n0 * DP, valid_n, tid);
-        if (tid < BN) sm.mask[tid] = tid < valid_n ? maskc[n0 + tid] : -1;
-        __syncthreads();
-        float acc[4][4];
-        score_tile<DP>(sm, ty, tx, acc);
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int lr = ty + 16 * r;
-            const int brow = c * L.npc + row0 + lr;  // batch row (padded numbering), what the filter names
-            float v[4];
-            float tmax = -INFINITY;
-#pragma unroll
-            for (int cc = 0; cc < 4; cc++) {
-                const int lc = tx + 16 * cc;
-                float sc = acc[r][cc];
-                if (sm.mask[lc] == brow) sc = kMasked;
-                v[cc] = lc < valid_n ? sc : -INFINITY;
-                tmax = fmaxf(tmax, v[cc]);
-                if (dump != nullptr && lr < valid_rows && lc < valid_n) dump[(int64_t)brow * d.N + n0 + lc] = sc;
-            }
-            if (tmax > -INFINITY) {
-                const float nm = fmaxf(run_m[r], tmax);
-                float add = 0.f;
-#pragma unroll
-                for (int cc = 0; cc < 4; cc++) add += expf(v[cc] - nm);  // exp(-inf) = 0 for absent columns
-                run_l[r] = run_l[r] * expf(run_m[r] - nm) + add;
-                run_m[r] = nm;
-            }
+    if (warp == kTmaWarpA && lane == 0) {
+        mbar_init(&bars[kAXFull], 1);
+        mbar_init(&bars[kAXEmpty], 1);
+        for (int k = 0; k < kLseStages; k++) {
+            mbar_init(&bars[kAYFull + k], 1);
+            mbar_init(&bars[kAYEmpty + k], 1);
         }
-    }
-    // combine the 16 threads that share a row (consecutive lanes of a half warp), fold in the positive score
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        float m = run_m[r], l = run_l[r];
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-            const float om = __shfl_xor_sync(0xffffffffu, m, o);
-            const float ol = __shfl_xor_sync(0xffffffffu, l, o);
-            const float nm = fmaxf(m, om);
-            if (nm > -INFINITY) {
-                l = l * expf(m - nm) + ol * expf(om - nm);
-                m = nm;
-            }
+        for (int k = 0; k < 2; k++) {
+            mbar_init(&bars[kASFull + k], 1);
+            mbar_init(&bars[kASEmpty + k], kSoftWarps);
+            mbar_init(&bars[kAXch + k], kSoftWarps / 2);
+            mbar_init(&bars[kAXchFree + k], kSoftWarps / 2);
         }
-        const int lr = ty + 16 * r;
-        if (tx == 0) {
-            float lse = 0.f;
-            if (lr < valid_rows) {
-                const float pos = L.pos[grow0 + lr];
-                const float nm = fmaxf(m, pos);
-                const float z = l * expf(m - nm) + expf(pos - nm);
-                lse = nm + logf(z);
-                L.lse[grow0 + lr] = lse;
-                sm.loss[lr] = lse - pos;
-            } else {
-                sm.loss[lr] = 0.f;
-            }
-            sm.lse[lr] = lse;
-        }
+        *s_abort = 0;
+        mbar_init_fence();
+        prefetch_tensormap(&tmQ);
+        prefetch_tensormap(&tmK);
     }
-
+    if (warp == kMmaWarpA) {
+        tmem_alloc(s_tmem, 128);
+        tmem_relinquish();
+    }
+    tc_fence_before();
     __syncthreads();
-    if (tid == 0) {  // one double-precision add per CTA into the step's loss
-        double acc = 0.0;
-        for (int r = 0; r < BM; r++) acc += (double)sm.loss[r];
-        atomicAdd(L.loss_acc, acc);
-    }
-    // ---- sweep 2: probabilities, dQ and dK ---------------------------------------------------------
-    constexpr int H = DP / 64;  // column groups of 64 floats; thread owns columns tx*4 + 64*h
-    float dq[4][H][4];
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-#pragma unroll
-        for (int hh = 0; hh < H; hh++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) dq[r][hh][e] = 0.f;
+    tc_fence_after();
+    griddep_wait();  // set-up done; from here on global memory written by the preceding kernel is read and its buffers rewritten
+    const uint32_t tmem = *s_tmem;
 
-    for (int t = 0; t < n_tiles; t++) {
-        const int n0 = t * BN;
-        const int valid_n = min(BN, d.N - n0);
-        __syncthreads();  // previous tile's K / P fully consumed; sm.lse visible
-        load_rows<DP>(sm.k, Kc + (int64_t)n0 * DP, valid_n, tid);
-        if (tid < BN) sm.mask[tid] = tid < valid_n ? maskc[n0 + tid] : -1;
-        __syncthreads();
-        float acc[4][4];
-        score_tile<DP>(sm, ty, tx, acc);
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int lr = ty + 16 * r;
-            const int brow = c * L.npc + row0 + lr;
-            const float lse = sm.lse[lr];
-#pragma unroll
-            for (int cc = 0; cc < 4; cc++) {
-                const int lc = tx + 16 * cc;
-                float pr = 0.f;  // masked entries were overwritten in place: no gradient reaches them
-                if (lr < valid_rows && lc < valid_n && sm.mask[lc] != brow) pr = expf(acc[r][cc] - lse);
-                sm.p[lr][lc] = pr;
+    if (warp == kTmaWarpA) {
+        int sg = -1;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            if (it == 0 || un.tile == 0) {
+                sg++;
+                if (!spin_wait(kAXEmpty, (sg & 1) ^ 1)) break;
+                mbar_expect_tx_warp(&bars[kAXFull], kPlanes * LY::kXPlane);
+                for (int p = 0; p < kPlanes; p++)
+                    for (int b = 0; b < LY::NB; b++)
+                        tma_load_3d_warp(smem + LY::kX + p * LY::kXPlane + b * LY::kXBlock, &tmQ, b * 64, un.rb * BM, p * sc.ZC + un.zc, &bars[kAXFull]);
             }
+            const int st = it % kLseStages, use = it / kLseStages;
+            if (!spin_wait(kAYEmpty + st, (use & 1) ^ 1)) break;
+            mbar_expect_tx_warp(&bars[kAYFull + st], kPlanes * LY::kYPlane);
+            for (int p = 0; p < kPlanes; p++)
+                for (int b = 0; b < LY::NB; b++)
+                    tma_load_3d_warp(smem + LY::kY + (st * kPlanes + p) * LY::kYPlane + b * LY::kYBlock, &tmK, b * 64, un.tile * BN, p * sc.ZC + un.zc,
+                                     &bars[kAYFull + st]);
         }
-        __syncthreads();
-        // dQ[rows ty+16r][cols] += sum_j P[row][j] * K[j][cols]
-#pragma unroll 2
-        for (int j4 = 0; j4 < BN / 4; j4++) {
-            float4 pa[4];
+    } else if (warp == kMmaWarpA) {
+        constexpr uint32_t kIdesc = idesc_bf16(BM, BN, 0, 0);
+        const uint32_t dX = desc_lo_sw128(smem_u32(smem + LY::kX), 16), dY0 = desc_lo_sw128(smem_u32(smem + LY::kY), 16);
+        const int KS = (d.D + kMmaK - 1) / kMmaK;
+        int sg = -1;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            if (it == 0 || un.tile == 0) {
+                sg++;
+                if (!spin_wait(kAXFull, sg & 1)) break;
+            }
+            const int st = it % kLseStages, use = it / kLseStages, sb = it & 1, su = it >> 1;
+            if (!spin_wait(kAYFull + st, use & 1)) break;
+            if (!spin_wait(kASEmpty + sb, (su & 1) ^ 1)) break;
+            tc_fence_after();
+            const uint32_t dY = dY0 + st * (kPlanes * LY::kYPlane >> 4);
+#pragma unroll 1
+            for (int p = 0; p < 6; p++) {
+                const uint32_t da = dX + ((kFirst >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY + ((kSecond >> (2 * p)) & 3) * (LY::kYPlane >> 4);
 #pragma unroll
-            for (int r = 0; r < 4; r++) pa[r] = *reinterpret_cast<const float4*>(&sm.p[ty + 16 * r][j4 * 4]);
+                for (int ks = 0; ks < DP / kMmaK; ks++)
+                    if (ks < KS)
+                        mma_f16_ss_warp(tmem + sb * BN, da + (((ks >> 2) * LY::kXBlock + (ks & 3) * 32) >> 4),
+                                        db + (((ks >> 2) * LY::kYBlock + (ks & 3) * 32) >> 4), kIdesc, (p > 0 || ks > 0) ? 1u : 0u);
+            }
+            mma_commit_warp(&bars[kAYEmpty + st]);
+            if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit_warp(&bars[kAXEmpty]);
+            mma_commit_warp(&bars[kASFull + sb]);  // last: whoever waits for it has seen the others' arrivals land before the CTA exits
+        }
+    } else if (warp >= kClearWarpA) {
+        // clear what the gradient pass will add to: dK, and the dQ rows of every block whose stream that pass cuts at a CTA boundary
+        const int wz = (warp - kClearWarpA) * 32 + lane;
+        const int64_t n4 = (int64_t)sc.ZC * d.N * (DP / 4);
+        const int64_t z0 = n4 * blockIdx.x / gridDim.x, z1 = n4 * (blockIdx.x + 1) / gridDim.x;
+        float4* p4 = reinterpret_cast<float4*>(L.dK);
+        for (int64_t k = z0 + wz; k < z1; k += kClearWarps * 32) p4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 1 + (int)blockIdx.x; j < sc.gridB; j += (int)gridDim.x) {
+            const int u = range_begin(j, sc.unitsB, sc.gridB);
+            if (u <= 0 || u >= sc.unitsB) continue;
+            const UnitA un = decode_a(u, sc);
+            if (un.tile == 0) continue;  // the boundary falls between two blocks: nothing is split
+            float4* q4 = reinterpret_cast<float4*>(L.dQ + ((int64_t)un.zc * L.npc + (int64_t)un.rb * BM) * DP);
+            const int n = min(BM, L.npc - un.rb * BM) * (DP / 4);
+            for (int k = wz; k < n; k += kClearWarps * 32) q4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    } else {
+        // ---- softmax warps: warp w takes rows 32 (w & 3) ... + 31 and columns 32 (w >> 2) ... + 31 of every tile ----
+        const int half = warp >> 2, my_row = tid & 127;
+        const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
+        float run_m = -INFINITY, run_l = 0.f;
+        int sg = -1;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            const int s = un.zc / d.C, c = un.zc - s * d.C, row0 = un.rb * BM, valid_rows = min(BM, L.npc - row0);
+            if (it == 0 || un.tile == 0) {
+                sg++;
+                run_m = -INFINITY;
+                run_l = 0.f;
+            }
+            const int n0 = un.tile * BN + half * 32, nv = min(32, d.N - n0);  // live columns among this warp's (may be <= 0)
+            const int brow = c * L.npc + row0 + my_row;  // batch row in the padded numbering the filter uses
+            const int32_t word = lane < nv ? __ldg(&L.mask[(int64_t)un.zc * d.N + n0 + lane]) : -1;
+            const uint32_t mb = mask_bits(word, brow - lane, brow);
+            const int sb = it & 1;
+            if (!warp_wait(kASFull + sb, (it >> 1) & 1)) break;
+            tc_fence_after();
+            float v[32];
+            tmem_ld_32x32(tmem + sb * BN + half * 32 + lane_sel, v);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[kASEmpty + sb]);
+            if (nv > 0) {
+                float* dump = s == 0 ? d.neg_scores : d.inv_neg_scores;
+                float mx = -INFINITY;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-#pragma unroll
-                for (int hh = 0; hh < H; hh++) {
-                    const float4 kb = *reinterpret_cast<const float4*>(&sm.k[j4 * 4 + q][tx * 4 + 64 * hh]);
-#pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        const float pv = q == 0 ? pa[r].x : q == 1 ? pa[r].y : q == 2 ? pa[r].z : pa[r].w;
-                        dq[r][hh][0] = fmaf(pv, kb.x, dq[r][hh][0]);
-                        dq[r][hh][1] = fmaf(pv, kb.y, dq[r][hh][1]);
-                        dq[r][hh][2] = fmaf(pv, kb.z, dq[r][hh][2]);
-                        dq[r][hh][3] = fmaf(pv, kb.w, dq[r][hh][3]);
-                    }
+                for (int j = 0; j < 32; j++) {
+                    v[j] = ((mb >> j) & 1u) ? kMasked : v[j];
+                    if (dump != nullptr && my_row < valid_rows && j < nv) dump[(int64_t)brow * d.N + n0 + j] = v[j];
+                    v[j] = j < nv ? v[j] : -INFINITY;
+                    mx = fmaxf(mx, v[j]);
                 }
+                const float nm = fmaxf(run_m, mx);
+                float add[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int j = 0; j < 32; j++) add[j & 3] += expf(v[j] - nm);  // exp(-inf) = 0 for absent columns
+                run_l = fmaf(run_l, expf(run_m - nm), (add[0] + add[1]) + (add[2] + add[3]));
+                run_m = nm;
             }
-        }
-        // dK[negatives ty*4+r][cols] = sum_i P[i][neg] * Q[i][cols]
-        float dk[4][H][4];
+            if (it == n_iter - 1 || un.tile == sc.T - 1) {
+                // end of the block, or of this CTA's share of it: the halves of a row meet
+                const int h = sg & 1;
+                if (half == 1) {
+                    if (!warp_wait(kAXchFree + h, ((sg >> 1) & 1) ^ 1)) break;
+                    s_xch[h * BM + my_row] = make_float2(run_m, run_l);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars[kAXch + h]);
+                } else {
+                    if (!warp_wait(kAXch + h, (sg >> 1) & 1)) break;
+                    const float2 o = s_xch[h * BM + my_row];
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars[kAXchFree + h]);
+                    float m = fmaxf(run_m, o.x), l = 0.f;
+                    if (m > -INFINITY) l = run_l * expf(run_m - m) + o.y * expf(o.x - m);
+                    const int first = cta_of_unit(un.item * sc.T, sc.unitsA, (int)gridDim.x);
+                    const bool whole = first == (int)blockIdx.x && un.tile == sc.T - 1;
+                    const int64_t grow = (int64_t)s * L.Bp + c * L.npc + row0 + my_row;
+                    if (!whole) {  // shared with a neighbouring CTA: the gradient pass combines the partials
+                        const int part = (int)blockIdx.x - first;
+                        if (my_row < valid_rows && part < kMaxParts) reinterpret_cast<float2*>(L.part)[grow * kMaxParts + part] = make_float2(m, l);
+                    } else {
+                        float lse = kDeadRow, loss = 0.f;
+                        if (my_row < valid_rows) {
+                            const float pos = __ldg(&L.pos[grow]), nm = fmaxf(m, pos);
+                            lse = nm + logf(l * expf(m - nm) + expf(pos - nm));
+                            L.lse[grow] = lse;
+                            loss = lse - pos;
+                        }
+                        L.lse2s[(int64_t)un.item * BM + my_row] = lse;
 #pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-            for (int hh = 0; hh < H; hh++)
-#pragma unroll
-                for (int e = 0; e < 4; e++) dk[r][hh][e] = 0.f;
-#pragma unroll 4
-        for (int i = 0; i < BM; i++) {
-            const float4 pa = *reinterpret_cast<const float4*>(&sm.p[i][ty * 4]);
-#pragma unroll
-            for (int hh = 0; hh < H; hh++) {
-                const float4 qb = *reinterpret_cast<const float4*>(&sm.q[i][tx * 4 + 64 * hh]);
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const float pv = r == 0 ? pa.x : r == 1 ? pa.y : r == 2 ? pa.z : pa.w;
-                    dk[r][hh][0] = fmaf(pv, qb.x, dk[r][hh][0]);
-                    dk[r][hh][1] = fmaf(pv, qb.y, dk[r][hh][1]);
-                    dk[r][hh][2] = fmaf(pv, qb.z, dk[r][hh][2]);
-                    dk[r][hh][3] = fmaf(pv, qb.w, dk[r][hh][3]);
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int ln = ty * 4 + r;
-            if (ln < valid_n) {
-#pragma unroll
-                for (int hh = 0; hh < H; hh++) {
-                    const int col = tx * 4 + 64 * hh;
-                    if (col < d.D) {  // padded columns of Q are zero: nothing to add there
-                        float4* dst = reinterpret_cast<float4*>(dKc + (int64_t)(n0 + ln) * DP + col);
-                        atomicAdd(dst, make_float4(dk[r][hh][0], dk[r][hh][1], dk[r][hh][2], dk[r][hh][3]));
+                        for (int k = 16; k > 0; k >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, k);
+                        if (lane == 0) atomicAdd(L.loss_acc, (double)loss);
                     }
                 }
             }
         }
     }
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const int lr = ty + 16 * r;
-        if (lr < valid_rows) {
-#pragma unroll
-            for (int hh = 0; hh < H; hh++) {
-                const int col = tx * 4 + 64 * hh;
-                *reinterpret_cast<float4*>(L.dQ + (grow0 + lr) * DP + col) = make_float4(dq[r][hh][0], dq[r][hh][1], dq[r][hh][2], dq[r][hh][3]);
+    // ---- common exit: every role ends here, normally or after an abort; then tensor memory is released ----------
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kMmaWarpA) {
+        if (*s_abort && lane == 0)  // copies still in flight get a bounded chance to land
+            for (int k = 0; k < kLseStages; k++) mbar_wait(&bars[kAYFull + k], 0, 1u << 14);
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem, 128);
+    }
+}
+
+// =====================================================================================================================
+// launch 2: both gradients
+// =====================================================================================================================
+constexpr int kDrainWarps = 8, kDrainWarp0 = kSoftWarps, kTmaWarpB = 16, kMmaWarpB = 17, kGradWarpB = 18, kThreadsB = 608;
+enum BarB { kBXFull = 0, kBXEmpty, kBYFull, kBYEmpty = kBYFull + kYSlots, kBSFull = kBYEmpty + kYSlots, kBSEmpty = kBSFull + 2, kBWFull = kBSEmpty + 2,
+            kBWEmpty, kBGFull, kBGEmpty = kBGFull + 2, kNumBarsB = kBGEmpty + 2 };
+// tensor memory: scores at 0 and 64, dK^T of a tile at 128 and 192, dQ of a tile at 256 and 384
+constexpr uint32_t kTmS = 0, kTmDk = 128, kTmDq = 256;
+
+template <int DP>
+__global__ void __launch_bounds__(kThreadsB, 1)
+    lp_grad32_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, LpKernelArgs a, Sched sc) {
+    using LY = Layout32<DP>;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = (uint64_t*)(smem + LY::kMiscB);
+    uint32_t* s_tmem = (uint32_t*)(smem + LY::kMiscB + kNumBarsB * 8);
+    volatile int* s_abort = (volatile int*)(smem + LY::kMiscB + kNumBarsB * 8 + 4);
+    const ge2_lp_desc& d = a.d;
+    const LpLayout& L = a.L;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ub = range_begin(blockIdx.x, sc.unitsB, gridDim.x), ue = range_begin(blockIdx.x + 1, sc.unitsB, gridDim.x);
+    const int n_iter = ue - ub;
+    auto spin_wait = [&](int bar, uint32_t parity) { return warp_spin_wait(&bars[bar], parity, s_abort, d.status); };
+    auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, d.status); };
+
+    if (warp == kTmaWarpB && lane == 0) {
+        mbar_init(&bars[kBXFull], 1);
+        mbar_init(&bars[kBXEmpty], 1);
+        for (int k = 0; k < kYSlots; k++) {
+            mbar_init(&bars[kBYFull + k], 1);
+            mbar_init(&bars[kBYEmpty + k], 1);
+        }
+        for (int k = 0; k < 2; k++) {
+            mbar_init(&bars[kBSFull + k], 1);
+            mbar_init(&bars[kBSEmpty + k], kSoftWarps);
+            mbar_init(&bars[kBGFull + k], 1);
+            mbar_init(&bars[kBGEmpty + k], kDrainWarps);
+        }
+        mbar_init(&bars[kBWFull], kSoftWarps);
+        mbar_init(&bars[kBWEmpty], 1);
+        *s_abort = 0;
+        mbar_init_fence();
+        prefetch_tensormap(&tmQ);
+        prefetch_tensormap(&tmK);
+    }
+    if (warp == kMmaWarpB) {
+        tmem_alloc(s_tmem, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    griddep_wait();  // set-up done; from here on global memory written by the preceding kernel is read and its buffers rewritten
+    const uint32_t tmem = *s_tmem;
+    const int KS = (d.D + kMmaK - 1) / kMmaK;
+
+    if (warp == kTmaWarpB) {
+        int sg = -1, slot = 0;
+        uint32_t phase = 1;
+        bool ok = true;
+        IterA un(ub, sc);
+        for (int it = 0; ok && it < n_iter; it++, un.next(sc)) {
+            if (it == 0 || un.tile == 0) {
+                sg++;
+                if (!spin_wait(kBXEmpty, (sg & 1) ^ 1)) break;
+                mbar_expect_tx_warp(&bars[kBXFull], kPlanes * LY::kXPlane);
+                for (int p = 0; p < kPlanes; p++)
+                    for (int b = 0; b < LY::NB; b++)
+                        tma_load_3d_warp(smem + LY::kX + p * LY::kXPlane + b * LY::kXBlock, &tmQ, b * 64, un.rb * BM, p * sc.ZC + un.zc, &bars[kBXFull]);
+            }
+            for (int k = 0; k < kPlanes; k++) {
+                ok = spin_wait(kBYEmpty + slot, phase);
+                if (!ok) break;
+                const int p = k == 0 ? 1 : k == 1 ? 0 : 2;  // m, h, l
+                mbar_expect_tx_warp(&bars[kBYFull + slot], LY::kYPlane);
+                for (int b = 0; b < LY::NB; b++)
+                    tma_load_3d_warp(smem + LY::kY + slot * LY::kYPlane + b * LY::kYBlock, &tmK, b * 64, un.tile * BN, p * sc.ZC + un.zc, &bars[kBYFull + slot]);
+                if (++slot == kYSlots) slot = 0, phase ^= 1;
             }
         }
+    } else if (warp == kMmaWarpB) {
+        // ---- S = X Y^T ----
+        constexpr uint32_t kIdesc = idesc_bf16(BM, BN, 0, 0);
+        const uint32_t dX = desc_lo_sw128(smem_u32(smem + LY::kX), 16), dY0 = desc_lo_sw128(smem_u32(smem + LY::kY), 16);
+        int sg = -1, slot0 = 0;
+        uint32_t ph0 = 0;
+        bool ok = true;
+        IterA un(ub, sc);
+        for (int it = 0; ok && it < n_iter; it++, un.next(sc)) {
+            if (it == 0 || un.tile == 0) {
+                sg++;
+                if (!spin_wait(kBXFull, sg & 1)) break;
+            }
+            const int sb = it & 1, su = it >> 1;
+            if (!spin_wait(kBSEmpty + sb, (su & 1) ^ 1)) break;
+            int seen = 0;  // planes of this tile known to have arrived, in the order m, h, l
+#pragma unroll 1
+            for (int p = 0; p < 6; p++) {
+                const int k = slot_of_plane((kSecondS >> (2 * p)) & 3);
+                const int slot = slot0 + k >= kYSlots ? slot0 + k - kYSlots : slot0 + k;
+                if (k >= seen) {
+                    ok = spin_wait(kBYFull + slot, slot0 + k >= kYSlots ? ph0 ^ 1 : ph0);
+                    if (!ok) break;
+                    seen = k + 1;
+                    tc_fence_after();
+                }
+                const uint32_t da = dX + ((kFirstS >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY0 + slot * (LY::kYPlane >> 4);
+#pragma unroll
+                for (int ks = 0; ks < DP / kMmaK; ks++)
+                    if (ks < KS)
+                        mma_f16_ss_warp(tmem + kTmS + sb * BN, da + (((ks >> 2) * LY::kXBlock + (ks & 3) * 32) >> 4),
+                                        db + (((ks >> 2) * LY::kYBlock + (ks & 3) * 32) >> 4), kIdesc, (p > 0 || ks > 0) ? 1u : 0u);
+            }
+            if (!ok) break;
+            mma_commit_warp(&bars[kBSFull + sb]);
+            slot0 += kPlanes;
+            if (slot0 >= kYSlots) slot0 -= kYSlots, ph0 ^= 1;
+        }
+    } else if (warp == kGradWarpB) {
+        // ---- dK^T [d x 64] = X^T W, then dQ [128 x D] of the tile = W Y ----
+        const uint32_t kIdescDk = idesc_bf16(128, BN, 1, 1), kIdescDq = idesc_bf16(BM, KS * kMmaK, 0, 1);
+        // X along its columns: the second 64 of them lie a block further (for D <= 64 there are none, and what is read there ends up in
+        // accumulator rows that nobody reads)
+        const uint32_t dXm = desc_lo_sw128(smem_u32(smem + LY::kX), LY::kXBlock), dWm = desc_lo_sw128(smem_u32(smem + LY::kW), 16 * 1024),
+                       dWk = desc_lo_sw128(smem_u32(smem + LY::kW), 16), dYm0 = desc_lo_sw128(smem_u32(smem + LY::kY), LY::kYBlock);
+        int slot0 = 0;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            const int pb = it & 1;
+            if (!spin_wait(kBGEmpty + pb, ((it >> 1) & 1) ^ 1)) break;
+            // (no wait on X or Y: W was made from scores that were made from them)
+            if (!spin_wait(kBWFull, it & 1)) break;
+            tc_fence_after();
+#pragma unroll 1
+            for (int p = 0; p < 6; p++) {
+                const uint32_t da = dXm + ((kFirst >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dWm + ((kSecond >> (2 * p)) & 3) * (LY::kWPlane >> 4);
+#pragma unroll
+                for (int ks = 0; ks < BM / kMmaK; ks++)
+                    mma_f16_ss_warp(tmem + kTmDk + pb * BN, da + ks * (2048 >> 4), db + ks * (2048 >> 4), kIdescDk, (p > 0 || ks > 0) ? 1u : 0u);
+            }
+#pragma unroll 1
+            for (int p = 0; p < 6; p++) {
+                const int k = slot_of_plane((kSecondDq >> (2 * p)) & 3);
+                const int slot = slot0 + k >= kYSlots ? slot0 + k - kYSlots : slot0 + k;
+                const uint32_t da = dWk + ((kFirstDq >> (2 * p)) & 3) * (LY::kWPlane >> 4), db = dYm0 + slot * (LY::kYPlane >> 4);
+#pragma unroll
+                for (int ks = 0; ks < BN / kMmaK; ks++)
+                    mma_f16_ss_warp(tmem + kTmDq + pb * 128, da + ks * (32 >> 4), db + ks * (2048 >> 4), kIdescDq, (p > 0 || ks > 0) ? 1u : 0u);
+                if (p == 1 || p == 2 || p == 5) mma_commit_warp(&bars[kBYEmpty + slot]);  // the last product with this plane of Y
+            }
+            mma_commit_warp(&bars[kBWEmpty]);
+            if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit_warp(&bars[kBXEmpty]);
+            mma_commit_warp(&bars[kBGFull + pb]);  // last: whoever waits for it has seen the others' arrivals land before the CTA exits
+            slot0 += kPlanes;
+            if (slot0 >= kYSlots) slot0 -= kYSlots;
+        }
+    } else if (warp < kSoftWarps) {
+        // ---- softmax warps: warp w takes rows 32 (w & 3) ... + 31 and columns 32 (w >> 2) ... + 31 of every tile ----
+        const int half = warp >> 2, my_row = tid & 127;
+        const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
+        float lrow = kDeadRow;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            const int s = un.zc / d.C, c = un.zc - s * d.C, row0 = un.rb * BM;
+            const int brow = c * L.npc + row0 + my_row;
+            if (it == 0 || un.tile == 0) {
+                // was the block run by one CTA of the logsumexp pass (that launch's grid and ranges are known here)?
+                const int first = cta_of_unit(un.item * sc.T, sc.unitsA, sc.gridA);
+                const int nparts = cta_of_unit(un.item * sc.T + sc.T - 1, sc.unitsA, sc.gridA) - first + 1;
+                if (nparts == 1) {
+                    lrow = __ldg(&L.lse2s[(int64_t)un.item * BM + my_row]);
+                } else {
+                    // combine the partial (max, sum) pairs its sharers left; the CTA that starts the block here also writes the lse for
+                    // the scatter kernel and adds the rows' loss terms
+                    const int64_t grow = (int64_t)s * L.Bp + brow;
+                    const bool writer = un.tile == 0 && half == 0;
+                    float loss = 0.f;
+                    lrow = kDeadRow;
+                    if (my_row < min(BM, L.npc - row0)) {
+                        const float2* part = reinterpret_cast<const float2*>(L.part) + grow * kMaxParts;
+                        float m = -INFINITY, l = 0.f;
+                        for (int k = 0; k < nparts && k < kMaxParts; k++) {
+                            const float2 pk = __ldg(&part[k]);
+                            const float nm = fmaxf(m, pk.x);
+                            if (nm > -INFINITY) {
+                                l = l * expf(m - nm) + pk.y * expf(pk.x - nm);
+                                m = nm;
+                            }
+                        }
+                        const float pos = __ldg(&L.pos[grow]), nm = fmaxf(m, pos);
+                        lrow = nm + logf(l * expf(m - nm) + expf(pos - nm));
+                        if (writer) {
+                            L.lse[grow] = lrow;
+                            loss = lrow - pos;
+                        }
+                    }
+                    if (writer) {
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+                        if (lane == 0) atomicAdd(L.loss_acc, (double)loss);
+                    }
+                }
+            }
+            const int n0 = un.tile * BN + half * 32, nv = min(32, d.N - n0);  // live columns among this warp's (may be <= 0)
+            const int32_t word = lane < nv ? __ldg(&L.mask[(int64_t)un.zc * d.N + n0 + lane]) : -1;
+            const uint32_t mb = mask_bits(word, brow - lane, brow);
+            const int sb = it & 1;
+            if (!warp_wait(kBSFull + sb, (it >> 1) & 1)) break;
+            tc_fence_after();
+            float v[32];
+            tmem_ld_32x32(tmem + kTmS + sb * BN + half * 32 + lane_sel, v);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[kBSEmpty + sb]);
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                const float p = expf(v[j] - lrow);
+                // masked entries were overwritten in place by the reference: no gradient reaches them; columns past the chunk have none
+                v[j] = j < nv && !((mb >> j) & 1u) ? p : 0.f;
+            }
+            if (!warp_wait(kBWEmpty, (it & 1) ^ 1)) break;
+            unsigned char* w0 = smem + LY::kW + my_row * 128;
+#pragma unroll 1
+            for (int p = 0; p < kPlanes; p++) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) {  // 8 values = one 16-byte chunk; what is left of them stays for the next plane
+                    uint32_t pk[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * q + 2 * e], v[8 * q + 2 * e + 1]);
+                        pk[e] = *reinterpret_cast<const uint32_t*>(&h);
+                        v[8 * q + 2 * e] -= __uint_as_float(pk[e] << 16);
+                        v[8 * q + 2 * e + 1] -= __uint_as_float(pk[e] & 0xffff0000u);
+                    }
+                    *reinterpret_cast<uint4*>(w0 + p * LY::kWPlane + (((half * 4 + q) ^ (my_row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                }
+            }
+            fence_proxy_async_smem();  // W was written with ordinary stores; the MMA reads it through the async proxy
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[kBWFull]);
+        }
+    } else {
+        // ---- drain warps: dK^T leaves by atomics (lanes run along a row of dK), dQ is summed in registers over the block's tiles ----
+        constexpr int kCols = DP / 2;  // columns of dQ a thread sums: its row, half of them
+        const int w = warp - kDrainWarp0, quarter = warp & 3, half = w >> 2;
+        const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
+        const int dcol = quarter * 32 + lane;  // dK^T: this lane's embedding column
+        float acc[kCols];
+        bool whole = false;
+        IterA un(ub, sc);
+        for (int it = 0; it < n_iter; it++, un.next(sc)) {
+            if (it == 0 || un.tile == 0) {
+                whole = un.tile == 0 && (ub + it + sc.T <= ue);  // this CTA runs the block's whole stream
+#pragma unroll
+                for (int k = 0; k < kCols; k++) acc[k] = 0.f;
+            }
+            const int pb = it & 1;
+            if (!warp_wait(kBGFull + pb, (it >> 1) & 1)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int k = 0; k < kCols; k += 16) {
+                float t[16];
+                tmem_ld_32x16(tmem + kTmDq + pb * 128 + half * kCols + k + lane_sel, t);
+#pragma unroll
+                for (int j = 0; j < 16; j++) acc[k + j] += t[j];
+            }
+            const int n0 = un.tile * BN + half * 32;
+            float* dk = L.dK + ((int64_t)un.zc * d.N + n0) * DP + dcol;
+#pragma unroll 1
+            for (int k = 0; k < 32; k += 16) {
+                float t[16];
+                tmem_ld_32x16(tmem + kTmDk + pb * BN + half * 32 + k + lane_sel, t);
+                if (k == 16) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars[kBGEmpty + pb]);
+                }
+                if (dcol < d.D) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        if (n0 + k + j < d.N) atomicAdd(dk + (int64_t)(k + j) * DP, t[j]);
+                }
+            }
+            if (it == n_iter - 1 || un.tile == sc.T - 1) {
+                const int row = un.rb * BM + dcol;  // dQ: this lane's row
+                if (row < L.npc) {
+                    float4* q4 = reinterpret_cast<float4*>(L.dQ + ((int64_t)un.zc * L.npc + row) * DP + half * kCols);
+#pragma unroll
+                    for (int k = 0; k < kCols; k += 4) {
+                        if (half * kCols + k >= d.D) continue;
+                        const float4 x = make_float4(acc[k], acc[k + 1], acc[k + 2], acc[k + 3]);
+                        if (whole) q4[k / 4] = x;
+                        else atomicAdd(q4 + k / 4, x);
+                    }
+                }
+            }
+        }
+    }
+    // ---- common exit: every role ends here, normally or after an abort; then tensor memory is released ----------
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kMmaWarpB) {
+        if (*s_abort && lane == 0) {  // copies and contractions still in flight get a bounded chance to land
+            for (int k = 0; k < kYSlots; k++) mbar_wait(&bars[kBYFull + k], 0, 1u << 14);
+            for (int k = 0; k < 2; k++) mbar_wait(&bars[kBGFull + k], 0, 1u << 14);
+        }
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
     }
 }
 
 template <int DP>
 int launch(const LpKernelArgs& a, cudaStream_t stream) {
-    const size_t smem = sizeof(Smem<DP>);
-    // per-device function attribute; setting it on every launch keeps multi-device processes correct and is not a stream operation
-    GE2_CUDA_TRY(cudaFuncSetAttribute(lp_scores_fp32_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)ceil_div(a.L.npc, BM), (unsigned)a.d.C, (unsigned)a.L.S);
-    lp_scores_fp32_kernel<DP><<<grid, kThreads, smem, stream>>>(a);
-    GE2_LAUNCH_CHECK();
+    using LY = Layout32<DP>;
+    const int ZC = a.L.S * a.d.C;
+    CUtensorMap tmQ, tmK;
+    int rc = make_operand_map(&tmQ, a.L.Qs, true, DP, a.L.npc, (int64_t)kPlanes * ZC, BM);
+    if (rc != GE2_OK) return rc;
+    rc = make_operand_map(&tmK, a.L.Ks, true, DP, a.d.N, (int64_t)kPlanes * ZC, BN);
+    if (rc != GE2_OK) return rc;
+    Sched sc;
+    sc.RB = ceil_div(a.L.npc, BM);
+    sc.T = ceil_div(a.d.N, BN);
+    sc.ZC = ZC;
+    const long long units = (long long)ZC * sc.RB * sc.T;
+    if (units > 0x3fffffff) return GE2_ERR_UNSUPPORTED;
+    sc.unitsA = sc.unitsB = (int)units;
+    // every CTA's range is at least ceil(T / 7) units long, so a row block is shared by at most kMaxParts CTAs
+    sc.gridA = std::max(1, std::min(kNumSMs, sc.unitsA / ceil_div(sc.T, kMaxParts - 1)));
+    sc.gridB = std::max(1, std::min(kNumSMs, sc.unitsB));
+    // per-device function attributes; setting them on every launch keeps multi-device processes correct and is not a stream operation
+    GE2_CUDA_TRY(cudaFuncSetAttribute(lp_lse32_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::kBytesA));
+    GE2_CUDA_TRY(cudaFuncSetAttribute(lp_grad32_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::kBytesB));
+    GE2_CUDA_TRY(launch_after(lp_lse32_kernel<DP>, dim3((unsigned)sc.gridA), dim3(kThreadsA), LY::kBytesA, stream, tmQ, tmK, a, sc));
+    GE2_CUDA_TRY(launch_after(lp_grad32_kernel<DP>, dim3((unsigned)sc.gridB), dim3(kThreadsB), LY::kBytesB, stream, tmQ, tmK, a, sc));
     return GE2_OK;
 }
 

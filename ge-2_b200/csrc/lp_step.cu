@@ -58,6 +58,25 @@ __device__ __forceinline__ void store_half4(__half* dst, float4 v) {
     *reinterpret_cast<uint2*>(dst) = pk;
 }
 
+// an fp32 value as the sum of three bf16 values, exactly (24 bits as 8 + 8 + 8; rounded to nearest, so the parts alternate in sign and
+// the later ones are at most 2^-8 and 2^-16 of it)
+__device__ __forceinline__ void store_split4(__nv_bfloat16* dst, int64_t plane, float4 v) {
+    const float x[4] = {v.x, v.y, v.z, v.w};
+    float r[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) r[e] = x[e];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(r[0], r[1]), b = __floats2bfloat162_rn(r[2], r[3]);
+        uint2 pk;
+        pk.x = *reinterpret_cast<const uint32_t*>(&a);
+        pk.y = *reinterpret_cast<const uint32_t*>(&b);
+        *reinterpret_cast<uint2*>(dst + k * plane) = pk;
+        const float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);
+        r[0] -= fa.x, r[1] -= fa.y, r[2] -= fb.x, r[3] -= fb.y;
+    }
+}
+
 // ---------------------------------------------------------------------------------------------------
 // prep: eight lanes per output row (four rows in flight per warp, so the dependent loads id -> row index -> embedding
 // row overlap), each lane 4 columns at a time.  Rows [0, S*Bp) are query rows, rows [S*Bp, S*Bp + S*CN) negative rows.
@@ -75,18 +94,14 @@ __global__ void __launch_bounds__(256) lp_prep_kernel(LpKernelArgs a) {
     const int D = d.D, h = D / 2, ld = L.ld;
     const bool vec_e = (d.emb_stride % 4 == 0) && (((uintptr_t)d.node_emb) & 15) == 0 && D % 4 == 0;
     const bool vec_r = D % 4 == 0 && ((((uintptr_t)d.rel) | ((uintptr_t)d.inv_rel)) & 15) == 0;
-    const bool write_k32 = d.precision != GE2_PRECISION_F16;  // the tensor path reads only the fp16 copy of the negatives
+    const int64_t q_plane = q_rows * ld, k_plane = (int64_t)L.S * L.CN * ld;
     griddep_wait();
     if (blockIdx.x == 0 && tid == 0) *L.loss_acc = 0.0;        // the scores kernel of this step adds every row's loss term to it
-    if (blockIdx.x == 0 && L.item_ctr != nullptr)               // arrival counters of the tensor path's logsumexp pass start at zero
-        for (int k = tid; k < L.n_items + 2; k += blockDim.x) L.item_ctr[k] = 0;
     for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + tid) >> 3; w < total_pad; w += groups) {
         if (w >= total) continue;
         if (w < q_rows) {
             const int s = (int)(w / L.Bp);
             const int i = (int)(w - (int64_t)s * L.Bp);
-            float* q = L.Q + ((int64_t)s * L.Bp + i) * ld;
-            __half* qh = L.Qh != nullptr ? L.Qh + ((int64_t)s * L.Bp + i) * ld : nullptr;
             bool ok = i < d.B;  // rows past B: zero rows appended by pad_and_reshape; their positive score is padded with 0
             int64_t sid = 0, did = 0, rid = 0;
             if (ok) {
@@ -134,8 +149,8 @@ __global__ void __launch_bounds__(256) lp_prep_kernel(LpKernelArgs a) {
                     const float4 y = load4(eb, k, D, vec_e);
                     dot += v.x * y.x + v.y * y.y + v.z * y.z + v.w * y.w;
                 }
-                if (write_k32) *reinterpret_cast<float4*>(q + k) = v;  // only the fp32 scores kernel reads the fp32 copies
-                if (qh != nullptr) store_half4(qh + k, v);
+                if (L.Qh != nullptr) store_half4(L.Qh + w * ld + k, v);
+                else store_split4(L.Qs + w * ld + k, q_plane, v);
             }
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) dot += __shfl_xor_sync(gmask, dot, o);
@@ -163,8 +178,8 @@ __global__ void __launch_bounds__(256) lp_prep_kernel(LpKernelArgs a) {
             const float* src = bad ? nullptr : emb_row(d, id);
             for (int k = gl * 4; k < ld; k += 32) {
                 const float4 v = bad ? make_float4(0.f, 0.f, 0.f, 0.f) : load4(src, k, D, vec_e);
-                if (write_k32) *reinterpret_cast<float4*>(L.K + e * ld + k) = v;
                 if (L.Kh != nullptr) store_half4(L.Kh + e * ld + k, v);
+                else store_split4(L.Ks + e * ld + k, k_plane, v);
             }
         }
     }
@@ -499,8 +514,6 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     cudaStream_t stream = as_stream(stream_);
 
     const int phases = desc->phases == 0 ? 7 : desc->phases;
-    // fp32 path: dK is reduced with atomics and starts from zero; the tensor path stores whole tiles and clears nothing
-    if ((phases & 2) && desc->precision == GE2_PRECISION_FP32) GE2_CUDA_TRY(cudaMemsetAsync(L.dK, 0, L.zero_bytes, stream));
     if ((phases & 4) && !(desc->flags & GE2_LP_NODE_GRAD_IS_ZERO))
         GE2_CUDA_TRY(cudaMemsetAsync(desc->node_grad, 0, (size_t)desc->U * desc->D * 4, stream));
     if (phases & 1) {

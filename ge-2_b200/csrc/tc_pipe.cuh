@@ -109,10 +109,10 @@ inline int encode_3d(CUtensorMap* map, CUtensorMapDataType type, int elem_bytes,
     return GE2_OK;
 }
 
-// [mats][rows][ld 16-bit elements] as a 3-D tensor of operand blocks: box = 64 elements x 128 rows of one matrix, 128-byte swizzle,
+// [mats][rows][ld 16-bit elements] as a 3-D tensor of operand blocks: box = 64 elements x box_rows rows of one matrix, 128-byte swizzle,
 // rows past the matrix end read as zero
-inline int make_operand_map(CUtensorMap* map, void* base, bool bf16, int64_t ld, int64_t rows, int64_t mats) {
-    return encode_3d(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, ld, rows, mats, 64, 128,
+inline int make_operand_map(CUtensorMap* map, void* base, bool bf16, int64_t ld, int64_t rows, int64_t mats, int box_rows = 128) {
+    return encode_3d(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, ld, rows, mats, 64, box_rows,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
 }
 

@@ -118,55 +118,50 @@ __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, int a_mn, int b_m
 }
 // the same with bf16 A and B (format code 1)
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int a_mn, int b_mn) { return idesc_f16(M, N, a_mn, b_mn) | (1u << 7) | (1u << 10); }
-__device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // ---- the same, issued from code that the whole warp runs -----------------------------------------------------------------
 // The asynchronous instructions need one thread, but a one-lane section is no place for a loop that juggles descriptors: with many of
 // them alive, values the compiler keeps in uniform registers were seen to come back wrong there (single k-steps of a contraction read
-// other operands).  These forms are run by all 32 lanes and predicated on `leader` (non-zero in one lane), so control flow and all
-// address arithmetic stay warp-uniform.  Descriptors are given by their low words: the high word of a 128-byte-swizzled operand
-// with 8-row groups 1024 bytes apart is a constant.
+// other operands).  These forms are run by all 32 lanes, converged, and elect.sync picks the (same) one that issues, so control flow
+// and all address arithmetic stay warp-uniform: 48 / 64 / 128 cycles a contraction of N = 64 / 128 / 256, the rate of the pipe (a lane
+// predicate instead of the election: 62 - 67 cycles at N <= 128).  Descriptors are given by their low words: the high word of a
+// 128-byte-swizzled operand with 8-row groups 1024 bytes apart is a constant.
 constexpr uint32_t kDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo_sw128(uint32_t addr, uint32_t lbo) { return ((addr & 0x3FFFFu) >> 4) | (((lbo >> 4) & 0x3FFFu) << 16); }
-__device__ __forceinline__ void mma_f16_ss_warp(uint32_t leader, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16_ss_warp(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 x;\n\t.reg .b64 da, db;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "mov.b64 da, {%1, %6};\n\t"
-        "mov.b64 db, {%2, %6};\n\t"
+        "elect.sync x|q, 0xffffffff;\n\t"
+        "mov.b64 da, {%1, %5};\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
-        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(leader), "r"(kDescHiSw128)
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHiSw128)
         : "memory");
 }
-__device__ __forceinline__ void mma_commit_warp(uint32_t leader, uint64_t* bar) {
+__device__ __forceinline__ void mma_commit_warp(uint64_t* bar) {
     asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(leader)
+        "{\n\t.reg .pred q;\n\t.reg .b32 x;\n\t"
+        "elect.sync x|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
         : "memory");
 }
-// expects one box of `bytes` on the barrier and starts its load
-__device__ __forceinline__ void tma_load_3d_warp(uint32_t leader, void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar, uint32_t bytes) {
+__device__ __forceinline__ void mbar_expect_tx_warp(uint64_t* bar, uint32_t bytes) {
     asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], %7;\n\t"
+        "{\n\t.reg .pred q;\n\t.reg .b32 x;\n\t"
+        "elect.sync x|q, 0xffffffff;\n\t"
+        "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+        "r"(bytes)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_warp(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t.reg .b32 e;\n\t"
+        "elect.sync e|q, 0xffffffff;\n\t"
         "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}" ::"r"(smem_u32(smem_dst)),
-        "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(leader), "r"(bytes)
+        "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
 
-// arrives on the mbarrier once every tcgen05.mma issued so far by this thread has completed
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // ---- tensor memory -> registers: this warp's 32 lanes x 32 consecutive 32-bit columns ------------------------------
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, float (&v)[32]) {
@@ -186,17 +181,18 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// this warp's 32 lanes x 64 consecutive 32-bit columns
-__device__ __forceinline__ void tmem_ld_32x64(uint32_t taddr, float (&v)[64]) {
-    uint32_t r[64];
+// this warp's 32 lanes x 16 consecutive 32-bit columns
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
         "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
 #pragma unroll
-    for (int i = 0; i < 64; i++) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
 }  // namespace tc

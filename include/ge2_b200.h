@@ -99,7 +99,8 @@ GE2_API int ge2_pack_ids(const int64_t *const parts[4], const int64_t lens[4], c
  * consumed the previous batch's gradients), so the step skips its own memset of U * D floats */
 #define GE2_LP_NODE_GRAD_IS_ZERO 1
 
-#define GE2_PRECISION_FP32 0 /* CUDA-core FFMA contraction, fp32 throughout (1e-4 relative parity)      */
+#define GE2_PRECISION_FP32 0 /* fp32 throughout (1e-4 relative parity): tcgen05 tiles of operands split exactly into three
+                                bf16 terms, small products first, tiles summed in fp32                   */
 #define GE2_PRECISION_F16 1  /* tcgen05 kind::f16 tiles (fp16 operands, 11-bit significand like TF32), fp32
                                 accumulate in TMEM, fp32 everywhere else (1e-2 relative parity)         */
 

@@ -206,3 +206,19 @@ def test_full_size_step_is_the_sum_of_its_chunks(capi, cuda_device, precision, B
     assert rel_err(whole["rel_grad"], rel_grad) < tol
     assert rel_err(whole["inv_rel_grad"], inv_rel_grad) < tol
     assert np.abs(node_grad).max() > 0
+
+
+@pytest.mark.parametrize("kind,B,C,N,D", [
+    ("DISTMULT", 129, 1, 63, 64), ("DISTMULT", 128, 1, 65, 65), ("COMPLEX", 257, 2, 1, 66),   # one row, one negative past a tile
+    ("DISTMULT", 7, 3, 200, 1), ("COMPLEX", 1500, 2, 900, 128), ("DISTMULT", 60, 1, 2000, 17),  # blocks cut between CTAs; narrow rows
+])
+def test_split_operand_tiles_at_their_edges(capi, cuda_device, kind, B, C, N, D):
+    """The fp32 path's exact bf16 splitting and its tile sums: gradients to a few fp32 roundings of float64 contractions."""
+    case = workloads.make_case(kind, B, C, N, D, 5, 150, N // 2, 31 + D)
+    o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
+    exp = dict(loss=o.loss, node_grad=o.node_grad, rel_grad=o.rel_grad, inv_rel_grad=o.inv_rel_grad)
+    got = run_lp_step(capi, case, cuda_device, "fp32", "pairs")
+    assert got["status"] == 0
+    assert abs(got["loss"] - exp["loss"]) <= 2e-6 * abs(exp["loss"])
+    for key in ("node_grad", "rel_grad", "inv_rel_grad"):
+        assert rel_err(got[key], exp[key]) <= 5e-6, key
