@@ -355,11 +355,8 @@ __global__ void __launch_bounds__(kCountThreads, 1)
                 ok = spin_wait(kAccEmpty + ab, ((ac / kAccs) & 1) ^ 1);
                 if (!ok) break;
                 const uint32_t acc = tmem + ab * kTileN;
-                // (straight-line issue: the tensor pipe is fed a 128-cycle contraction at a time)
-                auto product = [&](uint32_t da, uint32_t db, int b, bool first) {
-#pragma unroll
-                    for (int ks = 0; ks < 4; ks++)
-                        if (ks + 4 * b < KS) mma_f16_ss_warp(acc, da + ks * 2, db + b * kCandStep + ks * 2, kIdesc, (first && ks == 0) ? 0u : 1u);
+                auto product = [&](uint32_t da, uint32_t db, int b, bool first) {  // one 64-column block
+                    mma_kmajor<1, kBlockBytes, SM::kCandBlock>(min(4, KS - 4 * b), acc, da, db + b * kCandStep, kIdesc, first ? 0u : 1u);
                 };
 #pragma unroll
                 for (int k = 0; k < 2 * NB; k++) {

@@ -171,11 +171,7 @@ __global__ void __launch_bounds__(kThreadsA, 1)
 #pragma unroll 1
             for (int p = 0; p < 6; p++) {
                 const uint32_t da = dX + ((kFirst >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY + ((kSecond >> (2 * p)) & 3) * (LY::kYPlane >> 4);
-#pragma unroll
-                for (int ks = 0; ks < DP / kMmaK; ks++)
-                    if (ks < KS)
-                        mma_f16_ss_warp(tmem + sb * BN, da + (((ks >> 2) * LY::kXBlock + (ks & 3) * 32) >> 4),
-                                        db + (((ks >> 2) * LY::kYBlock + (ks & 3) * 32) >> 4), kIdesc, (p > 0 || ks > 0) ? 1u : 0u);
+                mma_kmajor<LY::NB, LY::kXBlock, LY::kYBlock>(KS, tmem + sb * BN, da, db, kIdesc, p > 0 ? 1u : 0u);
             }
             mma_commit_warp(&bars[kAYEmpty + st]);
             if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit_warp(&bars[kAXEmpty]);
@@ -398,11 +394,7 @@ __global__ void __launch_bounds__(kThreadsB, 1)
                     tc_fence_after();
                 }
                 const uint32_t da = dX + ((kFirstS >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY0 + slot * (LY::kYPlane >> 4);
-#pragma unroll
-                for (int ks = 0; ks < DP / kMmaK; ks++)
-                    if (ks < KS)
-                        mma_f16_ss_warp(tmem + kTmS + sb * BN, da + (((ks >> 2) * LY::kXBlock + (ks & 3) * 32) >> 4),
-                                        db + (((ks >> 2) * LY::kYBlock + (ks & 3) * 32) >> 4), kIdesc, (p > 0 || ks > 0) ? 1u : 0u);
+                mma_kmajor<LY::NB, LY::kXBlock, LY::kYBlock>(KS, tmem + kTmS + sb * BN, da, db, kIdesc, p > 0 ? 1u : 0u);
             }
             if (!ok) break;
             mma_commit_warp(&bars[kBSFull + sb]);

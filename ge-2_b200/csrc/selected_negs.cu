@@ -13,14 +13,13 @@
 //
 // Here a warp owns a query row: the row sits in registers (D <= 128, four values a lane), every chosen negative row is read
 // once with coalesced (16-byte, where the rows allow it) loads and serves the score, the query gradient and the negative gradient of its pair in one pass
-// (the reference's backward reads every pair twice, in two launches).  The tournament never stores the [rows x N] scores:
-// a CTA holds 128 query rows in shared memory, streams 128-column tiles whose edges fall on group boundaries, and scans each
-// tile for the group winners.  fp32 on the CUDA cores: the winner of a group is decided by comparing nearly equal scores.
+// (the reference's backward reads every pair twice, in two launches).  The tournament never stores the [rows x N] scores: they are
+// contracted tile by tile on the tensor cores, with fp32 operands split exactly, and the group winners are read off the tiles.
 #include <math_constants.h>
 
 #include <algorithm>
 
-#include "common.cuh"
+#include "tc_pipe.cuh"
 
 namespace ge2 {
 namespace {
@@ -203,157 +202,253 @@ __global__ void __launch_bounds__(kPairThreads) selected_scores_backward_kernel(
 // ---------------------------------------------------------------------------------------------------------------------------
 // tournament selection
 // ---------------------------------------------------------------------------------------------------------------------------
-constexpr int kTile = 128, kHalf = kTile / 2, kChunkD = 32, kTourThreads = 256;
-constexpr int kTileStride = kTile + 4;  // floats between the rows of Qt and Et: 16-byte aligned, banks shifted by 4 a row
-constexpr int kStStride = kTile + 1;
-constexpr int kFetch = kTile * kChunkD / kTourThreads;  // values of a negative slice a thread moves: 16 consecutive of one row
+// Scores are contracted on the tensor cores: both operands are split exactly into three bf16 terms in shared memory (x = xh + xm + xl) and
+// a tile of 128 query rows x 64 negatives is xl yh + xh yl + xm ym + xm yh + xh ym + xh yh, the small products first; what is left
+// out is below 2^-24 of |x y|, the sums are fp32 in tensor memory.  Two negatives with equal rows get equal scores, so ties stay ties.
+//
+// A CTA keeps a tile of query rows and takes a contiguous share of all (chunk, row tile, group) triples, so every SM is busy to the end and a
+// share begins and ends on a group boundary.  Warps by role: 8 warps convert rows (fp32, read along the row) into one of two tile
+// buffers, one issues the contractions, 4 epilogue warps walk the scores: a thread owns a row, keeps the running winner of the group
+// in registers and writes it where the group ends.  Groups need not fit tiles.
+// Bound by the contractions (6 ceil(D / 16) steps of 48 cycles a tile at best, 92 beside the conversion's shared-memory stores) and the
+// one epilogue warp a scheduler.  50 000 rows x 1 000 negatives, D = 100, 100 kept: 122 us (405 us as fp32 multiply-adds).
+using namespace tc;
+constexpr int kTourRows = 128, kTourCols = 64, kTourPlanes = 3;
+constexpr int kTourThreads = 512, kTourEpi0 = 0, kTourMma = 4, kTourConv0 = 8, kTourConvWarps = 8;
 
 struct TourArgs {
     const float* chunked;    // [chunks, R, D]
     const float* negatives;  // [chunks, N, D]
     int64_t R, N, K, T;      // T = N / K negatives in a group
-    int64_t units;           // work items of a (chunk, row tile): T <= 128: tiles of groups_per_unit whole groups; else one group
-    int64_t units_per_cta;   // a CTA takes this many consecutive units
-    int groups_per_unit;
+    int64_t row_tiles, shares_total;  // shares_total = chunks * row_tiles * K groups to deal out
     int D;
     float* out_scores;       // [chunks * R, K]
     int64_t* out_idx;        // [chunks * R, K] column of the winner in its chunk
+    int32_t* status;
 };
 
-inline size_t tour_smem_bytes(int D) { return (size_t)(D * kTileStride + kChunkD * kTileStride + kHalf * kStStride) * sizeof(float); }
+template <int NB>
+struct TourSmem {
+    static constexpr int kQBlock = kTourRows * 128, kYBlock = kTourCols * 128;
+    static constexpr int kQPlane = NB * kQBlock, kYPlane = NB * kYBlock;
+    static constexpr int kQ = 0, kY = kTourPlanes * kQPlane, kMisc = kY + 2 * kTourPlanes * kYPlane;
+    static constexpr int kBytes = (kMisc + 256 + 1024) > 120 * 1024 ? (kMisc + 256 + 1024) : 120 * 1024;  // one CTA an SM
+};
+enum TourBar { kTQFull = 0, kTQEmpty, kTYFull, kTYEmpty = kTYFull + 2, kTSFull = kTYEmpty + 2, kTSEmpty = kTSFull + 2, kTourBars = kTSEmpty + 2 };
 
-// the slice [c0, c0 + 32) of 128 negative rows starting at column n0: a thread holds 16 consecutive values of one row
-__device__ __forceinline__ void tour_fetch(float (&r)[kFetch], const float* __restrict__ Nc, int64_t n0, int64_t col_end, int c0, int D, int tid) {
-    const int64_t col = n0 + (tid >> 1);
-    const int d0 = c0 + (tid & 1) * kFetch;
-    const float* row = Nc + col * D;
-    const bool in = col < col_end;
-#pragma unroll
-    for (int k = 0; k < kFetch; k++) r[k] = (in && d0 + k < D) ? __ldg(row + d0 + k) : 0.f;
+// four consecutive columns of a row (zeros past D), read with the widest access its alignment allows
+template <int VEC>
+__device__ __forceinline__ float4 tour_load(const float* __restrict__ row, int c, int D, bool there) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (VEC == 4) {
+        if (there && c < D) v = __ldg(reinterpret_cast<const float4*>(row + c));
+    } else if (VEC == 2) {
+        float2 x = make_float2(0.f, 0.f), y = x;
+        if (there && c < D) x = __ldg(reinterpret_cast<const float2*>(row + c));
+        if (there && c + 2 < D) y = __ldg(reinterpret_cast<const float2*>(row + c + 2));
+        v = make_float4(x.x, x.y, y.x, y.y);
+    } else {
+        if (there && c < D) v.x = __ldg(row + c);
+        if (there && c + 1 < D) v.y = __ldg(row + c + 1);
+        if (there && c + 2 < D) v.z = __ldg(row + c + 2);
+        if (there && c + 3 < D) v.w = __ldg(row + c + 3);
+    }
+    return v;
 }
 
-// grid: x = tiles of 128 query rows, y = shares of the units, z = chunk.  256 threads as 16 x 16; a thread owns rows
-// {ty*4 .. +3} and {64 + ty*4 .. +3} and columns {tx*4 .. +3} and {64 + tx*4 .. +3} of the 128 x 128 tile: 64 multiply-adds
-// for four 16-byte shared-memory loads a step.  The slices of the negative tiles go global -> registers -> shared memory, the
-// next slice (of this tile or of the CTA's next tile) in flight while the current one is multiplied.  The tile's scores pass
-// through shared memory 64 rows at a time for the scan of the group winners.
-__global__ void __launch_bounds__(kTourThreads, 2) tournament_kernel(TourArgs a) {
-    extern __shared__ __align__(16) float tour_smem[];
-    float* Qt = tour_smem;                    // [D][132]: the CTA's query rows, transposed
-    float* Et = Qt + a.D * kTileStride;       // [32][132]: a slice of the negative tile, transposed
-    float* St = Et + kChunkD * kTileStride;   // [64][129]: half of the tile's scores
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int D = a.D;
-    const int64_t c = blockIdx.z, r0 = (int64_t)blockIdx.x * kTile;
-    const int rows_here = (int)(a.R - r0 < kTile ? a.R - r0 : kTile);
-    const float* Q = a.chunked + (c * a.R + r0) * D;
-    for (int k = tid; k < kTile * D; k += kTourThreads) {
-        const int row = k / D, cc = k - row * D;
-        Qt[cc * kTileStride + row] = row < rows_here ? __ldg(Q + k) : 0.f;
+// one CTA's walk over its share: segments of (chunk, row tile) with a run of groups each
+struct TourSegment {
+    int64_t chunk, row0, col, col_end, group;  // columns [col, col_end) of the chunk, the first of them the first of `group`
+};
+__device__ __forceinline__ bool tour_segment(const TourArgs& a, int64_t at, int64_t end, TourSegment& s, int64_t& next) {
+    if (at >= end) return false;
+    const int64_t item = at / a.K, g = at - item * a.K;
+    int64_t g_end = g + (end - at) < a.K ? g + (end - at) : a.K;
+    const int64_t most = a.T < (1 << 29) ? (1 << 29) / a.T : 1;  // columns of a segment are counted in 32 bits
+    if (g_end - g > most) g_end = g + most;
+    s.chunk = item / a.row_tiles;
+    s.row0 = (item - s.chunk * a.row_tiles) * kTourRows;
+    s.group = g;
+    s.col = g * a.T;
+    s.col_end = g_end * a.T;
+    next = at + (g_end - g);
+    return true;
+}
+
+template <int NB, int VEC>
+__global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __grid_constant__ TourArgs a) {
+    using SM = TourSmem<NB>;
+    extern __shared__ unsigned char tour_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)tour_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = (uint64_t*)(smem + SM::kMisc);
+    uint32_t* s_tmem = (uint32_t*)(smem + SM::kMisc + kTourBars * 8);
+    volatile int* s_abort = (volatile int*)(smem + SM::kMisc + kTourBars * 8 + 4);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t begin = a.shares_total * blockIdx.x / gridDim.x, end = a.shares_total * (blockIdx.x + 1) / gridDim.x;
+    auto spin_wait = [&](int bar, uint32_t parity) { return warp_spin_wait(&bars[bar], parity, s_abort, a.status); };
+    auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, a.status); };
+    if (tid == 0) {
+        mbar_init(&bars[kTQFull], kTourConvWarps);
+        mbar_init(&bars[kTQEmpty], 1);
+        for (int k = 0; k < 2; k++) {
+            mbar_init(&bars[kTYFull + k], kTourConvWarps);
+            mbar_init(&bars[kTYEmpty + k], 1);
+            mbar_init(&bars[kTSFull + k], 1);
+            mbar_init(&bars[kTSEmpty + k], 4);
+        }
+        *s_abort = 0;
+        mbar_init_fence();
     }
-    const float* Nc = a.negatives + c * a.N * D;
-    const bool whole_groups = a.T <= kTile;  // every group of a unit lies inside its one tile
-    const int64_t u_first = (int64_t)blockIdx.y * a.units_per_cta;
-    const int64_t u_last = u_first + a.units_per_cta < a.units ? u_first + a.units_per_cta : a.units;
-    auto unit_groups = [&](int64_t u) { return (int)(a.K - u * a.groups_per_unit < a.groups_per_unit ? a.K - u * a.groups_per_unit : a.groups_per_unit); };
-    float pre[kFetch];
-    if (u_first < u_last) tour_fetch(pre, Nc, u_first * a.groups_per_unit * a.T, (u_first * a.groups_per_unit + unit_groups(u_first)) * a.T, 0, D, tid);
-    for (int64_t u = u_first; u < u_last; u++) {
-        const int64_t g_begin = u * a.groups_per_unit;
-        const int g_count = unit_groups(u);
-        const int64_t col_begin = g_begin * a.T, col_end = col_begin + (int64_t)g_count * a.T;
-        // a group wider than a tile: thread t < 64 keeps the running winners of rows t and 64 + t over the group's tiles
-        float best_v[2] = {-CUDART_INF_F, -CUDART_INF_F};
-        int64_t best_i[2] = {col_begin, col_begin};
-        for (int64_t n0 = col_begin; n0 < col_end; n0 += kTile) {
-            float acc[8][8];
+    if (warp == kTourMma) {
+        tmem_alloc(s_tmem, 128);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *s_tmem;
+
+    if (warp >= kTourConv0) {
+        // ---- rows -> three bf16 planes, 128-byte-swizzled; a warp takes eight consecutive rows at a time ----
+        const int cw = warp - kTourConv0, D = a.D, c = lane * 4;
+        auto convert8 = [&](const float* base, int64_t valid, unsigned char* tile, int plane_bytes, int block_bytes, int r0) {
+            float4 v[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++)
+            for (int k = 0; k < 8; k++) v[k] = tour_load<VEC>(base + (int64_t)(r0 + k) * D, c, D, r0 + k < valid);
+            if (NB == 1 && lane >= 16) return;
+            unsigned char* at0 = tile + (lane >> 4) * block_bytes + r0 * 128 + (lane & 1) * 8;
 #pragma unroll
-                for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-            for (int c0 = 0; c0 < D; c0 += kChunkD) {
-                {
-                    const int node = tid >> 1, cc = (tid & 1) * kFetch;
+            for (int k = 0; k < 8; k++) {
+                unsigned char* at = at0 + k * 128 + ((((lane & 15) >> 1) ^ k) << 4);  // r0 is a multiple of 8: k = row % 8
 #pragma unroll
-                    for (int k = 0; k < kFetch; k++) Et[(cc + k) * kTileStride + node] = pre[k];
+                for (int p = 0; p < kTourPlanes; p++) {
+                    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[k].x, v[k].y), hi = __floats2bfloat162_rn(v[k].z, v[k].w);
+                    const uint2 pk = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                    *reinterpret_cast<uint2*>(at + p * plane_bytes) = pk;
+                    v[k].x -= __uint_as_float(pk.x << 16), v[k].y -= __uint_as_float(pk.x & 0xffff0000u);
+                    v[k].z -= __uint_as_float(pk.y << 16), v[k].w -= __uint_as_float(pk.y & 0xffff0000u);
                 }
-                __syncthreads();  // also orders the writes of Qt before its first use
-                // what comes after this slice: the tile's next slice, the unit's next tile, or the CTA's next unit
-                if (c0 + kChunkD < D) {
-                    tour_fetch(pre, Nc, n0, col_end, c0 + kChunkD, D, tid);
-                } else if (n0 + kTile < col_end) {
-                    tour_fetch(pre, Nc, n0 + kTile, col_end, 0, D, tid);
-                } else if (u + 1 < u_last) {
-                    const int64_t nb = (u + 1) * a.groups_per_unit * a.T;
-                    tour_fetch(pre, Nc, nb, nb + (int64_t)unit_groups(u + 1) * a.T, 0, D, tid);
-                }
-                const int kmax = D - c0 < kChunkD ? D - c0 : kChunkD;
-                for (int k = 0; k < kmax; k++) {
-                    const float* qrow = Qt + (c0 + k) * kTileStride + ty * 4;
-                    const float* erow = Et + k * kTileStride + tx * 4;
-                    const float4 q0 = *reinterpret_cast<const float4*>(qrow), q1 = *reinterpret_cast<const float4*>(qrow + kHalf);
-                    const float4 e0 = *reinterpret_cast<const float4*>(erow), e1 = *reinterpret_cast<const float4*>(erow + kHalf);
-                    const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-                    const float ev[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-#pragma unroll
-                        for (int j = 0; j < 8; j++) acc[i][j] = __fmaf_rn(qv[i], ev[j], acc[i][j]);
-                }
-                __syncthreads();
             }
-            // the scores of rows [64 h, 64 h + 64) go through St, then the (row, group) winners are read off it
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        St[(ty * 4 + i) * kStStride + (j < 4 ? tx * 4 + j : kHalf + tx * 4 + j - 4)] = acc[h * 4 + i][j];
-                __syncthreads();
-                if (whole_groups) {
-                    // one (row, group) per thread and turn; groups vary fastest, so a warp writes runs of adjacent winners
-                    const int T = (int)a.T;
-                    for (int it = tid; it < kHalf * g_count; it += kTourThreads) {
-                        const int lr = it / g_count, g = it - lr * g_count, row = h * kHalf + lr;
-                        const float* sc = St + lr * kStStride + g * T;
-                        float bv = sc[0];
-                        int bi = 0;
-                        for (int j = 1; j < T; j++)
-                            if (sc[j] > bv) {  // the first of equal scores wins
-                                bv = sc[j];
-                                bi = j;
-                            }
-                        if (row < rows_here) {
-                            const int64_t o = (c * a.R + r0 + row) * a.K + g_begin + g;
-                            a.out_scores[o] = bv;
-                            a.out_idx[o] = n0 + (int64_t)g * T + bi;
-                        }
+        };
+        uint32_t items = 0, tiles = 0;
+        TourSegment sg;
+        bool ok = true;
+        for (int64_t at = begin, next = 0; ok && tour_segment(a, at, end, sg, next); at = next, items++) {
+            ok = warp_wait(kTQEmpty, (items & 1) ^ 1);
+            if (!ok) break;
+#pragma unroll 1
+            for (int r = 0; r < 2; r++)
+                convert8(a.chunked + (sg.chunk * a.R + sg.row0) * D, a.R - sg.row0, smem + SM::kQ, SM::kQPlane, SM::kQBlock, cw * 16 + r * 8);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars[kTQFull]);
+            for (int64_t n0 = sg.col; n0 < sg.col_end; n0 += kTourCols, tiles++) {
+                const int b = tiles & 1;
+                ok = warp_wait(kTYEmpty + b, ((tiles >> 1) & 1) ^ 1);
+                if (!ok) break;
+                convert8(a.negatives + (sg.chunk * a.N + n0) * D, sg.col_end - n0, smem + SM::kY + b * kTourPlanes * SM::kYPlane, SM::kYPlane, SM::kYBlock, cw * 8);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars[kTYFull + b]);
+            }
+        }
+    } else if (warp == kTourMma) {
+        constexpr uint32_t kIdesc = idesc_bf16(kTourRows, kTourCols, 0, 0);
+        constexpr uint32_t kFirst = 2 | 0 << 2 | 1 << 4 | 1 << 6 | 0 << 8 | 0 << 10, kSecond = 0 | 2 << 2 | 1 << 4 | 0 << 6 | 1 << 8 | 0 << 10;
+        const uint32_t dQ = desc_lo_sw128(smem_u32(smem + SM::kQ), 16), dY0 = desc_lo_sw128(smem_u32(smem + SM::kY), 16);
+        const int KS = (a.D + kMmaK - 1) / kMmaK;
+        uint32_t items = 0, tiles = 0;
+        TourSegment sg;
+        bool ok = true;
+        for (int64_t at = begin, next = 0; ok && tour_segment(a, at, end, sg, next); at = next, items++) {
+            ok = spin_wait(kTQFull, items & 1);
+            if (!ok) break;
+            for (int64_t n0 = sg.col; n0 < sg.col_end; n0 += kTourCols, tiles++) {
+                const int b = tiles & 1;
+                const uint32_t use = (tiles >> 1) & 1;
+                ok = spin_wait(kTYFull + b, use) && spin_wait(kTSEmpty + b, use ^ 1);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll 1
+                for (int p = 0; p < 6; p++) {
+                    const uint32_t da = dQ + ((kFirst >> (2 * p)) & 3) * (SM::kQPlane >> 4),
+                                   db = dY0 + (b * kTourPlanes + ((kSecond >> (2 * p)) & 3)) * (SM::kYPlane >> 4);
+                    mma_kmajor<NB, SM::kQBlock, SM::kYBlock>(KS, tmem + b * kTourCols, da, db, kIdesc, p > 0 ? 1u : 0u);
+                }
+                mma_commit_warp(&bars[kTYEmpty + b]);
+                if (n0 + kTourCols >= sg.col_end) mma_commit_warp(&bars[kTQEmpty]);
+                mma_commit_warp(&bars[kTSFull + b]);  // last: whoever waits for it has seen the others' arrivals land before the CTA exits
+            }
+        }
+    } else if (warp < kTourEpi0 + 4) {
+        // ---- winners: thread = row; columns in order, the running winner of the group in registers ----
+        const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;
+        uint32_t tiles = 0;
+        TourSegment sg;
+        bool ok = true;
+        for (int64_t at = begin, next = 0; ok && tour_segment(a, at, end, sg, next); at = next) {
+            const bool live = sg.row0 + tid < a.R;
+            const int64_t first = (sg.chunk * a.R + sg.row0 + tid) * a.K + sg.group;
+            float* out_s = a.out_scores + first;
+            int64_t* out_i = a.out_idx + first;
+            const int T = (int)a.T;
+            int todo = (int)((sg.col_end - sg.col) / a.T);  // groups of this segment still to be written; columns are counted from its first
+            float best = -CUDART_INF_F;
+            int best_c = 0, left = T;  // left: columns from the current position to the end of the group
+            for (int64_t n0 = sg.col; n0 < sg.col_end; n0 += kTourCols, tiles++) {
+                const int b = tiles & 1;
+                ok = warp_wait(kTSFull + b, (tiles >> 1) & 1);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll 1
+                for (int k = 0; k < kTourCols; k += 16) {
+                    float v[16];
+                    tmem_ld_32x16(tmem + b * kTourCols + k + lane_sel, v);
+                    if (k == kTourCols - 16) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars[kTSEmpty + b]);
                     }
-                } else if (tid < kHalf) {
-                    const int len = (int)(col_end - n0 < kTile ? col_end - n0 : kTile);
-                    const float* sc = St + tid * kStStride;
-                    for (int j = 0; j < len; j++)
-                        if (sc[j] > best_v[h]) {
-                            best_v[h] = sc[j];
-                            best_i[h] = n0 + j;
-                        }
-                }
-                __syncthreads();  // the other half, or the next tile, overwrites St
-            }
-        }
-        if (!whole_groups && tid < kHalf) {
+                    const int col0 = (int)(n0 - sg.col) + k;
+                    // straight-line and predicated: with one warp a scheduler a branch per column, or a winner that is updated through a
+                    // compare, leaves it waiting for latencies (81 cycles a column)
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int row = h * kHalf + tid;
-                if (row < rows_here) {
-                    const int64_t o = (c * a.R + r0 + row) * a.K + g_begin;
-                    a.out_scores[o] = best_v[h];
-                    a.out_idx[o] = best_i[h];
+                    for (int j = 0; j < 16; j++) {
+                        best_c = v[j] > best ? col0 + j : best_c;  // the first of equal scores wins, a NaN never
+                        best = fmaxf(best, v[j]);
+                        const bool end = left == j + 1;            // the same for all threads
+                        if (end && live && todo > 0) {
+                            *out_s = best;
+                            *out_i = sg.col + best_c;
+                        }
+                        out_s += end ? 1 : 0;
+                        out_i += end ? 1 : 0;
+                        todo -= end ? 1 : 0;
+                        best = end ? -CUDART_INF_F : best;
+                        best_c = end ? col0 + j + 1 : best_c;
+                        left += end ? T : 0;
+                    }
+                    left -= 16;
                 }
             }
         }
     }
+    // ---- common exit ----
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kTourMma) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 128);
+    }
+}
+
+template <int NB, int VEC>
+int launch_tournament(const TourArgs& a, cudaStream_t stream) {
+    // per-device function attribute; setting it on every call keeps multi-device processes correct and is not a stream operation
+    GE2_CUDA_TRY(cudaFuncSetAttribute(tournament_kernel<NB, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, TourSmem<NB>::kBytes));
+    tournament_kernel<NB, VEC><<<(unsigned)std::min<int64_t>(kNumSMs, a.shares_total), kTourThreads, TourSmem<NB>::kBytes, stream>>>(a);
+    GE2_LAUNCH_CHECK();
+    return GE2_OK;
 }
 
 int check_pairs(int kind, const void* chunked, const void* negatives, const void* selected, int64_t chunks, int64_t rows_per_chunk,
@@ -455,6 +550,7 @@ extern "C" int ge2_tournament_select(const float* selector_chunked, const float*
     if (score_negatives == nullptr) score_negatives = selector_negatives;
     cudaStream_t stream = as_stream(stream_);
 
+    if (num_negs / num_selected > (1 << 30)) return GE2_ERR_UNSUPPORTED;
     TourArgs a;
     a.chunked = selector_chunked;
     a.negatives = selector_negatives;
@@ -463,34 +559,16 @@ extern "C" int ge2_tournament_select(const float* selector_chunked, const float*
     a.K = num_selected;
     a.T = num_negs / num_selected;
     a.D = D;
-    a.groups_per_unit = a.T <= kTile ? (int)(kTile / a.T) : 1;
-    a.units = ceil_div<int64_t>(num_selected, a.groups_per_unit);
+    a.row_tiles = ceil_div<int64_t>(rows_per_chunk, kTourRows);
+    a.shares_total = chunks * a.row_tiles * num_selected;
     a.out_scores = out_scores;
     a.out_idx = out_idx;
-    const int64_t row_tiles = ceil_div<int64_t>(rows_per_chunk, kTile);
-    if (row_tiles > 0x7fffffffLL) return GE2_ERR_UNSUPPORTED;
-    const size_t smem = tour_smem_bytes(D);
-    // How many CTAs share the units of a (row tile, chunk): the split with the shortest bound on the makespan of CTAs handed
-    // out greedily to `slots` resident places -- all work / slots + the work of one CTA, its query-tile load counted as a third
-    // of a unit.  Two CTAs an SM by registers.
-    const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(2, (int64_t)(227 * 1024) / (int64_t)(smem + 1024)));
-    const int64_t slots = (int64_t)kNumSMs * per_sm, base = row_tiles * chunks;
-    int64_t shares = 1;
-    double best_cost = 0.0;
-    for (int64_t s = 1; s <= std::min<int64_t>(a.units, 64); s++) {
-        const int64_t per = ceil_div<int64_t>(a.units, s), used = ceil_div<int64_t>(a.units, per);  // `used` CTAs get work
-        const double cost = ((double)(base * used) / (double)slots + 1.0) * ((double)per + 0.33);
-        if (s == 1 || cost < best_cost - 1e-9) {
-            best_cost = cost;
-            shares = used;
-            a.units_per_cta = per;
-        }
-    }
-    // per-device function attribute; setting it on every call keeps multi-device processes correct and is not a stream operation
-    GE2_CUDA_TRY(cudaFuncSetAttribute(tournament_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)row_tiles, (unsigned)shares, (unsigned)chunks);
-    tournament_kernel<<<grid, kTourThreads, smem, stream>>>(a);
-    GE2_LAUNCH_CHECK();
+    a.status = nullptr;
+    const uintptr_t mis = (uintptr_t)(D * 4) | (uintptr_t)selector_chunked | (uintptr_t)selector_negatives;
+    const int vec = (mis & 15) == 0 ? 4 : (mis & 7) == 0 ? 2 : 1;
+    const int rc = D <= 64 ? (vec == 4 ? launch_tournament<1, 4>(a, stream) : vec == 2 ? launch_tournament<1, 2>(a, stream) : launch_tournament<1, 1>(a, stream))
+                           : (vec == 4 ? launch_tournament<2, 4>(a, stream) : vec == 2 ? launch_tournament<2, 2>(a, stream) : launch_tournament<2, 1>(a, stream));
+    if (rc != GE2_OK) return rc;
     if (score_chunked != selector_chunked || score_negatives != selector_negatives) {
         // a selector separate from the scorer: the winners are scored again with the scorer's rows
         return ge2_selected_neg_scores(GE2_SELECTED_DOT, score_chunked, score_negatives, out_idx, chunks, rows_per_chunk, num_negs, num_selected,

@@ -77,6 +77,30 @@ __device__ __forceinline__ bool warp_pipe_wait(uint64_t* bar, uint32_t parity, v
     return __all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0) || warp_pipe_wait_slow(bar, parity, abort_flag, status);
 }
 
+// ---- contractions ---------------------------------------------------------------------------------------------------------
+// D (+)= A B^T over the first `steps` k-steps (1 ... 4 NB) of operands of NB 64-column blocks, both K-major.  The number of steps is made a
+// constant of straight-line code: with a test per step a contraction of N = 64 took 71 cycles to issue instead of 48.
+template <int STEPS, int A_BLOCK, int B_BLOCK>
+__device__ __forceinline__ void mma_kmajor_fixed(uint32_t acc, uint32_t da, uint32_t db, uint32_t idesc, uint32_t accumulate) {
+#pragma unroll
+    for (int ks = 0; ks < STEPS; ks++)
+        mma_f16_ss_warp(acc, da + (((ks >> 2) * A_BLOCK + (ks & 3) * 32) >> 4), db + (((ks >> 2) * B_BLOCK + (ks & 3) * 32) >> 4), idesc,
+                        ks > 0 ? 1u : accumulate);
+}
+template <int NB, int A_BLOCK, int B_BLOCK>
+__device__ __forceinline__ void mma_kmajor(int steps, uint32_t acc, uint32_t da, uint32_t db, uint32_t idesc, uint32_t accumulate) {
+    switch (steps) {
+        case 1: mma_kmajor_fixed<1, A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+        case 2: mma_kmajor_fixed<2, A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+        case 3: mma_kmajor_fixed<3, A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+        case 4: mma_kmajor_fixed<4, A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+        case 5: if (NB > 1) mma_kmajor_fixed<(NB > 1 ? 5 : 1), A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+        case 6: if (NB > 1) mma_kmajor_fixed<(NB > 1 ? 6 : 1), A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+        case 7: if (NB > 1) mma_kmajor_fixed<(NB > 1 ? 7 : 1), A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+        default: if (NB > 1) mma_kmajor_fixed<(NB > 1 ? 8 : 1), A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+    }
+}
+
 // ---- host: tensor maps ----------------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -132,3 +132,18 @@ def test_tournament_rejects_uneven_groups_and_accepts_empty_input(capi, cuda_dev
     scores, idx = capi.tournament_select(q, n, 5)
     torch.cuda.synchronize()
     assert torch.equal(idx.cpu().view(2, 5, 5), (torch.arange(5) * 2).expand(2, 5, 5)) and float(scores.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("C,R,N,D,K", [
+    (1, 127, 64, 63, 64), (2, 129, 65, 65, 5), (1, 1, 1, 1, 1), (300, 3, 20, 8, 4),  # one past a tile each way; more items than SMs
+    (3, 256, 640, 128, 3), (1, 128, 4096, 66, 64),                                    # groups over several tiles, shares cut inside a row tile
+])
+def test_tournament_at_tile_edges_and_on_ties(capi, cuda_device, C, R, N, D, K):
+    rng = np.random.default_rng(C + R + N + D)
+    q = rng.standard_normal((C, R, D)).astype(np.float32)
+    n = rng.standard_normal((C, N, D)).astype(np.float32)
+    n[:, N // 2:] = n[:, :N - N // 2]  # every negative twice: equal scores, within a group when there is one, and the first must win
+    scores, idx = capi.tournament_select(torch.from_numpy(q).to(cuda_device), torch.from_numpy(n).to(cuda_device), K)
+    _check_tournament(scores, idx, q, n, K)
+    if K == 1 and N > 1:
+        assert int(idx.max()) < N // 2
