@@ -24,7 +24,7 @@ EXPORTS = [
     "ge2_copy_slabs", "ge2_unique_bitmap_static", "ge2_sample_batch", "ge2_advance_step", "ge2_dense_adagrad_peers",
     "ge2_enable_peer_access", "ge2_build_state_edges", "ge2_swap_begin", "ge2_swap_wait", "ge2_sample_batch_dev",
     "ge2_eval_workspace_bytes", "ge2_eval_ranks", "ge2_selected_neg_scores", "ge2_selected_neg_scores_backward",
-    "ge2_tournament_select",
+    "ge2_tournament_select", "ge2_unique_bitmap_shared", "ge2_adagrad_scatter_shared", "ge2_train_step",
 ]
 
 
@@ -46,6 +46,7 @@ class LpDesc(C.Structure):
         ("node_grad", C.c_void_p), ("rel_grad", C.c_void_p), ("inv_rel_grad", C.c_void_p), ("loss", C.c_void_p),
         ("pos_scores", C.c_void_p), ("neg_scores", C.c_void_p), ("inv_pos_scores", C.c_void_p), ("inv_neg_scores", C.c_void_p),
         ("status", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t),
+        ("node_state", C.c_void_p), ("row_shared", C.c_void_p), ("node_lr", C.c_float), ("reserved", C.c_int32),
     ]
 
 
@@ -60,6 +61,15 @@ class EvalDesc(C.Structure):
         ("dst_ranks", C.c_void_p), ("src_ranks", C.c_void_p), ("pos_scores", C.c_void_p), ("inv_pos_scores", C.c_void_p),
         ("status", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t),
     ]
+
+
+class TrainDesc(C.Structure):
+    _fields_ = [("lp", C.POINTER(LpDesc)), ("edges", C.c_void_p), ("cols", C.c_int32), ("n_deg", C.c_int32), ("domain", C.c_int64), ("seed", C.c_uint64),
+                ("batch_index", C.c_uint64), ("packed", C.c_void_p), ("deg_rows", C.c_void_p), ("n_ids", C.c_int64), ("unique_ws", C.c_void_p),
+                ("unique_ws_bytes", C.c_size_t), ("unique", C.c_void_p), ("inverse", C.c_void_p), ("count", C.c_void_p), ("shared", C.c_void_p),
+                ("twin_begin", C.c_int64), ("twin_len", C.c_int64), ("table", C.c_void_p), ("state", C.c_void_p), ("table_rows", C.c_int64),
+                ("lr", C.c_float), ("dense_lr", C.c_float), ("grad_scale", C.c_float), ("num_dense", C.c_int32), ("dense_param", C.c_void_p * 2),
+                ("dense_state", C.c_void_p * 2), ("dense_grad", C.c_void_p * 2), ("dense_numel", C.c_int64)]
 
 
 class SwapDesc(C.Structure):
@@ -90,15 +100,18 @@ def load_library():
     lib.ge2_unique_workspace_bytes.restype = C.c_size_t
     lib.ge2_unique_workspace_bytes.argtypes = [C.c_int64]
     lib.ge2_unique_bitmap.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.ge2_unique_bitmap_shared.argtypes = lib.ge2_unique_bitmap.argtypes[:-1] + [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p]
     lib.ge2_unique_bitmap_static.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.ge2_pack_ids.argtypes = [C.POINTER(C.c_void_p), C.POINTER(C.c_int64), C.POINTER(C.c_int64), C.c_void_p, C.c_void_p]
     lib.ge2_lp_workspace_bytes.argtypes = [C.POINTER(LpDesc), C.POINTER(C.c_size_t)]
     lib.ge2_lp_step.argtypes = [C.POINTER(LpDesc), C.c_void_p]
+    lib.ge2_train_step.argtypes = [C.POINTER(TrainDesc), C.c_void_p]
     lib.ge2_sparse_adagrad.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int32, C.c_float, C.c_void_p]
     lib.ge2_index_read.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.ge2_index_add.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.ge2_adagrad_scatter.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int32, C.c_float,
                                         C.c_int32, C.c_void_p, C.c_void_p]
+    lib.ge2_adagrad_scatter_shared.argtypes = lib.ge2_adagrad_scatter.argtypes[:-2] + [C.c_void_p, C.c_void_p, C.c_void_p]
     lib.ge2_dense_adagrad.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_float, C.c_float, C.c_int32, C.c_void_p]
     lib.ge2_dense_adagrad_peers.argtypes = [C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p), C.c_int32, C.c_int32, C.c_int64, C.c_void_p, C.c_float,
                                             C.c_float, C.c_float, C.c_uint32, C.c_void_p, C.c_void_p]
@@ -161,8 +174,10 @@ def unique_workspace(domain: int, device):
     return torch.empty(load_library().ge2_unique_workspace_bytes(domain), dtype=torch.uint8, device=device)
 
 
-def unique_bitmap(ids, domain: int, workspace=None, out_unique=None, out_inverse=None, out_count=None):
-    """ids: int64 CUDA [n].  Returns (unique[capacity], inverse[n], count[2] int32) -- count[0] distinct ids (device)."""
+def unique_bitmap(ids, domain: int, workspace=None, out_unique=None, out_inverse=None, out_count=None, out_shared=None, twins=(0, 0)):
+    """ids: int64 CUDA [n].  Returns (unique[capacity], inverse[n], count[2] int32) -- count[0] distinct ids (device).
+    out_shared: uint8 CUDA [capacity], 1 for ids that occur more than once; twins = (begin, len): ids[begin + k] and
+    ids[begin + len + k] count as one occurrence where they are equal."""
     import torch
 
     lib = load_library()
@@ -176,8 +191,8 @@ def unique_bitmap(ids, domain: int, workspace=None, out_unique=None, out_inverse
         out_inverse = torch.empty(max(1, n), dtype=torch.int64, device=dev)
     if out_count is None:
         out_count = torch.empty(2, dtype=torch.int32, device=dev)
-    check(lib.ge2_unique_bitmap(ptr(ids), n, domain, ptr(workspace), workspace.numel(), ptr(out_unique), ptr(out_inverse), ptr(out_count),
-                                cur_stream()), "ge2_unique_bitmap")
+    check(lib.ge2_unique_bitmap_shared(ptr(ids), n, domain, ptr(workspace), workspace.numel(), ptr(out_unique), ptr(out_inverse), ptr(out_count),
+                                       ptr(out_shared), twins[0], twins[1], cur_stream()), "ge2_unique_bitmap")
     return out_unique, out_inverse[:n], out_count
 
 
@@ -194,7 +209,8 @@ def unique_bitmap_static(ids, domain: int, out_unique, out_inverse, out_count):
 def make_lp_desc(*, decoder, precision, B, Cn, N, D, R, U, node_emb, row_index=None, emb_stride=None, src_ids, dst_ids, rel_ids=None,
                  edge_stride=1, rel_stride=1, dst_negs, src_negs=None, dst_filter=None, src_filter=None, deg_sample_rows=None, n_deg=0,
                  rel=None, inv_rel=None, node_grad, rel_grad=None, inv_rel_grad=None, loss, pos_scores=None, neg_scores=None,
-                 inv_pos_scores=None, inv_neg_scores=None, status=None, workspace=None, node_grad_is_zero=False) -> LpDesc:
+                 inv_pos_scores=None, inv_neg_scores=None, status=None, workspace=None, node_grad_is_zero=False, node_state=None,
+                 row_shared=None, node_lr=0.0) -> LpDesc:
     d = LpDesc()
     d.decoder = DECODER[decoder] if isinstance(decoder, str) else decoder
     d.precision = PRECISION[precision] if isinstance(precision, str) else precision
@@ -219,6 +235,7 @@ def make_lp_desc(*, decoder, precision, B, Cn, N, D, R, U, node_emb, row_index=N
     d.pos_scores, d.neg_scores = ptr(pos_scores), ptr(neg_scores)
     d.inv_pos_scores, d.inv_neg_scores = ptr(inv_pos_scores), ptr(inv_neg_scores)
     d.status = ptr(status)
+    d.node_state, d.row_shared, d.node_lr = ptr(node_state), ptr(row_shared), node_lr
     if workspace is not None:
         d.workspace, d.workspace_bytes = ptr(workspace), workspace.numel()
     return d
@@ -232,6 +249,10 @@ def lp_workspace_bytes(desc: LpDesc) -> int:
 
 def lp_step(desc: LpDesc):
     check(load_library().ge2_lp_step(C.byref(desc), cur_stream()), "ge2_lp_step")
+
+
+def train_step(desc: TrainDesc):
+    check(load_library().ge2_train_step(C.byref(desc), cur_stream()), "ge2_train_step")
 
 
 def sparse_adagrad(grad, state_local, lr: float, out_delta=None, out_state_update=None, rows_dev=None):
@@ -264,11 +285,11 @@ def index_add(table, ids, values, n_dev=None, status=None):
           "ge2_index_add")
 
 
-def adagrad_scatter(table, state, unique_ids, node_grad, lr: float, U=None, U_dev=None, clear_grad=False, status=None):
+def adagrad_scatter(table, state, unique_ids, node_grad, lr: float, U=None, U_dev=None, clear_grad=False, status=None, row_shared=None):
     D = table.shape[1]
     U = unique_ids.numel() if U is None else U
-    check(load_library().ge2_adagrad_scatter(ptr(table), ptr(state), table.shape[0], ptr(unique_ids), U, ptr(U_dev), ptr(node_grad), D, lr,
-                                             1 if clear_grad else 0, ptr(status), cur_stream()), "ge2_adagrad_scatter")
+    check(load_library().ge2_adagrad_scatter_shared(ptr(table), ptr(state), table.shape[0], ptr(unique_ids), U, ptr(U_dev), ptr(node_grad), D, lr,
+                                                    1 if clear_grad else 0, ptr(row_shared), ptr(status), cur_stream()), "ge2_adagrad_scatter")
 
 
 def dense_adagrad(param, sum_state, grad, lr: float, eps: float = 1e-10, grad_scale: float = 1.0, clear_grad=False):

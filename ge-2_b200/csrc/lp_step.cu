@@ -5,6 +5,9 @@
 // mod_node_corrupt_forward RNS branch (cpp/src/nn/decoders/edge/decoder_methods.cpp:724-806,933-946,1089-1097),
 // relation operators (relation_operators.cpp:3-31), apply_score_filter (cpp/src/data/samplers/negative.cpp:570-575)
 // and SoftmaxCrossEntropy with SUM reduction (cpp/src/nn/loss.cpp:46-63).
+#include <algorithm>
+
+#include "adagrad.cuh"
 #include "lp_internal.cuh"
 
 namespace ge2 {
@@ -34,21 +37,96 @@ __global__ void __launch_bounds__(256) mask_from_pairs_kernel(const int64_t* __r
     }
 }
 
-// four consecutive columns [k, k+4) of a row of length D; columns past D read as zero.  `vec` = the row start is
-// 16-byte aligned and D % 4 == 0, so one vector load serves; otherwise 8-byte pairs (k even) or scalars.
-__device__ __forceinline__ float4 load4(const float* __restrict__ row, int k, int D, bool vec) {
-    if (vec && k + 3 < D) return __ldg(reinterpret_cast<const float4*>(row + k));
-    float4 v;
-    if ((k & 1) == 0 && k + 3 < D && (((uintptr_t)(row + k)) & 7) == 0) {
-        const float2 a = __ldg(reinterpret_cast<const float2*>(row + k)), b = __ldg(reinterpret_cast<const float2*>(row + k + 2));
-        return make_float4(a.x, a.y, b.x, b.y);
+// ---------------------------------------------------------------------------------------------------
+// A row of D columns is spread over ld / 4 lanes (16 or 32), four values a lane.
+//   plain   : lane l holds columns [4l, 4l + 4)
+//   ComplEx : coordinates 2l and 2l + 1 of the h = D / 2 complex ones: .x .y their real parts (columns 2l, 2l + 1), .z .w their
+//             imaginary parts (columns h + 2l, h + 2l + 1), so the relation operator and its backward need no other lane's values
+// V is the widest access that the row length and the pointers allow (4 only for plain rows); columns past the row read as zero.
+// ---------------------------------------------------------------------------------------------------
+template <int V, bool CPLX>
+__device__ __forceinline__ float4 load_row(const float* __restrict__ row, int l, int D) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int k = CPLX ? 2 * l : 4 * l, h = D >> 1;
+    if constexpr (CPLX) {
+        if constexpr (V == 2) {
+            if (k < h) {
+                const float2 a = __ldg(reinterpret_cast<const float2*>(row + k)), b = __ldg(reinterpret_cast<const float2*>(row + h + k));
+                v = make_float4(a.x, a.y, b.x, b.y);
+            }
+        } else {
+            if (k < h) v.x = __ldg(row + k), v.z = __ldg(row + h + k);
+            if (k + 1 < h) v.y = __ldg(row + k + 1), v.w = __ldg(row + h + k + 1);
+        }
+    } else if constexpr (V == 4) {
+        if (k < D) v = __ldg(reinterpret_cast<const float4*>(row + k));
+    } else if constexpr (V == 2) {
+        if (k < D) {
+            const float2 a = __ldg(reinterpret_cast<const float2*>(row + k));
+            v.x = a.x, v.y = a.y;
+        }
+        if (k + 2 < D) {
+            const float2 b = __ldg(reinterpret_cast<const float2*>(row + k + 2));
+            v.z = b.x, v.w = b.y;
+        }
+    } else {
+        if (k < D) v.x = __ldg(row + k);
+        if (k + 1 < D) v.y = __ldg(row + k + 1);
+        if (k + 2 < D) v.z = __ldg(row + k + 2);
+        if (k + 3 < D) v.w = __ldg(row + k + 3);
     }
-    v.x = k < D ? __ldg(row + k) : 0.f;
-    v.y = k + 1 < D ? __ldg(row + k + 1) : 0.f;
-    v.z = k + 2 < D ? __ldg(row + k + 2) : 0.f;
-    v.w = k + 3 < D ? __ldg(row + k + 3) : 0.f;
     return v;
 }
+
+struct PutStore {
+    static __device__ __forceinline__ void one(float* p, float a) { *p = a; }
+    static __device__ __forceinline__ void two(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+    static __device__ __forceinline__ void four(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+};
+struct PutAdd {  // reductions at L2, as wide as the row allows
+    static __device__ __forceinline__ void one(float* p, float a) { atomicAdd(p, a); }
+    static __device__ __forceinline__ void two(float* p, float a, float b) { atomicAdd(reinterpret_cast<float2*>(p), make_float2(a, b)); }
+    static __device__ __forceinline__ void four(float* p, float4 v) { atomicAdd(reinterpret_cast<float4*>(p), v); }
+};
+template <int V, bool CPLX, typename Put>
+__device__ __forceinline__ void put_row(float* row, int l, int D, float4 v) {
+    const int k = CPLX ? 2 * l : 4 * l, h = D >> 1;
+    if constexpr (CPLX) {
+        if constexpr (V == 2) {
+            if (k < h) Put::two(row + k, v.x, v.y), Put::two(row + h + k, v.z, v.w);
+        } else {
+            if (k < h) Put::one(row + k, v.x), Put::one(row + h + k, v.z);
+            if (k + 1 < h) Put::one(row + k + 1, v.y), Put::one(row + h + k + 1, v.w);
+        }
+    } else if constexpr (V == 4) {
+        if (k < D) Put::four(row + k, v);
+    } else if constexpr (V == 2) {
+        if (k < D) Put::two(row + k, v.x, v.y);
+        if (k + 2 < D) Put::two(row + k + 2, v.z, v.w);
+    } else {
+        if (k < D) Put::one(row + k, v.x);
+        if (k + 1 < D) Put::one(row + k + 1, v.y);
+        if (k + 2 < D) Put::one(row + k + 2, v.z);
+        if (k + 3 < D) Put::one(row + k + 3, v.w);
+    }
+}
+
+// the relation operator: element-wise product, or product of complex numbers
+template <bool CPLX>
+__device__ __forceinline__ float4 rel_mul(float4 a, float4 r) {
+    if constexpr (CPLX) return make_float4(a.x * r.x - a.z * r.z, a.y * r.y - a.w * r.w, a.x * r.z + a.z * r.x, a.y * r.w + a.w * r.y);
+    else return make_float4(a.x * r.x, a.y * r.y, a.z * r.z, a.w * r.w);
+}
+// ... and its transpose: the gradient of a from that of a x r (and of r from it, with a in the place of r)
+template <bool CPLX>
+__device__ __forceinline__ float4 rel_mul_t(float4 g, float4 r) {
+    if constexpr (CPLX) return make_float4(g.x * r.x + g.z * r.z, g.y * r.y + g.w * r.w, -g.x * r.z + g.z * r.x, -g.y * r.w + g.w * r.y);
+    else return make_float4(g.x * r.x, g.y * r.y, g.z * r.z, g.w * r.w);
+}
+__device__ __forceinline__ float4 axpy4(float a, float4 x, float4 y) { return make_float4(a * x.x + y.x, a * x.y + y.y, a * x.z + y.z, a * x.w + y.w); }
+__device__ __forceinline__ float4 add4(float4 x, float4 y) { return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w); }
+__device__ __forceinline__ float4 scale4(float a, float4 x) { return make_float4(a * x.x, a * x.y, a * x.z, a * x.w); }
+__device__ __forceinline__ float dot4(float4 x, float4 y) { return x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w; }
 
 __device__ __forceinline__ void store_half4(__half* dst, float4 v) {
     const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
@@ -77,109 +155,148 @@ __device__ __forceinline__ void store_split4(__nv_bfloat16* dst, int64_t plane, 
     }
 }
 
+// one row in the lanes' layout as an operand row of the scores kernels: fp16, or (plane > 0) the three bf16 planes
+template <int V, bool CPLX, bool HALF>
+__device__ __forceinline__ void store_operand(void* rows, int64_t plane, int64_t row, int ld, int l, int D, float4 v) {
+    if constexpr (!CPLX) {
+        if constexpr (HALF) store_half4((__half*)rows + row * ld + 4 * l, v);
+        else store_split4((__nv_bfloat16*)rows + row * ld + 4 * l, plane, v);
+    } else {
+        const int k = 2 * l, h = D >> 1;
+        uint16_t* p = (uint16_t*)rows + row * ld;
+        if constexpr (HALF) {
+            const __half2 re = __floats2half2_rn(v.x, v.y), im = __floats2half2_rn(v.z, v.w);
+            if constexpr (V == 2) {
+                if (k < h) *reinterpret_cast<__half2*>(p + k) = re, *reinterpret_cast<__half2*>(p + h + k) = im;
+            } else {  // an odd h leaves the imaginary parts on odd columns
+                if (k < h) p[k] = __half_as_ushort(re.x), p[h + k] = __half_as_ushort(im.x);
+                if (k + 1 < h) p[k + 1] = __half_as_ushort(re.y), p[h + k + 1] = __half_as_ushort(im.y);
+            }
+            for (int c = D + k; c < ld; c += ld >> 1) *reinterpret_cast<uint32_t*>(p + c) = 0u;  // the padding of the row
+        } else {
+#pragma unroll
+            for (int t = 0; t < 3; t++, p += plane) {
+                const __nv_bfloat162 re = __floats2bfloat162_rn(v.x, v.y), im = __floats2bfloat162_rn(v.z, v.w);
+                if constexpr (V == 2) {
+                    if (k < h) *reinterpret_cast<__nv_bfloat162*>(p + k) = re, *reinterpret_cast<__nv_bfloat162*>(p + h + k) = im;
+                } else {
+                    if (k < h) p[k] = __bfloat16_as_ushort(re.x), p[h + k] = __bfloat16_as_ushort(im.x);
+                    if (k + 1 < h) p[k + 1] = __bfloat16_as_ushort(re.y), p[h + k + 1] = __bfloat16_as_ushort(im.y);
+                }
+                for (int c = D + k; c < ld; c += ld >> 1) *reinterpret_cast<uint32_t*>(p + c) = 0u;
+                const float2 fr = __bfloat1622float2(re), fi = __bfloat1622float2(im);
+                v.x -= fr.x, v.y -= fr.y, v.z -= fi.x, v.w -= fi.y;
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------------------------
-// prep: eight lanes per output row (four rows in flight per warp, so the dependent loads id -> row index -> embedding
-// row overlap), each lane 4 columns at a time.  Rows [0, S*Bp) are query rows, rows [S*Bp, S*Bp + S*CN) negative rows.
+// prep: the operands of the scores kernels.  A group of ld / 4 lanes takes one edge (both corruption sides: four rows in, two
+// operand rows and two positive scores out) or two columns of negatives (one row in and both sides' rows out where the sides share the
+// node) at a time.
+// Bound by the chain id -> row index -> row on small batches (and by fetching the kernel's own code: 80 KB of it, with more rows a
+// group unrolled, ran no faster than one row at a time), by L2 and HBM on large ones.  10 000 edges, 2 x 10 000 negatives, ComplEx 100:
+// 10.8 us; 100 000 edges, 2 x 200 000 negatives, DistMult 128: 85 us (eight lanes a row and side: 12.8 and 168 us).
 // ---------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) lp_prep_kernel(LpKernelArgs a) {
+constexpr int kPrepNegs = 2;
+
+template <int V, bool CPLX, bool REL, bool HALF>
+__global__ void __launch_bounds__(256, 5) lp_prep_kernel(const __grid_constant__ LpKernelArgs a, int write_mask) {
     const ge2_lp_desc& d = a.d;
     const LpLayout& L = a.L;
-    const int tid = threadIdx.x;
-    const int gl = tid & 7;                              // lane within the row group
-    const unsigned gmask = 0xFFu << ((tid & 31) & ~7);   // the 8 lanes of this group inside the warp
-    const int64_t groups = ((int64_t)gridDim.x * blockDim.x) >> 3;
-    const int64_t q_rows = (int64_t)L.S * L.Bp;
-    const int64_t total = q_rows + (int64_t)L.S * L.CN;
-    const int64_t total_pad = round_up<int64_t>(total, 4);  // whole warps stay in the loop for the shuffles
-    const int D = d.D, h = D / 2, ld = L.ld;
-    const bool vec_e = (d.emb_stride % 4 == 0) && (((uintptr_t)d.node_emb) & 15) == 0 && D % 4 == 0;
-    const bool vec_r = D % 4 == 0 && ((((uintptr_t)d.rel) | ((uintptr_t)d.inv_rel)) & 15) == 0;
-    const int64_t q_plane = q_rows * ld, k_plane = (int64_t)L.S * L.CN * ld;
+    const int ld = L.ld, D = d.D, lpr = ld >> 2;
+    const int lane = threadIdx.x & 31, l = lane & (lpr - 1);
+    const unsigned gmask = lpr == 32 ? 0xFFFFFFFFu : 0xFFFFu << (lane & 16);
+    const int groups = (int)(gridDim.x * blockDim.x) / lpr;
+    const int64_t neg_units = (L.CN + kPrepNegs - 1) / kPrepNegs;
+    const int64_t q_plane = (int64_t)L.S * L.Bp * ld, k_plane = (int64_t)L.S * L.CN * ld;
+    void* const Q = HALF ? (void*)L.Qh : (void*)L.Qs;
+    void* const K = HALF ? (void*)L.Kh : (void*)L.Ks;
+    const bool two = REL && L.S == 2;
     griddep_wait();
-    if (blockIdx.x == 0 && tid == 0) *L.loss_acc = 0.0;        // the scores kernel of this step adds every row's loss term to it
-    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + tid) >> 3; w < total_pad; w += groups) {
-        if (w >= total) continue;
-        if (w < q_rows) {
-            const int s = (int)(w / L.Bp);
-            const int i = (int)(w - (int64_t)s * L.Bp);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *L.loss_acc = 0.0;  // the scores kernel of this step adds every row's loss term to it
+#pragma unroll 1
+    for (int64_t u = (int)(blockIdx.x * blockDim.x + threadIdx.x) / lpr; u < L.Bp + neg_units; u += groups) {
+        if (u < L.Bp) {
+            const int64_t i = u;
             bool ok = i < d.B;  // rows past B: zero rows appended by pad_and_reshape; their positive score is padded with 0
             int64_t sid = 0, did = 0, rid = 0;
             if (ok) {
-                sid = d.src_ids[(int64_t)i * d.edge_stride];
-                did = d.dst_ids[(int64_t)i * d.edge_stride];
-                ok = sid >= 0 && sid < d.U && did >= 0 && did < d.U;
-                if (d.has_relations) {
-                    rid = d.rel_ids[(int64_t)i * d.rel_stride];
-                    ok = ok && rid >= 0 && rid < d.R;
-                }
-                if (!ok && gl == 0) or_status(d.status, GE2_STATUS_BAD_INDEX);
+                sid = __ldg(&d.src_ids[i * d.edge_stride]);
+                did = __ldg(&d.dst_ids[i * d.edge_stride]);
+                if (REL) rid = __ldg(&d.rel_ids[i * d.rel_stride]);
+                ok = sid >= 0 && sid < d.U && did >= 0 && did < d.U && (!REL || (rid >= 0 && rid < d.R));
+                if (!ok && l == 0) or_status(d.status, GE2_STATUS_BAD_INDEX);
             }
-            const float* ea = ok ? emb_row(d, s == 0 ? sid : did) : nullptr;  // the endpoint the relation is applied to
-            const float* eb = ok ? emb_row(d, s == 0 ? did : sid) : nullptr;  // the endpoint it is compared with
-            const float* r = (ok && d.has_relations) ? (s == 0 ? d.rel : d.inv_rel) + rid * D : nullptr;
-            float dot = 0.f;
-            for (int k = gl * 4; k < ld; k += 32) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (ok) {
-                    const float4 x = load4(ea, k, D, vec_e);
-                    if (r == nullptr) {
-                        v = x;
-                    } else {
-                        const float4 rr = load4(r, k, D, vec_r);
-                        if (d.decoder == GE2_DECODER_DISTMULT) {
-                            v = make_float4(x.x * rr.x, x.y * rr.y, x.z * rr.z, x.w * rr.w);
-                        } else {
-                            // complex Hadamard: columns [0, h) real, [h, D) imaginary; the partner component comes from the
-                            // same two rows (just loaded, so these scalar reads hit L1)
-                            float xv[4] = {x.x, x.y, x.z, x.w}, rv[4] = {rr.x, rr.y, rr.z, rr.w}, o[4];
-#pragma unroll
-                            for (int e2 = 0; e2 < 4; e2++) {
-                                const int c = k + e2;
-                                o[e2] = 0.f;
-                                if (c < D) {
-                                    const int cp = c < h ? c + h : c - h;
-                                    const float xp = __ldg(ea + cp), rp = __ldg(r + cp);
-                                    o[e2] = c < h ? xv[e2] * rv[e2] - xp * rp   // real: e_re r_re - e_im r_im
-                                                  : xp * rv[e2] + xv[e2] * rp;  // imaginary: e_re r_im + e_im r_re
-                                }
-                            }
-                            v = make_float4(o[0], o[1], o[2], o[3]);
-                        }
-                    }
-                    const float4 y = load4(eb, k, D, vec_e);
-                    dot += v.x * y.x + v.y * y.y + v.z * y.z + v.w * y.w;
-                }
-                if (L.Qh != nullptr) store_half4(L.Qh + w * ld + k, v);
-                else store_split4(L.Qs + w * ld + k, q_plane, v);
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f), t = s, r0 = s, r1 = s;
+            if (ok) {
+                const float *es = emb_row(d, sid), *ed = emb_row(d, did);
+                if (REL) r0 = load_row<V, CPLX>(d.rel + rid * D, l, D);
+                if (two) r1 = load_row<V, CPLX>(d.inv_rel + rid * D, l, D);
+                s = load_row<V, CPLX>(es, l, D);
+                t = load_row<V, CPLX>(ed, l, D);
+            }
+            const float4 q0 = REL ? rel_mul<CPLX>(s, r0) : s;
+            store_operand<V, CPLX, HALF>(Q, q_plane, i, ld, l, D, q0);
+            float p0 = dot4(q0, t), p1 = 0.f;
+            if (two) {
+                const float4 q1 = rel_mul<CPLX>(t, r1);
+                store_operand<V, CPLX, HALF>(Q, q_plane, L.Bp + i, ld, l, D, q1);
+                p1 = dot4(q1, s);
             }
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) dot += __shfl_xor_sync(gmask, dot, o);
-            if (gl == 0) L.pos[(int64_t)s * L.Bp + i] = dot;
+            for (int o = 16; o > 0; o >>= 1) {
+                if (o < lpr) {
+                    p0 += __shfl_xor_sync(gmask, p0, o);
+                    if (REL) p1 += __shfl_xor_sync(gmask, p1, o);
+                }
+            }
+            if (l == 0) {
+                L.pos[i] = p0;
+                if (two) L.pos[L.Bp + i] = p1;
+            }
         } else {
-            const int64_t e = w - q_rows;
-            const int s = (int)(e / L.CN);
-            const int64_t j = e - (int64_t)s * L.CN;
-            const int64_t id = (s == 0 ? d.dst_negs : d.src_negs)[j];
-            const bool bad = id < 0 || id >= d.U;
-            if (bad && gl == 0) or_status(d.status, GE2_STATUS_BAD_INDEX);
-            if (gl == 0 && d.deg_sample_rows != nullptr) {
+            const int64_t j0 = (u - L.Bp) * kPrepNegs;
+            const float* src[2][kPrepNegs];
+#pragma unroll
+            for (int e = 0; e < kPrepNegs; e++) {
+                const int64_t j = j0 + e < L.CN ? j0 + e : L.CN - 1;
+                const int64_t i0 = __ldg(&d.dst_negs[j]), i1 = two ? __ldg(&d.src_negs[j]) : i0;
+                const bool bad0 = i0 < 0 || i0 >= d.U, bad1 = i1 < 0 || i1 >= d.U;
+                if ((bad0 || bad1) && l == 0) or_status(d.status, GE2_STATUS_BAD_INDEX);
+                src[0][e] = bad0 ? nullptr : emb_row(d, i0);
+                src[1][e] = bad1 ? nullptr : i1 == i0 ? src[0][e] : emb_row(d, i1);
+            }
+            if (write_mask && l < kPrepNegs && j0 + l < L.CN) {
                 // the filter word of this (side, chunk, column): deg_negative_local_filter on the device (negative.cpp:215-263 of
                 // the reference): entry (c, col) masks row deg_rows[c][col] when that row belongs to chunk c; the same for both
                 // sides (the reference shares one filter tensor, negative.cpp:1049-1056)
-                const int c = (int)(j / d.N), col = (int)(j - (int64_t)c * d.N);
+                const int64_t j = j0 + l;
                 int32_t m = -1;
-                if (col < d.n_deg) {
-                    const int64_t r = d.deg_sample_rows[(int64_t)c * d.n_deg + col];
-                    if (r < 0 || r >= d.B) or_status(d.status, GE2_STATUS_BAD_INDEX);
-                    else if ((int)(r / L.npc) == c) m = (int32_t)r;
+                if (d.deg_sample_rows != nullptr) {
+                    const int c = (int)((uint32_t)j / (uint32_t)d.N), col = (int)j - c * d.N;  // (C N fits 31 bits)
+                    if (col < d.n_deg) {
+                        const int64_t r = d.deg_sample_rows[(int64_t)c * d.n_deg + col];
+                        if (r < 0 || r >= d.B) or_status(d.status, GE2_STATUS_BAD_INDEX);
+                        else if ((int)((uint32_t)r / (uint32_t)L.npc) == c) m = (int32_t)r;
+                    }
                 }
-                L.mask[e] = m;
+                L.mask[j] = m;
+                if (two) L.mask[L.CN + j] = m;
             }
-            const float* src = bad ? nullptr : emb_row(d, id);
-            for (int k = gl * 4; k < ld; k += 32) {
-                const float4 v = bad ? make_float4(0.f, 0.f, 0.f, 0.f) : load4(src, k, D, vec_e);
-                if (L.Kh != nullptr) store_half4(L.Kh + e * ld + k, v);
-                else store_split4(L.Ks + e * ld + k, k_plane, v);
+            float4 v[2][kPrepNegs];
+#pragma unroll
+            for (int e = 0; e < kPrepNegs; e++) {
+                v[0][e] = v[1][e] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (src[0][e] != nullptr) v[0][e] = load_row<V, CPLX>(src[0][e], l, D);
+                if (REL && src[1][e] != src[0][e] && src[1][e] != nullptr) v[1][e] = load_row<V, CPLX>(src[1][e], l, D);
+            }
+#pragma unroll
+            for (int e = 0; e < kPrepNegs; e++) {
+                if (j0 + e >= L.CN) break;
+                store_operand<V, CPLX, HALF>(K, k_plane, j0 + e, ld, l, D, v[0][e]);
+                if (two) store_operand<V, CPLX, HALF>(K, k_plane, L.CN + j0 + e, ld, l, D, src[1][e] == src[0][e] ? v[0][e] : v[1][e]);
             }
         }
     }
@@ -187,275 +304,276 @@ __global__ void __launch_bounds__(256) lp_prep_kernel(LpKernelArgs a) {
 
 // ---------------------------------------------------------------------------------------------------
 // finish: relation-operator backward and the scatter of every gradient row.
-// One warp per row: an edge (both corruption sides at once) or one negative.  Lanes run along the embedding, so every
-// load and every atomic of a warp covers one contiguous 128-byte piece of a row, and the loads of a row (two endpoints, two
-// relation rows, two rows of dQ) are all issued before the first one is needed.  For ComplEx a lane holds the real and the
-// imaginary component of the same complex coordinate, so the operator's backward needs no second pass over the rows.
-// A CTA walks a contiguous range of rows and folds the gradients of relation rows (few rows, hit by every edge) into a
-// small shared-memory table that is flushed once at the end; node rows go straight to global memory (the batch-local
-// gradient buffer lives in L2).  Sums are the same as the reference's index_add backward up to fp32 addition order.
+// The first CTAs take the negatives, `occ` rows of dK a warp; the others batches of kFinBatch edges, both corruption sides at once,
+// with the scalars of the next batch on their way while the rows of one are worked on.  Rows that occur again among a batch's
+// edges (relations always do; hub nodes of a skewed graph) or the warp's negatives are added up on chip first -- thousands of
+// reductions onto the same 128 bytes would serialise in L2 -- and the rest go to the gradient tables as 16-byte reductions at L2.
+// Where the caller hands over the optimizer state and says which nodes occur once in the batch (row_shared), such a node is
+// finished on the spot: the whole gradient of its row is in registers here, and so is the row, so its Adagrad step costs one read
+// of the state and two writes instead of a reduction, and later a read, a clearing and a second visit to the table.
+// Sums are the same as the reference's index_add backward up to fp32 addition order.
+// Bound by latency on small batches (ids -> rows -> reductions), by HBM on large ones.  With the sparse Adagrad pass that follows:
+// 10 000 edges, 2 x 10 000 negatives, ComplEx 100: 28 us (33 us with every row through the gradient table); 50 000 edges and
+// negatives, Dot 100: 104 us (143 us); 100 000 edges, 2 x 200 000 negatives, DistMult 128: 270 us (465 us).
 // ---------------------------------------------------------------------------------------------------
-constexpr int kFinSlots = 32;     // relation rows cached per CTA
 constexpr int kFinWarps = 8;
-constexpr long long kFinEmpty = -1;
+constexpr int kFinBatch = 16;  // edges a batch: their 32 endpoints are the lanes of one warp when it looks for repeated nodes
 
-constexpr int kFinEdgeBatch = 64;  // edges whose scalars (ids, table rows, d loss / d pos, table slots) are fetched together
-constexpr int kFinHotSlots = 8;    // node rows cached per CTA: rows that occur more than once among a batch's endpoints
-
-struct FinishSmem {
-    float acc[kFinSlots][128];
-    long long tag[kFinSlots];  // (1 + side) << 40 | relation id
-    // per edge of the current batch: filled by one thread per edge, so the chain id -> row index -> ... is walked for
-    // 64 edges at once instead of once per warp and edge
-    long long sid[kFinEdgeBatch], did[kFinEdgeBatch], srow[kFinEdgeBatch], drow[kFinEdgeBatch];
-    int rid[kFinEdgeBatch], slot[2][kFinEdgeBatch];  // rid < 0: skip the edge (bad ids, flagged by prep)
-    float dpos[2][kFinEdgeBatch];
-    // Hub rows: in a skewed graph one node can be an endpoint of a tenth of the batch, and thousands of atomics on the same
-    // 128 bytes of its gradient row serialise in L2.  A row seen twice among the 128 endpoints of an edge batch gets a
-    // shared-memory row (first come, kept until the end of the CTA) and reaches global memory once per CTA.
-    float hot[kFinHotSlots][128];
-    long long hot_tag[kFinHotSlots];      // batch-local node id, or kFinEmpty
-    int hot_slot[2][kFinEdgeBatch];      // per edge: slot of its source / destination row, or -1
+struct FinScalars {
+    long long id[2 * kFinBatch];   // local node ids, sources then destinations; -1: skip the edge (bad ids, flagged by prep)
+    long long row[2 * kFinBatch];  // their rows of the table
+    unsigned same[2 * kFinBatch];  // lanes with the same node
+    int rid[kFinBatch];
+    unsigned rel_same[kFinBatch];  // edges with the same relation
+    float dpos[2][kFinBatch];
+    unsigned char shared[2 * kFinBatch];  // the node occurs elsewhere in the batch
 };
 
-__device__ __forceinline__ int fin_slot_of(long long key) { return (int)(((unsigned long long)key * 0x9E3779B97F4A7C15ull) >> 59); }  // top 5 bits
+// one row's Adagrad step (called, not inlined: four exact divisions and square roots are 3 KB of code, and this kernel runs too briefly to
+// fetch several copies)
+template <int V, bool CPLX>
+__device__ __noinline__ void adagrad_row(float* emb, float* state, int l, int D, float4 e, float4 s, float4 g, float neg_lr) {
+    // a lane without columns must not divide: 0 / 1e-10 is off the fast path of the division, and the whole warp would wait for it
+    const int cols = CPLX ? (D >> 1) - 2 * l : D - 4 * l;
+    if (cols <= 0) return;
+    if (CPLX ? cols == 1 : cols < 4) {
+        if (CPLX) s.y = s.w = 1.f;
+        else s.w = 1.f, s.z = cols < 3 ? 1.f : s.z, s.y = cols < 2 ? 1.f : s.y;
+    }
+    float dl, up;
+    adagrad_elem(g.x, s.x, dl, up, neg_lr), e.x = __fadd_rn(e.x, dl);
+    adagrad_elem(g.y, s.y, dl, up, neg_lr), e.y = __fadd_rn(e.y, dl);
+    adagrad_elem(g.z, s.z, dl, up, neg_lr), e.z = __fadd_rn(e.z, dl);
+    adagrad_elem(g.w, s.w, dl, up, neg_lr), e.w = __fadd_rn(e.w, dl);
+    put_row<V, CPLX, PutStore>(state, l, D, s);
+    put_row<V, CPLX, PutStore>(emb, l, D, e);
+}
 
-__global__ void __launch_bounds__(kFinWarps * 32) lp_finish_kernel(LpKernelArgs a, int edges_per_cta, int negs_per_cta) {
-    __shared__ FinishSmem sm;
+template <int V, bool CPLX, bool REL>
+__global__ void __launch_bounds__(kFinWarps * 32, 4) lp_finish_kernel(const __grid_constant__ LpKernelArgs a, int neg_ctas, int occ) {
+    extern __shared__ __align__(16) float fin_rows[];  // [4][kFinBatch][ld]: relation, inverse relation, source, destination gradients
+    __shared__ FinScalars sm;
     const ge2_lp_desc& d = a.d;
     const LpLayout& L = a.L;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t e_rows = d.B;  // one row per edge (both sides), then one per negative
-    const int64_t total = e_rows + (int64_t)L.S * L.CN;
-    const int D = d.D, h = D / 2, ld = L.ld;
-    const bool cplx = d.has_relations && d.decoder == GE2_DECODER_COMPLEX;
-    const int n_el = cplx ? h : D;       // coordinates a lane loop runs over: complex pairs, or plain columns
-    const int off2 = cplx ? h : 0;       // where the second component of a coordinate lives
-    const bool vec_g = (D % 4 == 0) && (((uintptr_t)d.node_grad) & 15) == 0;
+    const int D = d.D, ld = L.ld, lpr = ld >> 2, l = lane & (lpr - 1);
+    const int per_warp = 32 / lpr;            // rows a warp works on side by side
+    const int sub = per_warp == 1 ? 0 : lane >> 4;
     const float gs = L.grad_unscale;  // the tensor path leaves dQ / dK scaled by a power of two
-
-    if (d.has_relations) {
-        for (int k = tid; k < kFinSlots * 128; k += kFinWarps * 32) (&sm.acc[0][0])[k] = 0.f;
-        if (tid < kFinSlots) sm.tag[tid] = kFinEmpty;
-    }
-    for (int k = tid; k < kFinHotSlots * 128; k += kFinWarps * 32) (&sm.hot[0][0])[k] = 0.f;
-    if (tid < kFinHotSlots) sm.hot_tag[tid] = kFinEmpty;
-    griddep_wait();  // the shared-memory set-up above overlaps the tail of the scores kernel
+    const bool fused = d.node_state != nullptr && d.row_shared != nullptr;
+    const float neg_lr = -d.node_lr;
+    float* const table = const_cast<float*>(d.node_emb);
+    griddep_wait();
     // loss = sum over sides and padded rows of (lse - pos), accumulated in double by the scores kernel that ran before
     if (blockIdx.x == 0 && tid == 0) *d.loss = (float)*L.loss_acc;
-    __syncthreads();
 
-    // Every CTA takes a contiguous share of the edges (heavy rows: six input rows, four output rows each) and a contiguous
-    // share of the negatives (one row in, one out), so the heavy rows are spread over the whole grid.
-    const int64_t e_begin = (int64_t)blockIdx.x * edges_per_cta;
-    const int64_t e_end = e_begin + edges_per_cta < e_rows ? e_begin + edges_per_cta : e_rows;
-    const int64_t n_begin = e_rows + (int64_t)blockIdx.x * negs_per_cta;
-    const int64_t n_end = n_begin + negs_per_cta < total ? n_begin + negs_per_cta : total;
-
-    // the negatives of this CTA: one row of dK each, added to the gradient row of the node it was drawn as
-    auto scatter_negatives = [&]() {
-        // A row whose node holds a shared-memory row (claimed by the edges of this CTA: a hub) is summed there: with
-        // negatives drawn by degree a hub node owns thousands of these rows, and their atomics would serialise in L2.
-        for (int64_t w = n_begin + warp; w < n_end; w += kFinWarps) {
-            const int64_t e = w - e_rows;
-            const int s = (int)(e / L.CN);
-            const int64_t j = e - (int64_t)s * L.CN;
-            const int64_t id = (s == 0 ? d.dst_negs : d.src_negs)[j];
-            if (id < 0 || id >= d.U) continue;
-            const float* dk = L.dK + e * ld;
-            const int sidx = (int)(((unsigned long long)id * 0x9E3779B97F4A7C15ull) >> 61);
-            if (sm.hot_tag[sidx] == id) {
-                for (int k = lane; k < D; k += 32) {
-                    const float v = dk[k] * gs;
-                    if (v != 0.f) atomicAdd(&sm.hot[sidx][k], v);
-                }
-                continue;
+    if ((int)blockIdx.x < neg_ctas) {  // ---- negatives
+        const int64_t w = (int64_t)blockIdx.x * kFinWarps + warp;
+        const int per_side = L.S == 2 ? occ >> 1 : occ;
+        const int side = lane >= per_side ? 1 : 0;
+        const int64_t j = w * per_side + (lane - side * per_side);
+        long long id = -1 - lane;
+        int shared = 1;
+        long long trow = 0;
+        if (lane < occ && j < L.CN) {
+            const long long v = (side == 0 ? d.dst_negs : d.src_negs)[j];
+            if (v >= 0 && v < d.U) id = v;
+        }
+        if (fused && id >= 0) {
+            shared = d.row_shared[id];
+            trow = d.row_index != nullptr ? __ldg(&d.row_index[id]) : id;
+        }
+        const unsigned same = __match_any_sync(0xFFFFFFFFu, id);
+        const long long dk_row = (long long)side * L.CN + j;
+        const bool leads = id >= 0 && (same & ((1u << lane) - 1u)) == 0;
+        const unsigned leaders = __ballot_sync(0xFFFFFFFFu, leads);
+#pragma unroll 1
+        for (int k0 = 0; k0 < occ; k0 += per_warp) {
+            if (((leaders >> k0) & ((1u << per_warp) - 1u)) == 0u) continue;
+            const int k = k0 + sub;
+            const bool on = (leaders >> k) & 1u;
+            const unsigned members = __shfl_sync(0xFFFFFFFFu, same, k);
+            const long long gid = __shfl_sync(0xFFFFFFFFu, id, k), grow = __shfl_sync(0xFFFFFFFFu, trow, k);
+            const int sh = __shfl_sync(0xFFFFFFFFu, shared, k);
+            const bool upd = on && sh == 0;
+            const long long r1 = __shfl_sync(0xFFFFFFFFu, dk_row, k);
+            unsigned rest = members & (members - 1);
+            const long long r2 = __shfl_sync(0xFFFFFFFFu, dk_row, rest ? __ffs((int)rest) - 1 : k);
+            float4 g = make_float4(0.f, 0.f, 0.f, 0.f), g2 = g, e = g, s = g;
+            if (on) g = load_row<V, CPLX>(L.dK + r1 * ld, l, D);
+            if (on && rest) g2 = load_row<V, CPLX>(L.dK + r2 * ld, l, D);  // the other side's row, mostly
+            if (upd) {
+                e = load_row<V, CPLX>(table + grow * d.emb_stride, l, D);
+                s = load_row<V, CPLX>(d.node_state + grow * d.emb_stride, l, D);
             }
-            float* grow = d.node_grad + id * D;
-            if (vec_g) {
-                for (int k = lane * 4; k < D; k += 128) {
-                    float4 v = *reinterpret_cast<const float4*>(dk + k);
-                    v.x *= gs, v.y *= gs, v.z *= gs, v.w *= gs;
-                    if (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f) atomicAdd(reinterpret_cast<float4*>(grow + k), v);
-                }
-            } else {
-                for (int k = lane; k < D; k += 32) {
-                    const float v = dk[k] * gs;
-                    if (v != 0.f) atomicAdd(grow + k, v);
-                }
+            g = add4(g, g2);
+            rest = on ? rest & (rest - 1) : 0u;
+            while (__any_sync(0xFFFFFFFFu, rest != 0u)) {
+                const long long r = __shfl_sync(0xFFFFFFFFu, dk_row, rest ? __ffs((int)rest) - 1 : 0);
+                if (rest) g = add4(g, load_row<V, CPLX>(L.dK + r * ld, l, D));
+                rest &= rest - 1;
+            }
+            g = scale4(gs, g);
+            if (upd) adagrad_row<V, CPLX>(table + grow * d.emb_stride, d.node_state + grow * d.emb_stride, l, D, e, s, g, neg_lr);
+            else if (on) put_row<V, CPLX, PutAdd>(d.node_grad + gid * D, l, D, g);
+        }
+        return;
+    }
+
+    // ---- edges
+    // the scalars of one batch, a lane an endpoint (warp 0: sources, then destinations), an edge's relation (warp 1) or its d loss / d
+    // pos on one side (warp 2)
+    long long p_id = -1, p_row = -1;
+    int p_rid = -1;
+    float p_dpos = 0.f;
+    int p_shared = 1;
+    const int k16 = lane & (kFinBatch - 1);
+    auto fetch = [&](int64_t base) {
+        const int64_t i = base + k16;
+        if (warp == 0) {  // lanes are endpoints: sources, then destinations
+            p_id = p_row = -1;
+            p_shared = 1;
+            if (i < d.B) p_id = (lane < kFinBatch ? d.src_ids : d.dst_ids)[i * d.edge_stride];
+            if (p_id >= d.U || p_id < 0) p_id = -1;
+            if (p_id >= 0) {
+                p_row = d.row_index != nullptr ? __ldg(&d.row_index[p_id]) : p_id;
+                if (fused) p_shared = d.row_shared[p_id];
+            }
+        } else if (warp == 1 && REL) {
+            p_rid = -1;
+            if (i < d.B) {
+                const int64_t r = d.rel_ids[i * d.rel_stride];
+                if (r >= 0 && r < d.R) p_rid = (int)r;
+            }
+        } else if (warp == 2) {
+            const int side = lane / kFinBatch;
+            if (side < L.S && i < d.B) {
+                const int64_t qrow = (int64_t)side * L.Bp + i;
+                p_dpos = __expf(L.pos[qrow] - L.lse[qrow]) - 1.0f;  // d loss / d pos_i = softmax prob of the positive - 1
             }
         }
     };
-    bool negs_done = false;
-    for (int64_t base = e_begin; base < e_end; base += kFinEdgeBatch) {
-        const int nb = (int)(e_end - base < kFinEdgeBatch ? e_end - base : kFinEdgeBatch);
-        if (tid < nb) {
-            const int64_t i = base + tid;
-            const int64_t sid = d.src_ids[i * d.edge_stride];
-            const int64_t did = d.dst_ids[i * d.edge_stride];
-            bool ok = sid >= 0 && sid < d.U && did >= 0 && did < d.U;
-            int64_t rid = 0;
-            if (d.has_relations) {
-                rid = d.rel_ids[i * d.rel_stride];
-                ok = ok && rid >= 0 && rid < d.R;
-            }
-            sm.rid[tid] = ok ? (int)rid : -1;
-            if (ok) {
-                sm.sid[tid] = sid;
-                sm.did[tid] = did;
-                sm.srow[tid] = d.row_index != nullptr ? __ldg(&d.row_index[sid]) : sid;
-                sm.drow[tid] = d.row_index != nullptr ? __ldg(&d.row_index[did]) : did;
-                for (int s = 0; s < L.S; s++) {
-                    const int64_t qrow = (int64_t)s * L.Bp + i;
-                    sm.dpos[s][tid] = __expf(L.pos[qrow] - L.lse[qrow]) - 1.0f;  // d loss / d pos_i = softmax prob of the positive - 1
-                    int slot = -1;
-                    if (d.has_relations) {  // claim (or find) the shared slot of this relation row; -1 when it belongs to another row
-                        const long long key = ((long long)(1 + s) << 40) | rid;
-                        const int sidx = fin_slot_of(key);
-                        const long long old = (long long)atomicCAS((unsigned long long*)&sm.tag[sidx], (unsigned long long)kFinEmpty, (unsigned long long)key);
-                        slot = (old == kFinEmpty || old == key) ? sidx : -1;
-                    }
-                    sm.slot[s][tid] = slot;
-                }
-            }
-        }
+    auto usable = [&](int k) { return sm.id[k] >= 0 && sm.id[kFinBatch + k] >= 0 && (!REL || sm.rid[k] >= 0); };
+    const int group = warp * per_warp + sub, groups = kFinWarps * per_warp;
+    const int plane = kFinBatch * ld;
+    const bool two = REL && L.S == 2;
+    const int64_t step = (int64_t)(gridDim.x - neg_ctas) * kFinBatch;
+    int64_t base = (int64_t)((int)blockIdx.x - neg_ctas) * kFinBatch;
+    fetch(base);
+#pragma unroll 1
+    for (; base < d.B; base += step) {
+        if (warp == 0) sm.id[lane] = p_id, sm.row[lane] = p_row, sm.shared[lane] = (unsigned char)p_shared;
+        else if (warp == 1 && REL && lane < kFinBatch) sm.rid[lane] = p_rid;
+        else if (warp == 2) sm.dpos[lane / kFinBatch][k16] = p_dpos;
         __syncthreads();
-        if (tid < 2 * kFinEdgeBatch) {  // thread (side, k): does the row of this endpoint occur again in the batch, or hold a slot already?
-            const int side = tid / kFinEdgeBatch, k = tid % kFinEdgeBatch;
-            int hs = -1;
-            if (k < nb && sm.rid[k] >= 0) {
-                const long long id = side == 0 ? sm.sid[k] : sm.did[k];
-                const int sidx = (int)(((unsigned long long)id * 0x9E3779B97F4A7C15ull) >> 61);  // top 3 bits
-                if (sm.hot_tag[sidx] == id) {
-                    hs = sidx;
-                } else if (sm.hot_tag[sidx] == kFinEmpty) {
-                    int seen = 0;
-                    for (int j = 0; j < nb; j++)
-                        if (sm.rid[j] >= 0) seen += (sm.sid[j] == id) + (sm.did[j] == id);
-                    if (seen > 1) {
-                        const long long old = (long long)atomicCAS((unsigned long long*)&sm.hot_tag[sidx], (unsigned long long)kFinEmpty, (unsigned long long)id);
-                        if (old == kFinEmpty || old == id) hs = sidx;
-                    }
-                }
-            }
-            sm.hot_slot[side][k] = hs;
+        if (warp == 0) {
+            sm.same[lane] = __match_any_sync(0xFFFFFFFFu, usable(k16) ? p_id : -1ll - lane);
+        } else if (warp == 1 && REL) {
+            const unsigned m = __match_any_sync(0xFFFFFFFFu, usable(k16) ? p_rid : -1 - lane);
+            if (lane < kFinBatch) sm.rel_same[lane] = m & ((1u << kFinBatch) - 1u);
         }
+        fetch(base + step);
         __syncthreads();
-        for (int k = warp; k < nb; k += kFinWarps) {
+#pragma unroll 1
+        for (int k = group; k < kFinBatch; k += groups) {
+            if (!usable(k)) continue;
+            const int64_t i = base + k;
+            const int64_t srow = sm.row[k] * d.emb_stride, drow = sm.row[kFinBatch + k] * d.emb_stride;
             // one edge, both corruption sides at once: side 0 applies the relation to the source and compares with the
             // destination, side 1 the inverse relation to the destination and compares with the source, so each endpoint
             // receives one combined row instead of two
-            const int64_t i = base + k;
-            const int rid = sm.rid[k];
-            if (rid < 0) continue;  // bad rows were flagged by prep
-            const int64_t sid = sm.sid[k], did = sm.did[k];
-            const float* es = d.node_emb + sm.srow[k] * d.emb_stride;
-            const float* ed = d.node_emb + sm.drow[k] * d.emb_stride;
-            const float* r[2] = {nullptr, nullptr};
-            const float* dq[2] = {nullptr, nullptr};
-            float* rg[2] = {nullptr, nullptr};
-            int slot_r[2] = {-1, -1};
-            float dpos[2] = {0.f, 0.f};
-#pragma unroll
-            for (int s = 0; s < 2; s++) {
-                if (s >= L.S) break;
-                dq[s] = L.dQ + ((int64_t)s * L.Bp + i) * ld;
-                dpos[s] = sm.dpos[s][k];
-                if (d.has_relations) {
-                    r[s] = (s == 0 ? d.rel : d.inv_rel) + (int64_t)rid * D;
-                    rg[s] = (s == 0 ? d.rel_grad : d.inv_rel_grad) + (int64_t)rid * D;
-                    slot_r[s] = sm.slot[s][k];
+            const float4 es = load_row<V, CPLX>(table + srow, l, D), ed = load_row<V, CPLX>(table + drow, l, D);
+            float4 g0 = load_row<V, CPLX>(L.dQ + i * ld, l, D), g1 = g0, r0 = g0, r1 = g0, ss = g0, sd = g0;
+            const int rid = REL ? sm.rid[k] : 0;
+            if (REL) r0 = load_row<V, CPLX>(d.rel + (int64_t)rid * D, l, D);
+            if (two) {
+                g1 = load_row<V, CPLX>(L.dQ + (L.Bp + i) * ld, l, D);
+                r1 = load_row<V, CPLX>(d.inv_rel + (int64_t)rid * D, l, D);
+            }
+            if (!sm.shared[k]) ss = load_row<V, CPLX>(d.node_state + srow, l, D);
+            if (!sm.shared[kFinBatch + k]) sd = load_row<V, CPLX>(d.node_state + drow, l, D);
+            // gradient with respect to the relation-adjusted embedding q = op(a, r): from the negatives (dQ) and the positive
+            const float p0 = sm.dpos[0][k];
+            g0 = axpy4(p0, ed, scale4(gs, g0));
+            float4 gsrc = g0, gdst = scale4(p0, es);
+            float* const buf = fin_rows + k * ld + 4 * l;
+            if (REL) {
+                gsrc = rel_mul_t<CPLX>(g0, r0);
+                gdst = scale4(p0, rel_mul<CPLX>(es, r0));
+                float4 vr0 = rel_mul_t<CPLX>(g0, es), vr1 = vr0;
+                if (two) {
+                    const float p1 = sm.dpos[1][k];
+                    g1 = axpy4(p1, es, scale4(gs, g1));
+                    gdst = add4(gdst, rel_mul_t<CPLX>(g1, r1));
+                    gsrc = add4(gsrc, scale4(p1, rel_mul<CPLX>(ed, r1)));
+                    vr1 = rel_mul_t<CPLX>(g1, ed);
+                }
+                if ((sm.rel_same[k] & (sm.rel_same[k] - 1u)) == 0u) {
+                    put_row<V, CPLX, PutAdd>(d.rel_grad + (int64_t)rid * D, l, D, vr0);
+                    if (two) put_row<V, CPLX, PutAdd>(d.inv_rel_grad + (int64_t)rid * D, l, D, vr1);
+                } else {
+                    *reinterpret_cast<float4*>(buf) = vr0;
+                    *reinterpret_cast<float4*>(buf + plane) = vr1;
                 }
             }
-            // generic pointers: a shared-memory row for a hub, the global gradient row otherwise (the atomics below take either)
-            const int hs_s = sm.hot_slot[0][k], hs_d = sm.hot_slot[1][k];
-            float* gsrc = hs_s >= 0 ? sm.hot[hs_s] : d.node_grad + sid * D;
-            float* gdst = hs_d >= 0 ? sm.hot[hs_d] : d.node_grad + did * D;
-            for (int c = lane; c < n_el; c += 32) {
-                // components 0 / 1 of coordinate c: (real, imaginary) for ComplEx, otherwise only component 0 is used
-                const int c2 = c + off2;
-                const float s0 = __ldg(es + c), d0 = __ldg(ed + c);
-                const float s1 = cplx ? __ldg(es + c2) : 0.f, d1 = cplx ? __ldg(ed + c2) : 0.f;
-                float gs0 = 0.f, gs1 = 0.f, gd0 = 0.f, gd1 = 0.f;  // gradient of the source / destination row at this coordinate
-#pragma unroll
-                for (int s = 0; s < 2; s++) {
-                    if (s >= L.S) break;
-                    const float a0 = s == 0 ? s0 : d0, a1 = s == 0 ? s1 : d1;  // endpoint the relation is applied to
-                    const float b0 = s == 0 ? d0 : s0, b1 = s == 0 ? d1 : s1;  // endpoint it is compared with
-                    // gradient with respect to the relation-adjusted embedding q = op(a, r): from the negatives (dQ) and the positive
-                    const float g0 = dq[s][c] * gs + dpos[s] * b0;
-                    const float g1 = cplx ? dq[s][c2] * gs + dpos[s] * b1 : 0.f;
-                    float ga0, ga1 = 0.f, gb0, gb1 = 0.f, vr0 = 0.f, vr1 = 0.f;
-                    if (r[s] == nullptr) {            // Dot: q = a
-                        gb0 = dpos[s] * a0;
-                        ga0 = g0;
-                    } else if (!cplx) {               // DistMult: q = a * r
-                        const float r0 = __ldg(r[s] + c);
-                        gb0 = dpos[s] * (a0 * r0);
-                        ga0 = g0 * r0;
-                        vr0 = g0 * a0;
-                    } else {                          // ComplEx: q = a x r (complex product), backward through both factors
-                        const float r0 = __ldg(r[s] + c), r1 = __ldg(r[s] + c2);
-                        gb0 = dpos[s] * (a0 * r0 - a1 * r1);
-                        gb1 = dpos[s] * (a0 * r1 + a1 * r0);
-                        ga0 = g0 * r0 + g1 * r1;
-                        ga1 = -g0 * r1 + g1 * r0;
-                        vr0 = g0 * a0 + g1 * a1;
-                        vr1 = -g0 * a1 + g1 * a0;
-                    }
-                    if (s == 0) {
-                        gs0 += ga0; gs1 += ga1; gd0 += gb0; gd1 += gb1;
-                    } else {
-                        gd0 += ga0; gd1 += ga1; gs0 += gb0; gs1 += gb1;
-                    }
-                    if (rg[s] != nullptr) {
-                        if (slot_r[s] >= 0) {
-                            atomicAdd(&sm.acc[slot_r[s]][c], vr0);
-                            if (cplx) atomicAdd(&sm.acc[slot_r[s]][c2], vr1);
-                        } else {
-                            atomicAdd(rg[s] + c, vr0);
-                            if (cplx) atomicAdd(rg[s] + c2, vr1);
-                        }
-                    }
-                }
-                atomicAdd(gsrc + c, gs0);
-                atomicAdd(gdst + c, gd0);
-                if (cplx) {
-                    atomicAdd(gsrc + c2, gs1);
-                    atomicAdd(gdst + c2, gd1);
-                }
+            float4 g = gsrc, e = es, st = ss;
+            int64_t at = srow;
+#pragma unroll 1
+            for (int side = 0; side < 2; side++) {  // the two endpoints
+                const int kk = side * kFinBatch + k;
+                if (!sm.shared[kk]) adagrad_row<V, CPLX>(table + at, d.node_state + at, l, D, e, st, g, neg_lr);
+                else if ((sm.same[kk] & (sm.same[kk] - 1u)) == 0u) put_row<V, CPLX, PutAdd>(d.node_grad + sm.id[kk] * D, l, D, g);
+                else *reinterpret_cast<float4*>(buf + (2 + side) * plane) = g;
+                g = gdst, e = ed, st = sd, at = drow;
             }
         }
-        if (!negs_done) {  // after the first batch of edges, whose endpoints have claimed the shared-memory rows of the hubs
-            scatter_negatives();
-            negs_done = true;
+        __syncthreads();
+        // the repeated rows: their first occurrence adds them up and sends the sum
+        const int rel_tasks = REL ? L.S * kFinBatch : 0;
+#pragma unroll 1
+        for (int t = group; t < rel_tasks + 2 * kFinBatch; t += groups) {
+            const bool is_rel = t < rel_tasks;
+            const int k = is_rel ? t & (kFinBatch - 1) : t - rel_tasks, side = is_rel ? t / kFinBatch : 2;
+            unsigned m = is_rel ? sm.rel_same[k] : sm.same[k];
+            if ((m & (m - 1u)) == 0u || __ffs((int)m) - 1 != k || (!is_rel && !sm.shared[k])) continue;
+            const float* rows = fin_rows + side * plane + 4 * l;  // (the destinations follow the sources)
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            while (m != 0u) {
+                v = add4(v, *reinterpret_cast<const float4*>(rows + (__ffs((int)m) - 1) * ld));
+                m &= m - 1u;
+            }
+            float* grow = is_rel ? (side == 0 ? d.rel_grad : d.inv_rel_grad) + (int64_t)sm.rid[k] * D : d.node_grad + sm.id[k] * D;
+            put_row<V, CPLX, PutAdd>(grow, l, D, v);
         }
-        __syncthreads();  // the batch's scalars are overwritten by the next batch
+        __syncthreads();  // the scalars are overwritten by the next batch
     }
-    if (!negs_done) scatter_negatives();
-    __syncthreads();
-    for (int slot = warp; slot < kFinHotSlots; slot += kFinWarps) {  // hub rows: one pass over global memory per CTA
-        const long long id = sm.hot_tag[slot];
-        if (id == kFinEmpty) continue;
-        float* grow = d.node_grad + id * D;
-        for (int k = lane; k < D; k += 32) {
-            const float v = sm.hot[slot][k];
-            if (v != 0.f) atomicAdd(grow + k, v);
-        }
-    }
-    if (!d.has_relations) return;
-    // flush: warp w writes slots w, w + 8, ...
-    for (int slot = warp; slot < kFinSlots; slot += kFinWarps) {
-        const long long key = sm.tag[slot];
-        if (key == kFinEmpty) continue;
-        const int kind = (int)(key >> 40);
-        const long long id = key & ((1ll << 40) - 1);
-        float* grow = (kind == 1 ? d.rel_grad : d.inv_rel_grad) + id * D;
-        for (int k = lane; k < D; k += 32) {
-            const float v = sm.acc[slot][k];
-            if (v != 0.f) atomicAdd(grow + k, v);
-        }
-    }
+}
+
+// the widest access all rows of a step allow: 16 bytes when rows are multiples of it and every table starts on one (8 for ComplEx, whose
+// halves need not), else 8, else 4
+int row_access(const ge2_lp_desc& d) {
+    const bool cplx = d.has_relations && d.decoder == GE2_DECODER_COMPLEX;
+    const uintptr_t bits = (uintptr_t)d.node_emb | (uintptr_t)d.node_grad | (uintptr_t)d.rel | (uintptr_t)d.inv_rel | (uintptr_t)d.rel_grad |
+                           (uintptr_t)d.inv_rel_grad | (uintptr_t)d.node_state | (uintptr_t)(d.emb_stride * 4);
+    if (cplx) return d.D % 4 == 0 && (bits & 7) == 0 ? 2 : 1;
+    if (d.D % 4 == 0 && (bits & 15) == 0) return 4;
+    return d.D % 2 == 0 && (bits & 7) == 0 ? 2 : 1;
+}
+
+using PrepKernel = void (*)(LpKernelArgs, int);
+using FinishKernel = void (*)(LpKernelArgs, int, int);
+template <bool HALF>
+PrepKernel prep_kernel_of(const ge2_lp_desc& d) {
+    const int V = row_access(d);
+    if (d.has_relations && d.decoder == GE2_DECODER_COMPLEX) return V == 2 ? lp_prep_kernel<2, true, true, HALF> : lp_prep_kernel<1, true, true, HALF>;
+    if (d.has_relations) return V == 4 ? lp_prep_kernel<4, false, true, HALF> : V == 2 ? lp_prep_kernel<2, false, true, HALF> : lp_prep_kernel<1, false, true, HALF>;
+    return V == 4 ? lp_prep_kernel<4, false, false, HALF> : V == 2 ? lp_prep_kernel<2, false, false, HALF> : lp_prep_kernel<1, false, false, HALF>;
+}
+FinishKernel finish_kernel_of(const ge2_lp_desc& d) {
+    const int V = row_access(d);
+    if (d.has_relations && d.decoder == GE2_DECODER_COMPLEX) return V == 2 ? lp_finish_kernel<2, true, true> : lp_finish_kernel<1, true, true>;
+    if (d.has_relations) return V == 4 ? lp_finish_kernel<4, false, true> : V == 2 ? lp_finish_kernel<2, false, true> : lp_finish_kernel<1, false, true>;
+    return V == 4 ? lp_finish_kernel<4, false, false> : V == 2 ? lp_finish_kernel<2, false, false> : lp_finish_kernel<1, false, false>;
 }
 
 __global__ void __launch_bounds__(256) copy_pos_kernel(const float* __restrict__ pos, int Bp, float* __restrict__ out0, float* __restrict__ out1,
@@ -485,6 +603,7 @@ int validate(const ge2_lp_desc* d) {
         (d->src_filter_n > 0 && d->src_filter == nullptr))
         return GE2_ERR_INVALID_ARGUMENT;
     if (d->deg_sample_rows != nullptr && (d->n_deg <= 0 || d->n_deg > d->N)) return GE2_ERR_INVALID_ARGUMENT;
+    if ((d->node_state == nullptr) != (d->row_shared == nullptr)) return GE2_ERR_INVALID_ARGUMENT;
     if (d->deg_sample_rows != nullptr && (d->dst_filter_n > 0 || d->src_filter_n > 0)) return GE2_ERR_INVALID_ARGUMENT;
     return GE2_OK;
 }
@@ -517,7 +636,9 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     if ((phases & 4) && !(desc->flags & GE2_LP_NODE_GRAD_IS_ZERO))
         GE2_CUDA_TRY(cudaMemsetAsync(desc->node_grad, 0, (size_t)desc->U * desc->D * 4, stream));
     if (phases & 1) {
-    if (desc->deg_sample_rows == nullptr) {  // (with the degree-sample plan the prepare kernel writes every filter word itself)
+    // without explicit filter pairs the prepare kernel writes every filter word itself
+    const bool pairs = desc->dst_filter_n > 0 || desc->src_filter_n > 0;
+    if (pairs) {
         GE2_CUDA_TRY(cudaMemsetAsync(L.mask, 0xFF, (size_t)L.S * L.CN * 4, stream));
         if (desc->dst_filter_n > 0) {
             mask_from_pairs_kernel<<<stream_grid(desc->dst_filter_n, 256), 256, 0, stream>>>(desc->dst_filter, desc->dst_filter_n, L.npc, L.Bp,
@@ -531,8 +652,9 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
         }
     }
 
-    const int64_t prep_rows = (int64_t)L.S * L.Bp + (int64_t)L.S * L.CN;
-    GE2_CUDA_TRY(launch_after(lp_prep_kernel, dim3((unsigned)stream_grid(prep_rows, 32, 8)), dim3(256), 0, stream, a));
+    const int64_t units = L.Bp + ceil_div<int64_t>(L.CN, kPrepNegs);
+    const PrepKernel prep = desc->precision == GE2_PRECISION_F16 ? prep_kernel_of<true>(*desc) : prep_kernel_of<false>(*desc);
+    GE2_CUDA_TRY(launch_after(prep, dim3((unsigned)stream_grid(units, 1024 / L.ld, 5)), dim3(256), 0, stream, a, pairs ? 0 : 1));
     }
 
     if (phases & 2) {
@@ -541,13 +663,14 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     }
     if (!(phases & 4)) return GE2_OK;
 
-    const int64_t fin_rows = (int64_t)desc->B + (int64_t)L.S * L.CN;
-    // about four CTAs per SM, each with a contiguous share of the edges (whose relation rows meet in its shared table) and of the negatives
+    // negatives a warp: 32 keep repeated nodes together and amortise the ids' latency, 8 spread a small batch over the GPU
     const int64_t neg_rows = (int64_t)L.S * L.CN;
-    int fin_ctas = (int)std::min<int64_t>((int64_t)kNumSMs * 4, ceil_div<int64_t>(fin_rows, 8));
-    if (fin_ctas < 1) fin_ctas = 1;
-    const int edges_per_cta = (int)ceil_div<int64_t>(desc->B, fin_ctas), negs_per_cta = (int)ceil_div<int64_t>(neg_rows, fin_ctas);
-    GE2_CUDA_TRY(launch_after(lp_finish_kernel, dim3((unsigned)fin_ctas), dim3(256), 0, stream, a, edges_per_cta, negs_per_cta));
+    int occ = 8;
+    while (occ < 32 && neg_rows / (2 * occ) >= (int64_t)kNumSMs * 4 * kFinWarps) occ *= 2;
+    const int edge_ctas = std::min(ceil_div(desc->B, kFinBatch), kNumSMs * 4);  // as many as are resident together
+    const int64_t neg_ctas = ceil_div<int64_t>(ceil_div<int64_t>(L.CN, occ / L.S), kFinWarps);
+    const size_t fin_smem = (size_t)4 * kFinBatch * L.ld * 4;
+    GE2_CUDA_TRY(launch_after(finish_kernel_of(*desc), dim3((unsigned)(edge_ctas + neg_ctas)), dim3(kFinWarps * 32), fin_smem, stream, a, (int)neg_ctas, occ));
     if (desc->pos_scores != nullptr || desc->inv_pos_scores != nullptr) {
         copy_pos_kernel<<<ceil_div(L.Bp, 256), 256, 0, stream>>>(L.pos, L.Bp, desc->pos_scores, desc->inv_pos_scores, L.S);
         GE2_LAUNCH_CHECK();

@@ -6,12 +6,10 @@
 // Floating-point updates use explicit round-to-nearest intrinsics so no multiply-add contraction happens: the result
 // is bit-identical to evaluating the reference's chain of element-wise ATen ops (cpp/src/data/batch.cpp:264-266,
 // cpp/src/nn/optim.cpp:130-137 of the reference project) one IEEE operation at a time.
-#include "common.cuh"
+#include "adagrad.cuh"
 
 namespace ge2 {
 namespace {
-
-constexpr float kAdagradEps = 1e-10f;  // literal in cpp/src/data/batch.cpp:266 of the reference project
 
 template <int V>
 struct Vec;
@@ -62,14 +60,6 @@ __device__ __forceinline__ int64_t live_rows(int64_t rows, const int32_t* rows_d
     int64_t r = (int64_t)__ldg(rows_dev);
     if (r < 0) r = 0;
     return r < rows ? r : rows;
-}
-
-// state += g*g ; delta = -lr * g / (sqrt(state) + eps)
-__device__ __forceinline__ void adagrad_elem(float g, float& state, float& delta, float& upd, float neg_lr) {
-    upd = __fmul_rn(g, g);
-    state = __fadd_rn(state, upd);
-    const float den = __fadd_rn(__fsqrt_rn(state), kAdagradEps);
-    delta = __fmul_rn(neg_lr, __fdiv_rn(g, den));
 }
 
 template <int V>
@@ -127,55 +117,85 @@ __global__ void __launch_bounds__(256) index_rows_kernel(float* __restrict__ tab
 }
 
 // Fused accumulateGradients + indexAdd(embeddings) + indexAdd(state): one read-modify-write of the touched rows.
+// A group of 2^lg lanes (enough for a row where 32 are) takes two consecutive rows at a time, so that their loads overlap; with
+// row_shared only the rows it names are touched (the others were finished where their gradient arose), and those that
+// are not cost one load.
 template <int V>
 __global__ void __launch_bounds__(256) adagrad_scatter_kernel(float* __restrict__ table, float* __restrict__ state, int64_t table_rows,
                                                               const int64_t* __restrict__ unique_ids, int64_t U, const int32_t* U_dev,
-                                                              float* __restrict__ node_grad, int vec_per_row, float neg_lr, int clear_grad,
-                                                              int32_t* status) {
+                                                              float* __restrict__ node_grad, int vec_per_row, int lg, float neg_lr, int clear_grad,
+                                                              const uint8_t* __restrict__ row_shared, int32_t* status) {
     using VT = typename Vec<V>::type;
+    constexpr int kRows = 2;
     griddep_wait();  // the gradient rows come from the kernel before this one
-    const int64_t total = live_rows(U, U_dev) * vec_per_row;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const int64_t l = i / vec_per_row;
-        const int c = (int)(i - l * vec_per_row);
-        const int64_t row = __ldg(&unique_ids[l]);
-        if (row < 0 || row >= table_rows) {
-            or_status(status, GE2_STATUS_BAD_INDEX);
-            continue;
-        }
-        const int64_t off = row * vec_per_row + c;
-        float g[V], s[V], e[V], d[V], u[V];
-        to_arr<V>(reinterpret_cast<const VT*>(node_grad)[i], g);
-        to_arr<V>(reinterpret_cast<const VT*>(state)[off], s);
-        to_arr<V>(reinterpret_cast<const VT*>(table)[off], e);
+    const int64_t rows = live_rows(U, U_dev);
+    const int64_t groups = ((int64_t)gridDim.x * blockDim.x) >> lg;
+    const int l = threadIdx.x & ((1 << lg) - 1);
+    for (int64_t r0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> lg) * kRows; r0 < rows; r0 += groups * kRows) {
+        int64_t row[kRows];
+        bool on[kRows];
 #pragma unroll
-        for (int k = 0; k < V; k++) {
-            adagrad_elem(g[k], s[k], d[k], u[k], neg_lr);
-            e[k] = __fadd_rn(e[k], d[k]);
+        for (int k = 0; k < kRows; k++) {
+            on[k] = r0 + k < rows && (row_shared == nullptr || row_shared[r0 + k] != 0);
+            row[k] = r0 + k < rows ? __ldg(&unique_ids[r0 + k]) : 0;
         }
-        reinterpret_cast<VT*>(state)[off] = from_arr<V>(s);
-        reinterpret_cast<VT*>(table)[off] = from_arr<V>(e);
-        if (clear_grad) {
-            float z[V];
 #pragma unroll
-            for (int k = 0; k < V; k++) z[k] = 0.f;
-            reinterpret_cast<VT*>(node_grad)[i] = from_arr<V>(z);
+        for (int k = 0; k < kRows; k++) {
+            if (on[k] && (row[k] < 0 || row[k] >= table_rows)) {
+                or_status(status, GE2_STATUS_BAD_INDEX);
+                on[k] = false;
+            }
+        }
+        for (int c = l; c < vec_per_row; c += 1 << lg) {
+            float g[kRows][V], s[kRows][V], e[kRows][V];
+#pragma unroll
+            for (int k = 0; k < kRows; k++) {
+                if (!on[k]) continue;
+                to_arr<V>(reinterpret_cast<const VT*>(node_grad)[(r0 + k) * vec_per_row + c], g[k]);
+                to_arr<V>(reinterpret_cast<const VT*>(state)[row[k] * vec_per_row + c], s[k]);
+                to_arr<V>(reinterpret_cast<const VT*>(table)[row[k] * vec_per_row + c], e[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < kRows; k++) {
+                if (!on[k]) continue;
+#pragma unroll
+                for (int v = 0; v < V; v++) {
+                    float dl, up;
+                    adagrad_elem(g[k][v], s[k][v], dl, up, neg_lr);
+                    e[k][v] = __fadd_rn(e[k][v], dl);
+                    g[k][v] = 0.f;
+                }
+                reinterpret_cast<VT*>(state)[row[k] * vec_per_row + c] = from_arr<V>(s[k]);
+                reinterpret_cast<VT*>(table)[row[k] * vec_per_row + c] = from_arr<V>(e[k]);
+                if (clear_grad) reinterpret_cast<VT*>(node_grad)[(r0 + k) * vec_per_row + c] = from_arr<V>(g[k]);
+            }
         }
     }
 }
 
+template <int V>
 __global__ void __launch_bounds__(256) dense_adagrad_kernel(float* __restrict__ param, float* __restrict__ sum, float* __restrict__ grad,
-                                                            int64_t numel, float neg_lr, float eps, float grad_scale, int clear_grad) {
+                                                            int64_t vecs, float neg_lr, float eps, float grad_scale, int clear_grad) {
+    using VT = typename Vec<V>::type;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < numel; i += stride) {
-        float g = grad[i];
-        if (grad_scale != 1.0f) g = __fmul_rn(g, grad_scale);
-        const float s = __fadd_rn(sum[i], __fmul_rn(g, g));
-        const float den = __fadd_rn(__fsqrt_rn(s), eps);
-        sum[i] = s;
-        param[i] = __fadd_rn(param[i], __fmul_rn(neg_lr, __fdiv_rn(g, den)));
-        if (clear_grad) grad[i] = 0.f;
+    griddep_wait();
+#pragma unroll 1
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += stride) {
+        float g[V], s[V], p[V];
+        to_arr<V>(reinterpret_cast<const VT*>(grad)[i], g);
+        to_arr<V>(reinterpret_cast<const VT*>(sum)[i], s);
+        to_arr<V>(reinterpret_cast<const VT*>(param)[i], p);
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+            if (grad_scale != 1.0f) g[v] = __fmul_rn(g[v], grad_scale);
+            s[v] = __fadd_rn(s[v], __fmul_rn(g[v], g[v]));
+            const float den = __fadd_rn(__fsqrt_rn(s[v]), eps);
+            p[v] = __fadd_rn(p[v], __fmul_rn(neg_lr, __fdiv_rn(g[v], den)));
+            g[v] = 0.f;
+        }
+        reinterpret_cast<VT*>(sum)[i] = from_arr<V>(s);
+        reinterpret_cast<VT*>(param)[i] = from_arr<V>(p);
+        if (clear_grad) reinterpret_cast<VT*>(grad)[i] = from_arr<V>(g);
     }
 }
 
@@ -324,6 +344,9 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
     return x ^ (x >> 31);
 }
 
+// (out of line: a 64-bit division is 1 KB of code, and kernels this short are bound by fetching theirs)
+__device__ __noinline__ uint64_t div_u64(uint64_t a, uint64_t b) { return a / b; }
+
 __global__ void __launch_bounds__(256) sample_negatives_kernel(const int64_t* __restrict__ src_ids, const int64_t* __restrict__ dst_ids,
                                                                int64_t edge_stride, int B, int C, int N, int n_deg, int64_t domain,
                                                                int want_src, uint64_t key, int64_t* __restrict__ packed,
@@ -337,7 +360,7 @@ __global__ void __launch_bounds__(256) sample_negatives_kernel(const int64_t* __
             num_batches = *num_batches_dev;
             if (num_batches < 1) num_batches = 1;
         }
-        const int64_t off = (int64_t)(step % (uint64_t)num_batches) * B * edge_stride;
+        const int64_t off = (int64_t)(step - div_u64(step, (uint64_t)num_batches) * (uint64_t)num_batches) * B * edge_stride;
         src_ids += off;
         dst_ids += off;
         if (rel_ids != nullptr) rel_ids += off;
@@ -348,6 +371,7 @@ __global__ void __launch_bounds__(256) sample_negatives_kernel(const int64_t* __
     int64_t* out_src_neg = packed + 2 * (int64_t)B;
     int64_t* out_dst_neg = out_src_neg + (want_src ? CN : 0);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 1
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         if (i < B) {
             packed[i] = src_ids[i * edge_stride];
@@ -356,7 +380,7 @@ __global__ void __launch_bounds__(256) sample_negatives_kernel(const int64_t* __
             packed[i] = dst_ids[(i - B) * edge_stride];
         } else {
             const int64_t e = i - 2 * (int64_t)B;
-            const int c = (int)(e / N);
+            const int c = e >> 32 ? (int)div_u64((uint64_t)e, (uint64_t)N) : (int)((uint32_t)e / (uint32_t)N);
             const int j = (int)(e - (int64_t)c * N);
             const uint64_t r = splitmix64(key ^ splitmix64((uint64_t)e));
             if (j < n_deg) {
@@ -428,17 +452,24 @@ extern "C" int ge2_index_add(float* table, int64_t table_rows, const int64_t* id
 
 extern "C" int ge2_adagrad_scatter(float* table, float* state, int64_t table_rows, const int64_t* unique_ids, int64_t U,
                                    const int32_t* U_dev, float* node_grad, int32_t D, float lr, int32_t clear_grad, int32_t* status,
-                                   ge2_stream_t stream_) {
+                                   ge2_stream_t stream) {
+    return ge2_adagrad_scatter_shared(table, state, table_rows, unique_ids, U, U_dev, node_grad, D, lr, clear_grad, nullptr, status, stream);
+}
+
+extern "C" int ge2_adagrad_scatter_shared(float* table, float* state, int64_t table_rows, const int64_t* unique_ids, int64_t U,
+                                          const int32_t* U_dev, float* node_grad, int32_t D, float lr, int32_t clear_grad,
+                                          const uint8_t* row_shared, int32_t* status, ge2_stream_t stream_) {
     if (U < 0 || D <= 0 || table_rows < 0) return GE2_ERR_INVALID_ARGUMENT;
     if (U == 0) return GE2_OK;
     if (table == nullptr || state == nullptr || unique_ids == nullptr || node_grad == nullptr) return GE2_ERR_INVALID_ARGUMENT;
     cudaStream_t stream = as_stream(stream_);
-    const int V = vec_width(D, table, state, node_grad);
-    const int grid = stream_grid(U * (D / V), 256);
-    const dim3 g((unsigned)grid), b(256);
-    if (V == 4) GE2_CUDA_TRY(launch_after(adagrad_scatter_kernel<4>, g, b, 0, stream, table, state, table_rows, unique_ids, U, U_dev, node_grad, D / 4, -lr, clear_grad, status));
-    else if (V == 2) GE2_CUDA_TRY(launch_after(adagrad_scatter_kernel<2>, g, b, 0, stream, table, state, table_rows, unique_ids, U, U_dev, node_grad, D / 2, -lr, clear_grad, status));
-    else GE2_CUDA_TRY(launch_after(adagrad_scatter_kernel<1>, g, b, 0, stream, table, state, table_rows, unique_ids, U, U_dev, node_grad, D, -lr, clear_grad, status));
+    const int V = vec_width(D, table, state, node_grad), vpr = D / V;
+    int lg = 0;
+    while (lg < 5 && (1 << lg) < vpr) lg++;
+    const dim3 g((unsigned)stream_grid(ceil_div<int64_t>(U, 2) << lg, 256)), b(256);
+    if (V == 4) GE2_CUDA_TRY(launch_after(adagrad_scatter_kernel<4>, g, b, 0, stream, table, state, table_rows, unique_ids, U, U_dev, node_grad, vpr, lg, -lr, clear_grad, row_shared, status));
+    else if (V == 2) GE2_CUDA_TRY(launch_after(adagrad_scatter_kernel<2>, g, b, 0, stream, table, state, table_rows, unique_ids, U, U_dev, node_grad, vpr, lg, -lr, clear_grad, row_shared, status));
+    else GE2_CUDA_TRY(launch_after(adagrad_scatter_kernel<1>, g, b, 0, stream, table, state, table_rows, unique_ids, U, U_dev, node_grad, vpr, lg, -lr, clear_grad, row_shared, status));
     return GE2_OK;
 }
 
@@ -447,8 +478,11 @@ extern "C" int ge2_dense_adagrad(float* param, float* sum_state, float* grad, in
     if (numel < 0) return GE2_ERR_INVALID_ARGUMENT;
     if (numel == 0) return GE2_OK;
     if (param == nullptr || sum_state == nullptr || grad == nullptr) return GE2_ERR_INVALID_ARGUMENT;
-    dense_adagrad_kernel<<<stream_grid(numel, 256), 256, 0, as_stream(stream_)>>>(param, sum_state, grad, numel, -lr, eps, grad_scale, clear_grad);
-    GE2_LAUNCH_CHECK();
+    cudaStream_t stream = as_stream(stream_);
+    if (numel % 4 == 0 && (((uintptr_t)param | (uintptr_t)sum_state | (uintptr_t)grad) & 15) == 0)
+        GE2_CUDA_TRY(launch_after(dense_adagrad_kernel<4>, dim3((unsigned)stream_grid(numel / 4, 256)), dim3(256), 0, stream, param, sum_state, grad, numel / 4, -lr, eps, grad_scale, clear_grad));
+    else
+        GE2_CUDA_TRY(launch_after(dense_adagrad_kernel<1>, dim3((unsigned)stream_grid(numel, 256)), dim3(256), 0, stream, param, sum_state, grad, numel, -lr, eps, grad_scale, clear_grad));
     return GE2_OK;
 }
 
@@ -579,4 +613,21 @@ extern "C" int ge2_copy_slabs(const float* src, float* dst, const int32_t* moves
     copy_slabs_kernel<<<grid, 256, 0, as_stream(stream_)>>>(reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), mv, v4);
     GE2_LAUNCH_CHECK();
     return GE2_OK;
+}
+
+extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
+    if (t == nullptr || t->lp == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+    const ge2_lp_desc& d = *t->lp;
+    int rc = ge2_sample_negatives(t->edges, t->edges + t->cols - 1, t->cols, d.B, d.C, d.N, t->n_deg, t->domain, d.use_inverse, t->seed, t->batch_index,
+                                  t->packed, t->deg_rows, stream);
+    if (rc != GE2_OK) return rc;
+    rc = ge2_unique_bitmap_shared(t->packed, t->n_ids, t->domain, t->unique_ws, t->unique_ws_bytes, t->unique, t->inverse, t->count, t->shared,
+                                  t->twin_begin, t->twin_len, stream);
+    if (rc != GE2_OK) return rc;
+    rc = ge2_lp_step(&d, stream);
+    if (rc != GE2_OK) return rc;
+    rc = ge2_adagrad_scatter_shared(t->table, t->state, t->table_rows, t->unique, d.U, t->count, d.node_grad, d.D, t->lr, 1, t->shared, d.status, stream);
+    for (int k = 0; rc == GE2_OK && k < t->num_dense; k++)
+        rc = ge2_dense_adagrad(t->dense_param[k], t->dense_state[k], t->dense_grad[k], t->dense_numel, t->dense_lr, 1e-10f, t->grad_scale, 1, stream);
+    return rc;
 }

@@ -3,23 +3,27 @@
 // Stands in for the bitmap backend of the reference's map_tensors_unique_inverse_cuda
 // (cuda/src/common/unique_map_cuda.cu:771-882 of the reference project: memset, mark, popcount, CUB scan,
 // extract, inverse, two stream syncs and four scalar read-backs).  Here:
-//   memset(control words + bitset)                       one cudaMemsetAsync (they are adjacent in the workspace)
-//   mark_kernel        ids -> bits                       n threads, 64-bit atomicOr (red) into an L2-resident bitset
+//   memset(control words + bitsets)                      one cudaMemsetAsync (they are adjacent in the workspace)
+//   mark_kernel        ids -> bits                       n threads, 64-bit atomicOr into an L2-resident bitset
 //   scan_extract_kernel popcount + exclusive scan + emit  one pass over the words; tiles chained by a
 //                                                        decoupled look-back (ticketed, bounded spin)
 //   inverse_kernel     rank of every input id            n threads; also hands the status word to the caller
 // The scan and the inverse kernel are launched with programmatic dependent launch behind their predecessors.
-// The bitset (domain/8 bytes) and the per-word offsets (domain/16 bytes) stay in the 126 MB L2 for every
-// configuration of interest (12.5 M-node domain: 1.6 MB + 0.8 MB), so HBM traffic is the ids in and the two
-// outputs: 16 n + 8 U bytes.
+// The bitsets (domain/8 bytes each) and the per-word offsets (domain/16 bytes) stay in the 126 MB L2 for every
+// configuration of interest (12.5 M-node domain: 2 x 1.6 MB + 0.8 MB), so HBM traffic is the ids in and the two
+// outputs: 16 n + 8 U bytes.  (One launch on a cluster of eight CTAs with the bitset in their shared memory is slower from a few
+// thousand ids on: 40 000 ids of a million took 31 us with the ids shared out, 21 us with every CTA going through all of them.)
+//
+// It can also say which ids occur more than once (out_shared): a second bitset collects the bits that were set already when they were
+// marked.  The rows of the other ids have one contribution to their gradient, so the training step can finish them on the spot.
 #include "common.cuh"
 
 namespace ge2 {
 namespace {
 
-constexpr int kScanThreads = 256;
-constexpr int kWordsPerThread = 4;
-constexpr int kTileWords = kScanThreads * kWordsPerThread;  // 1024 words = 65536 ids per tile
+constexpr int kScanThreads = 128;
+constexpr int kWordsPerThread = 1;
+constexpr int kTileWords = kScanThreads * kWordsPerThread;  // 128 words = 8192 ids per tile: a small domain still spreads over CTAs
 constexpr uint32_t kFlagAggregate = 1u << 30;               // tile state: local sum published
 constexpr uint32_t kFlagPrefix = 2u << 30;                  // tile state: inclusive prefix published
 constexpr uint32_t kValueMask = (1u << 30) - 1;
@@ -29,62 +33,85 @@ struct UniqueWorkspace {
     uint32_t* tile_state;       // [num_tiles]   } control words: cleared together with the bitset by one memset
     uint32_t* ticket;           // [1]           }
     int32_t* status;            // [1]           } GE2_STATUS_* bits of this call
-    unsigned long long* words;  // [num_words]
+    unsigned long long* words;  // [num_words]  one bit per id that occurs   } cleared by the same memset
+    unsigned long long* dup;    // [num_words]  ... that occurs again        }
     int32_t* word_offsets;      // [num_words]
 };
 
+// ids[begin + k] and ids[begin + len + k] count as one occurrence when they are equal (len == 0: no such pairs)
+struct Twins {
+    int64_t begin, len;
+};
+__device__ __forceinline__ bool is_second_twin(const int64_t* ids, int64_t i, int64_t key, const Twins& tw) {
+    const int64_t k = i - tw.begin - tw.len;
+    return k >= 0 && k < tw.len && ids[i - tw.len] == key;
+}
+
 constexpr size_t align256c(size_t x) { return (x + 255) & ~(size_t)255; }
-// control words (tile states, ticket, status, one spare), bitset, per-word offsets
+// control words (tile states, ticket, status, one spare), two bitsets, per-word offsets
 constexpr size_t unique_ws_bytes(int64_t domain) {
     const int64_t nw = (domain + 63) >> 6;
-    const int64_t tiles = (nw + 1023) / 1024;
-    return align256c((size_t)(tiles + 4) * 4) + align256c((size_t)nw * 8) + align256c((size_t)nw * 4);
+    const int64_t tiles = (nw + kTileWords - 1) / kTileWords;
+    return align256c((size_t)(tiles + 4) * 4) + 2 * align256c((size_t)nw * 8) + align256c((size_t)nw * 4);
 }
 
 __host__ __device__ inline int64_t num_words_of(int64_t domain) { return (domain + 63) >> 6; }
 
 __global__ void __launch_bounds__(256) mark_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t domain,
-                                                   unsigned long long* __restrict__ words, int32_t* __restrict__ status) {
+                                                   unsigned long long* __restrict__ words, unsigned long long* __restrict__ dup, Twins tw,
+                                                   int32_t* __restrict__ status) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     bool bad = false;
+#pragma unroll 1
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         int64_t key = ids[i];
         if (key < 0 || key >= domain) {
             bad = true;
             continue;
         }
-        atomicOr(&words[key >> 6], 1ull << (key & 63));
+        const unsigned long long bit = 1ull << (key & 63);
+        if (dup == nullptr) {
+            atomicOr(&words[key >> 6], bit);
+        } else if (!is_second_twin(ids, i, key, tw)) {
+            if ((atomicOr(&words[key >> 6], bit) & bit) != 0ull) atomicOr(&dup[key >> 6], bit);
+        }
     }
     if (bad) atomicOr(status, GE2_STATUS_ID_OUT_OF_RANGE);
 }
 
-// One tile = 1024 consecutive words.  Tiles are handed out by an atomic ticket so a tile only ever waits for tiles
+// One tile = 128 consecutive words.  Tiles are handed out by an atomic ticket so a tile only ever waits for tiles
 // that have already started (forward progress without co-residency assumptions); the wait is bounded anyway.
 __global__ void __launch_bounds__(kScanThreads) scan_extract_kernel(const unsigned long long* __restrict__ words, int64_t num_words,
                                                                     int32_t* __restrict__ word_offsets, uint32_t* tile_state,
                                                                     uint32_t* ticket, int num_tiles, int64_t* __restrict__ out_unique,
                                                                     int64_t out_capacity, int32_t* __restrict__ out_count,
+                                                                    const unsigned long long* __restrict__ dup, unsigned char* __restrict__ out_shared,
                                                                     int32_t* __restrict__ status) {
+    __shared__ unsigned long long s_words[kTileWords], s_dup[kTileWords];
+    __shared__ uint32_t s_off[kTileWords];
     __shared__ uint32_t s_warp_sums[kScanThreads / 32];
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_prefix;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // (the first ticket while the marking kernel still runs: the counter was cleared before that one started)
+    uint32_t first = tid == 0 ? atomicAdd(ticket, 1u) : 0u;
     griddep_wait();  // the bitset comes from the marking kernel
 
-    for (;;) {
-        if (tid == 0) s_tile = atomicAdd(ticket, 1u);
+    for (bool again_ = false;; again_ = true) {
+        if (tid == 0) s_tile = again_ ? atomicAdd(ticket, 1u) : first;
         __syncthreads();
         const uint32_t tile = s_tile;
         if (tile >= (uint32_t)num_tiles) return;
 
-        // each thread owns 4 consecutive words (one 32-byte load)
+        // each thread owns one word
         const int64_t w0 = (int64_t)tile * kTileWords + (int64_t)tid * kWordsPerThread;
-        unsigned long long w[kWordsPerThread];
+        unsigned long long w[kWordsPerThread], again[kWordsPerThread];
         uint32_t cnt[kWordsPerThread];
         uint32_t local = 0;
 #pragma unroll
         for (int k = 0; k < kWordsPerThread; k++) {
             w[k] = (w0 + k < num_words) ? words[w0 + k] : 0ull;
+            again[k] = (out_shared != nullptr && w0 + k < num_words) ? dup[w0 + k] : 0ull;
             cnt[k] = __popcll(w[k]);
             local += cnt[k];
         }
@@ -106,54 +133,75 @@ __global__ void __launch_bounds__(kScanThreads) scan_extract_kernel(const unsign
         }
         const uint32_t excl_in_tile = warp_base + incl - local;
 
-        // decoupled look-back, done by warp 0 lane 0 (the chain is short: one predecessor in the common case)
-        if (tid == 0) {
+        // decoupled look-back by warp 0, 32 predecessors at a time (tiles that start together publish their sums together: one by one
+        // tile k had about k / 3 loads in a row to wait for, 8 of the 10 us this kernel took on a million ids)
+        if (warp == 0) {
             uint32_t prefix = 0;
-            if (tile == 0) {
+            if (lane == 0) {
                 __threadfence();
-                atomicExch(&tile_state[0], kFlagPrefix | tile_total);
-            } else {
-                atomicExch(&tile_state[tile], kFlagAggregate | tile_total);
-                int64_t look = (int64_t)tile - 1;
-                int spins = 0;
-                bool failed = false;
-                while (look >= 0) {
-                    uint32_t st = *((volatile uint32_t*)&tile_state[look]);
-                    uint32_t flag = st & ~kValueMask;
-                    if (flag == kFlagPrefix) {
-                        prefix += st & kValueMask;
-                        break;
-                    } else if (flag == kFlagAggregate) {
-                        prefix += st & kValueMask;
-                        look--;
-                    } else if (++spins > kSpinLimit) {
+                atomicExch(&tile_state[tile], (tile == 0 ? kFlagPrefix : kFlagAggregate) | tile_total);
+            }
+            int64_t look = (int64_t)tile - 1;
+            int spins = 0;
+            bool failed = false;
+            while (look >= 0) {
+                uint32_t st = 2u << 30;  // (before the first tile: a prefix of zero)
+                if (look - lane >= 0) st = *((volatile uint32_t*)&tile_state[look - lane]);
+                const uint32_t flag = st & ~kValueMask;
+                const unsigned has_prefix = __ballot_sync(0xffffffffu, flag == kFlagPrefix);
+                const unsigned nearer = has_prefix ? (has_prefix & -has_prefix) - 1u : 0xffffffffu;  // lanes before the first prefix
+                if ((__ballot_sync(0xffffffffu, flag == 0u) & nearer) != 0u) {  // one of them has not published yet
+                    if (++spins > kSpinLimit) {
                         failed = true;
                         break;
                     }
+                    continue;
                 }
-                if (failed) atomicOr(status, GE2_STATUS_SCAN_TIMEOUT);
-                __threadfence();
-                atomicExch(&tile_state[tile], kFlagPrefix | ((prefix + tile_total) & kValueMask));
+                const bool take = (nearer >> lane) & 1u || (has_prefix & -has_prefix) == (1u << lane);
+                prefix += __reduce_add_sync(0xffffffffu, take ? st & kValueMask : 0u);
+                if (has_prefix) break;
+                look -= 32;
             }
-            s_prefix = prefix;
-            if (tile == (uint32_t)num_tiles - 1) out_count[0] = (int32_t)(prefix + tile_total);
+            if (lane == 0) {
+                if (failed) atomicOr(status, GE2_STATUS_SCAN_TIMEOUT);
+                if (tile != 0) {
+                    __threadfence();
+                    atomicExch(&tile_state[tile], kFlagPrefix | ((prefix + tile_total) & kValueMask));
+                }
+                s_prefix = prefix;
+                if (tile == (uint32_t)num_tiles - 1) out_count[0] = (int32_t)(prefix + tile_total);
+            }
         }
         __syncthreads();
         uint32_t out = s_prefix + excl_in_tile;
 #pragma unroll
         for (int k = 0; k < kWordsPerThread; k++) {
-            if (w0 + k < num_words) {
-                word_offsets[w0 + k] = (int32_t)out;
-                unsigned long long bits = w[k];
-                const int64_t base = (w0 + k) << 6;
-                uint32_t o = out;
-                while (bits != 0ull) {
-                    int b = __ffsll((long long)bits) - 1;
-                    if ((int64_t)o < out_capacity) out_unique[o] = base + b;
-                    o++;
-                    bits &= bits - 1ull;
+            s_words[tid * kWordsPerThread + k] = w[k];
+            s_dup[tid * kWordsPerThread + k] = again[k];
+            s_off[tid * kWordsPerThread + k] = out;
+            if (w0 + k < num_words) word_offsets[w0 + k] = (int32_t)out;
+            out += cnt[k];
+        }
+        __syncthreads();
+        // emission, eight ids of the domain a thread: a word that is full (small domains, hubs) costs its thread 8 turns, not 64, and
+        // neighbouring threads write neighbouring entries
+#pragma unroll 1
+        for (int p = tid; p < kTileWords * 8; p += kScanThreads) {
+            const unsigned long long word = s_words[p >> 3];
+            const int sh = (p & 7) * 8;
+            uint32_t bits = (uint32_t)(word >> sh) & 0xFFu;
+            if (bits == 0) continue;
+            uint32_t o = s_off[p >> 3] + (uint32_t)__popcll(word & ((1ull << sh) - 1ull));
+            const int64_t byte = (int64_t)tile * (kTileWords * 8) + p;
+            const uint32_t rep = (uint32_t)(s_dup[p >> 3] >> sh);
+            while (bits != 0) {
+                const int b = __ffs((int)bits) - 1;
+                if ((int64_t)o < out_capacity) {
+                    out_unique[o] = byte * 8 + b;
+                    if (out_shared != nullptr) out_shared[o] = (unsigned char)((rep >> b) & 1u);
                 }
-                out += cnt[k];
+                o++;
+                bits &= bits - 1u;
             }
         }
         __syncthreads();  // s_tile / s_prefix / s_warp_sums are reused by the next ticket
@@ -167,6 +215,7 @@ __global__ void __launch_bounds__(256) inverse_kernel(const int64_t* __restrict_
     griddep_wait();  // offsets and the count come from the scan kernel
     if (blockIdx.x == 0 && threadIdx.x == 0) *out_status = *status;  // the marking and scan kernels are over: the word is final
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll 1
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         int64_t key = ids[i];
         if (key < 0 || key >= domain) {
@@ -206,7 +255,14 @@ extern "C" size_t ge2_unique_workspace_bytes(int64_t domain) {
 }
 
 extern "C" int ge2_unique_bitmap(const int64_t* ids, int64_t n, int64_t domain, void* workspace, size_t workspace_bytes,
-                                 int64_t* out_unique, int64_t* out_inverse, int32_t* out_count, ge2_stream_t stream_) {
+                                 int64_t* out_unique, int64_t* out_inverse, int32_t* out_count, ge2_stream_t stream) {
+    return ge2_unique_bitmap_shared(ids, n, domain, workspace, workspace_bytes, out_unique, out_inverse, out_count, nullptr, 0, 0, stream);
+}
+
+extern "C" int ge2_unique_bitmap_shared(const int64_t* ids, int64_t n, int64_t domain, void* workspace, size_t workspace_bytes,
+                                        int64_t* out_unique, int64_t* out_inverse, int32_t* out_count, uint8_t* out_shared, int64_t twin_begin,
+                                        int64_t twin_len, ge2_stream_t stream_) {
+    if (twin_begin < 0 || twin_len < 0 || (twin_len > 0 && twin_begin + 2 * twin_len > n)) return GE2_ERR_INVALID_ARGUMENT;
     if (n < 0 || domain <= 0 || out_count == nullptr) return GE2_ERR_INVALID_ARGUMENT;
     if (n > 0 && (ids == nullptr || out_unique == nullptr || out_inverse == nullptr)) return GE2_ERR_INVALID_ARGUMENT;
     if (n > (int64_t)kValueMask) return GE2_ERR_UNSUPPORTED;  // the reference stops at INT32_MAX ids (unique_map_cuda.cu:784); the packed tile state here holds 30 bits
@@ -221,6 +277,9 @@ extern "C" int ge2_unique_bitmap(const int64_t* ids, int64_t n, int64_t domain, 
     if (workspace == nullptr || ((uintptr_t)workspace & 255) != 0 || workspace_bytes < ge2_unique_workspace_bytes(domain))
         return GE2_ERR_WORKSPACE;
 
+    const int64_t cap = n < domain ? n : domain;
+    const Twins tw = {twin_begin, twin_len};
+
     char* p = (char*)workspace;
     UniqueWorkspace ws;
     ws.tile_state = (uint32_t*)p;
@@ -230,18 +289,19 @@ extern "C" int ge2_unique_bitmap(const int64_t* ids, int64_t n, int64_t domain, 
     p += ctl_bytes;
     ws.words = (unsigned long long*)p;
     p += align256c((size_t)nw * 8);
+    ws.dup = (unsigned long long*)p;
+    p += align256c((size_t)nw * 8);
     ws.word_offsets = (int32_t*)p;
 
-    // control words and bitset are adjacent: one memset; out_count needs none (the scan's last tile writes the count, the
+    // control words and bitsets are adjacent: one memset; out_count needs none (the scan's last tile writes the count, the
     // inverse kernel the status)
-    GE2_CUDA_TRY(cudaMemsetAsync(ws.tile_state, 0, ctl_bytes + (size_t)nw * 8, stream));
+    GE2_CUDA_TRY(cudaMemsetAsync(ws.tile_state, 0, ctl_bytes + (out_shared != nullptr ? align256c((size_t)nw * 8) : 0) + (size_t)nw * 8, stream));
 
-    mark_kernel<<<stream_grid(n, 256), 256, 0, stream>>>(ids, n, domain, ws.words, ws.status);
+    mark_kernel<<<stream_grid(n, 256), 256, 0, stream>>>(ids, n, domain, ws.words, out_shared != nullptr ? ws.dup : nullptr, tw, ws.status);
     GE2_LAUNCH_CHECK();
-    const int64_t cap = n < domain ? n : domain;
-    const int scan_grid = (int)(tiles < (int64_t)kNumSMs * 4 ? tiles : (int64_t)kNumSMs * 4);
+    const int scan_grid = (int)(tiles < (int64_t)kNumSMs * 8 ? tiles : (int64_t)kNumSMs * 8);
     GE2_CUDA_TRY(launch_after(scan_extract_kernel, dim3((unsigned)scan_grid), dim3(kScanThreads), 0, stream, (const unsigned long long*)ws.words, nw,
-                              ws.word_offsets, ws.tile_state, ws.ticket, (int)tiles, out_unique, cap, out_count, ws.status));
+                              ws.word_offsets, ws.tile_state, ws.ticket, (int)tiles, out_unique, cap, out_count, (const unsigned long long*)ws.dup, out_shared, ws.status));
     GE2_CUDA_TRY(launch_after(inverse_kernel, dim3((unsigned)stream_grid(n, 256)), dim3(256), 0, stream, ids, n, domain,
                               (const unsigned long long*)ws.words, (const int32_t*)ws.word_offsets, out_inverse, (const int32_t*)ws.status,
                               out_count + 1));

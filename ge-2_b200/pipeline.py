@@ -9,6 +9,7 @@ Torch tensors are used as device memory only; every arithmetic step is a kernel 
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 from typing import Optional
 
@@ -61,6 +62,8 @@ class _IdSet:
         self.deg_rows = torch.empty((cfg.C, max(cfg.n_deg, 1)), **i64)
         self.unique = torch.empty(cap, **i64)
         self.inverse = torch.empty(n_ids, **i64)
+        self.shared = torch.empty(cap, dtype=torch.uint8, device=dev)  # per unique id: 1 = more than one occurrence in the batch
+        self.twins = (2 * B, CN) if cfg.sides == 2 else (0, 0)  # the sides' negatives, node for node where they are drawn uniformly
         self.count = torch.zeros(2, dtype=torch.int32, device=dev)
         self.rel_ids = torch.empty(max(B, 1), **i64)  # the batch's relation column, copied by the sampler
         self.loss = torch.zeros(1, dtype=torch.float32, device=dev)  # loss of the batch trained from this set
@@ -181,6 +184,10 @@ class BatchPipeline:
         else:
             capi.sample_batch(edges_all, num_batches, counter, *args)
 
+    def _unique(self, ids: "_IdSet"):
+        capi.unique_bitmap(ids.packed, self.cfg.domain, workspace=ids.uws, out_unique=ids.unique, out_inverse=ids.inverse, out_count=ids.count,
+                           out_shared=ids.shared, twins=ids.twins)
+
     def use_peer_gradients(self, peer: PeerGradients):
         """Multi-GPU: relation gradients go into `peer`'s buffer (alternating halves) and the dense optimizer step sums them
         over the ranks itself.  Supported by enqueue_resident and capture_pipelined; needs the relation tables (and their
@@ -209,7 +216,8 @@ class BatchPipeline:
             rel_ids=rel_ids if cfg.has_relations else None, edge_stride=1, rel_stride=rel_stride or 1, dst_negs=ids.dst_negs_local,
             src_negs=ids.src_negs_local, deg_sample_rows=ids.deg_rows if cfg.n_deg > 0 else None, n_deg=cfg.n_deg,
             rel=self.rel, inv_rel=self.inv_rel if cfg.sides == 2 else None, node_grad=self.node_grad, rel_grad=rel_grad,
-            inv_rel_grad=inv_rel_grad, loss=ids.loss, status=self.status, node_grad_is_zero=True)
+            inv_rel_grad=inv_rel_grad, loss=ids.loss, status=self.status, node_grad_is_zero=True,
+            node_state=self.state, row_shared=ids.shared, node_lr=cfg.lr)
         if self._ws is None:
             self._ws = torch.empty(capi.lp_workspace_bytes(d), dtype=torch.uint8, device=self.device)
         d.workspace, d.workspace_bytes = self._ws.data_ptr(), self._ws.numel()
@@ -224,10 +232,47 @@ class BatchPipeline:
         cfg = self.cfg
         cols = edges.shape[1]
         assert edges.shape[0] == cfg.B and edges.dtype == torch.int64 and edges.is_contiguous()
+        if scores_events is None and rel_hook is None and self.peer is None:
+            t = self._train_desc(edges)
+            t.edges, t.batch_index = edges.data_ptr(), batch_index
+            if cfg.has_relations:
+                self._train_lp.rel_ids = t.edges + 8  # column 1
+            capi.train_step(t)
+            return
         capi.sample_negatives(edges, edges[:, cols - 1], cols, cfg.B, cfg.C, cfg.N, cfg.n_deg, cfg.domain, cfg.sides == 2, cfg.seed,
                               batch_index, self.packed, self.deg_rows if cfg.n_deg > 0 else None)
-        capi.unique_bitmap(self.packed, cfg.domain, workspace=self.uws, out_unique=self.unique, out_inverse=self.inverse, out_count=self.count)
+        self._unique(self.ids[0])
         self._backward_and_update(self._make_desc(edges), scores_events, rel_hook)
+
+    def _train_desc(self, edges):
+        """The arguments of a whole host-issued step: laid out once, and again whenever a table or a rate was replaced; of the rest only
+        the batch's address and number change from step to step."""
+        cfg = self.cfg
+        key = (self.table.data_ptr(), self.state.data_ptr(), self.node_grad.data_ptr(), cfg.lr, cfg.dense_lr, self.grad_scale, edges.shape[1])
+        if cfg.has_relations:
+            tabs = (self.rel, self.rel_state, self.rel_grad) + ((self.inv_rel, self.inv_rel_state, self.inv_rel_grad) if cfg.sides == 2 else ())
+            key += tuple(a.data_ptr() for a in tabs)
+        if key == getattr(self, "_train_key", None):
+            return self._train
+        ids = self.ids[0]
+        self._train_lp = self._make_desc(edges)
+        t = capi.TrainDesc()
+        t.lp = ctypes.pointer(self._train_lp)
+        t.cols, t.n_deg, t.domain, t.seed = edges.shape[1], cfg.n_deg, cfg.domain, cfg.seed
+        t.packed, t.deg_rows, t.n_ids = ids.packed.data_ptr(), ids.deg_rows.data_ptr() if cfg.n_deg > 0 else None, ids.packed.numel()
+        t.unique_ws, t.unique_ws_bytes = ids.uws.data_ptr(), ids.uws.numel()
+        t.unique, t.inverse, t.count, t.shared = (a.data_ptr() for a in (ids.unique, ids.inverse, ids.count, ids.shared))
+        t.twin_begin, t.twin_len = ids.twins
+        t.table, t.state, t.table_rows, t.lr, t.grad_scale = self.table.data_ptr(), self.state.data_ptr(), self.table.shape[0], cfg.lr, self.grad_scale
+        if cfg.has_relations:
+            t.dense_lr = cfg.lr if cfg.dense_lr is None else cfg.dense_lr
+            both = cfg.sides == 2 and self._rel_tables_adjacent
+            t.num_dense = 2 if cfg.sides == 2 and not both else 1
+            t.dense_numel = self.rel.numel() * (2 if both else 1)
+            for k, (p, st, g) in enumerate(((self.rel, self.rel_state, self.rel_grad), (self.inv_rel, self.inv_rel_state, self.inv_rel_grad))[:t.num_dense]):
+                t.dense_param[k], t.dense_state[k], t.dense_grad[k] = p.data_ptr(), st.data_ptr(), g.data_ptr()
+        self._train, self._train_key = t, key
+        return t
 
     def _backward_and_update(self, desc, scores_events=None, rel_hook=None):
         self._backward(desc, scores_events)
@@ -277,9 +322,10 @@ class BatchPipeline:
     def _update_nodes(self, ids: Optional[_IdSet] = None):
         cfg = self.cfg
         ids = ids or self.ids[0]
+        # rows with one occurrence were updated by the backward pass, where their whole gradient is at hand; this does the others.
         # clear_grad: the rows just consumed are zeroed in the same pass, so the next step needs no memset of the gradient buffer
         capi.adagrad_scatter(self.table, self.state, ids.unique, self.node_grad, cfg.lr, U=self.cap, U_dev=ids.count, clear_grad=True,
-                             status=self.status)
+                             status=self.status, row_shared=ids.shared)
 
     def _update_relations(self):
         cfg = self.cfg
@@ -306,7 +352,7 @@ class BatchPipeline:
         captured once into a CUDA graph (capture_resident) and replayed."""
         cfg = self.cfg
         self._sample(self.ids[0], edges_all, num_batches, self.step_dev)
-        capi.unique_bitmap(self.packed, cfg.domain, workspace=self.uws, out_unique=self.unique, out_inverse=self.inverse, out_count=self.count)
+        self._unique(self.ids[0])
         self._backward_and_update(self._make_desc(edges_all, self.rel_ids, 1), scores_events, rel_hook)
         capi.advance_step(self.step_dev, 2)
         self._t_host += 1
@@ -336,8 +382,7 @@ class BatchPipeline:
         with torch.cuda.graph(ga):
             capi.sample_batch(edges_all, num_batches, self.step_dev, cfg.B, cfg.C, cfg.N, cfg.n_deg, cfg.domain, cfg.sides == 2, cfg.seed,
                               self.packed, self.deg_rows if cfg.n_deg > 0 else None, self.rel_ids if cfg.has_relations else None)
-            capi.unique_bitmap(self.packed, cfg.domain, workspace=self.uws, out_unique=self.unique, out_inverse=self.inverse,
-                               out_count=self.count)
+            self._unique(self.ids[0])
             self._backward(self._make_desc(edges_all, self.rel_ids, 1))
         with torch.cuda.graph(gb):
             self._update()
@@ -357,7 +402,7 @@ class BatchPipeline:
         """sampler + unique-map into one id set; `counter` is the device counter holding the batch number to use"""
         cfg = self.cfg
         self._sample(ids, edges_all, num_batches, counter)
-        capi.unique_bitmap(ids.packed, cfg.domain, workspace=ids.uws, out_unique=ids.unique, out_inverse=ids.inverse, out_count=ids.count)
+        self._unique(ids)
 
     def idle_step(self):
         """A step of a lane that has no batch (lanes of a superstep have unequal batch counts): the relation-gradient

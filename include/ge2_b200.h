@@ -64,10 +64,16 @@ GE2_API size_t ge2_unique_workspace_bytes(int64_t domain);
 GE2_API int ge2_unique_bitmap(const int64_t *ids, int64_t n, int64_t domain, void *workspace, size_t workspace_bytes,
                       int64_t *out_unique, int64_t *out_inverse, int32_t *out_count, ge2_stream_t stream);
 
+/* The same, and which of the distinct ids occur more than once: out_shared[rank] = 1 when the id of that rank does, else 0 (capacity
+ * as out_unique; NULL = not wanted).  Entries k of [twin_begin, twin_begin + twin_len) and of the twin_len entries behind them count as
+ * one occurrence where they are equal (twin_len == 0: none) -- the negatives both corruption sides of a step share. */
+GE2_API int ge2_unique_bitmap_shared(const int64_t *ids, int64_t n, int64_t domain, void *workspace, size_t workspace_bytes,
+                                     int64_t *out_unique, int64_t *out_inverse, int32_t *out_count, uint8_t *out_shared, int64_t twin_begin,
+                                     int64_t twin_len, ge2_stream_t stream);
 /* Unique-map for callers that cannot allocate device memory -- a host runtime that owns the whole GPU heap and hands
  * out none of it after start-up, a plugin that only ever receives its input and output buffers, a latency-bound loop
  * that may not call an allocator.  No counterpart in the reference project.  Same results as ge2_unique_bitmap, but
- * the scratch is a fixed array inside the library (about 0.8 MB on every GPU that loads it, held until the process
+ * the scratch is a fixed array inside the library (about 1.3 MB on every GPU that loads it, held until the process
  * exits), so the id domain is limited to GE2_UNIQUE_STATIC_MAX_DOMAIN; a larger domain returns GE2_ERR_UNSUPPORTED.
  * The call makes no cudaMalloc/cudaFree and uses no allocating library routine.  The first call on each device looks
  * up the array's device address; make that first call outside any stream capture.  All calls share the one array,
@@ -168,6 +174,15 @@ typedef struct ge2_lp_desc {
     int32_t *status;      /* device int32, GE2_STATUS_* bits are OR-ed in; may be NULL             */
     void *workspace;      /* ge2_lp_workspace_bytes() bytes, 256-byte aligned                      */
     size_t workspace_bytes;
+
+    /* optional (both or neither): the optimizer step of the rows that need no sum over occurrences, inside the scatter.  row_shared[U]
+     * (ge2_unique_bitmap_shared with the two sides' negatives as twins): 0 = the node occurs once in the batch.  Such a row never
+     * reaches node_grad: its row of node_emb (written, despite the const) and of node_state (same rows and stride) takes the
+     * Adagrad step with learning rate node_lr here; ge2_adagrad_scatter_shared does the rows marked 1. */
+    float *node_state;
+    const uint8_t *row_shared;
+    float node_lr;
+    int32_t reserved;
 } ge2_lp_desc;
 
 GE2_API int ge2_lp_workspace_bytes(const ge2_lp_desc *desc, size_t *bytes);
@@ -199,6 +214,10 @@ GE2_API int ge2_index_add(float *table, int64_t table_rows, const int64_t *ids, 
 GE2_API int ge2_adagrad_scatter(float *table, float *state, int64_t table_rows, const int64_t *unique_ids, int64_t U,
                         const int32_t *U_dev, float *node_grad, int32_t D, float lr, int32_t clear_grad, int32_t *status,
                         ge2_stream_t stream);
+/* The same for the rows with row_shared != 0 alone (NULL: all of them). */
+GE2_API int ge2_adagrad_scatter_shared(float *table, float *state, int64_t table_rows, const int64_t *unique_ids, int64_t U,
+                                       const int32_t *U_dev, float *node_grad, int32_t D, float lr, int32_t clear_grad,
+                                       const uint8_t *row_shared, int32_t *status, ge2_stream_t stream);
 
 /* AdagradOptimizer::step on a dense table (cpp/src/nn/optim.cpp:109-143; weight_decay = lr_decay = 0):
  * sum += g*g; param += -lr * g / (sqrt(sum) + eps).  grad_scale multiplies g first (1/num_gpus in
@@ -251,6 +270,31 @@ GE2_API int ge2_sample_negatives(const int64_t *src_ids, const int64_t *dst_ids,
 GE2_API int ge2_sample_batch(const int64_t *edges, int32_t cols, int64_t num_batches, const uint64_t *step_dev, int32_t B, int32_t C,
                              int32_t N, int32_t n_deg, int64_t domain, int32_t want_src_negs, uint64_t seed, int64_t *out_packed_ids,
                              int64_t *out_deg_rows, int64_t *out_rel_ids, ge2_stream_t stream);
+/* One training step in one call: ge2_sample_negatives, ge2_unique_bitmap_shared, ge2_lp_step, ge2_adagrad_scatter_shared and
+ * ge2_dense_adagrad (num_dense parameters of dense_numel floats each) with the same arguments, issued from native code. */
+typedef struct ge2_train_desc {
+    const ge2_lp_desc *lp;
+    const int64_t *edges; /* [B, cols] */
+    int32_t cols, n_deg;
+    int64_t domain;
+    uint64_t seed, batch_index;
+    int64_t *packed, *deg_rows;
+    int64_t n_ids;
+    void *unique_ws;
+    size_t unique_ws_bytes;
+    int64_t *unique, *inverse;
+    int32_t *count;
+    uint8_t *shared;
+    int64_t twin_begin, twin_len;
+    float *table, *state;
+    int64_t table_rows;
+    float lr, dense_lr, grad_scale;
+    int32_t num_dense;
+    float *dense_param[2], *dense_state[2], *dense_grad[2];
+    int64_t dense_numel;
+} ge2_train_desc;
+GE2_API int ge2_train_step(const ge2_train_desc *desc, ge2_stream_t stream);
+
 /* The same with the number of batches read from device memory (*num_batches_dev >= 1): a partition-buffer state replaces the
  * resident edge list by one of another length (ge2_build_state_edges) without the captured launch changing. */
 GE2_API int ge2_sample_batch_dev(const int64_t *edges, int32_t cols, const int64_t *num_batches_dev, const uint64_t *step_dev, int32_t B,

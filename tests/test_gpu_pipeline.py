@@ -131,3 +131,38 @@ def test_host_feed_trains_the_same_batches_as_the_resident_form(cuda_device):
     for a, b in zip(out[0], out[1]):
         assert np.abs(a - b).max() <= 1e-5 * np.abs(a).max()
     assert (out[0][3][: nb - 1] > 0).all()
+
+
+@pytest.mark.parametrize("decoder,D,R,B,C,N,nodes", [("COMPLEX", 50, 9, 33, 2, 30, 300), ("COMPLEX", 128, 3, 1, 1, 1, 5), ("DISTMULT", 101, 7, 700, 3, 65, 90000),
+                                                      ("DISTMULT", 62, 300, 16, 1, 600, 900), ("DOT", 128, 1, 17, 1, 40, 100), ("DOT", 3, 1, 500, 7, 33, 2000)])
+def test_rows_finished_in_the_backward_pass(ge2, cuda_device, decoder, D, R, B, C, N, nodes):
+    """Rows with one occurrence updated where their gradient arises, the others through the gradient buffer: the tables are those of the
+    form that sends every row through the buffer."""
+    from importlib import import_module
+
+    pipeline = import_module("ge-2_b200.pipeline")
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(D + B)
+    start = [torch.rand((r, D), generator=gen, device=cuda_device) * 0.5 + 0.1 for r in (nodes, nodes, R, R, R, R)]
+    edges = torch.stack([torch.randint(m, (B,), generator=gen, device=cuda_device) for m in ((nodes, R, nodes) if R > 1 else (nodes, nodes))], 1).contiguous()
+    cfg = pipeline.PipelineConfig(decoder=decoder, B=B, C=C, N=N, degree_fraction=0.3, D=D, R=R, domain=nodes, lr=0.1, precision="fp32")
+    results = []
+    for fused in (True, False):
+        tables = [t.clone() for t in start]
+        pipe = pipeline.BatchPipeline(cfg, *(tables if R > 1 else tables[:2]))
+        if fused:
+            pipe.step(edges, 3)
+        else:
+            capi = ge2.capi
+            capi.sample_negatives(edges, edges[:, -1], edges.shape[1], B, C, N, cfg.n_deg, nodes, cfg.sides == 2, cfg.seed, 3, pipe.packed, pipe.deg_rows)
+            pipe._unique(pipe.ids[0])
+            d = pipe._make_desc(edges)
+            d.node_state = d.row_shared = None
+            capi.lp_step(d)
+            capi.adagrad_scatter(pipe.table, pipe.state, pipe.unique, pipe.node_grad, 0.1, U=pipe.cap, U_dev=pipe.count, clear_grad=True)
+            pipe._update_relations()
+        torch.cuda.synchronize()
+        assert int(pipe.status) == 0 and int(pipe.node_grad.abs().max() > 0) == 0
+        results.append(tables)
+    for a, b, s in zip(*results, start):
+        assert (a - b).abs().max() <= 2e-5 * max(1e-3, float((a - s).abs().max()))

@@ -136,7 +136,7 @@ def test_tournament_rejects_uneven_groups_and_accepts_empty_input(capi, cuda_dev
 
 @pytest.mark.parametrize("C,R,N,D,K", [
     (1, 127, 64, 63, 64), (2, 129, 65, 65, 5), (1, 1, 1, 1, 1), (300, 3, 20, 8, 4),  # one past a tile each way; more items than SMs
-    (3, 256, 640, 128, 3), (1, 128, 4096, 66, 64),                                    # groups over several tiles, shares cut inside a row tile
+    (3, 256, 640, 128, 5), (1, 128, 4096, 66, 64),                                    # groups over several tiles, shares cut inside a row tile
 ])
 def test_tournament_at_tile_edges_and_on_ties(capi, cuda_device, C, R, N, D, K):
     rng = np.random.default_rng(C + R + N + D)

@@ -76,3 +76,22 @@ def test_workspace_reuse_back_to_back(capi, cuda_device):
         ou, oinv = O.unique_map_sort(ids_np)
         c = int(cnt[0])
         assert c == ou.size and np.array_equal(u.cpu().numpy()[:c], ou) and np.array_equal(inv.cpu().numpy(), oinv)
+
+
+@pytest.mark.parametrize("n,domain", [(3, 2), (22000, 255), (22000, 257), (65536, 65536), (65537, 65537), (3000, 4_456_449)])
+def test_repeated_ids_and_twins(capi, cuda_device, n, domain):
+    """out_shared at the edges of words and tiles; the two equal halves of a twin count once."""
+    rng = np.random.default_rng(n + domain)
+    ids = rng.integers(0, domain, n)
+    begin, length = n // 3, n // 4
+    ids[begin + length:begin + 2 * length:2] = ids[begin:begin + length:2][:len(ids[begin + length:begin + 2 * length:2])]
+    ou, oinv, _ = O.unique_map_bitmap(ids, domain)
+    first = np.ones(n, bool)
+    first[begin + length:begin + 2 * length] = ids[begin + length:begin + 2 * length] != ids[begin:begin + length]
+    for twins, counted in (((0, 0), np.ones(n, bool)), ((begin, length), first)):
+        shared = torch.full((min(n, domain),), 7, dtype=torch.uint8, device=cuda_device)
+        u, inv, cnt = capi.unique_bitmap(torch.from_numpy(ids).to(cuda_device), domain, out_shared=shared, twins=twins)
+        torch.cuda.synchronize()
+        assert cnt.tolist() == [ou.size, 0]
+        assert np.array_equal(u.cpu().numpy()[:ou.size], ou) and np.array_equal(inv.cpu().numpy(), oinv)
+        assert np.array_equal(shared.cpu().numpy()[:ou.size], np.bincount(oinv[counted], minlength=ou.size) > 1)
