@@ -37,6 +37,7 @@ struct LpLayout {
     double* loss_acc; // [1] sum over rows of (lse - pos): zeroed by the prepare kernel, added to by the scores kernels
     float* part;      // [S][Bp][8][2] per-row partial (max, sum) of the logsumexp pass when a row block's tiles are split over CTAs
     float* lse2s;     // [S*C][row_blocks*128] row logsumexp in base-2 units minus the probability scale exponent; 1e30 for rows past the chunk
+    float* o_part;    // f16: [CTAs][2][128][ld] parts of dQ of the (at most two) row blocks a CTA of the query launch shares with others
     int n_items;        // S * C * row_blocks
     float grad_unscale; // factor the scatter kernel applies to what it reads from dQ / dK: 1, or 2^-14 on the tensor path
     size_t bytes;
@@ -50,6 +51,12 @@ struct LpKernelArgs {
 inline size_t lp_align(size_t x) { return (x + 255) & ~(size_t)255; }
 
 inline int lp_row_ld(int D) { return D <= 64 ? 64 : 128; }
+
+// Which of the two fp16 forms a step takes: while dK stays in the L2 beside the operands, adding the row blocks' parts up there is
+// the faster one: 25 000 edges, C N = 50 000, D = 128, two sides (49 MB of dK) 149 us against 156, 50 000 edges and 98 MB 403 against 283.
+inline bool lp_uses_flash(const ge2_lp_desc& d, int S, int64_t CN, int ld) {
+    return d.precision == GE2_PRECISION_F16 && S * CN * ld * 4 > (int64_t)64 << 20;
+}
 
 inline LpLayout lp_make_layout(const ge2_lp_desc& d, void* base) {
     LpLayout L;
@@ -79,6 +86,8 @@ inline LpLayout lp_make_layout(const ge2_lp_desc& d, void* base) {
     const int row_blocks = (L.npc + 127) / 128;
     L.n_items = L.S * d.C * row_blocks;
     size_t olse2 = take((size_t)L.n_items * 128 * 4);
+    size_t oopart = take(lp_uses_flash(d, L.S, L.CN, L.ld) ? (size_t)kNumSMs * 2 * 128 * L.ld * 4 : 0);
+    L.o_part = lp_uses_flash(d, L.S, L.CN, L.ld) ? (float*)(p + oopart) : nullptr;
     L.dQ = (float*)(p + odQ);
     L.dK = (float*)(p + odK);
     L.pos = (float*)(p + opos);
@@ -99,5 +108,7 @@ inline LpLayout lp_make_layout(const ge2_lp_desc& d, void* base) {
 // scores kernels (one per precision); both fill lse, dQ, dK (+ optional score dumps) from Q, K, pos, mask
 int lp_scores_fp32(const LpKernelArgs& a, cudaStream_t stream);
 int lp_scores_f16(const LpKernelArgs& a, cudaStream_t stream);
+int lp_flash_f16(const LpKernelArgs& a, cudaStream_t stream);
+
 
 }  // namespace ge2

@@ -658,7 +658,7 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     }
 
     if (phases & 2) {
-        rc = desc->precision == GE2_PRECISION_F16 ? lp_scores_f16(a, stream) : lp_scores_fp32(a, stream);
+        rc = desc->precision == GE2_PRECISION_FP32 ? lp_scores_fp32(a, stream) : L.o_part != nullptr ? lp_flash_f16(a, stream) : lp_scores_f16(a, stream);
         if (rc != GE2_OK) return rc;
     }
     if (!(phases & 4)) return GE2_OK;

@@ -222,3 +222,18 @@ def test_split_operand_tiles_at_their_edges(capi, cuda_device, kind, B, C, N, D)
     assert abs(got["loss"] - exp["loss"]) <= 2e-6 * abs(exp["loss"])
     for key in ("node_grad", "rel_grad", "inv_rel_grad"):
         assert rel_err(got[key], exp[key]) <= 5e-6, key
+
+
+@pytest.mark.parametrize("kind,B,C,N,D", [("DISTMULT", 130, 1, 66001, 128), ("COMPLEX", 210, 70, 1000, 66), ("DISTMULT", 300, 2, 70001, 50), ("COMPLEX", 1290, 10, 7003, 100)])
+def test_streaming_softmax_tiles_at_their_edges(capi, cuda_device, kind, B, C, N, D):
+    """The fp16 form for a dK that does not stay in the L2: blocks shared by many CTAs, chunks of three rows, one row past a tile; then scores
+    large enough that the reference of a row has to move."""
+    for scale in (1.0, 6.0):
+        case = workloads.make_case(kind, B, C, N, D, 5, 150, N // 2, 77 + D)
+        case.emb *= np.float32(scale)
+        o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
+        got = run_lp_step(capi, case, cuda_device, "f16", "pairs", dump_scores=False)
+        assert got["status"] == 0
+        assert abs(got["loss"] - o.loss) <= 1e-2 * abs(o.loss)
+        for key in ("node_grad", "rel_grad", "inv_rel_grad"):
+            assert rel_err(got[key], getattr(o, key)) <= 1e-2, key
