@@ -209,7 +209,9 @@ __global__ void __launch_bounds__(kPairThreads) selected_scores_backward_kernel(
 // A CTA keeps a tile of query rows and takes a contiguous share of all (chunk, row tile, group) triples, so every SM is busy to the end and a
 // share begins and ends on a group boundary.  Warps by role: 8 warps convert rows (fp32, read along the row) into one of two tile
 // buffers, one issues the contractions, 4 epilogue warps walk the scores: a thread owns a row, keeps the running winner of the group
-// in registers and writes it where the group ends.  Groups need not fit tiles.
+// in registers and writes it where the group ends.  Groups of less than eight end so often that their winners are put aside first, and 17 ... 32
+// of the warp's 32 rows leave together, a row at a time (groups of one, 33 000 x 1000 winners: 591 us written one by one, each to a sector
+// of its own, 178 us together; groups of ten are faster one by one).  Groups need not fit tiles.
 // Bound by the contractions (6 ceil(D / 16) steps of 48 cycles a tile at best, 92 beside the conversion's shared-memory stores) and the
 // one epilogue warp a scheduler.  50 000 rows x 1 000 negatives, D = 100, 100 kept: 122 us (405 us as fp32 multiply-adds).
 using namespace tc;
@@ -231,7 +233,8 @@ template <int NB>
 struct TourSmem {
     static constexpr int kQBlock = kTourRows * 128, kYBlock = kTourCols * 128;
     static constexpr int kQPlane = NB * kQBlock, kYPlane = NB * kYBlock;
-    static constexpr int kQ = 0, kY = kTourPlanes * kQPlane, kMisc = kY + 2 * kTourPlanes * kYPlane;
+    static constexpr int kQ = 0, kY = kTourPlanes * kQPlane, kStage = kY + 2 * kTourPlanes * kYPlane;
+    static constexpr int kMisc = kStage + 4 * 32 * 33 * 8;  // winners put aside: per epilogue warp [32 rows][33] scores, then columns
     static constexpr int kBytes = (kMisc + 256 + 1024) > 120 * 1024 ? (kMisc + 256 + 1024) : 120 * 1024;  // one CTA an SM
 };
 enum TourBar { kTQFull = 0, kTQEmpty, kTYFull, kTYEmpty = kTYFull + 2, kTSFull = kTYEmpty + 2, kTSEmpty = kTSFull + 2, kTourBars = kTSEmpty + 2 };
@@ -275,7 +278,7 @@ __device__ __forceinline__ bool tour_segment(const TourArgs& a, int64_t at, int6
     return true;
 }
 
-template <int NB, int VEC>
+template <int NB, int VEC, bool STAGED>
 __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __grid_constant__ TourArgs a) {
     using SM = TourSmem<NB>;
     extern __shared__ unsigned char tour_raw[];
@@ -383,14 +386,30 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
     } else if (warp < kTourEpi0 + 4) {
         // ---- winners: thread = row; columns in order, the running winner of the group in registers ----
         const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;
+        float* const st_s = reinterpret_cast<float*>(smem + SM::kStage) + warp * (32 * 33 * 2);
+        int* const st_c = reinterpret_cast<int*>(st_s) + 32 * 33;
         uint32_t tiles = 0;
         TourSegment sg;
         bool ok = true;
         for (int64_t at = begin, next = 0; ok && tour_segment(a, at, end, sg, next); at = next) {
-            const bool live = sg.row0 + tid < a.R;
-            const int64_t first = (sg.chunk * a.R + sg.row0 + tid) * a.K + sg.group;
-            float* out_s = a.out_scores + first;
-            int64_t* out_i = a.out_idx + first;
+            const int rows = (int)(a.R - sg.row0 - warp * 32 < 32 ? a.R - sg.row0 - warp * 32 : 32);  // of this warp
+            const int64_t first = (sg.chunk * a.R + sg.row0 + warp * 32) * a.K + sg.group;
+            float* out_s = a.out_scores + first + lane * a.K;
+            int64_t* out_i = a.out_idx + first + lane * a.K;
+            int cnt = 0, done = 0;  // winners put aside, and written
+            auto flush = [&]() {
+                __syncwarp();
+#pragma unroll 4
+                for (int r = 0; r < rows; r++) {
+                    if (lane < cnt) {
+                        a.out_scores[first + r * a.K + done + lane] = st_s[r * 33 + lane];
+                        a.out_idx[first + r * a.K + done + lane] = sg.col + st_c[r * 33 + lane];
+                    }
+                }
+                __syncwarp();
+                done += cnt;
+                cnt = 0;
+            };
             const int T = (int)a.T;
             int todo = (int)((sg.col_end - sg.col) / a.T);  // groups of this segment still to be written; columns are counted from its first
             float best = -CUDART_INF_F;
@@ -417,20 +436,31 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
                         best_c = v[j] > best ? col0 + j : best_c;  // the first of equal scores wins, a NaN never
                         best = fmaxf(best, v[j]);
                         const bool end = left == j + 1;            // the same for all threads
-                        if (end && live && todo > 0) {
-                            *out_s = best;
-                            *out_i = sg.col + best_c;
+                        const bool put = end && todo > 0;
+                        if (STAGED) {
+                            if (put) {
+                                st_s[lane * 33 + cnt] = best;
+                                st_c[lane * 33 + cnt] = best_c;
+                            }
+                            cnt += put ? 1 : 0;
+                        } else {
+                            if (put && lane < rows) {
+                                *out_s = best;
+                                *out_i = sg.col + best_c;
+                            }
+                            out_s += end ? 1 : 0;
+                            out_i += end ? 1 : 0;
                         }
-                        out_s += end ? 1 : 0;
-                        out_i += end ? 1 : 0;
                         todo -= end ? 1 : 0;
                         best = end ? -CUDART_INF_F : best;
                         best_c = end ? col0 + j + 1 : best_c;
                         left += end ? T : 0;
                     }
                     left -= 16;
+                    if (STAGED && cnt > 16) flush();
                 }
             }
+            if (STAGED && ok) flush();
         }
     }
     // ---- common exit ----
@@ -445,8 +475,9 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
 template <int NB, int VEC>
 int launch_tournament(const TourArgs& a, cudaStream_t stream) {
     // per-device function attribute; setting it on every call keeps multi-device processes correct and is not a stream operation
-    GE2_CUDA_TRY(cudaFuncSetAttribute(tournament_kernel<NB, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, TourSmem<NB>::kBytes));
-    tournament_kernel<NB, VEC><<<(unsigned)std::min<int64_t>(kNumSMs, a.shares_total), kTourThreads, TourSmem<NB>::kBytes, stream>>>(a);
+    auto kernel = a.T < 8 ? tournament_kernel<NB, VEC, true> : tournament_kernel<NB, VEC, false>;
+    GE2_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TourSmem<NB>::kBytes));
+    kernel<<<(unsigned)std::min<int64_t>(kNumSMs, a.shares_total), kTourThreads, TourSmem<NB>::kBytes, stream>>>(a);
     GE2_LAUNCH_CHECK();
     return GE2_OK;
 }
