@@ -25,6 +25,7 @@ EXPORTS = [
     "ge2_enable_peer_access", "ge2_build_state_edges", "ge2_swap_begin", "ge2_swap_wait", "ge2_sample_batch_dev",
     "ge2_eval_workspace_bytes", "ge2_eval_ranks", "ge2_selected_neg_scores", "ge2_selected_neg_scores_backward",
     "ge2_tournament_select", "ge2_unique_bitmap_shared", "ge2_adagrad_scatter_shared", "ge2_train_step",
+    "ge2_selected_neg_backward_workspace_bytes", "ge2_selected_neg_scores_backward_ws",
 ]
 
 
@@ -134,6 +135,9 @@ def load_library():
                                             C.c_void_p, C.c_void_p, C.c_void_p]
     lib.ge2_selected_neg_scores_backward.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64,
                                                      C.c_int64, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.ge2_selected_neg_scores_backward_ws.argtypes = lib.ge2_selected_neg_scores_backward.argtypes[:-1] + [C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.ge2_selected_neg_backward_workspace_bytes.restype = C.c_size_t
+    lib.ge2_selected_neg_backward_workspace_bytes.argtypes = [C.c_int, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int]
     lib.ge2_tournament_select.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int,
                                           C.c_void_p, C.c_void_p, C.c_void_p]
     lib.ge2_eval_workspace_bytes.restype = C.c_size_t
@@ -416,9 +420,12 @@ def selected_neg_scores_backward(kind, grad_out, chunked, negatives, selected, s
     chunks, rows, N, K, D = _selected_shapes(chunked, negatives, selected)
     assert tuple(grad_out.shape) == (chunks * rows, K) and grad_out.is_contiguous()
     grad_chunked, grad_negatives = torch.empty_like(chunked), torch.empty_like(negatives)
-    check(load_library().ge2_selected_neg_scores_backward(SELECTED_KINDS[kind], ptr(grad_out), ptr(chunked), ptr(negatives), ptr(selected),
-                                                          chunks, rows, N, K, D, ptr(grad_chunked), ptr(grad_negatives), ptr(status),
-                                                          cur_stream()), "ge2_selected_neg_scores_backward")
+    lib = load_library()
+    need = lib.ge2_selected_neg_backward_workspace_bytes(SELECTED_KINDS[kind], chunks, rows, N, K, D)
+    ws = torch.empty(need, dtype=torch.uint8, device=chunked.device) if need else None
+    check(lib.ge2_selected_neg_scores_backward_ws(SELECTED_KINDS[kind], ptr(grad_out), ptr(chunked), ptr(negatives), ptr(selected), chunks, rows, N, K,
+                                                  D, ptr(grad_chunked), ptr(grad_negatives), ptr(status), ptr(ws), need, cur_stream()),
+          "ge2_selected_neg_scores_backward")
     return grad_chunked, grad_negatives
 
 

@@ -200,6 +200,348 @@ __global__ void __launch_bounds__(kPairThreads) selected_scores_backward_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------
+// the same with the rows that are gathered in shared memory
+// ---------------------------------------------------------------------------------------------------------------------------
+// A pair moves 4 D bytes; from L2 that is what bounds the kernels above (2 GB at 50 000 rows x 100 pairs, D = 100: 282 us forward, and 495 us
+// backward, where every pair also sends 4 D bytes of reductions).  Here a CTA keeps what its pairs gather in shared memory:
+//   scores, query gradient (pair_rows_kernel): the negatives of a chunk, in as many slices of the columns as they need to fit; the CTA's
+//     rows are gone through once a slice
+//   negative gradient (pair_columns_kernel): a block of query rows; its pairs are sorted by negative first (counting sort), so that a
+//     negative's sum stays in registers and reaches L2 once a block instead of once a pair
+// Eight lanes take a pair, 16 bytes a lane and load, four pairs a warp side by side: conflict-free whatever the pairs, and the sums of 32
+// pairs fold in 7 shuffles.  Bound by shared memory (4 cycles a pair at D = 100) and the issue slots beside it (70 - 78 % of
+// its cycles in use): 50 000 rows x 100 pairs, D = 100: 146 us forward, 127 + 180 us backward.
+constexpr int kRowsThreads = 1024, kRowsWarps = kRowsThreads / 32;
+constexpr int kPairSmem = 208 * 1024;
+enum PairMode { kPairScores = 0, kPairCoeffs = 1, kPairQueryGrad = 2 };
+
+// four columns from column c of a row of D floats, zeros past it
+__device__ __forceinline__ float4 row_piece(const float* __restrict__ row, int c, int D, bool vec) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (vec) {
+        if (c < D) v = __ldg(reinterpret_cast<const float4*>(row + c));
+    } else {
+        if (c < D) v.x = __ldg(row + c);
+        if (c + 1 < D) v.y = __ldg(row + c + 1);
+        if (c + 2 < D) v.z = __ldg(row + c + 2);
+        if (c + 3 < D) v.w = __ldg(row + c + 3);
+    }
+    return v;
+}
+
+// mode scores: out = score of every pair.  coeffs (L2): out = grad / |q - n| (0 where the reference's gradient is).  query gradient:
+// out[row] = sum_k w n (dot) or w (q - n) (L2), w = the pairs' weights (grad, or the coefficients).
+// L: 16-byte pieces a lane has of a slice (W4 pieces wide, ns slices)
+template <int L, int KIND, int MODE>
+__global__ void __launch_bounds__(kRowsThreads, 1) pair_rows_kernel(PairArgs a, int ns, int W4, int cpc, int vec, const float* __restrict__ weights,
+                                                                    float* __restrict__ out) {
+    extern __shared__ __align__(16) float4 pr_tile[];  // [N][W4], then a row of zeros for pairs that do not exist
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, jl = lane & 7, g = lane >> 3;
+    const int64_t c = blockIdx.x / cpc;
+    const int part = (int)(blockIdx.x - c * cpc), N = (int)a.N, D = a.D, K = (int)a.K;
+    const int64_t r_begin = a.R * part / cpc, r_end = a.R * (part + 1) / cpc;
+    const float* negs = a.negatives + c * a.N * D;
+    const uint32_t tile = (uint32_t)__cvta_generic_to_shared(pr_tile) + jl * 16;
+    for (int s = 0; s < ns; s++) {
+        __syncthreads();
+#pragma unroll 4
+        for (int i = threadIdx.x; i < N * W4; i += kRowsThreads) {
+            const int j = (int)((uint32_t)i / (uint32_t)W4);
+            pr_tile[i] = row_piece(negs + (int64_t)j * D, (s * W4 + i - j * W4) * 4, D, vec);
+        }
+        for (int i = threadIdx.x; i < W4; i += kRowsThreads) pr_tile[N * W4 + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+        for (int64_t r = r_begin + warp; r < r_end; r += kRowsWarps) {
+            const int64_t row = c * a.R + r;
+            const int64_t* sel = a.selected + row * a.K;
+            float4 q[L], acc[L];
+#pragma unroll
+            for (int l = 0; l < L; l++) {
+                acc[l] = make_float4(0.f, 0.f, 0.f, 0.f);
+                q[l] = jl + 8 * l < W4 && (KIND == GE2_SELECTED_L2 || MODE != kPairQueryGrad) ? row_piece(a.chunked + row * D, (s * W4 + jl + 8 * l) * 4, D, vec) : acc[l];
+            }
+            // column and weight of pair k0 + lane; those of the next 32 pairs are on their way meanwhile
+            int64_t next = -2;
+            float next_w = 0.f;
+            auto fetch = [&](int k) {
+                next = -2;
+                next_w = 0.f;
+                if (k + lane < K) {
+                    next = __ldg(sel + k + lane);
+                    if (MODE == kPairQueryGrad) next_w = __ldg(weights + row * a.K + k + lane);
+                }
+            };
+            fetch(0);
+#pragma unroll 1
+            for (int k0 = 0; k0 < K; k0 += 32) {
+                int idx = N;
+                const float w = next_w;
+                if (next >= 0 && next < N) idx = (int)next;
+                else if (next != -2 && s == 0) or_status(a.status, GE2_STATUS_BAD_INDEX);
+                const int at0 = idx * (W4 * 16);
+                fetch(k0 + 32);
+                float val[8];
+                auto turn = [&](int i) {
+                    const uint32_t n = tile + __shfl_sync(0xffffffffu, at0, 4 * i + g);
+                    const float wp = MODE == kPairQueryGrad ? __shfl_sync(0xffffffffu, w, 4 * i + g) : 0.f;
+                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int l = 0; l < L; l++) {
+                        float4 x = q[l];  // (past the slice: a difference of zero, or zero)
+                        if (l + 1 < L || jl + 8 * l < W4) asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(n + l * 128));
+                        if (MODE == kPairQueryGrad) {
+                            if (KIND == GE2_SELECTED_L2) x = make_float4(q[l].x - x.x, q[l].y - x.y, q[l].z - x.z, q[l].w - x.w);
+                            acc[l].x = fmaf(wp, x.x, acc[l].x), acc[l].y = fmaf(wp, x.y, acc[l].y);
+                            acc[l].z = fmaf(wp, x.z, acc[l].z), acc[l].w = fmaf(wp, x.w, acc[l].w);
+                        } else if (KIND == GE2_SELECTED_DOT) {
+                            sum.x = fmaf(q[l].x, x.x, sum.x), sum.y = fmaf(q[l].y, x.y, sum.y), sum.z = fmaf(q[l].z, x.z, sum.z), sum.w = fmaf(q[l].w, x.w, sum.w);
+                        } else {
+                            const float dx = q[l].x - x.x, dy = q[l].y - x.y, dz = q[l].z - x.z, dw = q[l].w - x.w;
+                            sum.x = fmaf(dx, dx, sum.x), sum.y = fmaf(dy, dy, sum.y), sum.z = fmaf(dz, dz, sum.z), sum.w = fmaf(dw, dw, sum.w);
+                        }
+                    }
+                    val[i] = (sum.x + sum.y) + (sum.z + sum.w);
+                };
+                if (K - k0 > 28) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++) turn(i);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        val[i] = 0.f;
+                        if (k0 + 4 * i < K) turn(i);  // warp-uniform
+                    }
+                }
+                if (MODE != kPairQueryGrad) {
+                    // lane jl of a group ends up with the sum of the group's pair of turn jl
+#pragma unroll
+                    for (int h = 4; h > 0; h >>= 1) {
+#pragma unroll
+                        for (int i = 0; i < h; i++) {
+                            const bool up = (jl & h) != 0;
+                            const float keep = up ? val[i + h] : val[i], send = up ? val[i] : val[i + h];
+                            val[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+                        }
+                    }
+                    const int p = 4 * jl + g;
+                    const bool there = __shfl_sync(0xffffffffu, idx, p) < N;
+                    if (k0 + p < K) {
+                        float* at = out + row * a.K + k0 + p;
+                        float sum = val[0];
+                        if (s > 0) sum += *at;
+                        if (s == ns - 1) {
+                            if (MODE == kPairScores) sum = there ? finish_score<KIND>(sum) : 0.f;
+                            else sum = there && sum > kL2Floor ? __ldg(weights + row * a.K + k0 + p) / sqrtf(sum) : 0.f;
+                        }
+                        *at = sum;
+                    }
+                }
+            }
+            if (MODE == kPairQueryGrad) {
+#pragma unroll
+                for (int l = 0; l < L; l++) {
+#pragma unroll
+                    for (int o = 8; o < 32; o <<= 1) {
+                        acc[l].x += __shfl_xor_sync(0xffffffffu, acc[l].x, o), acc[l].y += __shfl_xor_sync(0xffffffffu, acc[l].y, o);
+                        acc[l].z += __shfl_xor_sync(0xffffffffu, acc[l].z, o), acc[l].w += __shfl_xor_sync(0xffffffffu, acc[l].w, o);
+                    }
+                    const int col = (s * W4 + jl + 8 * l) * 4;
+                    if (g == 0 && jl + 8 * l < W4 && col < D) {
+                        float* at = out + row * D + col;
+                        if (vec) {
+                            *reinterpret_cast<float4*>(at) = acc[l];
+                        } else {
+                            at[0] = acc[l].x;
+                            if (col + 1 < D) at[1] = acc[l].y;
+                            if (col + 2 < D) at[2] = acc[l].z;
+                            if (col + 3 < D) at[3] = acc[l].w;
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+// out[n] += sum over the block's pairs of negative n of w q (dot) or -w (q - n) (L2)
+template <int L, int KIND>
+__global__ void __launch_bounds__(kRowsThreads, 1) pair_columns_kernel(PairArgs a, int cpc, int vec, const float* __restrict__ weights, float2* __restrict__ sorted,
+                                                                       float* __restrict__ out) {
+    extern __shared__ __align__(16) float4 pc_rows[];  // [rows of the block and a row of zeros][D4], then the counters [N]
+    __shared__ int s_warp[kRowsWarps], s_base;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, jl = lane & 7, g = lane >> 3;
+    const int64_t c = blockIdx.x / cpc;
+    const int part = (int)(blockIdx.x - c * cpc), N = (int)a.N, D = a.D, D4 = (D + 3) >> 2;
+    const int64_t r_begin = a.R * part / cpc;
+    const int rows = (int)(a.R * (part + 1) / cpc - r_begin);
+    const int64_t row0 = c * a.R + r_begin;
+    int* count = reinterpret_cast<int*>(pc_rows + (a.R / cpc + 2) * D4);
+    for (int j = tid; j < N; j += kRowsThreads) count[j] = 0;
+    if (tid == 0) s_base = 0;
+#pragma unroll 4
+    for (int i = tid; i < rows * D4; i += kRowsThreads) {
+        const int r = (int)((uint32_t)i / (uint32_t)D4);
+        pc_rows[i] = row_piece(a.chunked + (row0 + r) * D, (i - r * D4) * 4, D, vec);
+    }
+    for (int i = tid; i < D4; i += kRowsThreads) pc_rows[rows * D4 + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    // counting sort of the block's pairs by negative
+    const int64_t p0 = row0 * a.K;
+    const int pairs = rows * (int)a.K;
+#pragma unroll 4
+    for (int i = tid; i < pairs; i += kRowsThreads) {
+        const int64_t j = __ldg(a.selected + p0 + i);
+        if (j >= 0 && j < a.N) atomicAdd(&count[j], 1);
+    }
+    __syncthreads();
+    for (int b = 0; b < N; b += kRowsThreads) {  // exclusive scan of the counters, in place
+        const int own = b + tid < N ? count[b + tid] : 0;
+        int incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        int before = s_base;
+        for (int w = 0; w < warp; w++) before += s_warp[w];
+        if (b + tid < N) count[b + tid] = before + incl - own;
+        __syncthreads();
+        if (tid == kRowsThreads - 1) s_base = before + incl;
+        __syncthreads();
+    }
+    float2* mine = sorted + p0;  // (weight, row of the block)
+#pragma unroll 4
+    for (int i = tid; i < pairs; i += kRowsThreads) {
+        const int64_t j = __ldg(a.selected + p0 + i);
+        if (j >= 0 && j < a.N) mine[atomicAdd(&count[j], 1)] = make_float2(__ldg(weights + p0 + i), __int_as_float((int)((uint32_t)i / (uint32_t)a.K) * D4));
+    }
+    __syncthreads();  // (also orders the block's own global writes before the reads below)
+    // count[j] is now the end of negative j's pairs, count[j - 1] their begin
+    for (int j = warp; j < N; j += kRowsWarps) {
+        const int begin = j == 0 ? 0 : count[j - 1], end = count[j];
+        if (begin == end) continue;
+        float4 acc[L], nv[L];
+#pragma unroll
+        for (int l = 0; l < L; l++) {
+            acc[l] = make_float4(0.f, 0.f, 0.f, 0.f);
+            nv[l] = KIND == GE2_SELECTED_L2 && jl + 8 * l < D4 ? row_piece(a.negatives + (c * a.N + j) * D, (jl + 8 * l) * 4, D, vec) : acc[l];
+        }
+#pragma unroll 1
+        for (int k0 = begin; k0 < end; k0 += 32) {
+            float2 e = make_float2(0.f, __int_as_float(rows * D4));
+            if (k0 + lane < end) e = __ldcg(mine + k0 + lane);
+            auto turn = [&](int i) {
+                const float w = __shfl_sync(0xffffffffu, e.x, 4 * i + g);
+                const float4* q = pc_rows + __float_as_int(__shfl_sync(0xffffffffu, e.y, 4 * i + g)) + jl;
+#pragma unroll
+                for (int l = 0; l < L; l++) {
+                    float4 x = nv[l];  // (past the row: a difference of zero, or zero)
+                    if (l + 1 < L || jl + 8 * l < D4) x = q[8 * l];
+                    if (KIND == GE2_SELECTED_L2) x = make_float4(nv[l].x - x.x, nv[l].y - x.y, nv[l].z - x.z, nv[l].w - x.w);
+                    acc[l].x = fmaf(w, x.x, acc[l].x), acc[l].y = fmaf(w, x.y, acc[l].y);
+                    acc[l].z = fmaf(w, x.z, acc[l].z), acc[l].w = fmaf(w, x.w, acc[l].w);
+                }
+            };
+            if (end - k0 > 28) {
+#pragma unroll 4
+                for (int i = 0; i < 8; i++) turn(i);
+            } else {
+#pragma unroll 1
+                for (int i = 0; k0 + 4 * i < end; i++) turn(i);
+            }
+        }
+        // the four groups' sums; group l then sends piece jl + 8 l
+        float4 send = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int l = 0; l < L; l++) {
+#pragma unroll
+            for (int o = 8; o < 32; o <<= 1) {
+                acc[l].x += __shfl_xor_sync(0xffffffffu, acc[l].x, o), acc[l].y += __shfl_xor_sync(0xffffffffu, acc[l].y, o);
+                acc[l].z += __shfl_xor_sync(0xffffffffu, acc[l].z, o), acc[l].w += __shfl_xor_sync(0xffffffffu, acc[l].w, o);
+            }
+            if (g == l) send = acc[l];
+        }
+        const int col = (jl + 8 * g) * 4;
+        if (g < L && col < D) {
+            float* at = out + (c * a.N + j) * D + col;
+            if (vec) {
+                atomicAdd(reinterpret_cast<float4*>(at), send);
+            } else {
+                atomicAdd(at, send.x);
+                if (col + 1 < D) atomicAdd(at + 1, send.y);
+                if (col + 2 < D) atomicAdd(at + 2, send.z);
+                if (col + 3 < D) atomicAdd(at + 3, send.w);
+            }
+        }
+    }
+}
+
+// How a problem is cut for the kernels above; usable == false: the rows are gathered from L2.
+struct PairCut {
+    bool usable;
+    int ns, W4, L;      // slices of the negatives
+    int cpc, cpc_rows;  // CTAs a chunk: negatives resident, query rows resident
+    int L_rows;
+};
+inline PairCut pair_cut(const PairArgs& a) {
+    PairCut p = {};
+    const int64_t chunks = a.R > 0 ? a.rows / a.R : 0;
+    const int D4 = (a.D + 3) / 4;
+    const int64_t w4 = a.N > 0 ? kPairSmem / (16 * (a.N + 1)) : 0;
+    // Filling shared memory costs every CTA its chunk's negatives once (4 N D bytes); it pays when the CTA's pairs gather several times
+    // that.  A slice narrower than four pieces would leave most lanes idle, and a block's pairs are counted in 31 bits.
+    if (chunks < 1 || a.K < 1 || w4 < 4 || chunks > 65535 || a.K > (1 << 20) || a.R > (1 << 24)) return p;
+    p.ns = (int)ceil_div<int64_t>(D4, w4);
+    p.W4 = ceil_div(D4, p.ns);
+    p.L = ceil_div(p.W4, 8);
+    p.cpc = (int)std::max<int64_t>(1, std::min<int64_t>(kNumSMs / chunks, a.R));
+    const int64_t most_rows = (kPairSmem - 4 * a.N) / (16 * D4) - 2;
+    p.cpc_rows = (int)std::max<int64_t>(p.cpc, ceil_div<int64_t>(a.R, most_rows));
+    p.L_rows = ceil_div(D4, 8);
+    const int64_t per_cta = ceil_div<int64_t>(a.R, p.cpc) * a.K;
+    p.usable = per_cta >= 4 * a.N && per_cta < (1 << 30);
+    return p;
+}
+
+template <int KIND, int MODE>
+int launch_pair_rows(const PairArgs& a, const PairCut& p, bool vec, const float* weights, float* out, cudaStream_t stream) {
+    const size_t smem = (size_t)(a.N + 1) * p.W4 * 16;
+    const dim3 grid((unsigned)(a.rows / a.R * p.cpc));
+    auto go = [&](auto kernel) {
+        GE2_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
+        kernel<<<grid, kRowsThreads, smem, stream>>>(a, p.ns, p.W4, p.cpc, vec ? 1 : 0, weights, out);
+        GE2_LAUNCH_CHECK();
+        return GE2_OK;
+    };
+    switch (p.L) {
+        case 1: return go(pair_rows_kernel<1, KIND, MODE>);
+        case 2: return go(pair_rows_kernel<2, KIND, MODE>);
+        case 3: return go(pair_rows_kernel<3, KIND, MODE>);
+        default: return go(pair_rows_kernel<4, KIND, MODE>);
+    }
+}
+
+template <int KIND>
+int launch_pair_columns(const PairArgs& a, const PairCut& p, bool vec, const float* weights, float2* sorted, float* out, cudaStream_t stream) {
+    const size_t smem = (size_t)(a.R / p.cpc_rows + 2) * ((a.D + 3) / 4) * 16 + (size_t)a.N * 4;
+    const dim3 grid((unsigned)(a.rows / a.R * p.cpc_rows));
+    auto go = [&](auto kernel) {
+        GE2_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
+        kernel<<<grid, kRowsThreads, smem, stream>>>(a, p.cpc_rows, vec ? 1 : 0, weights, sorted, out);
+        GE2_LAUNCH_CHECK();
+        return GE2_OK;
+    };
+    switch (p.L_rows) {
+        case 1: return go(pair_columns_kernel<1, KIND>);
+        case 2: return go(pair_columns_kernel<2, KIND>);
+        case 3: return go(pair_columns_kernel<3, KIND>);
+        default: return go(pair_columns_kernel<4, KIND>);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------
 // tournament selection
 // ---------------------------------------------------------------------------------------------------------------------------
 // Scores are contracted on the tensor cores: both operands are split exactly into three bf16 terms in shared memory (x = xh + xm + xl) and
@@ -527,6 +869,10 @@ extern "C" int ge2_selected_neg_scores(int kind, const float* chunked, const flo
     if (out_scores == nullptr) return GE2_ERR_INVALID_ARGUMENT;
     const PairArgs a = pair_args(kind, chunked, negatives, selected, chunks, rows_per_chunk, num_negs, num_selected, D, status);
     const bool vec = rows_are_vectors(D, chunked, negatives, nullptr, nullptr);
+    const PairCut cut = pair_cut(a);
+    if (cut.usable)
+        return kind == GE2_SELECTED_DOT ? launch_pair_rows<GE2_SELECTED_DOT, kPairScores>(a, cut, vec, nullptr, out_scores, as_stream(stream_))
+                                        : launch_pair_rows<GE2_SELECTED_L2, kPairScores>(a, cut, vec, nullptr, out_scores, as_stream(stream_));
     const dim3 grid((unsigned)stream_grid(rows, kPairWarps));
     cudaStream_t stream = as_stream(stream_);
     if (kind == GE2_SELECTED_DOT) {
@@ -543,7 +889,22 @@ extern "C" int ge2_selected_neg_scores(int kind, const float* chunked, const flo
 extern "C" int ge2_selected_neg_scores_backward(int kind, const float* grad_out, const float* chunked, const float* negatives,
                                                 const int64_t* selected, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs,
                                                 int64_t num_selected, int D, float* grad_chunked, float* grad_negatives, int32_t* status,
-                                                ge2_stream_t stream_) {
+                                                ge2_stream_t stream) {
+    return ge2_selected_neg_scores_backward_ws(kind, grad_out, chunked, negatives, selected, chunks, rows_per_chunk, num_negs, num_selected, D,
+                                               grad_chunked, grad_negatives, status, nullptr, 0, stream);
+}
+
+extern "C" size_t ge2_selected_neg_backward_workspace_bytes(int kind, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs, int64_t num_selected, int D) {
+    if (chunks <= 0 || rows_per_chunk <= 0 || num_negs <= 0 || num_selected <= 0 || D <= 0 || D > kMaxD) return 0;
+    const PairArgs a = pair_args(kind, nullptr, nullptr, nullptr, chunks, rows_per_chunk, num_negs, num_selected, D, nullptr);
+    if (!pair_cut(a).usable) return 0;
+    return (size_t)(a.rows * a.K) * (kind == GE2_SELECTED_L2 ? 12 : 8);  // sorted (weight, row) pairs; L2: the weights themselves too
+}
+
+extern "C" int ge2_selected_neg_scores_backward_ws(int kind, const float* grad_out, const float* chunked, const float* negatives,
+                                                   const int64_t* selected, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs,
+                                                   int64_t num_selected, int D, float* grad_chunked, float* grad_negatives, int32_t* status,
+                                                   void* workspace, size_t workspace_bytes, ge2_stream_t stream_) {
     const int rc = check_pairs(kind, chunked, negatives, selected, chunks, rows_per_chunk, num_negs, num_selected, D);
     if (rc != GE2_OK) return rc;
     const int64_t rows = chunks * rows_per_chunk;
@@ -557,6 +918,19 @@ extern "C" int ge2_selected_neg_scores_backward(int kind, const float* grad_out,
     // with nothing selected the kernel still writes the zero query gradient
     const PairArgs a = pair_args(kind, chunked, negatives, selected, chunks, rows_per_chunk, num_negs, num_selected, D, status);
     const bool vec = rows_are_vectors(D, chunked, negatives, grad_chunked, grad_negatives);
+    const size_t need = ge2_selected_neg_backward_workspace_bytes(kind, chunks, rows_per_chunk, num_negs, num_selected, D);
+    if (need > 0 && workspace != nullptr && workspace_bytes >= need && ((uintptr_t)workspace & 7) == 0) {
+        const PairCut cut = pair_cut(a);
+        float2* sorted = reinterpret_cast<float2*>(workspace);
+        float* coeffs = reinterpret_cast<float*>(sorted + rows * num_selected);
+        if (kind == GE2_SELECTED_DOT) {
+            const int rc2 = launch_pair_rows<GE2_SELECTED_DOT, kPairQueryGrad>(a, cut, vec, grad_out, grad_chunked, stream);
+            return rc2 != GE2_OK ? rc2 : launch_pair_columns<GE2_SELECTED_DOT>(a, cut, vec, grad_out, sorted, grad_negatives, stream);
+        }
+        int rc2 = launch_pair_rows<GE2_SELECTED_L2, kPairCoeffs>(a, cut, vec, grad_out, coeffs, stream);
+        if (rc2 == GE2_OK) rc2 = launch_pair_rows<GE2_SELECTED_L2, kPairQueryGrad>(a, cut, vec, coeffs, grad_chunked, stream);
+        return rc2 != GE2_OK ? rc2 : launch_pair_columns<GE2_SELECTED_L2>(a, cut, vec, coeffs, sorted, grad_negatives, stream);
+    }
     const dim3 grid((unsigned)stream_grid(rows, kPairWarps));
     if (kind == GE2_SELECTED_DOT) {
         if (vec) selected_scores_backward_kernel<true, GE2_SELECTED_DOT><<<grid, kPairThreads, 0, stream>>>(a, grad_out, grad_chunked, grad_negatives);

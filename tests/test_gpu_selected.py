@@ -46,6 +46,29 @@ def test_selected_scores_forward_and_backward(capi, cuda_device, C, R, N, D, K, 
     assert int(status.item()) == 0
 
 
+@pytest.mark.parametrize("C,R,N,D,K", [
+    (100, 9, 7, 128, 5), (80, 33, 130, 101, 17), (74, 70, 1664, 128, 200),  # one slice; a ragged row; four slices of the negatives
+    (149, 3, 5, 1, 33), (60, 100, 3300, 18, 300), (3, 700, 64, 50, 100),    # more chunks than SMs; the narrowest slice; many CTAs a chunk
+])
+@pytest.mark.parametrize("kind,code", [("DOT", O.SELECTED_DOT), ("L2", O.SELECTED_L2)])
+def test_rows_resident_in_shared_memory(capi, cuda_device, C, R, N, D, K, kind, code):
+    assert capi.load_library().ge2_selected_neg_backward_workspace_bytes(code, C, R, N, K, D) > 0  # this form is the one taken
+    rng = np.random.default_rng(N + D)
+    q, n, sel = _pairs(rng, C, R, N, D, K)
+    grad = rng.standard_normal((C * R, K)).astype(np.float32)
+    sel[C - 1, R * K - 1], grad[C * R - 1, K - 1] = 0, 0.0
+    exp_s, (exp_dq, exp_dn) = O.selected_neg_scores(q, n, sel, code), O.selected_neg_scores_backward(grad, q, n, sel, code)
+    sel[C - 1, R * K - 1] = N  # the last pair does not exist
+    exp_s[C * R - 1, K - 1] = 0.0
+    t = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
+    status = torch.zeros(1, dtype=torch.int32, device=cuda_device)
+    _close(capi.selected_neg_scores(kind, t(q), t(n), t(sel), status), exp_s)
+    assert int(status.item()) == 8
+    dq, dn = capi.selected_neg_scores_backward(kind, t(grad), t(q), t(n), t(sel), status)
+    _close(dq, exp_dq)
+    _close(dn, exp_dn)
+
+
 def test_selected_column_out_of_range_is_reported_and_skipped(capi, cuda_device):
     rng = np.random.default_rng(3)
     C, R, N, D, K = 2, 20, 30, 40, 4
