@@ -83,7 +83,7 @@ PYBIND11_MODULE(ge2_host, m) {
         .def_readwrite("batch_id", &DataLoader::batch_id_);
     py::class_<InMemory, std::shared_ptr<InMemory>>(m, "InMemory")
         .def(py::init<torch::Tensor>())
-        .def("indexRead", &InMemory::indexRead)
+        .def("indexRead", [](InMemory& s, torch::Tensor indices) { return s.indexRead(indices); })
         .def("indexAdd", &InMemory::indexAdd)
         .def("checkStatus", &InMemory::checkStatus)
         .def_readwrite("data", &InMemory::data_);

@@ -205,10 +205,13 @@ std::tuple<torch::Tensor, torch::Tensor> selected_neg_scores_cuda_backward(torch
     auto grad = grad_out.contiguous().to(torch::kFloat32);
     auto chunked = chunked_adjusted_embeddings.contiguous(), negatives = negative_embeddings.contiguous(), selected = selected_neg_indices.contiguous();
     auto grad_chunked = torch::empty_like(chunked), grad_negatives = torch::empty_like(negatives);  // the call zeroes grad_negatives
-    check(ge2_selected_neg_scores_backward((int)score_kind, grad.data_ptr<float>(), chunked.data_ptr<float>(), negatives.data_ptr<float>(),
-                                           selected.data_ptr<int64_t>(), s.chunks, s.rows, s.negs, s.selected, s.D, grad_chunked.data_ptr<float>(),
-                                           grad_negatives.data_ptr<float>(), selected_status_word(chunked.device()).data_ptr<int32_t>(),
-                                           current_stream(chunked)),
+    const size_t need = ge2_selected_neg_backward_workspace_bytes((int)score_kind, s.chunks, s.rows, s.negs, s.selected, s.D);
+    torch::Tensor ws;
+    if (need > 0) ws = torch::empty({(int64_t)need}, chunked.options().dtype(torch::kUInt8));
+    check(ge2_selected_neg_scores_backward_ws((int)score_kind, grad.data_ptr<float>(), chunked.data_ptr<float>(), negatives.data_ptr<float>(),
+                                              selected.data_ptr<int64_t>(), s.chunks, s.rows, s.negs, s.selected, s.D, grad_chunked.data_ptr<float>(),
+                                              grad_negatives.data_ptr<float>(), selected_status_word(chunked.device()).data_ptr<int32_t>(),
+                                              need > 0 ? ws.data_ptr() : nullptr, need, current_stream(chunked)),
           "ge2_selected_neg_scores_backward");
     return {grad_chunked, grad_negatives};
 }
@@ -375,8 +378,7 @@ void Model::check_status() {
 
 void Model::clear_grad() {
     if (!device_models_.empty()) return;  // replicated form: all_reduce clears the half the round after next accumulates into
-    relations_grad_.zero_();
-    if (inverse_relations_grad_.defined()) inverse_relations_grad_.zero_();
+    grad_buf_.narrow(0, 0, rel_both_.numel()).zero_();  // both tables' gradients: one launch
 }
 
 void Model::step() { step_after_all_reduce(1.0f); }
@@ -459,15 +461,18 @@ void Model::train_batch(std::shared_ptr<Batch> batch, bool call_step) {
     if (batch->node_embeddings_.defined()) batch->accumulateGradients(sparse_lr_);  // model.cpp:403-405
 }
 
-torch::Tensor InMemory::indexRead(Indices indices) {
+torch::Tensor InMemory::indexRead(Indices indices) { return indexRead(indices, torch::Tensor()); }
+
+torch::Tensor InMemory::indexRead(Indices indices, torch::Tensor count) {
     if (indices.sizes().size() != 1) throw std::runtime_error("");  // storage.cpp:1174-1177
     require_cuda(data_, "storage data");
     c10::cuda::CUDAGuard guard(data_.device());
     indices = indices.to(data_.device()).contiguous();
     auto out = torch::empty({indices.size(0), data_.size(1)}, data_.options());
     if (!status_.defined()) status_ = torch::zeros({1}, data_.options().dtype(torch::kInt32));
-    check(ge2_index_read(data_.data_ptr<float>(), data_.size(0), indices.data_ptr<int64_t>(), indices.size(0), nullptr, (int32_t)data_.size(1),
-                         out.data_ptr<float>(), status_.data_ptr<int32_t>(), current_stream(data_)),
+    check(ge2_index_read(data_.data_ptr<float>(), data_.size(0), indices.data_ptr<int64_t>(), indices.size(0),
+                         count.defined() ? count.data_ptr<int32_t>() : nullptr, (int32_t)data_.size(1), out.data_ptr<float>(),
+                         status_.data_ptr<int32_t>(), current_stream(data_)),
           "ge2_index_read");
     return out;
 }
@@ -712,7 +717,8 @@ DataLoader::DataLoader(torch::Tensor edges, std::shared_ptr<InMemory> node_embed
     want_src_ = edges_.size(1) == 3 && inverse_edges;                // dataloader.cpp:1321
     const int64_t n_ids = 2 * B_ + (want_src_ ? 2 : 1) * (int64_t)C_ * N_;
     packed_ = torch::empty({n_ids}, edges_.options());
-    deg_rows_ = torch::empty({C_, std::max(n_deg_, 1)}, edges_.options());
+    count_ = torch::empty({2}, edges_.options().dtype(torch::kInt32));
+    count_host_ = torch::empty({2}, torch::dtype(torch::kInt32).pinned_memory(true));
 }
 
 std::shared_ptr<Batch> DataLoader::getBatch() {
@@ -721,26 +727,47 @@ std::shared_ptr<Batch> DataLoader::getBatch() {
     const int64_t domain = emb_->data_.size(0);
     auto slice = edges_.narrow(0, b * B_, B_);
     const int64_t* e = slice.data_ptr<int64_t>();
+    auto batch = std::make_shared<Batch>();
+    if (n_deg_ > 0) batch->deg_sample_rows_ = torch::empty({C_, n_deg_}, edges_.options());
+    const ge2_stream_t stream = current_stream(edges_);
     check(ge2_sample_negatives(e, e + cols - 1, cols, (int32_t)B_, C_, N_, n_deg_, domain, want_src_ ? 1 : 0, seed_, (uint64_t)batch_id_,
-                               packed_.data_ptr<int64_t>(), n_deg_ > 0 ? deg_rows_.data_ptr<int64_t>() : nullptr, current_stream(edges_)),
+                               packed_.data_ptr<int64_t>(), n_deg_ > 0 ? batch->deg_sample_rows_.data_ptr<int64_t>() : nullptr, stream),
           "ge2_sample_negatives");
     batch_id_ += 1;
-    auto tup = map_tensors_unique_inverse_cuda(packed_, true, domain);
-    auto batch = std::make_shared<Batch>();
-    batch->unique_node_indices_ = std::get<0>(tup);
-    const auto& inv = std::get<1>(tup);
-    const int64_t CN = (int64_t)C_ * N_;
-    auto src_l = inv.narrow(0, 0, B_), dst_l = inv.narrow(0, B_, B_);
-    batch->edges_ = cols == 3 ? torch::stack({src_l, slice.select(1, 1), dst_l}, 1) : torch::stack({src_l, dst_l}, 1);
-    int64_t off = 2 * B_;
-    if (want_src_) {
-        batch->src_neg_indices_mapping_ = inv.narrow(0, off, CN).view({C_, N_});
-        off += CN;
+    // map_tensors and loadGPUParameters (dataloader.cpp:1354-1379).  Exactly sized results need the number of unique ids on the host, but
+    // nothing on the device waits for it: the copy of the count is queued behind the unique-map, the gathers (into buffers for as many
+    // rows as there can be, with the count read on the device) behind the copy, and the host waits for the copy alone, while they run.
+    const int64_t n = packed_.numel(), cap = std::min(n, domain), CN = (int64_t)C_ * N_;
+    const size_t need = ge2_unique_workspace_bytes(domain);
+    if (!unique_ws_.defined() || (size_t)unique_ws_.numel() < need) unique_ws_ = torch::empty({(int64_t)need}, edges_.options().dtype(torch::kUInt8));
+    auto unique = torch::empty({cap}, edges_.options()), inv = torch::empty({n}, edges_.options());
+    check(ge2_unique_bitmap(packed_.data_ptr<int64_t>(), n, domain, unique_ws_.data_ptr(), (size_t)unique_ws_.numel(), unique.data_ptr<int64_t>(),
+                            inv.data_ptr<int64_t>(), count_.data_ptr<int32_t>(), stream),
+          "ge2_unique_bitmap");
+    count_host_.copy_(count_, /*non_blocking=*/true);
+    counted_.record();
+    auto emb = emb_->indexRead(unique, count_), state = state_->indexRead(unique, count_);
+    auto split = [&]() {  // the mapped ids, back where they came from
+        auto src_l = inv.narrow(0, 0, B_), dst_l = inv.narrow(0, B_, B_);
+        batch->edges_ = cols == 3 ? torch::stack({src_l, slice.select(1, 1), dst_l}, 1) : torch::stack({src_l, dst_l}, 1);
+        if (want_src_) batch->src_neg_indices_mapping_ = inv.narrow(0, 2 * B_, CN).view({C_, N_});
+        batch->dst_neg_indices_mapping_ = inv.narrow(0, n - CN, CN).view({C_, N_});
+    };
+    split();
+    counted_.synchronize();
+    const int32_t* count = count_host_.data_ptr<int32_t>();
+    if (count[1] & GE2_STATUS_ID_OUT_OF_RANGE) {  // an edge names a node outside the table: map_tensors falls back to sorting
+        std::tie(unique, inv) = map_tensors_unique_inverse_cuda(packed_, true, domain);
+        split();
+        batch->unique_node_indices_ = unique;
+        batch->node_embeddings_ = emb_->indexRead(unique);
+        batch->node_embeddings_state_ = state_->indexRead(unique);
+        return batch;
     }
-    batch->dst_neg_indices_mapping_ = inv.narrow(0, off, CN).view({C_, N_});
-    if (n_deg_ > 0) batch->deg_sample_rows_ = deg_rows_.narrow(1, 0, n_deg_).clone();
-    batch->node_embeddings_ = emb_->indexRead(batch->unique_node_indices_);            // loadGPUParameters, dataloader.cpp:1354-1379
-    batch->node_embeddings_state_ = state_->indexRead(batch->unique_node_indices_);
+    if (count[1] != 0) throw GegeRuntimeException("unique-map failed on the device (status " + std::to_string(count[1]) + ")");
+    batch->unique_node_indices_ = unique.narrow(0, 0, count[0]);
+    batch->node_embeddings_ = emb.narrow(0, 0, count[0]);
+    batch->node_embeddings_state_ = state.narrow(0, 0, count[0]);
     return batch;
 }
 

@@ -15,6 +15,7 @@
 //   selected_neg_scores (autograd), selected_neg_scores_cuda_forward / _backward, distmult_tiled_tournament_selected_scores
 //                                       include/nn/decoders/edge/distmult_selected_neg_cuda.h:5-29
 #pragma once
+#include <ATen/cuda/CUDAEvent.h>
 #include <torch/torch.h>
 
 #include <array>
@@ -131,6 +132,7 @@ class InMemory {
    public:
     explicit InMemory(torch::Tensor data) : data_(std::move(data)) {}
     torch::Tensor indexRead(Indices indices);
+    torch::Tensor indexRead(Indices indices, torch::Tensor count);  // only the first count[0] (device, int32) rows of the result are filled
     void indexAdd(Indices indices, torch::Tensor values);
     // An index outside the table is skipped on the device (rows read as zero) and recorded in a status word; the reference's
     // index ops throw at once, here the word is read where the caller synchronises anyway: throws GegeRuntimeException.
@@ -202,7 +204,8 @@ class DataLoader {
     int64_t batch_id_ = 0;
 
    private:
-    torch::Tensor edges_, packed_, deg_rows_, rel_ids_, step_dev_;
+    torch::Tensor edges_, packed_, unique_ws_, count_, count_host_;  // count_host_: pinned copy of {unique ids, status}
+    at::cuda::CUDAEvent counted_;
     std::shared_ptr<InMemory> emb_, state_;
     int64_t B_;
     int32_t C_, N_, n_deg_;
