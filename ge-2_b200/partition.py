@@ -390,11 +390,12 @@ class RelayBuffer:
         return self.bufs[self.parity if parity is None else parity][t]
 
     def swap(self, next_states: Sequence[Optional[Sequence[int]]], wait_budget_us: int = 0):
-        """Enqueues the swap on the current stream (all ranks call this with the same argument): the barrier kernel, then one
-        pull kernel per table.  Afterwards `parity` names the buffers that hold the new state."""
+        """Enqueues the swap on the current stream (all ranks call this with the same argument): the barrier kernel, then the
+        pull kernels (one for all tables with rows of one length).  Afterwards `parity` names the buffers that hold the new state."""
         new_slots, pulls = plan_relay(self.place, next_states)
         self.epoch += 1
         old, new = self.parity, self.parity ^ 1
+        lists = []
         for t in range(len(self.home)):
             sb = self.slab_bytes[t]
             lst = []
@@ -402,8 +403,14 @@ class RelayBuffer:
                 src = (self.buf_ptrs[old][t][sr] if src_kind == "buf" else self.home_ptrs[t][sr]) + si * sb
                 dst = (self.bufs[new][t].data_ptr() if dst_kind == "buf" else self.home[t].data_ptr()) + di * sb
                 lst.append((src, dst))
-            # the barrier goes with the first table's pulls; the others follow it on the same stream
-            if t == 0:
+            # tables with rows of one length share a launch (no tail between them) as far as its list of slabs goes
+            if lists and lists[-1][1] == sb and len(lists[-1][0]) + len(lst) <= 32:
+                lists[-1][0].extend(lst)
+            else:
+                lists.append((lst, sb))
+        for k, (lst, sb) in enumerate(lists):
+            # the barrier goes with the first launch's pulls; the others follow it on the same stream
+            if k == 0:
                 self.capi.swap_begin(self.world, self.rank, self.flag_ptrs, self.epoch, lst, sb, self.status, wait_budget_us)
             elif lst:
                 self.capi.swap_begin(1, 0, None, self.epoch, lst, sb, self.status)

@@ -278,3 +278,18 @@ def test_two_rank_partitioned_epoch_matches_sequential_oracle(tmp_path):
         assert np.abs(f["rels"][1] - inv).max() <= 5e-4 * np.abs(inv).max()
     # every replica ends with bit-identical relation tables
     assert np.array_equal(np.load(tmp_path / "final_0.npz")["rels"], np.load(tmp_path / "final_1.npz")["rels"])
+
+
+@pytest.mark.parametrize("n", [1, 2, 5, 4097, (1 << 26) + 3])  # the last one is too long for the tabulated round function
+def test_state_edges_are_a_permutation_of_the_buckets(ge2, cuda_device, n):
+    capi, half = ge2.capi, 1 << 13
+    rows = torch.arange(n, device=cuda_device)
+    edges = torch.stack([rows // half, rows % half], 1).contiguous()
+    out = torch.zeros(2 * n + 1, dtype=torch.int64, device=cuda_device)[1:].view(n, 2)  # rows on odd 8-byte addresses
+    status = torch.zeros(1, dtype=torch.int32, device=cuda_device)
+    first = n // 3
+    total = capi.build_state_edges(edges, [first, 0], [n - first, first], torch.zeros(1, dtype=torch.int64, device=cuda_device), 2 * half, 77, out, status)
+    got = out[:, 0] * half + out[:, 1]
+    assert total == n and int(status) == 0
+    assert bool((torch.bincount(got, minlength=n) == 1).all())
+    assert n < 100 or int((got == rows).sum()) < n // 10
