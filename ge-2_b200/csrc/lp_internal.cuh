@@ -50,7 +50,7 @@ struct LpKernelArgs {
 
 inline size_t lp_align(size_t x) { return (x + 255) & ~(size_t)255; }
 
-inline int lp_row_ld(int D) { return D <= 64 ? 64 : 128; }
+__host__ __device__ inline int lp_row_ld(int D) { return D <= 64 ? 64 : 128; }
 
 // Which of the two fp16 forms a step takes: while dK stays in the L2 beside the operands, adding the row blocks' parts up there is
 // the faster one: 25 000 edges, C N = 50 000, D = 128, two sides (49 MB of dK) 149 us against 156, 50 000 edges and 98 MB 403 against 283.

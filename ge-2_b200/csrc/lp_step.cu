@@ -39,7 +39,8 @@ __global__ void __launch_bounds__(256) mask_from_pairs_kernel(const int64_t* __r
 
 // ---------------------------------------------------------------------------------------------------
 // A row of D columns is spread over ld / 4 lanes (16 or 32), four values a lane.
-//   plain   : lane l holds columns [4l, 4l + 4)
+//   plain   : lane l holds columns [4l, 4l + 4), or (V == 1) columns l, l + ld / 4, l + 2 ld / 4, l + 3 ld / 4, so that scalar accesses
+//             of neighbouring lanes are neighbours
 //   ComplEx : coordinates 2l and 2l + 1 of the h = D / 2 complex ones: .x .y their real parts (columns 2l, 2l + 1), .z .w their
 //             imaginary parts (columns h + 2l, h + 2l + 1), so the relation operator and its backward need no other lane's values
 // V is the widest access that the row length and the pointers allow (4 only for plain rows); columns past the row read as zero.
@@ -70,10 +71,11 @@ __device__ __forceinline__ float4 load_row(const float* __restrict__ row, int l,
             v.z = b.x, v.w = b.y;
         }
     } else {
-        if (k < D) v.x = __ldg(row + k);
-        if (k + 1 < D) v.y = __ldg(row + k + 1);
-        if (k + 2 < D) v.z = __ldg(row + k + 2);
-        if (k + 3 < D) v.w = __ldg(row + k + 3);
+        const int n = lp_row_ld(D) >> 2;
+        if (l < D) v.x = __ldg(row + l);
+        if (l + n < D) v.y = __ldg(row + l + n);
+        if (l + 2 * n < D) v.z = __ldg(row + l + 2 * n);
+        if (l + 3 * n < D) v.w = __ldg(row + l + 3 * n);
     }
     return v;
 }
@@ -104,10 +106,11 @@ __device__ __forceinline__ void put_row(float* row, int l, int D, float4 v) {
         if (k < D) Put::two(row + k, v.x, v.y);
         if (k + 2 < D) Put::two(row + k + 2, v.z, v.w);
     } else {
-        if (k < D) Put::one(row + k, v.x);
-        if (k + 1 < D) Put::one(row + k + 1, v.y);
-        if (k + 2 < D) Put::one(row + k + 2, v.z);
-        if (k + 3 < D) Put::one(row + k + 3, v.w);
+        const int n = lp_row_ld(D) >> 2;
+        if (l < D) Put::one(row + l, v.x);
+        if (l + n < D) Put::one(row + l + n, v.y);
+        if (l + 2 * n < D) Put::one(row + l + 2 * n, v.z);
+        if (l + 3 * n < D) Put::one(row + l + 3 * n, v.w);
     }
 }
 
@@ -158,7 +161,24 @@ __device__ __forceinline__ void store_split4(__nv_bfloat16* dst, int64_t plane, 
 // one row in the lanes' layout as an operand row of the scores kernels: fp16, or (plane > 0) the three bf16 planes
 template <int V, bool CPLX, bool HALF>
 __device__ __forceinline__ void store_operand(void* rows, int64_t plane, int64_t row, int ld, int l, int D, float4 v) {
-    if constexpr (!CPLX) {
+    if constexpr (!CPLX && V == 1) {
+        const int n = ld >> 2;
+        float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            uint16_t* p = (uint16_t*)rows + row * ld + l + e * n;
+            if constexpr (HALF) {
+                *p = __half_as_ushort(__float2half_rn(x[e]));
+            } else {
+#pragma unroll
+                for (int t = 0; t < 3; t++, p += plane) {
+                    const __nv_bfloat16 b = __float2bfloat16_rn(x[e]);
+                    *p = __bfloat16_as_ushort(b);
+                    x[e] -= __bfloat162float(b);
+                }
+            }
+        }
+    } else if constexpr (!CPLX) {
         if constexpr (HALF) store_half4((__half*)rows + row * ld + 4 * l, v);
         else store_split4((__nv_bfloat16*)rows + row * ld + 4 * l, plane, v);
     } else {
@@ -334,7 +354,8 @@ struct FinScalars {
 template <int V, bool CPLX>
 __device__ __noinline__ void adagrad_row(float* emb, float* state, int l, int D, float4 e, float4 s, float4 g, float neg_lr) {
     // a lane without columns must not divide: 0 / 1e-10 is off the fast path of the division, and the whole warp would wait for it
-    const int cols = CPLX ? (D >> 1) - 2 * l : D - 4 * l;
+    const int n = lp_row_ld(D) >> 2;
+    const int cols = CPLX ? (D >> 1) - 2 * l : V == 1 ? (D - l + n - 1) / n : D - 4 * l;  // values of this lane that exist (at least)
     if (cols <= 0) return;
     if (CPLX ? cols == 1 : cols < 4) {
         if (CPLX) s.y = s.w = 1.f;
@@ -663,11 +684,15 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     }
     if (!(phases & 4)) return GE2_OK;
 
-    // negatives a warp: 32 keep repeated nodes together and amortise the ids' latency, 8 spread a small batch over the GPU
+    // negatives a warp: as few as give half the warps that fit the GPU something to do, since a warp goes through them one by one (3000 of
+    // them in groups of 16: 28 us, a step of 55 us instead of 40), up to the 32 that one lane each can hold; more of them together
+    // merge more repeated nodes (9000 drawn half by degree: 15.4 us in groups of 2, 12.5 in groups of 8)
     const int64_t neg_rows = (int64_t)L.S * L.CN;
-    int occ = 8;
-    while (occ < 32 && neg_rows / (2 * occ) >= (int64_t)kNumSMs * 4 * kFinWarps) occ *= 2;
-    const int edge_ctas = std::min(ceil_div(desc->B, kFinBatch), kNumSMs * 4);  // as many as are resident together
+    int occ = 2;
+    while (occ < 32 && neg_rows / occ > (int64_t)kNumSMs * 2 * kFinWarps) occ *= 2;
+    // As many as are resident together.  More (one batch each) take 5 % off this kernel alone and put 4 % on the pipelined step, whose
+    // sampler and unique-map for the next batch run beside it.
+    const int edge_ctas = std::min(ceil_div(desc->B, kFinBatch), kNumSMs * 4);
     const int64_t neg_ctas = ceil_div<int64_t>(ceil_div<int64_t>(L.CN, occ / L.S), kFinWarps);
     const size_t fin_smem = (size_t)4 * kFinBatch * L.ld * 4;
     GE2_CUDA_TRY(launch_after(finish_kernel_of(*desc), dim3((unsigned)(edge_ctas + neg_ctas)), dim3(kFinWarps * 32), fin_smem, stream, a, (int)neg_ctas, occ));
