@@ -684,12 +684,12 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     }
     if (!(phases & 4)) return GE2_OK;
 
-    // negatives a warp: as few as give half the warps that fit the GPU something to do, since a warp goes through them one by one (3000 of
-    // them in groups of 16: 28 us, a step of 55 us instead of 40), up to the 32 that one lane each can hold; more of them together
+    // negatives a warp: as few as fill the GPU once, since a warp goes through them one by one (3000 of them in groups of 16: 28 us, a
+    // step of 55 us instead of 40), but at least four and up to the 32 that one lane each can hold: more of them together
     // merge more repeated nodes (9000 drawn half by degree: 15.4 us in groups of 2, 12.5 in groups of 8)
     const int64_t neg_rows = (int64_t)L.S * L.CN;
-    int occ = 2;
-    while (occ < 32 && neg_rows / occ > (int64_t)kNumSMs * 2 * kFinWarps) occ *= 2;
+    int occ = 4;
+    while (occ < 32 && neg_rows / occ > (int64_t)kNumSMs * 4 * kFinWarps) occ *= 2;
     // As many as are resident together.  More (one batch each) take 5 % off this kernel alone and put 4 % on the pipelined step, whose
     // sampler and unique-map for the next batch run beside it.
     const int edge_ctas = std::min(ceil_div(desc->B, kFinBatch), kNumSMs * 4);

@@ -22,15 +22,8 @@ namespace ge2 {
 namespace {
 
 constexpr int kScanThreads = 128;
-// Words a thread: one while that makes few tiles (a small domain then still spreads over CTAs), more for larger domains, so that the
-// look-back, 32 tiles a step, stays short.
-constexpr int kMaxWordsPerThread = 8, kFewTiles = 160;
-constexpr int64_t kMinTileWords = kScanThreads;
-__host__ __device__ inline int scan_words_per_thread(int64_t num_words) {
-    int w = 1;
-    while (w < kMaxWordsPerThread && num_words > (int64_t)kFewTiles * kScanThreads * w) w *= 2;
-    return w;
-}
+constexpr int kWordsPerThread = 1;
+constexpr int kTileWords = kScanThreads * kWordsPerThread;  // 128 words = 8192 ids per tile: a small domain still spreads over CTAs
 constexpr uint32_t kFlagAggregate = 1u << 30;               // tile state: local sum published
 constexpr uint32_t kFlagPrefix = 2u << 30;                  // tile state: inclusive prefix published
 constexpr uint32_t kValueMask = (1u << 30) - 1;
@@ -58,7 +51,7 @@ constexpr size_t align256c(size_t x) { return (x + 255) & ~(size_t)255; }
 // control words (tile states, ticket, status, one spare), two bitsets, per-word offsets
 constexpr size_t unique_ws_bytes(int64_t domain) {
     const int64_t nw = (domain + 63) >> 6;
-    const int64_t tiles = (nw + kMinTileWords - 1) / kMinTileWords;
+    const int64_t tiles = (nw + kTileWords - 1) / kTileWords;
     return align256c((size_t)(tiles + 4) * 4) + 2 * align256c((size_t)nw * 8) + align256c((size_t)nw * 4);
 }
 
@@ -86,16 +79,14 @@ __global__ void __launch_bounds__(256) mark_kernel(const int64_t* __restrict__ i
     if (bad) atomicOr(status, GE2_STATUS_ID_OUT_OF_RANGE);
 }
 
-// One tile = 128 x kWordsPerThread consecutive words.  Tiles are handed out by an atomic ticket so a tile only ever waits for tiles
+// One tile = 128 consecutive words.  Tiles are handed out by an atomic ticket so a tile only ever waits for tiles
 // that have already started (forward progress without co-residency assumptions); the wait is bounded anyway.
-template <int kWordsPerThread>
 __global__ void __launch_bounds__(kScanThreads) scan_extract_kernel(const unsigned long long* __restrict__ words, int64_t num_words,
                                                                     int32_t* __restrict__ word_offsets, uint32_t* tile_state,
                                                                     uint32_t* ticket, int num_tiles, int64_t* __restrict__ out_unique,
                                                                     int64_t out_capacity, int32_t* __restrict__ out_count,
                                                                     const unsigned long long* __restrict__ dup, unsigned char* __restrict__ out_shared,
                                                                     int32_t* __restrict__ status) {
-    constexpr int kTileWords = kScanThreads * kWordsPerThread;
     __shared__ unsigned long long s_words[kTileWords], s_dup[kTileWords];
     __shared__ uint32_t s_off[kTileWords];
     __shared__ uint32_t s_warp_sums[kScanThreads / 32];
@@ -112,7 +103,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_extract_kernel(const unsign
         const uint32_t tile = s_tile;
         if (tile >= (uint32_t)num_tiles) return;
 
-        // each thread owns kWordsPerThread consecutive words
+        // each thread owns one word
         const int64_t w0 = (int64_t)tile * kTileWords + (int64_t)tid * kWordsPerThread;
         unsigned long long w[kWordsPerThread], again[kWordsPerThread];
         uint32_t cnt[kWordsPerThread];
@@ -282,8 +273,7 @@ extern "C" int ge2_unique_bitmap_shared(const int64_t* ids, int64_t n, int64_t d
     }
     const int64_t nw = num_words_of(domain);
     if (nw > (int64_t)kValueMask) return GE2_ERR_UNSUPPORTED;
-    const int words_per_thread = scan_words_per_thread(nw);
-    const int64_t tiles = ceil_div<int64_t>(nw, (int64_t)kScanThreads * words_per_thread);
+    const int64_t tiles = ceil_div<int64_t>(nw, kTileWords);
     if (workspace == nullptr || ((uintptr_t)workspace & 255) != 0 || workspace_bytes < ge2_unique_workspace_bytes(domain))
         return GE2_ERR_WORKSPACE;
 
@@ -309,12 +299,8 @@ extern "C" int ge2_unique_bitmap_shared(const int64_t* ids, int64_t n, int64_t d
 
     mark_kernel<<<stream_grid(n, 256), 256, 0, stream>>>(ids, n, domain, ws.words, out_shared != nullptr ? ws.dup : nullptr, tw, ws.status);
     GE2_LAUNCH_CHECK();
-    auto scan = words_per_thread == 1   ? scan_extract_kernel<1>
-                : words_per_thread == 2 ? scan_extract_kernel<2>
-                : words_per_thread == 4 ? scan_extract_kernel<4>
-                                        : scan_extract_kernel<8>;
     const int scan_grid = (int)(tiles < (int64_t)kNumSMs * 8 ? tiles : (int64_t)kNumSMs * 8);
-    GE2_CUDA_TRY(launch_after(scan, dim3((unsigned)scan_grid), dim3(kScanThreads), 0, stream, (const unsigned long long*)ws.words, nw,
+    GE2_CUDA_TRY(launch_after(scan_extract_kernel, dim3((unsigned)scan_grid), dim3(kScanThreads), 0, stream, (const unsigned long long*)ws.words, nw,
                               ws.word_offsets, ws.tile_state, ws.ticket, (int)tiles, out_unique, cap, out_count, (const unsigned long long*)ws.dup, out_shared, ws.status));
     GE2_CUDA_TRY(launch_after(inverse_kernel, dim3((unsigned)stream_grid(n, 256)), dim3(256), 0, stream, ids, n, domain,
                               (const unsigned long long*)ws.words, (const int32_t*)ws.word_offsets, out_inverse, (const int32_t*)ws.status,

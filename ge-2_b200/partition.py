@@ -398,11 +398,9 @@ class RelayBuffer:
         lists = []
         for t in range(len(self.home)):
             sb = self.slab_bytes[t]
-            lst = []
-            for src_kind, sr, si, dst_kind, di in pulls[self.rank]:
-                src = (self.buf_ptrs[old][t][sr] if src_kind == "buf" else self.home_ptrs[t][sr]) + si * sb
-                dst = (self.bufs[new][t].data_ptr() if dst_kind == "buf" else self.home[t].data_ptr()) + di * sb
-                lst.append((src, dst))
+            buf_src, home_src, buf_dst, home_dst = self.buf_ptrs[old][t], self.home_ptrs[t], self.bufs[new][t].data_ptr(), self.home[t].data_ptr()
+            lst = [((buf_src[sr] if src_kind == "buf" else home_src[sr]) + si * sb, (buf_dst if dst_kind == "buf" else home_dst) + di * sb)
+                   for src_kind, sr, si, dst_kind, di in pulls[self.rank]]
             # tables with rows of one length share a launch (no tail between them) as far as its list of slabs goes
             if lists and lists[-1][1] == sb and len(lists[-1][0]) + len(lst) <= 32:
                 lists[-1][0].extend(lst)
