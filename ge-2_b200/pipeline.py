@@ -533,7 +533,7 @@ class BatchPipeline:
         cfg = self.cfg
         n = 1 + 3                              # sampler; unique-map: mark, scan, inverse
         n += 1                                 # prepare (gather + relation operator + positive scores + filter words)
-        n += 2 if cfg.precision == "f16" else 1  # scores: logsumexp pass + gradient pass (persistent launches), or the fp32 kernel
+        n += 2                                 # scores: logsumexp pass + gradient pass, or both passes of the streaming form
         n += 1                                 # finish (operator backward + scatter)
         n += 1                                 # sparse Adagrad scatter
         if cfg.has_relations:
