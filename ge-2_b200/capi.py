@@ -15,6 +15,7 @@ PKG = Path(__file__).resolve().parent
 GE2_OK = 0
 DECODER = {"DISTMULT": 0, "DOT": 0, "COMPLEX": 1}
 PRECISION = {"fp32": 0, "f16": 1}
+LP_NODE_GRAD_IS_ZERO, LP_HAS_ROW_UPDATE = 1, 2  # ge2_lp_desc.flags
 STATUS_BITS = {1: "id out of range", 2: "scan timeout", 4: "filter collision", 8: "bad index", 16: "pipeline timeout", 32: "peer timeout"}
 
 EXPORTS = [
@@ -233,7 +234,7 @@ def make_lp_desc(*, decoder, precision, B, Cn, N, D, R, U, node_emb, row_index=N
     if d.src_filter_n == 0:
         d.src_filter = None
     d.deg_sample_rows, d.n_deg = ptr(deg_sample_rows), n_deg
-    d.flags = 1 if node_grad_is_zero else 0
+    d.flags = (LP_NODE_GRAD_IS_ZERO if node_grad_is_zero else 0) | LP_HAS_ROW_UPDATE
     d.rel, d.inv_rel = ptr(rel), ptr(inv_rel)
     d.node_grad, d.rel_grad, d.inv_rel_grad, d.loss = ptr(node_grad), ptr(rel_grad), ptr(inv_rel_grad), ptr(loss)
     d.pos_scores, d.neg_scores = ptr(pos_scores), ptr(neg_scores)

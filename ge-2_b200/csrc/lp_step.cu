@@ -6,6 +6,8 @@
 // relation operators (relation_operators.cpp:3-31), apply_score_filter (cpp/src/data/samplers/negative.cpp:570-575)
 // and SoftmaxCrossEntropy with SUM reduction (cpp/src/nn/loss.cpp:46-63).
 #include <algorithm>
+#include <cstddef>
+#include <cstring>
 
 #include "adagrad.cuh"
 #include "lp_internal.cuh"
@@ -606,6 +608,13 @@ __global__ void __launch_bounds__(256) copy_pos_kernel(const float* __restrict__
     }
 }
 
+// the descriptor as the kernels see it: what the caller did not say it has is zero
+ge2_lp_desc whole_desc(const ge2_lp_desc* d) {
+    ge2_lp_desc whole = {};
+    memcpy(&whole, d, (d->flags & GE2_LP_HAS_ROW_UPDATE) ? sizeof(whole) : offsetof(ge2_lp_desc, node_state));
+    return whole;
+}
+
 int validate(const ge2_lp_desc* d) {
     if (d == nullptr) return GE2_ERR_INVALID_ARGUMENT;
     if (d->B <= 0 || d->C <= 0 || d->N <= 0 || d->D <= 0 || d->U <= 0) return GE2_ERR_INVALID_ARGUMENT;
@@ -624,7 +633,7 @@ int validate(const ge2_lp_desc* d) {
         (d->src_filter_n > 0 && d->src_filter == nullptr))
         return GE2_ERR_INVALID_ARGUMENT;
     if (d->deg_sample_rows != nullptr && (d->n_deg <= 0 || d->n_deg > d->N)) return GE2_ERR_INVALID_ARGUMENT;
-    if ((d->node_state == nullptr) != (d->row_shared == nullptr)) return GE2_ERR_INVALID_ARGUMENT;
+    if ((d->flags & GE2_LP_HAS_ROW_UPDATE) && (d->node_state == nullptr) != (d->row_shared == nullptr)) return GE2_ERR_INVALID_ARGUMENT;
     if (d->deg_sample_rows != nullptr && (d->dst_filter_n > 0 || d->src_filter_n > 0)) return GE2_ERR_INVALID_ARGUMENT;
     return GE2_OK;
 }
@@ -646,7 +655,7 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     int rc = validate(desc);
     if (rc != GE2_OK) return rc;
     LpKernelArgs a;
-    a.d = *desc;
+    a.d = whole_desc(desc);
     if (desc->workspace == nullptr || ((uintptr_t)desc->workspace & 255) != 0) return GE2_ERR_WORKSPACE;
     a.L = lp_make_layout(*desc, desc->workspace);
     if (desc->workspace_bytes < a.L.bytes) return GE2_ERR_WORKSPACE;
@@ -674,7 +683,7 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     }
 
     const int64_t units = L.Bp + ceil_div<int64_t>(L.CN, kPrepNegs);
-    const PrepKernel prep = desc->precision == GE2_PRECISION_F16 ? prep_kernel_of<true>(*desc) : prep_kernel_of<false>(*desc);
+    const PrepKernel prep = desc->precision == GE2_PRECISION_F16 ? prep_kernel_of<true>(a.d) : prep_kernel_of<false>(a.d);
     GE2_CUDA_TRY(launch_after(prep, dim3((unsigned)stream_grid(units, 1024 / L.ld, 5)), dim3(256), 0, stream, a, pairs ? 0 : 1));
     }
 
@@ -695,7 +704,7 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     const int edge_ctas = std::min(ceil_div(desc->B, kFinBatch), kNumSMs * 4);
     const int64_t neg_ctas = ceil_div<int64_t>(ceil_div<int64_t>(L.CN, occ / L.S), kFinWarps);
     const size_t fin_smem = (size_t)4 * kFinBatch * L.ld * 4;
-    GE2_CUDA_TRY(launch_after(finish_kernel_of(*desc), dim3((unsigned)(edge_ctas + neg_ctas)), dim3(kFinWarps * 32), fin_smem, stream, a, (int)neg_ctas, occ));
+    GE2_CUDA_TRY(launch_after(finish_kernel_of(a.d), dim3((unsigned)(edge_ctas + neg_ctas)), dim3(kFinWarps * 32), fin_smem, stream, a, (int)neg_ctas, occ));
     if (desc->pos_scores != nullptr || desc->inv_pos_scores != nullptr) {
         copy_pos_kernel<<<ceil_div(L.Bp, 256), 256, 0, stream>>>(L.pos, L.Bp, desc->pos_scores, desc->inv_pos_scores, L.S);
         GE2_LAUNCH_CHECK();

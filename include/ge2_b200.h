@@ -44,6 +44,9 @@ extern "C" {
 
 typedef void *ge2_stream_t; /* cudaStream_t */
 
+/* "ge2_b200 <major>.<minor> (...)".  0.2: ge2_lp_desc grew by the members behind GE2_LP_HAS_ROW_UPDATE; ge2_train_step,
+ * ge2_unique_bitmap_shared, ge2_adagrad_scatter_shared and the selected-negative backward with scratch are new.  A descriptor laid
+ * out as in 0.1 (without that flag) is still understood. */
 GE2_API const char *ge2_version(void);
 GE2_API int ge2_last_cuda_error(void);            /* cudaError_t of the last failing runtime call on this thread */
 GE2_API const char *ge2_status_string(int status);
@@ -104,6 +107,9 @@ GE2_API int ge2_pack_ids(const int64_t *const parts[4], const int64_t lens[4], c
 /* ge2_lp_desc.flags: the caller guarantees node_grad is all zero on entry (e.g. ge2_adagrad_scatter with clear_grad
  * consumed the previous batch's gradients), so the step skips its own memset of U * D floats */
 #define GE2_LP_NODE_GRAD_IS_ZERO 1
+/* ... the descriptor has the members from node_state on, which callers built against version 0.1 may not have: without this bit the
+ * library reads none of them */
+#define GE2_LP_HAS_ROW_UPDATE 2
 
 #define GE2_PRECISION_FP32 0 /* fp32 throughout (1e-4 relative parity): tcgen05 tiles of operands split exactly into three
                                 bf16 terms, small products first, tiles summed in fp32                   */
@@ -175,7 +181,7 @@ typedef struct ge2_lp_desc {
     void *workspace;      /* ge2_lp_workspace_bytes() bytes, 256-byte aligned                      */
     size_t workspace_bytes;
 
-    /* optional (both or neither): the optimizer step of the rows that need no sum over occurrences, inside the scatter.  row_shared[U]
+    /* read when flags has GE2_LP_HAS_ROW_UPDATE; optional (both pointers or neither): the optimizer step of the rows that need no sum over occurrences, inside the scatter.  row_shared[U]
      * (ge2_unique_bitmap_shared with the two sides' negatives as twins): 0 = the node occurs once in the batch.  Such a row never
      * reaches node_grad: its row of node_emb (written, despite the const) and of node_state (same rows and stride) takes the
      * Adagrad step with learning rate node_lr here; ge2_adagrad_scatter_shared does the rows marked 1. */

@@ -97,3 +97,52 @@ def test_swap_and_eval_structs_match_header(ge2):
     S, E = ge2.capi.SwapDesc, ge2.capi.EvalDesc
     assert ctypes.sizeof(S) == s_size and S.slab_bytes.offset == s_slab and S.status.offset == s_status
     assert ctypes.sizeof(E) == e_size and E.neg_ids.offset == e_neg and E.workspace.offset == e_ws
+
+
+def _old_caller(code):
+    """runs `code` in a process of its own with `lib` loaded, `D` the ctypes descriptor, and `d`: a valid descriptor as a caller built against
+    version 0.1 lays it out, ending with workspace_bytes, on the last bytes of a page behind which nothing can be read"""
+    import subprocess
+    import sys
+
+    head = f"""
+import ctypes, importlib, mmap, sys
+sys.path.insert(0, {str(ROOT)!r})
+capi = importlib.import_module("ge-2_b200.capi")
+lib, D = capi.load_library(), capi.LpDesc
+size = D.node_state.offset
+libc = ctypes.CDLL(None, use_errno=True)
+pages = mmap.mmap(-1, 2 * mmap.PAGESIZE)
+base = ctypes.addressof(ctypes.c_char.from_buffer(pages))
+assert libc.mprotect(ctypes.c_void_p(base + mmap.PAGESIZE), mmap.PAGESIZE, 0) == 0
+full = D(B=8, C=2, N=4, D=16, U=40, emb_stride=16, edge_stride=1)
+for name in ("node_emb", "src_ids", "dst_ids", "dst_negs", "node_grad", "loss"):
+    setattr(full, name, 4096)
+at = base + mmap.PAGESIZE - size
+ctypes.memmove(at, ctypes.addressof(full), size)
+d = ctypes.cast(at, ctypes.POINTER(D))
+need = ctypes.c_size_t()
+"""
+    return subprocess.run([sys.executable, "-c", head + code], capture_output=True, text=True)
+
+
+def test_descriptor_of_version_0_1_is_read_no_further_than_it_reaches():
+    r = _old_caller("""
+assert lib.ge2_lp_workspace_bytes(d, ctypes.byref(need)) == 0 and need.value > 0
+assert lib.ge2_lp_step(d, None) == 3  # no workspace: found out before any CUDA call, after the descriptor was copied
+""")
+    assert r.returncode == 0, (r.returncode, r.stderr)
+
+
+def test_row_update_members_count_only_with_their_flag(ge2):
+    """what lies behind an old descriptor must not switch the in-place optimizer on, nor have the call refused"""
+    lib, capi = ge2.load_library(), ge2.capi
+    d = capi.LpDesc(B=8, C=2, N=4, D=16, U=40, emb_stride=16, edge_stride=1)
+    for name in ("node_emb", "src_ids", "dst_ids", "dst_negs", "node_grad", "loss"):
+        setattr(d, name, 4096)
+    d.node_state = 4096  # without row_shared
+    need = ctypes.c_size_t()
+    assert lib.ge2_lp_workspace_bytes(ctypes.byref(d), ctypes.byref(need)) == 0
+    d.flags = capi.LP_HAS_ROW_UPDATE
+    assert lib.ge2_lp_workspace_bytes(ctypes.byref(d), ctypes.byref(need)) == 1
+    assert b" 0.1 " not in lib.ge2_version()
