@@ -49,6 +49,7 @@ class LpDesc(C.Structure):
         ("pos_scores", C.c_void_p), ("neg_scores", C.c_void_p), ("inv_pos_scores", C.c_void_p), ("inv_neg_scores", C.c_void_p),
         ("status", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t),
         ("node_state", C.c_void_p), ("row_shared", C.c_void_p), ("node_lr", C.c_float), ("reserved", C.c_int32),
+        ("table_rows", C.c_int64),
     ]
 
 
@@ -215,7 +216,7 @@ def make_lp_desc(*, decoder, precision, B, Cn, N, D, R, U, node_emb, row_index=N
                  edge_stride=1, rel_stride=1, dst_negs, src_negs=None, dst_filter=None, src_filter=None, deg_sample_rows=None, n_deg=0,
                  rel=None, inv_rel=None, node_grad, rel_grad=None, inv_rel_grad=None, loss, pos_scores=None, neg_scores=None,
                  inv_pos_scores=None, inv_neg_scores=None, status=None, workspace=None, node_grad_is_zero=False, node_state=None,
-                 row_shared=None, node_lr=0.0) -> LpDesc:
+                 row_shared=None, node_lr=0.0, table_rows=None) -> LpDesc:
     d = LpDesc()
     d.decoder = DECODER[decoder] if isinstance(decoder, str) else decoder
     d.precision = PRECISION[precision] if isinstance(precision, str) else precision
@@ -241,6 +242,7 @@ def make_lp_desc(*, decoder, precision, B, Cn, N, D, R, U, node_emb, row_index=N
     d.inv_pos_scores, d.inv_neg_scores = ptr(inv_pos_scores), ptr(inv_neg_scores)
     d.status = ptr(status)
     d.node_state, d.row_shared, d.node_lr = ptr(node_state), ptr(row_shared), node_lr
+    d.table_rows = node_emb.shape[0] if table_rows is None else table_rows
     if workspace is not None:
         d.workspace, d.workspace_bytes = ptr(workspace), workspace.numel()
     return d

@@ -15,11 +15,12 @@
 namespace ge2 {
 namespace {
 
+// The row of a local node id; the first row in the place of one that the table does not have (the finish kernel reports it and leaves its
+// gradient out).  Dropping what was read instead, here, is a dozen instructions more a row: 0.5 us of a step of 88.
 __device__ __forceinline__ const float* emb_row(const ge2_lp_desc& d, int64_t local) {
     const int64_t row = d.row_index != nullptr ? __ldg(&d.row_index[local]) : local;
-    return d.node_emb + row * d.emb_stride;
+    return d.node_emb + ((uint64_t)row < (uint64_t)d.table_rows ? row : 0) * d.emb_stride;
 }
-
 
 // ---------------------------------------------------------------------------------------------------
 // mask: one int per (side, chunk, column) = the batch row whose score there is overwritten with -1e9
@@ -339,6 +340,7 @@ __global__ void __launch_bounds__(256, 5) lp_prep_kernel(const __grid_constant__
 // negatives, Dot 100: 104 us (143 us); 100 000 edges, 2 x 200 000 negatives, DistMult 128: 270 us (465 us).
 // ---------------------------------------------------------------------------------------------------
 constexpr int kFinWarps = 8;
+constexpr int kNoRow = 2;      // in the place of a node's "occurs again": its row is not one of the table, so nothing is done with it
 constexpr int kFinBatch = 16;  // edges a batch: their 32 endpoints are the lanes of one warp when it looks for repeated nodes
 
 struct FinScalars {
@@ -402,22 +404,26 @@ __global__ void __launch_bounds__(kFinWarps * 32, 4) lp_finish_kernel(const __gr
             const long long v = (side == 0 ? d.dst_negs : d.src_negs)[j];
             if (v >= 0 && v < d.U) id = v;
         }
-        if (fused && id >= 0) {
-            shared = d.row_shared[id];
+        if (id >= 0) {
+            if (fused) shared = d.row_shared[id];
             trow = d.row_index != nullptr ? __ldg(&d.row_index[id]) : id;
         }
         const unsigned same = __match_any_sync(0xFFFFFFFFu, id);
         const long long dk_row = (long long)side * L.CN + j;
         const bool leads = id >= 0 && (same & ((1u << lane) - 1u)) == 0;
         const unsigned leaders = __ballot_sync(0xFFFFFFFFu, leads);
+        if ((uint64_t)trow >= (uint64_t)d.table_rows) {  // (here: the row may arrive while the ids are matched)
+            shared = kNoRow;
+            or_status(d.status, GE2_STATUS_BAD_INDEX);
+        }
 #pragma unroll 1
         for (int k0 = 0; k0 < occ; k0 += per_warp) {
             if (((leaders >> k0) & ((1u << per_warp) - 1u)) == 0u) continue;
             const int k = k0 + sub;
-            const bool on = (leaders >> k) & 1u;
             const unsigned members = __shfl_sync(0xFFFFFFFFu, same, k);
             const long long gid = __shfl_sync(0xFFFFFFFFu, id, k), grow = __shfl_sync(0xFFFFFFFFu, trow, k);
             const int sh = __shfl_sync(0xFFFFFFFFu, shared, k);
+            const bool on = ((leaders >> k) & 1u) && sh != kNoRow;
             const bool upd = on && sh == 0;
             const long long r1 = __shfl_sync(0xFFFFFFFFu, dk_row, k);
             unsigned rest = members & (members - 1);
@@ -485,7 +491,13 @@ __global__ void __launch_bounds__(kFinWarps * 32, 4) lp_finish_kernel(const __gr
     fetch(base);
 #pragma unroll 1
     for (; base < d.B; base += step) {
-        if (warp == 0) sm.id[lane] = p_id, sm.row[lane] = p_row, sm.shared[lane] = (unsigned char)p_shared;
+        if (warp == 0) {
+            if (p_id >= 0 && (uint64_t)p_row >= (uint64_t)d.table_rows) {  // (here and not where it is fetched: the load is not waited for until now)
+                p_id = -1;
+                or_status(d.status, GE2_STATUS_BAD_INDEX);
+            }
+            sm.id[lane] = p_id, sm.row[lane] = p_row, sm.shared[lane] = (unsigned char)p_shared;
+        }
         else if (warp == 1 && REL && lane < kFinBatch) sm.rid[lane] = p_rid;
         else if (warp == 2) sm.dpos[lane / kFinBatch][k16] = p_dpos;
         __syncthreads();
@@ -612,6 +624,7 @@ __global__ void __launch_bounds__(256) copy_pos_kernel(const float* __restrict__
 ge2_lp_desc whole_desc(const ge2_lp_desc* d) {
     ge2_lp_desc whole = {};
     memcpy(&whole, d, (d->flags & GE2_LP_HAS_ROW_UPDATE) ? sizeof(whole) : offsetof(ge2_lp_desc, node_state));
+    if (whole.table_rows == 0) whole.table_rows = INT64_MAX;  // not told: every row is taken for one of the table
     return whole;
 }
 
@@ -633,7 +646,10 @@ int validate(const ge2_lp_desc* d) {
         (d->src_filter_n > 0 && d->src_filter == nullptr))
         return GE2_ERR_INVALID_ARGUMENT;
     if (d->deg_sample_rows != nullptr && (d->n_deg <= 0 || d->n_deg > d->N)) return GE2_ERR_INVALID_ARGUMENT;
-    if ((d->flags & GE2_LP_HAS_ROW_UPDATE) && (d->node_state == nullptr) != (d->row_shared == nullptr)) return GE2_ERR_INVALID_ARGUMENT;
+    if (d->flags & GE2_LP_HAS_ROW_UPDATE) {
+        if ((d->node_state == nullptr) != (d->row_shared == nullptr) || d->table_rows < 0) return GE2_ERR_INVALID_ARGUMENT;
+        if (d->node_state != nullptr && d->table_rows == 0) return GE2_ERR_INVALID_ARGUMENT;  // rows are written only where they are known to exist
+    }
     if (d->deg_sample_rows != nullptr && (d->dst_filter_n > 0 || d->src_filter_n > 0)) return GE2_ERR_INVALID_ARGUMENT;
     return GE2_OK;
 }

@@ -6,6 +6,8 @@
 // Floating-point updates use explicit round-to-nearest intrinsics so no multiply-add contraction happens: the result
 // is bit-identical to evaluating the reference's chain of element-wise ATen ops (cpp/src/data/batch.cpp:264-266,
 // cpp/src/nn/optim.cpp:130-137 of the reference project) one IEEE operation at a time.
+#include <algorithm>
+
 #include "adagrad.cuh"
 
 namespace ge2 {
@@ -621,7 +623,8 @@ extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
     int rc = ge2_sample_negatives(t->edges, t->edges + t->cols - 1, t->cols, d.B, d.C, d.N, t->n_deg, t->domain, d.use_inverse, t->seed, t->batch_index,
                                   t->packed, t->deg_rows, stream);
     if (rc != GE2_OK) return rc;
-    rc = ge2_unique_bitmap_shared(t->packed, t->n_ids, t->domain, t->unique_ws, t->unique_ws_bytes, t->unique, t->inverse, t->count, t->shared,
+    // ids past the table get no local id: they are flagged here, and no later kernel meets them
+    rc = ge2_unique_bitmap_shared(t->packed, t->n_ids, std::min(t->domain, t->table_rows), t->unique_ws, t->unique_ws_bytes, t->unique, t->inverse, t->count, t->shared,
                                   t->twin_begin, t->twin_len, stream);
     if (rc != GE2_OK) return rc;
     rc = ge2_lp_step(&d, stream);

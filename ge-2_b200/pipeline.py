@@ -185,8 +185,12 @@ class BatchPipeline:
             capi.sample_batch(edges_all, num_batches, counter, *args)
 
     def _unique(self, ids: "_IdSet"):
-        capi.unique_bitmap(ids.packed, self.cfg.domain, workspace=ids.uws, out_unique=ids.unique, out_inverse=ids.inverse, out_count=ids.count,
+        capi.unique_bitmap(ids.packed, self._mapped_domain(), workspace=ids.uws, out_unique=ids.unique, out_inverse=ids.inverse, out_count=ids.count,
                            out_shared=ids.shared, twins=ids.twins)
+
+    def _mapped_domain(self):
+        """ids that get a local id: those with a row in the table (others are flagged, and neither read nor written)"""
+        return min(self.cfg.domain, self.table.shape[0])
 
     def use_peer_gradients(self, peer: PeerGradients):
         """Multi-GPU: relation gradients go into `peer`'s buffer (alternating halves) and the dense optimizer step sums them

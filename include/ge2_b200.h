@@ -189,6 +189,10 @@ typedef struct ge2_lp_desc {
     const uint8_t *row_shared;
     float node_lr;
     int32_t reserved;
+    /* rows of node_emb (and node_state); needed with node_state, else 0 = not told.  A node whose row is not below it (row_index can name
+     * any row of an id domain) sets GE2_STATUS_BAD_INDEX: no memory past the table is read or written (the first row stands in for what
+     * would be read), and the node's edges and negatives have no gradient. */
+    int64_t table_rows;
 } ge2_lp_desc;
 
 GE2_API int ge2_lp_workspace_bytes(const ge2_lp_desc *desc, size_t *bytes);

@@ -146,3 +146,14 @@ def test_row_update_members_count_only_with_their_flag(ge2):
     d.flags = capi.LP_HAS_ROW_UPDATE
     assert lib.ge2_lp_workspace_bytes(ctypes.byref(d), ctypes.byref(need)) == 1
     assert b" 0.1 " not in lib.ge2_version()
+
+
+def test_row_update_needs_the_number_of_table_rows(ge2):
+    lib, capi = ge2.load_library(), ge2.capi
+    d = capi.LpDesc(B=8, C=2, N=4, D=16, U=40, emb_stride=16, edge_stride=1, flags=capi.LP_HAS_ROW_UPDATE)
+    for name in ("node_emb", "src_ids", "dst_ids", "dst_negs", "node_grad", "loss", "node_state", "row_shared"):
+        setattr(d, name, 4096)
+    need = ctypes.c_size_t()
+    for rows, rc in ((0, 1), (-1, 1), (40, 0)):
+        d.table_rows = rows
+        assert lib.ge2_lp_workspace_bytes(ctypes.byref(d), ctypes.byref(need)) == rc

@@ -166,3 +166,44 @@ def test_rows_finished_in_the_backward_pass(ge2, cuda_device, decoder, D, R, B, 
         results.append(tables)
     for a, b, s in zip(*results, start):
         assert (a - b).abs().max() <= 2e-5 * max(1e-3, float((a - s).abs().max()))
+
+
+@pytest.mark.parametrize("decoder,precision,D,R,form", [
+    ("COMPLEX", "f16", 100, 9, "issued"), ("DISTMULT", "fp32", 64, 9, "resident"), ("DOT", "f16", 50, 1, "resident"), ("COMPLEX", "fp32", 50, 9, "lp_step"),
+    ("DOT", "f16", 100, 1, "lp_step")])
+def test_ids_past_the_table_are_reported_and_write_nothing(ge2, cuda_device, decoder, precision, D, R, form):
+    """The id domain may be larger than the table (a partition buffer that is not full): an id between the two is flagged, and neither the
+    rows behind the table nor the gradient buffer are touched, whether the id occurs once in the batch or more often."""
+    from importlib import import_module
+
+    pipeline = import_module("ge-2_b200.pipeline")
+    rng = np.random.default_rng(D)
+    nodes, past, B, C, N = 700, 900, 96, 3, 64
+    both = [torch.from_numpy(rng.random((nodes + past, D), dtype=np.float32) + 0.1).to(cuda_device) for _ in range(2)]
+    before = [t.clone() for t in both]
+    rels = [torch.from_numpy(rng.random((R, D), dtype=np.float32)).to(cuda_device) for _ in range(4)] if R > 1 else []
+    cfg = pipeline.PipelineConfig(decoder, B, C, N, 0.5, D, R, nodes + past, lr=0.1, precision=precision)
+    pipe = pipeline.BatchPipeline(cfg, both[0][:nodes], both[1][:nodes], *rels)
+    cols = [rng.integers(0, nodes, B)] + ([rng.integers(0, R, B)] if R > 1 else []) + [rng.integers(0, nodes, B)]
+    edges = torch.from_numpy(np.stack(cols, 1).astype(np.int64)).to(cuda_device)
+    edges[3, 0] = nodes + 5                    # once (unless it is drawn too) and twice, as source and destination
+    edges[7, -1] = edges[9, 0] = nodes + past - 1
+    if form == "issued":
+        pipe.step(edges, 0)
+    elif form == "resident":
+        pipe.enqueue_resident(edges, 1)
+    else:                                      # the entry points one by one, every id of the domain mapped: the kernels' own check
+        capi = ge2.capi
+        capi.sample_negatives(edges, edges[:, -1], edges.shape[1], B, C, N, cfg.n_deg, cfg.domain, cfg.sides == 2, 1, 0, pipe.packed, pipe.deg_rows)
+        capi.unique_bitmap(pipe.packed, cfg.domain, out_unique=pipe.unique, out_inverse=pipe.inverse, out_count=pipe.count, out_shared=pipe.ids[0].shared,
+                           twins=pipe.ids[0].twins)
+        capi.lp_step(pipe._make_desc(edges))
+        pipe._update()
+    torch.cuda.synchronize()
+    drawn = pipe.packed[2 * B:]
+    assert int((drawn >= nodes).sum()) > 0     # uniform negatives fall there as well
+    assert int(pipe.status) & 8
+    for t, old in zip(both, before):
+        assert torch.equal(t[nodes:], old[nodes:])
+        assert bool(torch.isfinite(t[:nodes]).all()) and not torch.equal(t[:nodes], old[:nodes])
+    assert float(pipe.node_grad.abs().max()) == 0.0
