@@ -618,13 +618,36 @@ extern "C" int ge2_copy_slabs(const float* src, float* dst, const int32_t* moves
 }
 
 extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
+    // everything is looked at before the first launch: a call that is refused has changed nothing
     if (t == nullptr || t->lp == nullptr) return GE2_ERR_INVALID_ARGUMENT;
     const ge2_lp_desc& d = *t->lp;
-    int rc = ge2_sample_negatives(t->edges, t->edges + t->cols - 1, t->cols, d.B, d.C, d.N, t->n_deg, t->domain, d.use_inverse, t->seed, t->batch_index,
-                                  t->packed, t->deg_rows, stream);
+    size_t need = 0;
+    int rc = ge2_lp_workspace_bytes(&d, &need);  // also: is the descriptor a valid one?
     if (rc != GE2_OK) return rc;
-    // ids past the table get no local id: they are flagged here, and no later kernel meets them
-    rc = ge2_unique_bitmap_shared(t->packed, t->n_ids, std::min(t->domain, t->table_rows), t->unique_ws, t->unique_ws_bytes, t->unique, t->inverse, t->count, t->shared,
+    if (d.workspace == nullptr || ((uintptr_t)d.workspace & 255) != 0 || d.workspace_bytes < need) return GE2_ERR_WORKSPACE;
+    if (t->edges == nullptr || t->cols <= 0 || t->n_deg < 0 || t->n_deg > d.N || t->domain <= 0 || t->table_rows <= 0) return GE2_ERR_INVALID_ARGUMENT;
+    if (t->packed == nullptr || t->unique == nullptr || t->inverse == nullptr || t->count == nullptr || (t->n_deg > 0 && t->deg_rows == nullptr))
+        return GE2_ERR_INVALID_ARGUMENT;
+    if (t->n_ids != 2 * (int64_t)d.B + (d.use_inverse ? 2 : 1) * (int64_t)d.C * d.N) return GE2_ERR_INVALID_ARGUMENT;  // what the sampler packs
+    if (t->twin_begin < 0 || t->twin_len < 0 || (t->twin_len > 0 && t->twin_begin + 2 * t->twin_len > t->n_ids)) return GE2_ERR_INVALID_ARGUMENT;
+    if (d.deg_sample_rows != nullptr && d.deg_sample_rows == t->deg_rows && d.n_deg != t->n_deg) return GE2_ERR_INVALID_ARGUMENT;
+    if (t->table == nullptr || t->state == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+    // the two halves of the row update, the finish kernel's and the scatter's, share the rows out by the same bytes and have one rate, table and state
+    const bool fused = (d.flags & GE2_LP_HAS_ROW_UPDATE) != 0 && d.node_state != nullptr;
+    if (t->shared != (fused ? d.row_shared : nullptr)) return GE2_ERR_INVALID_ARGUMENT;
+    if (fused && (d.node_emb != t->table || d.node_state != t->state || d.row_index != t->unique || d.emb_stride != d.D || d.node_lr != t->lr ||
+                  d.table_rows != t->table_rows))
+        return GE2_ERR_INVALID_ARGUMENT;
+    if (t->num_dense < 0 || t->num_dense > 2 || t->dense_numel < 0) return GE2_ERR_INVALID_ARGUMENT;
+    for (int k = 0; k < t->num_dense && t->dense_numel > 0; k++)
+        if (t->dense_param[k] == nullptr || t->dense_state[k] == nullptr || t->dense_grad[k] == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+    const int64_t mapped = std::min(t->domain, t->table_rows);  // ids past the table get no local id: they are flagged, and no later kernel meets them
+    if (t->unique_ws == nullptr || ((uintptr_t)t->unique_ws & 255) != 0 || t->unique_ws_bytes < ge2_unique_workspace_bytes(mapped)) return GE2_ERR_WORKSPACE;
+
+    rc = ge2_sample_negatives(t->edges, t->edges + t->cols - 1, t->cols, d.B, d.C, d.N, t->n_deg, t->domain, d.use_inverse, t->seed, t->batch_index,
+                              t->packed, t->deg_rows, stream);
+    if (rc != GE2_OK) return rc;
+    rc = ge2_unique_bitmap_shared(t->packed, t->n_ids, mapped, t->unique_ws, t->unique_ws_bytes, t->unique, t->inverse, t->count, t->shared,
                                   t->twin_begin, t->twin_len, stream);
     if (rc != GE2_OK) return rc;
     rc = ge2_lp_step(&d, stream);

@@ -157,3 +157,59 @@ def test_row_update_needs_the_number_of_table_rows(ge2):
     for rows, rc in ((0, 1), (-1, 1), (40, 0)):
         d.table_rows = rows
         assert lib.ge2_lp_workspace_bytes(ctypes.byref(d), ctypes.byref(need)) == rc
+
+
+def _train_desc(capi):
+    """a whole step that is right in everything but its unique-map workspace, which is looked at last: GE2_ERR_WORKSPACE, and no launch"""
+    p, q = 4096, 8192  # never dereferenced
+    lp = capi.LpDesc(B=8, C=2, N=4, D=16, R=5, U=40, emb_stride=16, edge_stride=1, rel_stride=3, has_relations=1, use_inverse=1,
+                     flags=capi.LP_HAS_ROW_UPDATE, node_lr=0.1, table_rows=100, node_emb=p, node_state=q, row_index=p, row_shared=p, deg_sample_rows=p,
+                     n_deg=2, workspace=p, workspace_bytes=1 << 30)
+    for name in ("src_ids", "dst_ids", "rel_ids", "dst_negs", "src_negs", "node_grad", "loss", "rel", "inv_rel", "rel_grad", "inv_rel_grad"):
+        setattr(lp, name, p)
+    t = capi.TrainDesc(lp=ctypes.pointer(lp), edges=p, cols=3, n_deg=2, domain=100, packed=p, deg_rows=p, n_ids=2 * 8 + 2 * 2 * 4, unique=p, inverse=p, count=p,
+                       shared=p, twin_begin=16, twin_len=8, table=p, state=q, table_rows=100, lr=0.1, dense_lr=0.1, grad_scale=1.0, num_dense=2,
+                       dense_numel=80)
+    for k in range(2):
+        t.dense_param[k] = t.dense_state[k] = t.dense_grad[k] = p
+    return t, lp
+
+
+def test_whole_step_refuses_what_does_not_fit_together(ge2):
+    lib, capi = ge2.load_library(), ge2.capi
+    call = lambda t: lib.ge2_train_step(ctypes.byref(t), None)  # noqa: E731
+    t, lp = _train_desc(capi)
+    assert call(t) == 3
+    t.dense_param[1] = None
+    assert call(t) == 1
+    for name, value in [("num_dense", 3), ("num_dense", -1), ("n_ids", 31), ("n_ids", 24), ("shared", 8192), ("shared", None), ("lr", 0.2), ("table", 8192),
+                        ("state", 4096), ("unique", 8192), ("table_rows", 99), ("table_rows", 0), ("domain", 0), ("cols", 0), ("n_deg", 5), ("n_deg", 1),
+                        ("edges", None), ("packed", None), ("inverse", None), ("count", None), ("deg_rows", None), ("twin_len", 9), ("twin_begin", -1)]:
+        t, lp = _train_desc(capi)
+        setattr(t, name, value)
+        assert call(t) == 1, (name, value)
+    for name, value in [("B", 0), ("emb_stride", 32), ("flags", 0), ("node_lr", 0.3), ("table_rows", 101), ("use_inverse", 0)]:
+        t, lp = _train_desc(capi)
+        setattr(lp, name, value)
+        assert call(t) == 1, (name, value)
+    t, lp = _train_desc(capi)
+    lp.workspace_bytes = 0
+    assert call(t) == 3
+
+
+def test_train_struct_matches_header(ge2):
+    import subprocess
+    import tempfile
+
+    src = ('#include "ge2_b200.h"\n#include <stdio.h>\n#include <stddef.h>\nint main(){printf("%zu %zu %zu %zu", sizeof(ge2_train_desc), '
+           'offsetof(ge2_train_desc, shared), offsetof(ge2_train_desc, num_dense), offsetof(ge2_train_desc, dense_numel));return 0;}')
+    with tempfile.TemporaryDirectory() as td:
+        c = Path(td) / "p.c"
+        c.write_text(src)
+        exe = Path(td) / "p"
+        r = subprocess.run(["gcc", "-std=c99", "-I", str(ROOT / "include"), str(c), "-o", str(exe)], capture_output=True, text=True)
+        if r.returncode != 0:
+            pytest.skip("no C compiler: " + r.stderr[:80])
+        size, shared, dense, numel = map(int, subprocess.run([str(exe)], capture_output=True, text=True).stdout.split())
+    T = ge2.capi.TrainDesc
+    assert ctypes.sizeof(T) == size and T.shared.offset == shared and T.num_dense.offset == dense and T.dense_numel.offset == numel
