@@ -44,7 +44,7 @@ struct EvalArgs {
     __half* Qsplit;               // [2][S * Bp][ld] the same, divided by qinv, as a sum of two fp16 terms (the second holds what the first leaves)
     float* qinv;                  // [S][Bp] a power of two: the row's largest element divided by it is near 2^8
     float* pos;                   // [S][Bp] positive scores; +inf for rows without a rank
-    float* qnorm;                 // [S][Bp] 2-norm of the query rows, rounded up; -1 for rows without a rank (padding, bad ids)
+    float* qnorm;                 // [S][Bp] 2-norm of the query rows, rounded up (infinity: decide nothing); -1 for rows without a rank (padding, bad ids)
     unsigned long long* hash;     // open-addressing set of filter pairs already applied (keys are pair + 1, 0 = empty)
     int64_t hash_slots;           // power of two
     uint2* open_list;             // (query row, candidate column) of comparisons the counting pass left open
@@ -181,8 +181,10 @@ __global__ void __launch_bounds__(kPrepThreads) eval_prep_kernel(EvalArgs a) {
     } else if (tid < 2 * kPrepRows) {
         const int lr = tid - kPrepRows;
         float sumsq = 0.f;
-        for (int k = 0; k < D; k++) sumsq = fmaf(sq[lr][k], sq[lr][k], sumsq);
-        a.qnorm[w0 + lr] = s_a[lr] >= 0 ? sqrtf(sumsq) * 1.001f : -1.f;
+        // of the scaled row, whose largest element is 2^8 or more: squares of the row itself vanish below 2.6e-23.  A row that has no such
+        // scale (zeros, elements at the end of the range, infinities and NaN) leaves everything undecided.
+        for (int k = 0; k < D; k++) sumsq = fmaf(sq[lr][k] * s_scale[lr], sq[lr][k] * s_scale[lr], sumsq);
+        a.qnorm[w0 + lr] = s_a[lr] < 0 ? -1.f : sumsq >= 65536.f ? sqrtf(sumsq) * 1.001f / s_scale[lr] : INFINITY;
     }
 }
 

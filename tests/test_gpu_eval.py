@@ -111,3 +111,22 @@ def test_ranks_are_exact_at_tile_edges_and_on_ties(capi, cuda_device, nodes, B, 
     t = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
     got, none = capi.eval_ranks("DISTMULT", t(table), t(edges), dst_filter=t(filt))
     assert none is None and np.array_equal(got.cpu().numpy(), exp)
+
+
+@pytest.mark.parametrize("D,size", [(64, 1e-23), (64, 3e-23), (100, 1e-22), (50, 1e-28), (64, 2e-36), (128, 1e-36), (64, 1e-38), (64, 1e-41), (100, 1e19), (64, 3e37)])
+def test_ranks_are_exact_for_query_rows_of_any_size(capi, cuda_device, D, size):
+    """Query rows (source times relation) so small that their squares vanish, down to numbers that are not normal, and so large that they
+    overflow: a comparison may be decided on the tensor cores only by a bound that holds there too."""
+    rng = np.random.default_rng(D)
+    nodes, R, B = 700, 4, 150
+    cand = 5e-3 if size < 1 else 1.0
+    table = (rng.standard_normal((nodes, D)) * cand).astype(np.float32)
+    table[5] = table[6]
+    rel = (rng.standard_normal((R, D)) * (size / cand)).astype(np.float32)
+    edges = np.stack([rng.integers(0, nodes, B), rng.integers(0, R, B), rng.integers(0, nodes, B)], 1).astype(np.int64)
+    filt = np.stack([rng.integers(0, B, B), rng.integers(0, nodes, B)], 1).astype(np.int64)
+    with np.errstate(over="ignore", invalid="ignore", under="ignore"):
+        exp_d, exp_s = O.eval_ranks("DISTMULT", table, rel, rel, edges, filt, filt)
+    t = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
+    got_d, got_s = capi.eval_ranks("DISTMULT", t(table), t(edges), t(rel), t(rel), dst_filter=t(filt), src_filter=t(filt))
+    assert np.array_equal(got_d.cpu().numpy(), exp_d) and np.array_equal(got_s.cpu().numpy(), exp_s)
