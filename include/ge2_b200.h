@@ -443,16 +443,7 @@ GE2_API int ge2_eval_ranks(const ge2_eval_desc *desc, ge2_stream_t stream);
  * selector's, which is also what equal pointers mean).  The reference's groups_per_tile only sizes its temporary score
  * matrix; no score matrix is stored here.  chunks <= 65535.
  * ===================================================================================================== */
-#define GE2_SELECTED_DOT 1 /* The same with scratch for the form that sorts the pairs by negative (8-byte aligned; 0 bytes: the sizes do not call for it, and
- * without the scratch the gradients are the same, summed in another order). */
-GE2_API size_t ge2_selected_neg_backward_workspace_bytes(int kind, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs, int64_t num_selected,
-                                                         int D);
-GE2_API int ge2_selected_neg_scores_backward_ws(int kind, const float *grad_out, const float *chunked, const float *negatives,
-                                                const int64_t *selected, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs,
-                                                int64_t num_selected, int D, float *grad_chunked, float *grad_negatives, int32_t *status,
-                                                void *workspace, size_t workspace_bytes, ge2_stream_t stream);
-
-/* the values of the reference's SelectedNegScoreKind */
+#define GE2_SELECTED_DOT 1 /* the values of the reference's SelectedNegScoreKind */
 #define GE2_SELECTED_L2 2
 GE2_API int ge2_selected_neg_scores(int kind, const float *chunked, const float *negatives, const int64_t *selected, int64_t chunks,
                                     int64_t rows_per_chunk, int64_t num_negs, int64_t num_selected, int D, float *out_scores,
@@ -461,6 +452,14 @@ GE2_API int ge2_selected_neg_scores_backward(int kind, const float *grad_out, co
                                              const int64_t *selected, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs,
                                              int64_t num_selected, int D, float *grad_chunked, float *grad_negatives, int32_t *status,
                                              ge2_stream_t stream);
+/* The same with scratch for the form that sorts the pairs by negative: ge2_selected_neg_backward_workspace_bytes() bytes, 8-byte aligned
+ * (0 bytes: the sizes do not call for it).  Without the scratch the gradients are the same, summed in another order. */
+GE2_API size_t ge2_selected_neg_backward_workspace_bytes(int kind, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs, int64_t num_selected,
+                                                         int D);
+GE2_API int ge2_selected_neg_scores_backward_ws(int kind, const float *grad_out, const float *chunked, const float *negatives,
+                                                const int64_t *selected, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs,
+                                                int64_t num_selected, int D, float *grad_chunked, float *grad_negatives, int32_t *status,
+                                                void *workspace, size_t workspace_bytes, ge2_stream_t stream);
 GE2_API int ge2_tournament_select(const float *selector_chunked, const float *selector_negatives, const float *score_chunked,
                                   const float *score_negatives, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs,
                                   int64_t num_selected, int D, float *out_scores, int64_t *out_idx, ge2_stream_t stream);

@@ -213,3 +213,13 @@ def test_train_struct_matches_header(ge2):
         size, shared, dense, numel = map(int, subprocess.run([str(exe)], capture_output=True, text=True).stdout.split())
     T = ge2.capi.TrainDesc
     assert ctypes.sizeof(T) == size and T.shared.offset == shared and T.num_dense.offset == dense and T.dense_numel.offset == numel
+
+
+def test_comments_of_the_header_stand_where_they_belong():
+    """a comment that runs on behind a #define must not swallow the declarations after it or be swallowed by them"""
+    text = (ROOT / "include" / "ge2_b200.h").read_text()
+    for line in text.splitlines():
+        if line.startswith("#define") and "/*" in line and "GE2_PRECISION" not in line:
+            assert line.rstrip().endswith("*/"), line
+    kinds = text[text.index("#define GE2_SELECTED_DOT"):].splitlines()[:2]
+    assert kinds[0].split()[:3] == ["#define", "GE2_SELECTED_DOT", "1"] and kinds[1].split() == ["#define", "GE2_SELECTED_L2", "2"]
