@@ -249,13 +249,14 @@ class BatchPipeline:
         self._backward_and_update(self._make_desc(edges), scores_events, rel_hook)
 
     def _train_desc(self, edges):
-        """The arguments of a whole host-issued step: laid out once, and again whenever a table or a rate was replaced; of the rest only
-        the batch's address and number change from step to step."""
+        """The arguments of a whole host-issued step: laid out once, and again whenever a table was replaced or any field of the
+        configuration changed; of the rest only the batch's address and number change from step to step."""
         cfg = self.cfg
-        key = (self.table.data_ptr(), self.state.data_ptr(), self.node_grad.data_ptr(), cfg.lr, cfg.dense_lr, self.grad_scale, edges.shape[1])
+        key = (*vars(cfg).values(), self.table.data_ptr(), self.table.shape[0], self.state.data_ptr(), self.node_grad.data_ptr(), self.status.data_ptr(),
+               self.grad_scale, edges.shape[1])
         if cfg.has_relations:
             tabs = (self.rel, self.rel_state, self.rel_grad) + ((self.inv_rel, self.inv_rel_state, self.inv_rel_grad) if cfg.sides == 2 else ())
-            key += tuple(a.data_ptr() for a in tabs)
+            key += (self.rel.numel(), *(a.data_ptr() for a in tabs))
         if key == getattr(self, "_train_key", None):
             return self._train
         ids = self.ids[0]

@@ -207,3 +207,35 @@ def test_ids_past_the_table_are_reported_and_write_nothing(ge2, cuda_device, dec
         assert torch.equal(t[nodes:], old[nodes:])
         assert bool(torch.isfinite(t[:nodes]).all()) and not torch.equal(t[:nodes], old[:nodes])
     assert float(pipe.node_grad.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("change", [dict(seed=7), dict(degree_fraction=0.25), dict(domain=2500), dict(decoder="COMPLEX"), dict(lr=0.01), dict(dense_lr=0.02)])
+def test_issued_steps_follow_changes_of_the_configuration(ge2, cuda_device, change):
+    """step() keeps its launch arguments between calls: a field that the caller changes in between counts from the next step on, as in a
+    pipeline that was made with it."""
+    from dataclasses import replace
+    from importlib import import_module
+
+    pipeline = import_module("ge-2_b200.pipeline")
+    nodes, B, C, N, D, R = 3000, 200, 2, 64, 32, 6
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(5)
+    start = [torch.rand((r, D), generator=gen, device=cuda_device) * 0.5 + 0.1 for r in (nodes, nodes, R, R, R, R)]
+    edges = [torch.stack([torch.randint(m, (B,), generator=gen, device=cuda_device) for m in (2500, R, 2500)], 1).contiguous() for _ in range(2)]
+    results = []
+    for made_with_it in (False, True):
+        cfg = pipeline.PipelineConfig("DISTMULT", B, C, N, 0.5, D, R, nodes, lr=0.1)
+        tables = [t.clone() for t in start]
+        pipe = pipeline.BatchPipeline(cfg, *tables)
+        pipe.step(edges[0], 0)
+        if made_with_it:
+            pipe = pipeline.BatchPipeline(replace(cfg, **change), *tables)
+        else:
+            for name, value in change.items():
+                setattr(cfg, name, value)
+        pipe.step(edges[1], 1)
+        pipe.check_status()
+        results.append([pipe.packed.clone()] + tables)
+    assert torch.equal(results[0][0], results[1][0])
+    for a, b in zip(results[0][1:], results[1][1:]):
+        assert (a - b).abs().max() <= 2e-5 * b.abs().max()  # sums of gradients in another order
