@@ -302,9 +302,21 @@ class BatchPipeline:
         """Milliseconds per scores phase (the clearing of dK plus the scores launches) as it runs inside a replayed graph:
         `reps` phases captured back to back on the operands the last step left in the workspace, bracketed by events.
         Host-issued launches of the same phase carry a few microseconds of launch gaps that a graph replay does not have.
-        (phases: 1 = prepare, 2 = scores, 4 = finish, as in ge2_lp_desc.)"""
+        (phases: 1 = prepare, 2 = scores, 4 = finish, as in ge2_lp_desc.  The finish kernel trains rows and adds to the gradient
+        buffers: it is timed on copies of them.)"""
         desc = self._make_desc(edges_all, self.ids[0].rel_ids, 1)
         desc.phases = phases
+        scratch = []
+        if phases & 4:
+            def copy(name, t):
+                scratch.append(t.clone())
+                setattr(desc, name, scratch[-1].data_ptr())
+
+            copy("node_emb", self.table), copy("node_state", self.state), copy("node_grad", self.node_grad), copy("loss", self.loss)
+            if self.cfg.has_relations:
+                copy("rel_grad", self.rel_grad)
+                if self.cfg.sides == 2:
+                    copy("inv_rel_grad", self.inv_rel_grad)
         capi.lp_step(desc)
         torch.cuda.synchronize(self.device)
         g = torch.cuda.CUDAGraph()

@@ -239,3 +239,23 @@ def test_issued_steps_follow_changes_of_the_configuration(ge2, cuda_device, chan
     assert torch.equal(results[0][0], results[1][0])
     for a, b in zip(results[0][1:], results[1][1:]):
         assert (a - b).abs().max() <= 2e-5 * b.abs().max()  # sums of gradients in another order
+
+
+def test_timing_a_phase_trains_nothing(ge2, cuda_device):
+    from importlib import import_module
+
+    pipeline = import_module("ge-2_b200.pipeline")
+    nodes, B, C, N, D, R = 3000, 200, 2, 64, 100, 6
+    gen = torch.Generator(device=cuda_device)
+    gen.manual_seed(8)
+    tables = [torch.rand((r, D), generator=gen, device=cuda_device) + 0.1 for r in (nodes, nodes, R, R, R, R)]
+    edges = torch.stack([torch.randint(m, (B,), generator=gen, device=cuda_device) for m in (nodes, R, nodes)], 1).contiguous()
+    pipe = pipeline.BatchPipeline(pipeline.PipelineConfig("COMPLEX", B, C, N, 0.5, D, R, nodes, precision="f16"), *tables)
+    pipe.enqueue_resident(edges, 1)
+    kept = tables + [pipe.node_grad, pipe.rel_grads, pipe.loss]
+    before = [t.clone() for t in kept]
+    for phase in (4, 1, 2):
+        assert pipe.time_scores_phase(edges, 3, phase) > 0
+    for t, old in zip(kept, before):
+        assert torch.equal(t, old)
+    pipe.check_status()
