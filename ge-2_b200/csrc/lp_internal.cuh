@@ -9,6 +9,7 @@
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <math.h>
 
 #include "common.cuh"
 
@@ -52,10 +53,25 @@ inline size_t lp_align(size_t x) { return (x + 255) & ~(size_t)255; }
 
 __host__ __device__ inline int lp_row_ld(int D) { return D <= 64 ? 64 : 128; }
 
-// Which of the two fp16 forms a step takes: while dK stays in the L2 beside the operands, adding the row blocks' parts up there is
-// the faster one: 25 000 edges, C N = 50 000, D = 128, two sides (49 MB of dK) 149 us against 156, 50 000 edges and 98 MB 403 against 283.
+// Which of the two fp16 forms a step takes.  The two-pass form adds every row block's part into dK, which is the faster way while dK stays in
+// the L2 beside the operands.  The streaming form writes every row once, but each of its blocks costs a fill and a drain of the pipeline,
+// and more where a block is cut between CTAs: of its two launches the one over the negatives has T blocks a chunk (T tiles of 128 negatives) with
+// only as many tiles each as the chunk has row blocks.  So the line in bytes of dK rises with T and falls with the row blocks, less steeply
+// for rows of 64 columns, whose tiles are half the traffic; without cuts it stays at 64 MB.  And where T is small and the last tile
+// mostly padding, the line is twice as high: the two-pass form skips the columns that do not exist.
+// Both forms at 2 370 shapes (chunks of 64 ... 2 000 rows, 100 ... 66 001 negatives, dK of 60 ... 290 MB, two sides); D = 100, us, two-pass : streaming
+//   10 000 negatives, 68 MB: 64 rows a chunk 46 : 149, 2 000 rows 331 : 353    1 300 negatives, 66 MB: 64 rows 47 : 76, 2 000 rows 398 : 380
+//   2 000 negatives, 96 MB: 64 rows 76 : 88, 384 rows 141 : 126, 2 000 rows 672 : 468    300 negatives, 153 MB: 64 rows 129 : 137, 500 rows 318 : 357
+//   1 000 negatives, 72 MB, 74 chunks (no cuts): 64 rows 54 : 46, 2 000 rows 540 : 352
+// At 96 of them the line takes the form that is more than 5 % slower (with 64 MB whatever the shape: at 520, up to 3.2 times slower).
 inline bool lp_uses_flash(const ge2_lp_desc& d, int S, int64_t CN, int ld) {
-    return d.precision == GE2_PRECISION_F16 && S * CN * ld * 4 > (int64_t)64 << 20;
+    if (d.precision != GE2_PRECISION_F16) return false;
+    const int64_t T = ceil_div<int64_t>(d.N, 128);
+    const double row_blocks = ceil_div(rows_per_chunk(d.B, d.C), 128), mb = (double)S * CN * ld * 4 / (1 << 20);
+    if (S * d.C * T % kNumSMs == 0) return mb > 64;
+    const double over = ld == 128 ? 4.0 * (T - 1) : T > 8 ? 2.0 * (T - 8) : 0.0;
+    const bool padded = ld == 128 && T >= 3 && T <= 6 && 128 * T * 8 > 9 * (int64_t)d.N;
+    return mb > (64 + over / (row_blocks * sqrt(row_blocks))) * (padded ? 2 : 1);
 }
 
 inline LpLayout lp_make_layout(const ge2_lp_desc& d, void* base) {

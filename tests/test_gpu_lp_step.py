@@ -226,10 +226,43 @@ def test_split_operand_tiles_at_their_edges(capi, cuda_device, kind, B, C, N, D)
 
 @pytest.mark.parametrize("kind,B,C,N,D", [("DISTMULT", 130, 1, 66001, 128), ("COMPLEX", 210, 70, 1000, 66), ("DISTMULT", 300, 2, 70001, 50), ("COMPLEX", 1290, 10, 7003, 100)])
 def test_streaming_softmax_tiles_at_their_edges(capi, cuda_device, kind, B, C, N, D):
-    """The fp16 form for a dK that does not stay in the L2: blocks shared by many CTAs, chunks of three rows, one row past a tile; then scores
-    large enough that the reference of a row has to move."""
+    """The fp16 path with a dK that does not stay in the L2 (which of its forms a shape gets: lp_uses_flash; the streaming one at sizes of its
+    own below): blocks shared by many CTAs, chunks of three rows, one row past a tile; then scores large enough that the reference of a row
+    has to move."""
     for scale in (1.0, 6.0):
         case = workloads.make_case(kind, B, C, N, D, 5, 150, N // 2, 77 + D)
+        case.emb *= np.float32(scale)
+        o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
+        got = run_lp_step(capi, case, cuda_device, "f16", "pairs", dump_scores=False)
+        assert got["status"] == 0
+        assert abs(got["loss"] - o.loss) <= 1e-2 * abs(o.loss)
+        for key in ("node_grad", "rel_grad", "inv_rel_grad"):
+            assert rel_err(got[key], getattr(o, key)) <= 1e-2, key
+
+
+@pytest.mark.parametrize("kind,B,C,N,D", [
+    ("DISTMULT", 98, 49, 2000, 128), ("DISTMULT", 136, 68, 2000, 128),      # one row block a chunk, many tiles: either side of the line
+    ("COMPLEX", 9472, 74, 1000, 66), ("COMPLEX", 9576, 76, 1000, 66),       # as many chunk sides as SMs, so no block is cut, and a few more
+    ("DISTMULT", 1500, 500, 300, 66), ("DISTMULT", 1440, 480, 300, 66),     # a last tile that is mostly padding
+    ("DISTMULT", 200, 90, 2000, 50), ("DISTMULT", 200, 70, 2000, 50),       # rows of 64 columns
+])
+def test_both_fp16_forms_where_the_rule_between_them_lies(capi, cuda_device, kind, B, C, N, D):
+    case = workloads.make_case(kind, B, C, N, D, 5, 150, min(N, 50), 9 + D)
+    o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
+    got = run_lp_step(capi, case, cuda_device, "f16", "pairs", dump_scores=False)
+    assert got["status"] == 0
+    assert abs(got["loss"] - o.loss) <= 1e-2 * abs(o.loss)
+    for key in ("node_grad", "rel_grad", "inv_rel_grad"):
+        assert rel_err(got[key], getattr(o, key)) <= 1e-2, key
+
+
+@pytest.mark.parametrize("kind,B,C,N,D", [
+    ("DISTMULT", 3870, 30, 4001, 128), ("COMPLEX", 330, 110, 1000, 66), ("DISTMULT", 7740, 60, 3001, 50), ("COMPLEX", 640, 160, 1000, 50)])
+def test_streaming_softmax_where_it_is_taken(capi, cuda_device, kind, B, C, N, D):
+    """as test_streaming_softmax_tiles_at_their_edges, at sizes that the rule gives to that form: blocks cut between many CTAs, chunks of three
+    rows, one row past a tile, scores large enough that the reference of a row has to move"""
+    for scale in (1.0, 6.0):
+        case = workloads.make_case(kind, B, C, N, D, 5, 150, min(N, 500), 77 + D)
         case.emb *= np.float32(scale)
         o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
         got = run_lp_step(capi, case, cuda_device, "f16", "pairs", dump_scores=False)
