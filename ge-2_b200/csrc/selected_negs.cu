@@ -478,20 +478,50 @@ __global__ void __launch_bounds__(kRowsThreads, 1) pair_columns_kernel(PairArgs 
     }
 }
 
-// How a problem is cut for the kernels above; usable == false: the rows are gathered from L2.
+// How a problem is cut for the kernels above.  possible: they can take it; taken: they do, otherwise the rows are gathered from L2.
 struct PairCut {
-    bool usable;
+    bool possible, taken;
     int ns, W4, L;      // slices of the negatives
     int cpc, cpc_rows;  // CTAs a chunk: negatives resident, query rows resident
     int L_rows;
 };
-inline PairCut pair_cut(const PairArgs& a) {
+enum PairOp { kOpScores = 0, kOpBackwardDot = 1, kOpBackwardL2 = 2 };
+inline PairOp backward_op(int kind) { return kind == GE2_SELECTED_L2 ? kOpBackwardL2 : kOpBackwardDot; }
+
+// Which form is the faster one, as an estimate of both in us: sums of what either spends its time on, fitted to both forms' times at 1 400
+// shapes (1 ... 320 chunks of 20 ... 5 000 rows, 50 ... 2 500 negatives, 1 ... 500 chosen, D = 16 ... 128; 10 to 15 % off a time on average).
+//   gather    a pair, and its columns; the longest warp's pairs one after the other; a row; a pair read element by element
+//   resident  a wave of CTAs (chunks beyond one an SM, or that do not divide the SMs, leave some of them idle); filling shared memory once
+//             a slice; a turn of the CTA's warps over a row, over 32 of its pairs, over their columns; for the negatives' gradient also a
+//             block's rows and pairs (sorted, then summed) and the negatives that it goes through
+// Backward, dot, gathered : resident: 7 chunks of 1 428 rows x 4 pairs, 2 310 negatives, D = 128: 11 : 84 us; 5 x 2 192 x 31, 1 980, 50: 34 : 81;
+// 14 x 353 x 179, 461, 128: 107 : 74; 128 x 613 x 60, 966, 16: 322 : 159.  At 900 further shapes the form taken is 0.5 - 0.7 % behind the better
+// one on average (with a line at four pairs a negative and CTA: 19 - 34 %, up to 11 times).
+inline bool resident_pays(const PairArgs& a, const PairCut& p, PairOp op) {
+    static constexpr double kGather[3][6] = {
+        {2.7, 3.0e-5, 1.8e-7, 0.15, 1.9e-4, 4.0e-6}, {4.1, 1.94e-5, 1.83e-6, 0.20, 1.7e-4, 1.42e-5}, {4.25, 6.44e-5, 7.5e-7, 0.36, 1.9e-4, 1.97e-5}};
+    static constexpr double kRows[3][5] = {{2.6, 3.7e-4, 0.99, 0.40, 0.0127}, {0.0, 7.5e-4, 0.61, 0.42, 0.0038}, {0.0, 1.34e-3, 1.48, 1.26, 0.0079}};
+    static constexpr double kColumns[3][5] = {{0.0, 0.0, 0.0, 0.0, 0.0}, {9.8, 9.9e-4, 6.9e-3, 1.12e-3, 1.05e-3}, {12.5, 1.63e-3, 7.6e-3, 1.13e-3, 1.53e-3}};
+    const int64_t chunks = a.rows / a.R, warps = (int64_t)kNumSMs * 8 * kPairWarps;
+    const double pairs = (double)a.rows * a.K, D4 = (a.D + 3) / 4;
+    const double* g = kGather[op];
+    const double gather = g[0] + pairs * (g[1] + g[2] * D4 + (a.D % 4 != 0 ? g[5] : 0.0)) + g[3] * ceil_div<int64_t>(a.rows, warps) * a.K + g[4] * a.rows;
+    const double turns = (double)p.ns * ceil_div<int64_t>(ceil_div<int64_t>(a.R, p.cpc), kRowsWarps);
+    const double* r = kRows[op];
+    double resident = ceil_div<int64_t>(chunks * p.cpc, kNumSMs) *
+                      (r[0] + r[1] * p.ns * a.N * p.W4 + turns * (r[2] + r[3] * ceil_div<int64_t>(a.K, 32) + r[4] * a.K * p.L));
+    const double block = (double)ceil_div<int64_t>(a.R, p.cpc_rows);
+    const double* c = kColumns[op];
+    resident += ceil_div<int64_t>(chunks * p.cpc_rows, kNumSMs) * (c[0] + c[2] * a.N + block * (c[1] * D4 + a.K * (c[3] + c[4] * p.L_rows)));
+    return resident < gather;
+}
+
+inline PairCut pair_cut(const PairArgs& a, PairOp op) {
     PairCut p = {};
     const int64_t chunks = a.R > 0 ? a.rows / a.R : 0;
     const int D4 = (a.D + 3) / 4;
     const int64_t w4 = a.N > 0 ? kPairSmem / (16 * (a.N + 1)) : 0;
-    // Filling shared memory costs every CTA its chunk's negatives once (4 N D bytes); it pays when the CTA's pairs gather several times
-    // that.  A slice narrower than four pieces would leave most lanes idle, and a block's pairs are counted in 31 bits.
+    // A slice narrower than four pieces would leave most lanes idle, and a block's pairs are counted in 31 bits.
     if (chunks < 1 || a.K < 1 || w4 < 4 || chunks > 65535 || a.K > (1 << 20) || a.R > (1 << 24)) return p;
     p.ns = (int)ceil_div<int64_t>(D4, w4);
     p.W4 = ceil_div(D4, p.ns);
@@ -500,8 +530,8 @@ inline PairCut pair_cut(const PairArgs& a) {
     const int64_t most_rows = (kPairSmem - 4 * a.N) / (16 * D4) - 2;
     p.cpc_rows = (int)std::max<int64_t>(p.cpc, ceil_div<int64_t>(a.R, most_rows));
     p.L_rows = ceil_div(D4, 8);
-    const int64_t per_cta = ceil_div<int64_t>(a.R, p.cpc) * a.K;
-    p.usable = per_cta >= 4 * a.N && per_cta < (1 << 30);
+    p.possible = ceil_div<int64_t>(a.R, p.cpc) * a.K < (1 << 30);
+    p.taken = p.possible && resident_pays(a, p, op);
     return p;
 }
 
@@ -869,8 +899,8 @@ extern "C" int ge2_selected_neg_scores(int kind, const float* chunked, const flo
     if (out_scores == nullptr) return GE2_ERR_INVALID_ARGUMENT;
     const PairArgs a = pair_args(kind, chunked, negatives, selected, chunks, rows_per_chunk, num_negs, num_selected, D, status);
     const bool vec = rows_are_vectors(D, chunked, negatives, nullptr, nullptr);
-    const PairCut cut = pair_cut(a);
-    if (cut.usable)
+    const PairCut cut = pair_cut(a, kOpScores);
+    if (cut.taken)
         return kind == GE2_SELECTED_DOT ? launch_pair_rows<GE2_SELECTED_DOT, kPairScores>(a, cut, vec, nullptr, out_scores, as_stream(stream_))
                                         : launch_pair_rows<GE2_SELECTED_L2, kPairScores>(a, cut, vec, nullptr, out_scores, as_stream(stream_));
     const dim3 grid((unsigned)stream_grid(rows, kPairWarps));
@@ -897,7 +927,7 @@ extern "C" int ge2_selected_neg_scores_backward(int kind, const float* grad_out,
 extern "C" size_t ge2_selected_neg_backward_workspace_bytes(int kind, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs, int64_t num_selected, int D) {
     if (chunks <= 0 || rows_per_chunk <= 0 || num_negs <= 0 || num_selected <= 0 || D <= 0 || D > kMaxD) return 0;
     const PairArgs a = pair_args(kind, nullptr, nullptr, nullptr, chunks, rows_per_chunk, num_negs, num_selected, D, nullptr);
-    if (!pair_cut(a).usable) return 0;
+    if (!pair_cut(a, backward_op(kind)).possible) return 0;
     return (size_t)(a.rows * a.K) * (kind == GE2_SELECTED_L2 ? 12 : 8);  // sorted (weight, row) pairs; L2: the weights themselves too
 }
 
@@ -919,8 +949,8 @@ extern "C" int ge2_selected_neg_scores_backward_ws(int kind, const float* grad_o
     const PairArgs a = pair_args(kind, chunked, negatives, selected, chunks, rows_per_chunk, num_negs, num_selected, D, status);
     const bool vec = rows_are_vectors(D, chunked, negatives, grad_chunked, grad_negatives);
     const size_t need = ge2_selected_neg_backward_workspace_bytes(kind, chunks, rows_per_chunk, num_negs, num_selected, D);
-    if (need > 0 && workspace != nullptr && workspace_bytes >= need && ((uintptr_t)workspace & 7) == 0) {
-        const PairCut cut = pair_cut(a);
+    const PairCut cut = pair_cut(a, backward_op(kind));
+    if (cut.taken && workspace != nullptr && workspace_bytes >= need && ((uintptr_t)workspace & 7) == 0) {
         float2* sorted = reinterpret_cast<float2*>(workspace);
         float* coeffs = reinterpret_cast<float*>(sorted + rows * num_selected);
         if (kind == GE2_SELECTED_DOT) {

@@ -52,7 +52,7 @@ def test_selected_scores_forward_and_backward(capi, cuda_device, C, R, N, D, K, 
 ])
 @pytest.mark.parametrize("kind,code", [("DOT", O.SELECTED_DOT), ("L2", O.SELECTED_L2)])
 def test_rows_resident_in_shared_memory(capi, cuda_device, C, R, N, D, K, kind, code):
-    assert capi.load_library().ge2_selected_neg_backward_workspace_bytes(code, C, R, N, K, D) > 0  # this form is the one taken
+    assert capi.load_library().ge2_selected_neg_backward_workspace_bytes(code, C, R, N, K, D) > 0  # this form can take them
     rng = np.random.default_rng(N + D)
     q, n, sel = _pairs(rng, C, R, N, D, K)
     grad = rng.standard_normal((C * R, K)).astype(np.float32)
@@ -67,6 +67,41 @@ def test_rows_resident_in_shared_memory(capi, cuda_device, C, R, N, D, K, kind, 
     dq, dn = capi.selected_neg_scores_backward(kind, t(grad), t(q), t(n), t(sel), status)
     _close(dq, exp_dq)
     _close(dn, exp_dn)
+
+
+@pytest.mark.parametrize("C,R,N,D,K,resident", [
+    (148, 400, 130, 101, 60, True), (74, 600, 1664, 128, 250, True), (149, 400, 5, 1, 90, True),   # a ragged row; many slices of the negatives; two waves
+    (74, 400, 3300, 18, 300, True), (3, 3000, 64, 50, 100, True), (62, 900, 299, 128, 90, True),     # the narrowest slice; many CTAs a chunk
+    (7, 1428, 2310, 128, 4, False), (203, 60, 300, 99, 7, False), (1, 40, 50, 16, 3, False),       # few pairs a negative, a second wave, next to nothing
+])
+@pytest.mark.parametrize("kind,code", [("DOT", O.SELECTED_DOT), ("L2", O.SELECTED_L2)])
+def test_the_form_that_the_estimate_takes(capi, cuda_device, C, R, N, D, K, resident, kind, code):
+    """Gradients of either form against the oracle; which one ran shows in the scratch, which only the form with resident rows writes."""
+    lib = capi.load_library()
+    rng = np.random.default_rng(N + D)
+    q, n, sel = _pairs(rng, C, R, N, D, K)
+    grad = rng.standard_normal((C * R, K)).astype(np.float32)
+    t = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
+    dq, dn, scores = torch.empty((C, R, D), device=cuda_device), torch.empty((C, N, D), device=cuda_device), None
+    tq, tn, ts, tg = t(q), t(n), t(sel), t(grad)
+    status = torch.zeros(1, dtype=torch.int32, device=cuda_device)
+    scores = capi.selected_neg_scores(kind, tq, tn, ts, status)
+    need = lib.ge2_selected_neg_backward_workspace_bytes(code, C, R, N, K, D)
+    ws = torch.full((need,), 0xCD, dtype=torch.uint8, device=cuda_device)
+    capi.check(lib.ge2_selected_neg_scores_backward_ws(code, tg.data_ptr(), tq.data_ptr(), tn.data_ptr(), ts.data_ptr(), C, R, N, K, D, dq.data_ptr(),
+                                                       dn.data_ptr(), status.data_ptr(), ws.data_ptr(), need, capi.cur_stream()), "backward")
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    if kind == "DOT":
+        assert bool((ws != 0xCD).any()) == resident
+    some = sorted({0, C // 2, C - 1})  # the oracle for a few chunks: they do not interact
+    pick = lambda a: np.ascontiguousarray(a[some])  # noqa: E731
+    rows = lambda a: np.concatenate([a[c * R:(c + 1) * R] for c in some])  # noqa: E731
+    exp_s = O.selected_neg_scores(pick(q), pick(n), pick(sel), code)
+    exp_dq, exp_dn = O.selected_neg_scores_backward(rows(grad), pick(q), pick(n), pick(sel), code)
+    _close(torch.cat([scores[c * R:(c + 1) * R] for c in some]), exp_s)
+    _close(dq[some], exp_dq)
+    _close(dn[some], exp_dn)
 
 
 def test_selected_column_out_of_range_is_reported_and_skipped(capi, cuda_device):
