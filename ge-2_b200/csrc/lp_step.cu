@@ -44,8 +44,8 @@ __global__ void __launch_bounds__(256) mask_from_pairs_kernel(const int64_t* __r
 // A row of D columns is spread over ld / 4 lanes (16 or 32), four values a lane.
 //   plain   : lane l holds columns [4l, 4l + 4), or (V == 1) columns l, l + ld / 4, l + 2 ld / 4, l + 3 ld / 4, so that scalar accesses
 //             of neighbouring lanes are neighbours
-//   ComplEx : coordinates 2l and 2l + 1 of the h = D / 2 complex ones: .x .y their real parts (columns 2l, 2l + 1), .z .w their
-//             imaginary parts (columns h + 2l, h + 2l + 1), so the relation operator and its backward need no other lane's values
+//   ComplEx : coordinates 2l and 2l + 1 of the h = D / 2 complex ones, or (V == 1) l and l + ld / 4: .x .y their real parts (columns k, k'),
+//             .z .w their imaginary parts (columns h + k, h + k'), so the relation operator and its backward need no other lane's values
 // V is the widest access that the row length and the pointers allow (4 only for plain rows); columns past the row read as zero.
 // ---------------------------------------------------------------------------------------------------
 template <int V, bool CPLX>
@@ -59,8 +59,9 @@ __device__ __forceinline__ float4 load_row(const float* __restrict__ row, int l,
                 v = make_float4(a.x, a.y, b.x, b.y);
             }
         } else {
-            if (k < h) v.x = __ldg(row + k), v.z = __ldg(row + h + k);
-            if (k + 1 < h) v.y = __ldg(row + k + 1), v.w = __ldg(row + h + k + 1);
+            const int n = lp_row_ld(D) >> 2;
+            if (l < h) v.x = __ldg(row + l), v.z = __ldg(row + h + l);
+            if (l + n < h) v.y = __ldg(row + l + n), v.w = __ldg(row + h + l + n);
         }
     } else if constexpr (V == 4) {
         if (k < D) v = __ldg(reinterpret_cast<const float4*>(row + k));
@@ -100,8 +101,9 @@ __device__ __forceinline__ void put_row(float* row, int l, int D, float4 v) {
         if constexpr (V == 2) {
             if (k < h) Put::two(row + k, v.x, v.y), Put::two(row + h + k, v.z, v.w);
         } else {
-            if (k < h) Put::one(row + k, v.x), Put::one(row + h + k, v.z);
-            if (k + 1 < h) Put::one(row + k + 1, v.y), Put::one(row + h + k + 1, v.w);
+            const int n = lp_row_ld(D) >> 2;
+            if (l < h) Put::one(row + l, v.x), Put::one(row + h + l, v.z);
+            if (l + n < h) Put::one(row + l + n, v.y), Put::one(row + h + l + n, v.w);
         }
     } else if constexpr (V == 4) {
         if (k < D) Put::four(row + k, v);
@@ -185,15 +187,15 @@ __device__ __forceinline__ void store_operand(void* rows, int64_t plane, int64_t
         if constexpr (HALF) store_half4((__half*)rows + row * ld + 4 * l, v);
         else store_split4((__nv_bfloat16*)rows + row * ld + 4 * l, plane, v);
     } else {
-        const int k = 2 * l, h = D >> 1;
+        const int k = 2 * l, h = D >> 1, n = ld >> 2;
         uint16_t* p = (uint16_t*)rows + row * ld;
         if constexpr (HALF) {
             const __half2 re = __floats2half2_rn(v.x, v.y), im = __floats2half2_rn(v.z, v.w);
             if constexpr (V == 2) {
                 if (k < h) *reinterpret_cast<__half2*>(p + k) = re, *reinterpret_cast<__half2*>(p + h + k) = im;
             } else {  // an odd h leaves the imaginary parts on odd columns
-                if (k < h) p[k] = __half_as_ushort(re.x), p[h + k] = __half_as_ushort(im.x);
-                if (k + 1 < h) p[k + 1] = __half_as_ushort(re.y), p[h + k + 1] = __half_as_ushort(im.y);
+                if (l < h) p[l] = __half_as_ushort(re.x), p[h + l] = __half_as_ushort(im.x);
+                if (l + n < h) p[l + n] = __half_as_ushort(re.y), p[h + l + n] = __half_as_ushort(im.y);
             }
             for (int c = D + k; c < ld; c += ld >> 1) *reinterpret_cast<uint32_t*>(p + c) = 0u;  // the padding of the row
         } else {
@@ -203,8 +205,8 @@ __device__ __forceinline__ void store_operand(void* rows, int64_t plane, int64_t
                 if constexpr (V == 2) {
                     if (k < h) *reinterpret_cast<__nv_bfloat162*>(p + k) = re, *reinterpret_cast<__nv_bfloat162*>(p + h + k) = im;
                 } else {
-                    if (k < h) p[k] = __bfloat16_as_ushort(re.x), p[h + k] = __bfloat16_as_ushort(im.x);
-                    if (k + 1 < h) p[k + 1] = __bfloat16_as_ushort(re.y), p[h + k + 1] = __bfloat16_as_ushort(im.y);
+                    if (l < h) p[l] = __bfloat16_as_ushort(re.x), p[h + l] = __bfloat16_as_ushort(im.x);
+                    if (l + n < h) p[l + n] = __bfloat16_as_ushort(re.y), p[h + l + n] = __bfloat16_as_ushort(im.y);
                 }
                 for (int c = D + k; c < ld; c += ld >> 1) *reinterpret_cast<uint32_t*>(p + c) = 0u;
                 const float2 fr = __bfloat1622float2(re), fi = __bfloat1622float2(im);
@@ -338,6 +340,9 @@ __global__ void __launch_bounds__(256, 5) lp_prep_kernel(const __grid_constant__
 // Bound by latency on small batches (ids -> rows -> reductions), by HBM on large ones.  With the sparse Adagrad pass that follows:
 // 10 000 edges, 2 x 10 000 negatives, ComplEx 100: 28 us (33 us with every row through the gradient table); 50 000 edges and
 // negatives, Dot 100: 104 us (143 us); 100 000 edges, 2 x 200 000 negatives, DistMult 128: 270 us (465 us).
+// A node in half of the edges and of the degree negatives: the first of these 28 us (31 us with its rows summed in shared memory for a CTA's
+// lifetime), the last with half of the negatives by degree 275 us (461 us).  Scalar reductions feel it most: 7919 edges, 2 x 4571 negatives,
+// ComplEx 50 (25 columns a half): 20 us, 25 us with neighbouring lanes two columns apart (17 us and 17 us without such a node).
 // ---------------------------------------------------------------------------------------------------
 constexpr int kFinWarps = 8;
 constexpr int kNoRow = 2;      // in the place of a node's "occurs again": its row is not one of the table, so nothing is done with it
@@ -359,7 +364,8 @@ template <int V, bool CPLX>
 __device__ __noinline__ void adagrad_row(float* emb, float* state, int l, int D, float4 e, float4 s, float4 g, float neg_lr) {
     // a lane without columns must not divide: 0 / 1e-10 is off the fast path of the division, and the whole warp would wait for it
     const int n = lp_row_ld(D) >> 2;
-    const int cols = CPLX ? (D >> 1) - 2 * l : V == 1 ? (D - l + n - 1) / n : D - 4 * l;  // values of this lane that exist (at least)
+    // values of this lane that exist (at least); ComplEx: pairs of them
+    const int cols = CPLX ? (V == 1 ? ((D >> 1) - l + n - 1) / n : (D >> 1) - 2 * l) : V == 1 ? (D - l + n - 1) / n : D - 4 * l;
     if (cols <= 0) return;
     if (CPLX ? cols == 1 : cols < 4) {
         if (CPLX) s.y = s.w = 1.f;
