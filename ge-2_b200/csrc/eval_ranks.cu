@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kCountThreads, 1)
     __syncthreads();
     if (warp == kMmaWarp) {
         if (*s_abort && lane == 0)  // copies still in flight get a bounded chance to land
-            for (int k = 0; k < SM::kSlots; k++) mbar_wait(&bars[kQFull + k], 0, 1u << 14);
+            for (int k = 0; k < SM::kSlots; k++) settle_bar(&bars[kQFull + k]);
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem, 512);

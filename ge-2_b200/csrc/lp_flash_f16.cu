@@ -649,9 +649,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (*s_abort && lane == 0) {
             // a wait ran out somewhere: give copies and contractions still in flight a bounded chance to land before the SM's shared and
             // tensor memory are handed to the next CTA
-            for (int k = 0; k < kStages; k++) mbar_wait(&bars[kBarYFull + k], 0, 1u << 14);
-            for (int k = 0; k < 2; k++) mbar_wait(&bars[kBarSFull + k], 0, 1u << 14);
-            mbar_wait(&bars[kBarOFull], 0, 1u << 14);
+            for (int k = 0; k < kStages; k++) settle_bar(&bars[kBarYFull + k]);
+            for (int k = 0; k < 2; k++) settle_bar(&bars[kBarSFull + k]);
+            settle_bar(&bars[kBarOFull]);
         }
         __syncwarp();
         tc_fence_after();

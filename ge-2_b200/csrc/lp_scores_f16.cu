@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (*s_abort && lane == 0) {
             // a wait ran out somewhere: give copies still in flight a bounded chance to land before the SM's shared and
             // tensor memory are handed to the next CTA
-            for (int k = 0; k < kStagesA; k++) mbar_wait(&bars[kBarYFull + k], 0, 1u << 14);
+            for (int k = 0; k < kStagesA; k++) settle_bar(&bars[kBarYFull + k]);
         }
         __syncwarp();
         tc_fence_after();
@@ -834,9 +834,9 @@ __global__ void __launch_bounds__(kThreadsB, 1)
     __syncthreads();
     if (warp == kMmaWarp) {
         if (*s_abort && lane == 0) {
-            for (int k = 0; k < kStages; k++) mbar_wait(&bars[kBarYFull + k], 0, 1u << 14);
-            for (int k = 0; k < 2; k++) mbar_wait(&bars[kBarDkFull + k], 0, 1u << 14);
-            mbar_wait(&bars[kBarDqFull], 0, 1u << 14);
+            for (int k = 0; k < kStages; k++) settle_bar(&bars[kBarYFull + k]);
+            for (int k = 0; k < 2; k++) settle_bar(&bars[kBarDkFull + k]);
+            settle_bar(&bars[kBarDqFull]);
         }
         __syncwarp();
         tc_fence_after();

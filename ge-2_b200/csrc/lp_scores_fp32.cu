@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kThreadsA, 1)
     __syncthreads();
     if (warp == kMmaWarpA) {
         if (*s_abort && lane == 0)  // copies still in flight get a bounded chance to land
-            for (int k = 0; k < kLseStages; k++) mbar_wait(&bars[kAYFull + k], 0, 1u << 14);
+            for (int k = 0; k < kLseStages; k++) settle_bar(&bars[kAYFull + k]);
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem, 128);
@@ -586,8 +586,8 @@ __global__ void __launch_bounds__(kThreadsB, 1)
     __syncthreads();
     if (warp == kMmaWarpB) {
         if (*s_abort && lane == 0) {  // copies and contractions still in flight get a bounded chance to land
-            for (int k = 0; k < kYSlots; k++) mbar_wait(&bars[kBYFull + k], 0, 1u << 14);
-            for (int k = 0; k < 2; k++) mbar_wait(&bars[kBGFull + k], 0, 1u << 14);
+            for (int k = 0; k < kYSlots; k++) settle_bar(&bars[kBYFull + k]);
+            for (int k = 0; k < 2; k++) settle_bar(&bars[kBGFull + k]);
         }
         __syncwarp();
         tc_fence_after();

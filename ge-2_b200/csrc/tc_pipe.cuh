@@ -77,6 +77,11 @@ __device__ __forceinline__ bool warp_pipe_wait(uint64_t* bar, uint32_t parity, v
     return __all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0) || warp_pipe_wait_slow(bar, parity, abort_flag, status);
 }
 
+// What may still be on its way when the roles of a kernel have left their loops after a wait that ran out -- a copy into shared memory, a
+// contraction -- gets a bounded chance to land before that memory goes to the next CTA.  The barrier it arrives on is in either phase: one that
+// has completed its phase 0 is in its phase 1.
+__device__ __forceinline__ void settle_bar(uint64_t* bar) { mbar_wait(bar, mbar_try_wait(bar, 0) ? 1u : 0u, 1u << 14); }
+
 // ---- contractions ---------------------------------------------------------------------------------------------------------
 // D (+)= A B^T over the first `steps` k-steps (1 ... 4 NB) of operands of NB 64-column blocks, both K-major.  The number of steps is made a
 // constant of straight-line code: with a test per step a contraction of N = 64 took 71 cycles to issue instead of 48.
