@@ -34,7 +34,7 @@ struct UniqueWorkspace {
     uint32_t* ticket;           // [1]           }
     int32_t* status;            // [1]           } GE2_STATUS_* bits of this call
     unsigned long long* words;  // [num_words]  one bit per id that occurs   } cleared by the same memset
-    unsigned long long* dup;    // [num_words]  ... that occurs again        }
+    unsigned long long* dup;    // [num_words]  ... that occurs again        } (null without out_shared)
     int32_t* word_offsets;      // [num_words]
 };
 
@@ -48,11 +48,11 @@ __device__ __forceinline__ bool is_second_twin(const int64_t* ids, int64_t i, in
 }
 
 constexpr size_t align256c(size_t x) { return (x + 255) & ~(size_t)255; }
-// control words (tile states, ticket, status, one spare), two bitsets, per-word offsets
-constexpr size_t unique_ws_bytes(int64_t domain) {
+// control words (tile states, ticket, status, one spare), one bitset or (for out_shared) two, per-word offsets
+constexpr size_t unique_ws_bytes(int64_t domain, int bitsets) {
     const int64_t nw = (domain + 63) >> 6;
     const int64_t tiles = (nw + kTileWords - 1) / kTileWords;
-    return align256c((size_t)(tiles + 4) * 4) + 2 * align256c((size_t)nw * 8) + align256c((size_t)nw * 4);
+    return align256c((size_t)(tiles + 4) * 4) + bitsets * align256c((size_t)nw * 8) + align256c((size_t)nw * 4);
 }
 
 __host__ __device__ inline int64_t num_words_of(int64_t domain) { return (domain + 63) >> 6; }
@@ -251,7 +251,7 @@ using namespace ge2;
 
 extern "C" size_t ge2_unique_workspace_bytes(int64_t domain) {
     if (domain <= 0) return 0;
-    return unique_ws_bytes(domain);
+    return unique_ws_bytes(domain, 2);  // enough for either form
 }
 
 extern "C" int ge2_unique_bitmap(const int64_t* ids, int64_t n, int64_t domain, void* workspace, size_t workspace_bytes,
@@ -274,7 +274,7 @@ extern "C" int ge2_unique_bitmap_shared(const int64_t* ids, int64_t n, int64_t d
     const int64_t nw = num_words_of(domain);
     if (nw > (int64_t)kValueMask) return GE2_ERR_UNSUPPORTED;
     const int64_t tiles = ceil_div<int64_t>(nw, kTileWords);
-    if (workspace == nullptr || ((uintptr_t)workspace & 255) != 0 || workspace_bytes < ge2_unique_workspace_bytes(domain))
+    if (workspace == nullptr || ((uintptr_t)workspace & 255) != 0 || workspace_bytes < unique_ws_bytes(domain, out_shared != nullptr ? 2 : 1))
         return GE2_ERR_WORKSPACE;
 
     const int64_t cap = n < domain ? n : domain;
@@ -289,15 +289,18 @@ extern "C" int ge2_unique_bitmap_shared(const int64_t* ids, int64_t n, int64_t d
     p += ctl_bytes;
     ws.words = (unsigned long long*)p;
     p += align256c((size_t)nw * 8);
-    ws.dup = (unsigned long long*)p;
-    p += align256c((size_t)nw * 8);
+    ws.dup = nullptr;
+    if (out_shared != nullptr) {
+        ws.dup = (unsigned long long*)p;
+        p += align256c((size_t)nw * 8);
+    }
     ws.word_offsets = (int32_t*)p;
 
     // control words and bitsets are adjacent: one memset; out_count needs none (the scan's last tile writes the count, the
     // inverse kernel the status)
     GE2_CUDA_TRY(cudaMemsetAsync(ws.tile_state, 0, ctl_bytes + (out_shared != nullptr ? align256c((size_t)nw * 8) : 0) + (size_t)nw * 8, stream));
 
-    mark_kernel<<<stream_grid(n, 256), 256, 0, stream>>>(ids, n, domain, ws.words, out_shared != nullptr ? ws.dup : nullptr, tw, ws.status);
+    mark_kernel<<<stream_grid(n, 256), 256, 0, stream>>>(ids, n, domain, ws.words, ws.dup, tw, ws.status);
     GE2_LAUNCH_CHECK();
     const int scan_grid = (int)(tiles < (int64_t)kNumSMs * 8 ? tiles : (int64_t)kNumSMs * 8);
     GE2_CUDA_TRY(launch_after(scan_extract_kernel, dim3((unsigned)scan_grid), dim3(kScanThreads), 0, stream, (const unsigned long long*)ws.words, nw,
@@ -338,7 +341,7 @@ namespace ge2 {
 namespace {
 
 constexpr int64_t kStaticMaxDomain = GE2_UNIQUE_STATIC_MAX_DOMAIN;
-constexpr size_t kStaticBytes = unique_ws_bytes(kStaticMaxDomain);
+constexpr size_t kStaticBytes = unique_ws_bytes(kStaticMaxDomain, 1);
 
 static __device__ __align__(256) unsigned char g_unique_static_scratch[kStaticBytes];
 

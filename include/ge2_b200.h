@@ -76,7 +76,7 @@ GE2_API int ge2_unique_bitmap_shared(const int64_t *ids, int64_t n, int64_t doma
 /* Unique-map for callers that cannot allocate device memory -- a host runtime that owns the whole GPU heap and hands
  * out none of it after start-up, a plugin that only ever receives its input and output buffers, a latency-bound loop
  * that may not call an allocator.  No counterpart in the reference project.  Same results as ge2_unique_bitmap, but
- * the scratch is a fixed array inside the library (about 1.3 MB on every GPU that loads it, held until the process
+ * the scratch is a fixed array inside the library (about 0.8 MB on every GPU that loads it, held until the process
  * exits), so the id domain is limited to GE2_UNIQUE_STATIC_MAX_DOMAIN; a larger domain returns GE2_ERR_UNSUPPORTED.
  * The call makes no cudaMalloc/cudaFree and uses no allocating library routine.  The first call on each device looks
  * up the array's device address; make that first call outside any stream capture.  All calls share the one array,

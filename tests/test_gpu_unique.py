@@ -95,3 +95,22 @@ def test_repeated_ids_and_twins(capi, cuda_device, n, domain):
         assert cnt.tolist() == [ou.size, 0]
         assert np.array_equal(u.cpu().numpy()[:ou.size], ou) and np.array_equal(inv.cpu().numpy(), oinv)
         assert np.array_equal(shared.cpu().numpy()[:ou.size], np.bincount(oinv[counted], minlength=ou.size) > 1)
+
+
+@pytest.mark.parametrize("domain", [1, 64, 8192, 8193, 1_000_003])
+def test_the_form_without_out_shared_needs_one_bitset(capi, cuda_device, domain):
+    """scratch of control words, one bitset and the per-word offsets is enough where repeated ids are not asked for, and nothing behind it is
+    written; with out_shared it is refused"""
+    words, up = (domain + 63) // 64, lambda x: (x + 255) // 256 * 256
+    small = up(((words + 127) // 128 + 4) * 4) + up(words * 8) + up(words * 4)
+    rng = np.random.default_rng(domain)
+    ids_np = rng.integers(0, domain, 5000)
+    ids = torch.from_numpy(ids_np).to(cuda_device)
+    ws = torch.full((small + 4096,), 0xCD, dtype=torch.uint8, device=cuda_device)
+    u, inv, cnt = capi.unique_bitmap(ids, domain, workspace=ws[:small])
+    torch.cuda.synchronize()
+    ou, oinv = O.unique_map_sort(ids_np)
+    assert cnt.tolist() == [ou.size, 0] and np.array_equal(u.cpu().numpy()[:ou.size], ou) and np.array_equal(inv.cpu().numpy(), oinv)
+    assert bool((ws[small:] == 0xCD).all())
+    with pytest.raises(capi.Ge2Error, match="workspace"):
+        capi.unique_bitmap(ids, domain, workspace=ws[:small], out_shared=torch.empty(5000, dtype=torch.uint8, device=cuda_device))
