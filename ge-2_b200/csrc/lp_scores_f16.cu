@@ -44,9 +44,9 @@
 //   warps 16-19 lse pass: warp 16 combines the softmax warps' partials at the end of a block; warps 17-19 clear dK and
 //               the dQ rows of split blocks.  Gradient pass: drain (with warps 23-26): accumulator -> swizzled staging
 //               slab -> TMA store / reduce-add, each warp its lane quarter and every second 32-column slab
-//   warp  20    lane 0: TMA producer (X at the start of a block, the Y ring)
-//   warp  21    lane 0: issues the score contractions; the warp also allocates and frees tensor memory
-//   warp  22    lane 0: issues the dK and dQ contractions of the gradient pass
+//   warp  20    TMA producer (X at the start of a block, the Y ring)
+//   warp  21    issues the score contractions; the warp also allocates and frees tensor memory
+//   warp  22    issues the dK and dQ contractions of the gradient pass
 //   warps 23-26 gradient pass only (864 threads): the second set of drain warps
 // Every mbarrier wait is bounded; a wait that runs out raises GE2_STATUS_PIPE_TIMEOUT and sets a block-wide abort flag
 // that every other wait polls, so all roles fall through to the common exit where tensor memory is released.
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!produce(tma_it)) break;
     } else if (warp == kMmaWarp) {
         // ================================ score contractions ================================
-        // (the whole warp walks the loop; the asynchronous instructions are lane 0's)
+        // (the whole warp walks the loop; elect.sync picks the lane that issues)
         constexpr uint32_t kIdescS = idesc_f16(BM, BN, 0, 0);
         const uint32_t dX = desc_lo_sw128(smem_u32(sX), 16), dY0 = desc_lo_sw128(smem_u32(sY), 16);
         int sg = -1;
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(kThreadsB, 1)
             if (!produce(tma_it)) break;
     } else if (warp == kMmaWarp) {
         // ================================ MMA issuer 1: score contractions S = Q K^T ================================
-        // (the whole warp walks the loop; the asynchronous instructions are lane 0's)
+        // (the whole warp walks the loop; elect.sync picks the lane that issues)
         constexpr uint32_t kIdescS = idesc_f16(BM, BN, 0, 0);
         const uint32_t dX = desc_lo_sw128(smem_u32(sX), 16), dY0 = desc_lo_sw128(smem_u32(sY), 16);
         int sg = -1;

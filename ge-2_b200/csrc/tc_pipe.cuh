@@ -18,11 +18,9 @@ constexpr int kMmaK = 16;               // k extent of one kind::f16 MMA (32 byt
 // Descriptors are built once per tile; a k-step only adds its byte offset (>> 4) to the start-address field, which cannot
 // carry out of the field because shared-memory addresses stay below 256 KB.
 // K-major operand: k-step `ks` (16 elements = 32 bytes) sits in column block ks/4 at byte (ks%4)*32; 8-row groups are 1024 bytes apart
-__device__ __forceinline__ uint64_t desc_kmajor_base(uint32_t tile) { return smem_desc_sw128(tile, 16, 1024); }
 __host__ __device__ constexpr uint64_t koff_kmajor(int ks) { return (uint64_t)(((ks >> 2) * kBlockBytes + (ks & 3) * 32) >> 4); }
 // MN-major operand: k-step `ks` is rows [16 ks, 16 ks + 16) = two 8-row groups of 1024 bytes; the 64-element MN blocks are
 // kBlockBytes apart
-__device__ __forceinline__ uint64_t desc_mnmajor_base(uint32_t tile) { return smem_desc_sw128(tile, kBlockBytes, 1024); }
 __host__ __device__ constexpr uint64_t koff_mnmajor(int ks) { return (uint64_t)((ks * 2048) >> 4); }
 
 // byte offset of the 16-byte chunk holding elements [col, col + 8) of row `row` in the swizzled block layout (col % 8 == 0)
@@ -47,9 +45,6 @@ static __device__ __noinline__ bool pipe_wait_slow(uint64_t* bar, uint32_t parit
     *abort_flag = 1;
     or_status(status, GE2_STATUS_PIPE_TIMEOUT);
     return false;
-}
-__device__ __forceinline__ bool pipe_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
-    return mbar_try_wait(bar, parity) || pipe_wait_slow(bar, parity, abort_flag, status);
 }
 // For the warps that feed the tensor pipe and its copies: the whole warp polls, and nobody sleeps (a slot is refilled within a few
 // hundred nanoseconds, about as long as a sleeping lane takes to come back)

@@ -41,13 +41,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     return false;
 }
 
-// ---- TMA: tiled 3-D load global -> shared, completion counted on an mbarrier -------------------------------------
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
-        "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
-        : "memory");
-}
+// ---- bulk copies ---------------------------------------------------------------------------------------------------
 // Untiled bulk copy global -> shared (both addresses 16-byte aligned, size a multiple of 16), counted on the same kind of mbarrier
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)), "l"(gsrc),
@@ -99,16 +93,6 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // ---- tcgen05.mma, A and B from shared memory ---------------------------------------------------------------------
-// Shared-memory matrix descriptor, 128-byte swizzle.  addr/lbo/sbo in bytes (16-byte granular).
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFFu) >> 4);        // start address           bits [0,14)
-    d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;    // leading byte offset     bits [16,30)
-    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;    // stride byte offset      bits [32,46)
-    d |= (uint64_t)1 << 46;                         // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;                         // layout type: SWIZZLE_128B
-    return d;
-}
 // Instruction descriptor for kind::f16 with fp16 A and B (format code 0) and fp32 accumulate (code 1).
 // a_mn / b_mn: 1 = operand is MN-major in shared memory.  (32-bit operands cannot share one swizzled tile between a
 // K-major and an MN-major use -- the hardware only transposes them from a 32-byte-atom layout -- 16-bit operands can.)
@@ -123,8 +107,10 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int a_mn, int b_
 // them alive, values the compiler keeps in uniform registers were seen to come back wrong there (single k-steps of a contraction read
 // other operands).  These forms are run by all 32 lanes, converged, and elect.sync picks the (same) one that issues, so control flow
 // and all address arithmetic stay warp-uniform: 48 / 64 / 128 cycles a contraction of N = 64 / 128 / 256, the rate of the pipe (a lane
-// predicate instead of the election: 62 - 67 cycles at N <= 128).  Descriptors are given by their low words: the high word of a
-// 128-byte-swizzled operand with 8-row groups 1024 bytes apart is a constant.
+// predicate instead of the election: 62 - 67 cycles at N <= 128).
+// Shared-memory matrix descriptors (addresses and offsets in units of 16 bytes) are given by their low words, start address in bits [0, 14) and
+// leading byte offset in [16, 30); the high word of a 128-byte-swizzled operand with 8-row groups 1024 bytes apart is a constant: stride
+// byte offset in [0, 14), descriptor version 1 (sm_100) at 14, layout type 2 (SWIZZLE_128B) at 29.
 constexpr uint32_t kDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo_sw128(uint32_t addr, uint32_t lbo) { return ((addr & 0x3FFFFu) >> 4) | (((lbo >> 4) & 0x3FFFu) << 16); }
 __device__ __forceinline__ void mma_f16_ss_warp(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
