@@ -50,7 +50,7 @@ PARTITIONED = {
 
 # dram__bytes_read.sum + dram__bytes_write.sum of the scores launches of one step on this workload, taken from one ncu
 # capture of those launches (operands and partial gradients stay in the 126 MB L2, so it is far below the operand bytes)
-NCU_TRAFFIC = {"f16": 38_685_952, "fp32": None}
+NCU_TRAFFIC = {"f16": 38_682_112, "fp32": 80_261_120}
 REPEATS = 9  # the K-step timed region is run this many times; `value` is total steps over total time, the spread is reported
 
 
@@ -259,6 +259,9 @@ def reference_arm(args):
         return
     cfg = CFG
     cpu = CpuReference(cfg, 20262)
+    if cpu.kind != "reference":  # a restatement in numpy is not the reference
+        print(json.dumps(dict(impl="reference", unavailable="the reference's sources are not here: oracle/_ref/gege_ref.so was not built")), flush=True)
+        return
     for w in range(min(args.warmup, 2)):
         cpu.step(w)
     t0 = time.perf_counter()
@@ -270,8 +273,8 @@ def reference_arm(args):
         cpu.step(200 + k)
     dt = time.perf_counter() - t0
     value = steps_run * cfg["B"] / dt
-    sample = f"{steps_run} batches of {cfg['B']} edges of the same workload on CPU ({cpu.kind}: " + (
-        "reference C++/libtorch decoder+loss+autograd+accumulateGradients, torch.unique for its broken CPU map_tensors" if cpu.kind == "reference" else "numpy restatement") + ")"
+    sample = (f"{steps_run} batches of {cfg['B']} edges of the same workload on CPU (reference C++/libtorch decoder+loss+autograd+accumulateGradients, "
+              "torch.unique for its broken CPU map_tensors)")
     line = dict(metric="train edges/sec/box", value=value, unit="edges/s", n_gpus=args.gpus, steps=args.steps, warmup=args.warmup,
                 ms_per_step=1e3 * dt / steps_run, higher_is_better=True, scaling="weak", vs_baseline=None, dtype="f32", data="synthetic",
                 impl="reference", config=dict(workload=cfg["name"] + (f", weak-scaled: {args.gpus} x nodes and triples, {4 * args.gpus} partitions" if args.gpus > 1 else ""),
@@ -557,20 +560,24 @@ def per_kernel_rooflines(pipe, pcfg, capi, edges, num_batches, reps=20):
         gbs = nbytes / (ms * 1e-3) / 1e9
         out[name] = dict(ms=ms, bytes=nbytes, achieved=gbs, unit="GB/s", peak=pk["hbm"], frac=gbs / pk["hbm"], bound="hbm", bytes_are=what)
 
-    add("unique_map", tg(lambda: capi.unique_bitmap(ids.packed, pcfg.domain, workspace=ids.uws, out_unique=ids.unique, out_inverse=ids.inverse,
-                                                      out_count=ids.count)),
-        16 * n_ids + 8 * U, "16 B per id (read id, write rank) + 8 B per distinct id; the domain-sized bitset passes (0.19 B per node) not counted")
+    add("unique_map", tg(lambda: pipe._unique(ids)), 16 * n_ids + 9 * U,
+        "16 B per id (read id, write rank) + 9 B per distinct id (id, does it occur again); the domain-sized bitset passes (0.31 B per node) not counted")
     add("gather_prepare", pipe.time_scores_phase(edges, reps, 1),
         ((2 + S) * B + S * CN) * D * 4 + (S * pcfg.B + S * CN) * 128 * 2, "embedding / relation rows read (fp32) + fp16 operand rows written")
+    shared = ids.shared[:U].bool()
+    U_shared = int(shared.sum())
+    negs_once = int((~shared[ids.inverse[2 * B:].unique()]).sum())   # their rows are read here; an endpoint's is read for its edge anyway
+    ends_once = U - U_shared - negs_once
+    rel_rows = S if pcfg.has_relations else 0
     add("scatter_finish", pipe.time_scores_phase(edges, reps, 4),
-        (B * (6 + 4) + S * CN * 2) * D * 4, "per edge 6 rows in + 4 gradient rows out, per negative 1 row in + 1 out (fp32)")
-    t2, s2 = pipe.table.clone(), pipe.state.clone()  # scratch copies: the timing must not train the real tables
-    pipe.node_grad.normal_()
-    add("adagrad_scatter", tg(lambda: capi.adagrad_scatter(t2, s2, ids.unique, pipe.node_grad, 0.1, U=pipe.cap, U_dev=ids.count,
-                                                            clear_grad=False, status=pipe.status)),
-        20 * U * D, "per touched row: embedding + state read and written (16 B per float) + gradient read (4 B)")
-    pipe.node_grad.zero_()
-    del t2, s2
+        (B * (2 + S + 2 * rel_rows) + S * CN + 3 * ends_once + 4 * negs_once + U_shared) * D * 4,
+        "per edge its embedding, dQ and relation rows in and its relation gradients out, per negative its dK row in; a node that occurs once has its "
+        "state read and both rows written (a negative's embedding read too), any other one gradient row out (fp32)")
+    t2, s2, g2 = pipe.table.clone(), pipe.state.clone(), torch.randn_like(pipe.node_grad)  # the timing must not train the real tables
+    add("adagrad_scatter", tg(lambda: capi.adagrad_scatter(t2, s2, ids.unique, g2, 0.1, U=pipe.cap, U_dev=ids.count, clear_grad=True, status=pipe.status,
+                                                            row_shared=ids.shared)),
+        24 * U_shared * D + U, "per row that occurs more than once: embedding + state read and written, gradient read and cleared (24 B per float); a byte per distinct id")
+    del t2, s2, g2
     return out
 
 
@@ -847,9 +854,9 @@ def main():
                     help="2: the single-GPU configuration (weak-scaled over partitions at N > 1); 3, 4, 5: the stated partitioned configurations "
                          "(need --gpus 2, 4, 8)")
     ap.add_argument("--precision", default=os.environ.get("GE2_PRECISION", "f16"), choices=["fp32", "f16"],
-                    help="f16: tcgen05 fp16-operand tiles with fp32 accumulation (1e-2 parity, the designed path); fp32: CUDA-core path (1e-4 parity)")
+                    help="f16: tcgen05 fp16-operand tiles with fp32 accumulation (1e-2 parity, the designed path); fp32: operands split exactly into three bf16 terms (1e-4 parity)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--no-fp32-path", action="store_true", help="skip the side measurement of the fp32 CUDA-core path")
+    ap.add_argument("--no-fp32-path", action="store_true", help="skip the side measurement of the fp32 path")
     ap.add_argument("--no-reference-gpu", action="store_true", help="skip timing the reference's own GPU code (oracle/_ref/gege_ref_cuda.so) on this GPU")
     ap.add_argument("--no-host-cpp", action="store_true", help="N = 1: skip the side measurement through the C++ host layer")
     ap.add_argument("--no-epoch", action="store_true", help="N = 1: skip the one-epoch (triples / B steps) timed region")
@@ -1051,7 +1058,7 @@ def main():
             roofline_kernels=kernel_rooflines,
         )
         if world == 1 and args.precision == "f16" and not args.no_fp32_path:
-            # the same step on the fp32 CUDA-core path (1e-4 parity), for reference next to the headline
+            # the same step on the fp32 path (1e-4 parity), for reference next to the headline
             pc32 = pipeline.PipelineConfig(cfg["decoder"], B, C, N, cfg["degree_fraction"], D, R, nodes, lr=cfg["lr"], precision="fp32")
             p32 = pipeline.BatchPipeline(pc32, table, state, rel, torch.zeros_like(rel), inv_rel, torch.zeros_like(inv_rel))
             g32 = p32.capture_resident(edges, num_batches)
