@@ -535,6 +535,13 @@ inline PairCut pair_cut(const PairArgs& a, PairOp op) {
     return p;
 }
 
+// Scratch of the backward pass.  None where the rows are gathered, so that a small call costs its caller no allocation -- but where a CTA has four
+// pairs a negative it is asked for all the same, as it was when that was the line: a caller may have sized its scratch once.
+inline size_t pair_scratch_bytes(const PairArgs& a, const PairCut& p) {
+    if (!p.possible || !(p.taken || ceil_div<int64_t>(a.R, p.cpc) * a.K >= 4 * a.N)) return 0;
+    return (size_t)(a.rows * a.K) * (a.kind == GE2_SELECTED_L2 ? 12 : 8);  // sorted (weight, row) pairs; L2: the weights themselves too
+}
+
 template <int KIND, int MODE>
 int launch_pair_rows(const PairArgs& a, const PairCut& p, bool vec, const float* weights, float* out, cudaStream_t stream) {
     const size_t smem = (size_t)(a.N + 1) * p.W4 * 16;
@@ -927,8 +934,7 @@ extern "C" int ge2_selected_neg_scores_backward(int kind, const float* grad_out,
 extern "C" size_t ge2_selected_neg_backward_workspace_bytes(int kind, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs, int64_t num_selected, int D) {
     if (chunks <= 0 || rows_per_chunk <= 0 || num_negs <= 0 || num_selected <= 0 || D <= 0 || D > kMaxD) return 0;
     const PairArgs a = pair_args(kind, nullptr, nullptr, nullptr, chunks, rows_per_chunk, num_negs, num_selected, D, nullptr);
-    if (!pair_cut(a, backward_op(kind)).possible) return 0;
-    return (size_t)(a.rows * a.K) * (kind == GE2_SELECTED_L2 ? 12 : 8);  // sorted (weight, row) pairs; L2: the weights themselves too
+    return pair_scratch_bytes(a, pair_cut(a, backward_op(kind)));
 }
 
 extern "C" int ge2_selected_neg_scores_backward_ws(int kind, const float* grad_out, const float* chunked, const float* negatives,
@@ -948,9 +954,8 @@ extern "C" int ge2_selected_neg_scores_backward_ws(int kind, const float* grad_o
     // with nothing selected the kernel still writes the zero query gradient
     const PairArgs a = pair_args(kind, chunked, negatives, selected, chunks, rows_per_chunk, num_negs, num_selected, D, status);
     const bool vec = rows_are_vectors(D, chunked, negatives, grad_chunked, grad_negatives);
-    const size_t need = ge2_selected_neg_backward_workspace_bytes(kind, chunks, rows_per_chunk, num_negs, num_selected, D);
     const PairCut cut = pair_cut(a, backward_op(kind));
-    if (cut.taken && workspace != nullptr && workspace_bytes >= need && ((uintptr_t)workspace & 7) == 0) {
+    if (cut.taken && workspace != nullptr && workspace_bytes >= pair_scratch_bytes(a, cut) && ((uintptr_t)workspace & 7) == 0) {
         float2* sorted = reinterpret_cast<float2*>(workspace);
         float* coeffs = reinterpret_cast<float*>(sorted + rows * num_selected);
         if (kind == GE2_SELECTED_DOT) {

@@ -453,7 +453,7 @@ GE2_API int ge2_selected_neg_scores_backward(int kind, const float *grad_out, co
                                              int64_t num_selected, int D, float *grad_chunked, float *grad_negatives, int32_t *status,
                                              ge2_stream_t stream);
 /* The same with scratch for the form that sorts the pairs by negative: ge2_selected_neg_backward_workspace_bytes() bytes, 8-byte aligned
- * (0 bytes: the sizes rule it out; otherwise the call takes the form that is the faster one at its sizes).  Without the scratch the
+ * (0 bytes: the sizes do not call for it; otherwise the call takes the form that is the faster one at its sizes).  Without the scratch the
  * gradients are the same, summed in another order. */
 GE2_API size_t ge2_selected_neg_backward_workspace_bytes(int kind, int64_t chunks, int64_t rows_per_chunk, int64_t num_negs, int64_t num_selected,
                                                          int D);

@@ -87,9 +87,10 @@ def test_the_form_that_the_estimate_takes(capi, cuda_device, C, R, N, D, K, resi
     status = torch.zeros(1, dtype=torch.int32, device=cuda_device)
     scores = capi.selected_neg_scores(kind, tq, tn, ts, status)
     need = lib.ge2_selected_neg_backward_workspace_bytes(code, C, R, N, K, D)
-    ws = torch.full((need,), 0xCD, dtype=torch.uint8, device=cuda_device)
+    assert need > 0 or not resident
+    ws = torch.full((max(need, 12 * C * R * K),), 0xCD, dtype=torch.uint8, device=cuda_device)
     capi.check(lib.ge2_selected_neg_scores_backward_ws(code, tg.data_ptr(), tq.data_ptr(), tn.data_ptr(), ts.data_ptr(), C, R, N, K, D, dq.data_ptr(),
-                                                       dn.data_ptr(), status.data_ptr(), ws.data_ptr(), need, capi.cur_stream()), "backward")
+                                                       dn.data_ptr(), status.data_ptr(), ws.data_ptr(), ws.numel(), capi.cur_stream()), "backward")
     torch.cuda.synchronize()
     assert int(status) == 0
     if kind == "DOT":
