@@ -340,18 +340,13 @@ __global__ void __launch_bounds__(256, 5) lp_prep_kernel(const __grid_constant__
 // Bound by latency on small batches (ids -> rows -> reductions), by HBM on large ones.  With the sparse Adagrad pass that follows:
 // 10 000 edges, 2 x 10 000 negatives, ComplEx 100: 28 us (33 us with every row through the gradient table); 50 000 edges and
 // negatives, Dot 100: 104 us (143 us); 100 000 edges, 2 x 200 000 negatives, DistMult 128: 270 us (465 us).
-// A node in half of the edges and of the degree negatives: the first of these 26 us (31 us with its rows summed in shared memory for a CTA's
-// lifetime), the last with half of the negatives by degree 269 us (461 us).  Scalar reductions feel it most: 7919 edges, 2 x 4571 negatives,
+// A node in half of the edges and of the degree negatives: the first of these 28 us (31 us with its rows summed in shared memory for a CTA's
+// lifetime), the last with half of the negatives by degree 275 us (461 us).  Scalar reductions feel it most: 7919 edges, 2 x 4571 negatives,
 // ComplEx 50 (25 columns a half): 20 us, 25 us with neighbouring lanes two columns apart (17 us and 17 us without such a node).
 // ---------------------------------------------------------------------------------------------------
 constexpr int kFinWarps = 8;
 constexpr int kNoRow = 2;      // in the place of a node's "occurs again": its row is not one of the table, so nothing is done with it
 constexpr int kFinBatch = 16;  // edges a batch: their 32 endpoints are the lanes of one warp when it looks for repeated nodes
-
-// the repeated node of each warp of negatives whose row meets the other warps' on chip
-struct FinHubs {
-    long long id[kFinWarps];
-};
 
 struct FinScalars {
     long long id[2 * kFinBatch];   // local node ids, sources then destinations; -1: skip the edge (bad ids, flagged by prep)
@@ -389,7 +384,6 @@ template <int V, bool CPLX, bool REL>
 __global__ void __launch_bounds__(kFinWarps * 32, 4) lp_finish_kernel(const __grid_constant__ LpKernelArgs a, int neg_ctas, int occ) {
     extern __shared__ __align__(16) float fin_rows[];  // [4][kFinBatch][ld]: relation, inverse relation, source, destination gradients
     __shared__ FinScalars sm;
-    __shared__ FinHubs hubs;
     const ge2_lp_desc& d = a.d;
     const LpLayout& L = a.L;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -428,15 +422,6 @@ __global__ void __launch_bounds__(kFinWarps * 32, 4) lp_finish_kernel(const __gr
             shared = kNoRow;
             or_status(d.status, GE2_STATUS_BAD_INDEX);
         }
-        // Negatives drawn by degree: the node that most of the warp's are, if it is one that repeats.  Its sum goes to shared memory, where those
-        // of the CTA's warps that have the same one meet before they leave (10 000 edges, half of them at one node, 2 x 10 000 negatives, nine in
-        // ten by degree, ComplEx 100, with the sparse Adagrad: 29 us instead of 32; without such a node 26 us either way).
-        const bool by_degree = d.deg_sample_rows != nullptr;
-        int hub = -1;
-        if (by_degree) {
-            const unsigned most = __reduce_max_sync(0xFFFFFFFFu, leads && shared == 1 && __popc(same) > 2 ? (unsigned)__popc(same) << 5 | (unsigned)lane : 0u);
-            if (most != 0u) hub = (int)(most & 31u);
-        }
 #pragma unroll 1
         for (int k0 = 0; k0 < occ; k0 += per_warp) {
             if (((leaders >> k0) & ((1u << per_warp) - 1u)) == 0u) continue;
@@ -465,21 +450,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 4) lp_finish_kernel(const __gr
             }
             g = scale4(gs, g);
             if (upd) adagrad_row<V, CPLX>(table + grow * d.emb_stride, d.node_state + grow * d.emb_stride, l, D, e, s, g, neg_lr);
-            else if (on && k == hub) *reinterpret_cast<float4*>(fin_rows + warp * ld + 4 * l) = g;
             else if (on) put_row<V, CPLX, PutAdd>(d.node_grad + gid * D, l, D, g);
-        }
-        if (!by_degree) return;
-        const long long hub_id = __shfl_sync(0xFFFFFFFFu, id, hub < 0 ? 0 : hub);
-        if (lane == 0) hubs.id[warp] = hub < 0 ? -1 : hub_id;
-        if (__syncthreads_or(hub >= 0)) {
-            const long long mine = hubs.id[warp];
-            if (mine < 0) return;
-            for (int w2 = 0; w2 < warp; w2++)
-                if (hubs.id[w2] == mine) return;  // an earlier warp sends the sum
-            float4 g = *reinterpret_cast<const float4*>(fin_rows + warp * ld + 4 * l);
-            for (int w2 = warp + 1; w2 < kFinWarps; w2++)
-                if (hubs.id[w2] == mine) g = add4(g, *reinterpret_cast<const float4*>(fin_rows + w2 * ld + 4 * l));
-            if (sub == 0) put_row<V, CPLX, PutAdd>(d.node_grad + mine * D, l, D, g);
         }
         return;
     }

@@ -274,7 +274,7 @@ def test_streaming_softmax_where_it_is_taken(capi, cuda_device, kind, B, C, N, D
 
 @pytest.mark.parametrize("kind,B,C,N,D", [("COMPLEX", 600, 3, 300, 50), ("COMPLEX", 500, 2, 7001, 100), ("DISTMULT", 300, 2, 3000, 128), ("DISTMULT", 257, 2, 640, 3)])
 def test_one_node_in_most_edges_and_negatives(capi, cuda_device, kind, B, C, N, D):
-    """Rows of a node that most of the degree negatives are meet on chip, warp by warp, before they leave."""
+    """Rows of a node that most edges and degree negatives have are added up where they meet, and leave as sums."""
     case = workloads.make_case(kind, B, C, N, D, 5, 400, int(0.9 * N), seed=B + D, relations=True, inverse=True, alpha=3.0)
     o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
     res = run_lp_step(capi, case, cuda_device, "fp32", "deg_rows", dump_scores=False)
