@@ -21,23 +21,29 @@
 // Shared memory holds two X blocks and a ring of Y tiles [128 x DP], fp16 in the 128-byte-swizzled layout TMA writes (64-element
 // column blocks of 128 rows at a 128-byte pitch); a tile read along its rows is the K-major operand of S, read along its columns the
 // MN-major operand of O.
-// Tensor memory (512 columns): two score accumulators at 0 and 128, two O accumulators at 256 and 384.  Two groups of eight softmax
-// warps take alternate tiles, each with its own score accumulator (and, for the queries, its own m and O), so one group
-// exponentiates while the other's contractions run.
-// Bound by the chain scores -> exponentials -> O -> scores of a group, 4900 ... 5800 cycles for its tile (the exp unit alone would take
-// 1024 a tile): B = 100 000, N = 2000, D = 128, two sides: 282 + 235 us, with the other kernels 213 + 687 us.
+// Tensor memory (512 columns): two score accumulators at 0 and 128, two O accumulators at 256 and 384.  Two groups of four softmax
+// warps, a thread a row, take alternate tiles, each with its own score accumulator, its own O and (queries) its own m, so one group
+// exponentiates while the other's contractions run.  P goes to the contraction in two halves of 64 columns, the first while the second is
+// exponentiated.
+// Bound by the chain scores -> exponentials -> O -> scores of a group, about 4200 cycles for its tile: 2300 ... 2800 of exponentials (2048 if
+// the unit for them were never idle, for both groups' tiles), 768 of contractions behind the last of them, the hand-overs.  The tensor pipe,
+// 1024 cycles a tile, is half busy.  B = 100 000, N = 2000, D = 128, two sides: 225 + 220 us on fresh tables, 230 + 224 inside training steps.
+// Measured before and on the way there (fresh tables; on one GPU the last of these forms took 229 + 227): two warps a row with a pass over the
+// scores for the maximum and an exchange of it, 258 + 230 (285 + 234 in training); one issuing warp for both groups, 261 + 235; an issuing warp a
+// group without turns, 246 + 244; with turns at the second half of O only, 229 + 227; halves of a tile as score tiles of their own (the
+// tensor pipe then has 1280 cycles a tile, and every hand-over twice), 264 + 278; an L2 prefetch of tiles to come, 227 + 224; five stages and
+// one X, 221 + 230; three stages, 325 + 287.
 // P carries a factor 2^14, so that probabilities down to 2^-38 keep their full significand instead of falling into fp16's subnormal
 // range; dQ and dK leave this kernel with that factor still on them and the scatter kernel, their only reader, takes it off
 // (LpLayout::grad_unscale).
 //
 // Warp roles, connected by mbarrier pipelines (no block-wide barrier inside the loops):
-//   warps 0-15  softmax: warp w takes rows 32 (w & 3) ... + 31 (its quarter of the tensor-memory lanes) and columns 64 ((w >> 2) & 1)
-//               ... + 63 of its group's (w >> 3) tiles
-//   warps 16-19 drain: O -> registers (-> weighted sum of the two groups) -> staging slab -> TMA store / reduce-add
-//   warp  20    TMA producer
-//   warp  21    issues the contractions; also allocates and frees tensor memory
-//   warps 22-23 what the softmax warps need to know about coming tiles (each for its group): which entries are masked and, for the
-//               negatives, the columns' lse.  Queries: they first clear the dK rows the second launch reduces into
+//   warps 0-7   softmax: warp w takes rows 32 (w & 3) ... + 31 (its quarter of the tensor-memory lanes) of its group's (w >> 2) tiles
+//   warps 8-11  drain: O -> registers (-> weighted sum of the two groups) -> staging slab -> TMA store / reduce-add
+//   warp  12    TMA producer
+//   warps 13-14 issue the contractions of a group each; warp 13 also allocates and frees tensor memory
+//   warp  15    what the softmax warps need to know about coming tiles: which entries are masked and, for the negatives, the columns'
+//               lse.  Queries: it first clears the dK rows the second launch reduces into
 // Every mbarrier wait is bounded; a wait that runs out raises GE2_STATUS_PIPE_TIMEOUT and sets a block-wide abort flag
 // that every other wait polls, so all roles fall through to the common exit where tensor memory is released.
 #include <algorithm>
@@ -52,9 +58,11 @@ using namespace tc;
 
 constexpr int BM = 128;                 // rows of the stationary block (MMA M)
 constexpr int BN = 128;                 // rows of a streamed tile
-constexpr int kSoftmaxWarps = 16;
-constexpr int kThreads = 768;
-constexpr int kDrainWarp0 = kSoftmaxWarps, kDrainWarps = 4, kTmaWarp = 20, kMmaWarp = 21, kHelpWarp = 22;
+constexpr int kGroupWarps = 4;          // softmax warps of a group: one a quarter of the tensor-memory lanes
+constexpr int kSoftmaxWarps = 2 * kGroupWarps;
+constexpr int kThreads = 512;           // 128 registers each at the launch; the drain warps take some of warps 12-15 (setmaxnreg)
+constexpr int kLaunchRegs = 128, kDrainRegs = 184, kServiceRegs = 2 * kLaunchRegs - kDrainRegs;
+constexpr int kDrainWarps = 4, kTmaWarp = 12, kMmaWarp = 13, kHelpWarp = 15;  // (an issuing warp a group)
 constexpr int kStages = 4;              // Y ring: two tiles wait for their O contraction, two are on their way
 constexpr int kInfoStages = 4;          // ring of what warps 22-23 find out about tiles
 constexpr uint32_t kTmemCols = 512;
@@ -62,11 +70,12 @@ constexpr float kMasked = -1e9f;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr int kWShift = 14;             // P is scaled by 2^14; undone by the reader of dQ / dK (kLpF16GradUnscale)
 constexpr float kHeadStart = 3.f;       // queries: log2 of how far the reference is set above the maximum it is taken from
+constexpr float kNoReference = -1e30f;  // queries: no score of the block has been seen by this group yet
 constexpr float kDeadRow = 1e30f;       // "lse" of a row past the end of its chunk: exp2(anything - 1e30) = 0
 
-enum Bar { kBarXFull = 0, kBarXEmpty = 2, kBarYFull = 4, kBarYEmpty = kBarYFull + kStages, kBarSFull = kBarYEmpty + kStages, kBarPFull = kBarSFull + 2,
-           kBarOFull = kBarPFull + 2, kBarOEmpty, kBarStat, kBarStatFree = kBarStat + 2, kBarMax = kBarStatFree + 2, kBarInfoFull = kBarMax + 8,
-           kBarInfoEmpty = kBarInfoFull + kInfoStages, kNumBars = kBarInfoEmpty + kInfoStages };
+enum Bar { kBarXFull = 0, kBarXEmpty = 2, kBarYFull = 6, kBarYEmpty = kBarYFull + kStages, kBarSFull = kBarYEmpty + kStages, kBarPFull = kBarSFull + 2,
+           kBarHalf = kBarPFull + 4, kBarTurn = kBarHalf + 2, kBarOFull = kBarTurn + 2, kBarOEmpty = kBarOFull + 2, kBarStat = kBarOEmpty + 2, kBarStatFree = kBarStat + 2,
+           kBarInfoFull = kBarStatFree + 2, kBarInfoEmpty = kBarInfoFull + kInfoStages, kNumBars = kBarInfoEmpty + kInfoStages };
 
 template <int DP>
 struct Layout {
@@ -74,11 +83,10 @@ struct Layout {
     static constexpr int kTileBytes = NB * kBlockBytes;
     static constexpr int kX = 0;
     static constexpr int kY = kX + 2 * kTileBytes;
-    static constexpr int kDrain = kY + kStages * kTileBytes;   // 4 drain warps x one slab (32 rows x 128 bytes), 128-byte swizzled
+    static constexpr int kDrain = kY + kStages * kTileBytes;       // 4 drain warps x one slab (32 rows x 128 bytes), 128-byte swizzled
     static constexpr int kMisc = kDrain + kDrainWarps * 4096;  // barriers, tensor-memory address, abort flag
-    static constexpr int kMax = kMisc + 1024;                  // row maxima of the column halves: [group][buffer][half][128]
-    static constexpr int kStat = kMax + 2 * 2 * 2 * 128 * 4;   // (m, sum) at the end of a block: [buffer][group * 2 + half][128]
-    static constexpr int kLse = kStat + 2 * 4 * 128 * 8;       // [kInfoStages][128]
+    static constexpr int kStat = kMisc + 1024;                     // (m, sum) at the end of a block: [buffer][group][128]
+    static constexpr int kLse = kStat + 2 * 2 * 128 * 8;           // [kInfoStages][128]: minus the columns' lse
     static constexpr int kMask = kLse + kInfoStages * 128 * 4; // [kInfoStages][128]
     static constexpr int kRange = kMask + kInfoStages * 128 * 4;  // first unit of every CTA of the query launch, and the end
     static constexpr int kEnd = kRange + (kNumSMs + 4) * 4;
@@ -99,8 +107,35 @@ __device__ __forceinline__ float exp2f_fast(float x) {  // one MUFU.EX2; 2^-inf 
     return y;
 }
 
+// two at a time: one instruction, the same roundings
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
+// Registers of a warpgroup (four warps, all of which run this): given back to the CTA, taken from what others gave back.  The CTA is launched
+// with kThreads x kLaunchRegs of them, and the shares add up to that, so the wait of the second form ends.
+template <int N>
+__device__ __forceinline__ void regs_dec() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void regs_inc() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 // base-2 logsumexp of a row from its positive score and the parts its sharers left
-__device__ __noinline__ float combine_parts(const float2* part, int nparts, float pos2) {
+__device__ __forceinline__ float combine_parts(const float2* part, int nparts, float pos2) {
     float m = pos2, l = 1.f;
 #pragma unroll 1
     for (int k = 0; k < nparts && k < kMaxParts; k++) {
@@ -114,6 +149,7 @@ __device__ __noinline__ float combine_parts(const float2* part, int nparts, floa
 
 struct FlashSched {
     Sched q, n;  // T, RB of each launch; units and grid of the launch in unitsA / gridA
+    int masks;   // are any scores masked in this step?
 };
 
 template <int DP, bool NEG>
@@ -128,7 +164,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t* bars = (uint64_t*)(smem + LY::kMisc);
     uint32_t* s_tmem = (uint32_t*)(smem + LY::kMisc + kNumBars * 8);
     volatile int* s_abort = (volatile int*)(smem + LY::kMisc + kNumBars * 8 + 4);
-    float* s_max = reinterpret_cast<float*>(smem + LY::kMax);
     float2* s_stat = reinterpret_cast<float2*>(smem + LY::kStat);
     float* s_lse = reinterpret_cast<float*>(smem + LY::kLse);
     int* s_mask = reinterpret_cast<int*>(smem + LY::kMask);    // partner of the entry that is masked: queries: a column's row, negatives: a row's column; -1
@@ -143,29 +178,29 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int n_iter = ue - ub;
     const int x_rows = NEG ? d.N : L.npc, y_rows = NEG ? L.npc : d.N;  // rows a chunk has on either side
     constexpr int NB = LY::NB;
-    auto spin_wait = [&](int bar, uint32_t parity) { return warp_spin_wait(&bars[bar], parity, s_abort, d.status); };
-    auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, d.status); };
+    auto warp_wait = [&](int bar, uint32_t parity) { return warp_wait_inline(&bars[bar], parity, s_abort, d.status); };
 
     if (warp == kTmaWarp && lane == 0) {
         for (int k = 0; k < 2; k++) {
             mbar_init(&bars[kBarXFull + k], 1);
-            mbar_init(&bars[kBarXEmpty + k], 1);
+            mbar_init(&bars[kBarXEmpty + 2 * k], 1), mbar_init(&bars[kBarXEmpty + 2 * k + 1], 1);  // [buffer][group]
             mbar_init(&bars[kBarSFull + k], 1);
-            mbar_init(&bars[kBarPFull + k], kSoftmaxWarps / 2);  // one arrival per warp of the group that owns the tile
+            mbar_init(&bars[kBarHalf + k], 1);
+            mbar_init(&bars[kBarTurn + k], 1);
+            mbar_init(&bars[kBarOFull + k], 1);
+            mbar_init(&bars[kBarOEmpty + k], kDrainWarps);
             mbar_init(&bars[kBarStat + k], kSoftmaxWarps);
             mbar_init(&bars[kBarStatFree + k], kDrainWarps);
         }
+        for (int k = 0; k < 4; k++) mbar_init(&bars[kBarPFull + k], kGroupWarps);  // [group][half of the tile's columns]: one arrival a warp
         for (int k = 0; k < kStages; k++) {
             mbar_init(&bars[kBarYFull + k], 1);
             mbar_init(&bars[kBarYEmpty + k], 1);
         }
-        for (int k = 0; k < 8; k++) mbar_init(&bars[kBarMax + k], 2);  // the two column halves of 32 rows
         for (int k = 0; k < kInfoStages; k++) {
             mbar_init(&bars[kBarInfoFull + k], 1);
-            mbar_init(&bars[kBarInfoEmpty + k], kSoftmaxWarps / 2);
+            mbar_init(&bars[kBarInfoEmpty + k], kGroupWarps);
         }
-        mbar_init(&bars[kBarOFull], 1);
-        mbar_init(&bars[kBarOEmpty], kDrainWarps);
         *s_abort = 0;
         mbar_init_fence();
         prefetch_tensormap(&tmX);
@@ -183,215 +218,172 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t tmem = *s_tmem;
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;  // this warp's quarter of the 128 tensor-memory lanes
 
-    if (warp == kTmaWarp) {
-        int sg = -1;
-        IterA un(ub, sc);
-        for (int it = 0; it < n_iter; it++, un.next(sc)) {
-            if (it == 0 || un.tile == 0) {  // a new block
-                sg++;
-                const int xs = sg & 1;
-                if (!spin_wait(kBarXEmpty + xs, ((sg >> 1) & 1) ^ 1)) break;
-                mbar_expect_tx_warp(&bars[kBarXFull + xs], LY::kTileBytes);
-#pragma unroll
-                for (int b = 0; b < NB; b++) tma_load_3d_warp(sX + xs * LY::kTileBytes + b * kBlockBytes, &tmX, b * 64, un.rb * BM, un.zc, &bars[kBarXFull + xs]);
-            }
-            const int st = it % kStages;
-            if (!spin_wait(kBarYEmpty + st, ((it / kStages) & 1) ^ 1)) break;
-            mbar_expect_tx_warp(&bars[kBarYFull + st], LY::kTileBytes);
-#pragma unroll
-            for (int b = 0; b < NB; b++)
-                tma_load_3d_warp(sY + st * LY::kTileBytes + b * kBlockBytes, &tmY, b * 64, un.tile * BN, un.zc, &bars[kBarYFull + st]);
-        }
-    } else if (warp == kMmaWarp) {
-        // ================================ contractions ================================
-        // S of the tile after next follows O of this one, so a score accumulator is overwritten only behind the contraction that reads
-        // the P in it, and "S complete" also says that the group's previous O contraction is.
-        const int D16 = ((d.D + kMmaK - 1) / kMmaK) * kMmaK;  // the embedding dimension rounded up to the MMA k step
-        constexpr uint32_t kIdescS = idesc_f16(BM, BN, 0, 0);
-        const uint32_t idesc_o = idesc_f16(BM, D16, 0, 1);
-        const uint32_t dXk = desc_lo_sw128(smem_u32(sX), 16), dYk = desc_lo_sw128(smem_u32(sY), 16), dYm = desc_lo_sw128(smem_u32(sY), kBlockBytes);
-        const int T = sc.T;
-        int ts = decode_a(ub, sc).tile, tp = ts, sg = -1, so = -1, st_s = 0, st_p = 0, use = 0;  // tile within the block, block and stage of the next S and O
-        uint32_t used = 0;  // accumulators that hold something of the current block
-#pragma unroll 1
-        for (int k = 0; k < n_iter + 2; k++) {
-            const bool do_s = k < n_iter, do_p = k >= 2, last = k == n_iter - 1, first_s = k == 0 || ts == 0, first_p = k == 2 || tp == 0;
-            if (do_s) {
-                sg += first_s ? 1 : 0;
-                if (first_s && !spin_wait(kBarXFull + (sg & 1), (sg >> 1) & 1)) break;
-                if (!spin_wait(kBarYFull + st_s, use & 1)) break;
-            }
-            if (do_p) {
-                if (first_p) {
-                    used = 0;
-                    so++;
-                    if (!spin_wait(kBarOEmpty, (so & 1) ^ 1)) break;  // the drain has read the previous block's O
-                }
-                if (!spin_wait(kBarPFull + (k & 1), ((k - 2) >> 1) & 1)) break;
-            }
-            tc_fence_after();
-            const uint32_t s = tmem + (k & 1) * 128;
-            if (do_p) {
-                const uint32_t o = tmem + 256 + (NEG ? 0 : (k & 1) * 128), p0 = s + 32, b0 = dYm + st_p * (LY::kTileBytes >> 4);
-                const uint32_t more = (used >> (NEG ? 0 : k & 1)) & 1u;
-#pragma unroll
-                for (int ks = 0; ks < BN / kMmaK; ks++)  // P sits in columns 32 ... 63 and 96 ... 127 of the score accumulator
-                    mma_f16_ts_warp(o, p0 + (ks >> 2) * 64 + (ks & 3) * 8, b0 + (uint32_t)koff_mnmajor(ks), idesc_o, ks > 0 ? 1u : more);
-                used |= 1u << (NEG ? 0 : k & 1);
-                mma_commit_warp(&bars[kBarYEmpty + st_p]);
-                if (k == n_iter + 1 || tp == T - 1) mma_commit_warp(&bars[kBarOFull]);
-                tp = tp == T - 1 ? 0 : tp + 1;
-                st_p = st_p == kStages - 1 ? 0 : st_p + 1;
-            }
-            if (do_s) {
-                const uint32_t x0 = dXk + (sg & 1) * (LY::kTileBytes >> 4), y0 = dYk + st_s * (LY::kTileBytes >> 4);
-#pragma unroll
-                for (int ks = 0; ks < DP / kMmaK; ks++) mma_f16_ss_warp(s, x0 + (uint32_t)koff_kmajor(ks), y0 + (uint32_t)koff_kmajor(ks), kIdescS, ks > 0);
-                mma_commit_warp(&bars[kBarSFull + (k & 1)]);
-                if (last || ts == T - 1) mma_commit_warp(&bars[kBarXEmpty + (sg & 1)]);
-                ts = ts == T - 1 ? 0 : ts + 1;
-                if (++st_s == kStages) st_s = 0, use++;
-            }
-        }
-    } else if (warp < kSoftmaxWarps) {
-        // ================================ softmax warps (0-15) ================================
-        const int grp = warp >> 3, ch = (warp >> 2) & 1, wq = warp & 3;
+    if (warp < kSoftmaxWarps) {
+        // ================================ softmax warps (0-7) ================================
+        const int grp = warp >> 2, wq = warp & 3;
         const int my_row = tid & 127;   // accumulator row / tensor-memory lane
-        const uint32_t tS = tmem + grp * 128 + ch * 64 + lane_sel;  // this warp's 64 score columns
+        const uint32_t tS = tmem + grp * 128 + lane_sel;
         IterA un(ub, sc);
-        float m = -INFINITY, l = 0.f;  // queries: reference and sum (scaled by 2^14) of this group's tiles of the block; the reference is shared by the halves
-        int sg = -1;
-#pragma unroll 1
-        for (int it = 0; it < n_iter; it++, un.next(sc)) {
-            if (it == 0 || un.tile == 0) {
-                sg++;
-                m = -INFINITY;
+        float m = kNoReference, l = 0.f;  // queries: reference and sum (scaled by 2^14) of this group's tiles of the block
+        if (grp == 1) un.next(sc);
+        int item = decode_a(ub, sc).item, sg = 0;  // the block at hand, and how many came before it
+        float pos2 = 0.f;  // positive score of my row in the block at hand
+        auto leave = [&](int next) -> bool {  // queries: what this group knows about the blocks before `next`
+            for (; item < next; item++, sg++) {
+                const int h = sg & 1;
+                if (!warp_wait(kBarStatFree + h, ((sg >> 1) & 1) ^ 1)) return false;
+                s_stat[(h * 2 + grp) * 128 + my_row] = make_float2(m, l);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars[kBarStat + h]);
+                m = kNoReference;
                 l = 0.f;
             }
-            if ((it & 1) == grp) {
-                const int nth = it >> 1, stage = it & (kInfoStages - 1);
-                const int nv = y_rows - un.tile * BN - ch * 64;  // columns of this warp's 64 that exist
-                if (!warp_wait(kBarInfoFull + stage, (it / kInfoStages) & 1)) break;
-                uint32_t mb[2] = {0u, 0u};  // bits of those masked for my row
-                if (s_any[stage]) {
-                    const int* msk = s_mask + stage * 128;
-                    if (NEG) {
-                        const int col = msk[my_row] - ch * 64;
-                        if ((unsigned)col < 64u) (col < 32 ? mb[0] : mb[1]) = 1u << (col & 31);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 2; k++) {
-                            const int row = msk[ch * 64 + k * 32 + lane];
-                            unsigned ballot = __ballot_sync(0xffffffffu, row >= 0 && (row >> 5) == wq);
-                            while (ballot != 0) {
-                                const int src = __ffs(ballot) - 1;
-                                ballot &= ballot - 1;
-                                if (__shfl_sync(0xffffffffu, row, src) == my_row) mb[k] |= 1u << src;
-                            }
-                        }
+            return true;
+        };
+        bool ok = true;
+#pragma unroll 1
+        for (int it = grp; it < n_iter; it += 2, un.next(sc), un.next(sc)) {
+            if (!NEG && !(ok = leave(un.item))) break;
+            if (!NEG && (it == grp || un.tile < 2)) {  // (a block's first tile for this group)
+                const int r = un.rb * BM + my_row;
+                pos2 = r < x_rows ? __ldg(&L.pos[(int64_t)un.zc * L.npc + r]) * kLog2e : kNoReference;
+            }
+            const int nth = it >> 1, stage = it & (kInfoStages - 1);
+            const int nv = y_rows - un.tile * BN;  // columns of the tile that exist (negatives: the others' lse leaves nothing of them)
+            if ((NEG || fs.masks) && !warp_wait(kBarInfoFull + stage, (it / kInfoStages) & 1)) break;
+            const bool masked = fs.masks && s_any[stage];
+            if (!warp_wait(kBarSFull + grp, nth & 1)) break;
+            tc_fence_after();
+            if (masked || (!NEG && nv < BN)) {
+                // scores of masked entries, and of columns that do not exist, are replaced in tensor memory: few tiles have any
+                const float value = NEG ? -INFINITY : kMasked;
+                const int* msk = s_mask + stage * 128;
+#pragma unroll 1
+                for (int k = masked ? 0 : 4; k < 4; k++) {
+                    const int w = msk[NEG ? my_row : k * 32 + lane];  // negatives: the column of my row, queries: the row of a column
+                    unsigned left = __ballot_sync(0xffffffffu, NEG ? (w >> 5) == k : (w >> 5) == wq);
+                    while (left != 0) {
+                        const int src = __ffs(left) - 1;
+                        left &= left - 1;
+                        const int of = __shfl_sync(0xffffffffu, w, src);
+                        const uint32_t at = tS + (NEG ? of : k * 32 + src);
+                        const float x = tmem_ld_32x1(at);
+                        tmem_st_32x1(at, (NEG ? lane == src : my_row == of) ? value : x);
+                        tmem_st_wait();
                     }
                 }
-                const bool odd = __any_sync(0xffffffffu, (mb[0] | mb[1]) != 0u) || nv < 64;
-                if (!warp_wait(kBarSFull + grp, nth & 1)) break;
-                tc_fence_after();
-                // 32 scores: masked and absent ones replaced
-                auto load = [&](int k, float (&v)[32]) {
-                    tmem_ld_32x32(tS + k * 32, v);
-                    if (odd) {
-                        const float masked = NEG ? -INFINITY : kMasked;
-                        const uint32_t bits = k == 0 ? mb[0] : mb[1];
-                        const int live = nv - k * 32;
-#pragma unroll
-                        for (int j = 0; j < 32; j++) v[j] = j >= live ? -INFINITY : ((bits >> j) & 1u) ? masked : v[j];
-                    }
-                };
-                float v[32];
-                float shift = 0.f;
                 if (!NEG) {
-                    float tmax = -INFINITY;
-                    float* dump = un.zc < d.C ? d.neg_scores : d.inv_neg_scores;
 #pragma unroll 1
-                    for (int k = 0; k < 2; k++) {
-                        load(k, v);
-                        float mx[4];
-#pragma unroll
-                        for (int q = 0; q < 4; q++) mx[q] = v[q];
-#pragma unroll
-                        for (int j = 4; j < 32; j++) mx[j & 3] = fmaxf(mx[j & 3], v[j]);
-                        tmax = fmaxf(tmax, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
-                        if (dump != nullptr && my_row < x_rows - un.rb * BM) {  // the score dump of the tests
-                            float* drow = dump + ((int64_t)(un.zc >= d.C ? un.zc - d.C : un.zc) * L.npc + un.rb * BM + my_row) * d.N + un.tile * BN + ch * 64 + k * 32;
-#pragma unroll
-                            for (int j = 0; j < 32; j++)
-                                if (k * 32 + j < nv) drow[j] = v[j];
-                        }
+                    for (int c = nv; c < BN; c++) tmem_st_32x1(tS + c, -INFINITY);
+                }
+                tmem_st_wait();
+            }
+            if (!NEG) {
+                float* dump = un.zc < d.C ? d.neg_scores : d.inv_neg_scores;
+                if (__builtin_expect(dump != nullptr, 0)) {  // the score dump of the tests
+                    float* drow = dump + ((int64_t)(un.zc >= d.C ? un.zc - d.C : un.zc) * L.npc + un.rb * BM + my_row) * d.N + un.tile * BN;
+#pragma unroll 1
+                    for (int c = 0; c < min(nv, BN); c++) {
+                        const float x = tmem_ld_32x1(tS + c);
+                        if (my_row < x_rows - un.rb * BM) drow[c] = x;
                     }
-                    // the row's maximum over both halves of the tile
-                    float* mine = s_max + ((grp * 2 + (nth & 1)) * 2 + ch) * 128 + my_row;
-                    *mine = tmax;
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars[kBarMax + grp * 4 + wq]);
-                    if (!warp_wait(kBarMax + grp * 4 + wq, nth & 1)) break;
-                    tmax = fmaxf(tmax, mine[ch == 0 ? 128 : -128]) * kLog2e;
-                    // The reference starts 2^3 above the first tile's maximum and follows only when it would be left more than a factor 2
-                    // behind (P <= 2^15 fits fp16): O and the sum have to be rescaled when that happens, for 32 rows at a time, so it
-                    // should be rare (without the head start some row of a warp did in nearly every tile).
-                    const bool first = m == -INFINITY, up = tmax > m + 1.f;
+                }
+            }
+            // P over the lower half of the 64 score columns it is made from, with the next 64 on their way
+            const float* neg_lse = s_lse + stage * 128;
+            float va[32], vb[32];
+            tmem_ld_32x32_start(tS + 64, va);
+            tmem_ld_32x32_start(tS + 96, vb);
+#pragma unroll 1
+            for (int h = 1; h >= 0; h--) {
+                uint32_t wa[16], wb[16];
+                float2 sum[2];  // of this half
+                bool settled = false;
+                tmem_ld_wait(va, vb);
+#pragma unroll 1
+                for (;;) {
+                    // Queries: the reference starts 2^3 above the larger of the positive score (which is in the lse, so nothing is lost below
+                    // it) and the maximum of the group's first scores, and follows only when a P might leave fp16's range: O and the sum have to
+                    // be rescaled when that happens, for 32 rows at a time, so it should be rare (without the head start some row of a warp did
+                    // in nearly every tile, with the first scores alone in many while the positive ones are being learned).  It is
+                    // looked for in sums of the exponentials (of 16 of them: none is larger), not in a pass over the scores.
+                    if (NEG || settled || !__any_sync(0xffffffffu, m == kNoReference)) {
+                        const float neg_shift = (float)kWShift - m;
+                        sum[0] = sum[1] = make_float2(0.f, 0.f);
+#pragma unroll
+                        for (int k = 0; k < 2; k++) {
+                            float (&v)[32] = k == 0 ? va : vb;
+                            uint32_t (&w)[16] = k == 0 ? wa : wb;
+#pragma unroll
+                            for (int q = 0; q < 8; q++) {
+                                float4 sh = make_float4(neg_shift, neg_shift, neg_shift, neg_shift);
+                                if (NEG) sh = *reinterpret_cast<const float4*>(neg_lse + h * 64 + k * 32 + 4 * q);
+                                float2 a = fma2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(kLog2e, kLog2e), make_float2(sh.x, sh.y));
+                                float2 b = fma2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(kLog2e, kLog2e), make_float2(sh.z, sh.w));
+                                a.x = exp2f_fast(a.x), a.y = exp2f_fast(a.y), b.x = exp2f_fast(b.x), b.y = exp2f_fast(b.y);
+                                if (!NEG) sum[0] = add2(sum[0], a), sum[1] = add2(sum[1], b);
+                                w[2 * q] = pack_half2(a.x, a.y);
+                                w[2 * q + 1] = pack_half2(b.x, b.y);
+                                asm volatile("" : "+r"(w[2 * q]), "+r"(w[2 * q + 1]));  // (packed before anything else is looked at)
+                            }
+                        }
+                        if (NEG || settled) break;
+                        if (__builtin_expect(!__any_sync(0xffffffffu, fmaxf(fmaxf(sum[0].x, sum[0].y), fmaxf(sum[1].x, sum[1].y)) > 65504.f), 1)) break;
+                    }
+                    settled = true;  // (whatever is found, everything is done again: nothing has to be kept meanwhile)
+                    float tmax = -INFINITY;
+#pragma unroll
+                    for (int j = 0; j < 32; j++) tmax = fmaxf(tmax, fmaxf(va[j], vb[j]));
+                    tmax *= kLog2e;
+                    if (m == kNoReference) tmax = fmaxf(tmax, pos2);
+                    const bool up = tmax > m - 2.f;  // (by at least a factor 2)
                     tmax += kHeadStart;
-                    if (__any_sync(0xffffffffu, up && !first)) {
+                    if (__any_sync(0xffffffffu, up && m != kNoReference)) {
+                        // (the contraction of this tile's first half may be adding to O)
+                        if (h == 0 && !(ok = warp_wait(kBarHalf + grp, nth & 1))) break;
+                        tc_fence_after();
                         const float f = up ? exp2f_fast(m - tmax) : 1.f;
                         l *= f;
 #pragma unroll 1
-                        for (int q = ch; q * 16 < d.D; q += 2) {
-                            float o[16];
-                            uint32_t w[16];
-                            const uint32_t at = tmem + 256 + grp * 128 + lane_sel + q * 16;
-                            tmem_ld_32x16(at, o);
+                        for (int q = 0; q * 32 < d.D; q++) {
+                            const uint32_t at = tmem + 256 + grp * 128 + lane_sel + q * 32;
+                            float o[32];
+                            tmem_ld_32x32(at, o);
 #pragma unroll
-                            for (int j = 0; j < 16; j++) w[j] = __float_as_uint(o[j] * f);
-                            tmem_st_32x16(at, w);
+                            for (int k = 0; k < 2; k++) {
+                                uint32_t x[16];
+#pragma unroll
+                                for (int j = 0; j < 16; j++) x[j] = __float_as_uint(o[k * 16 + j] * f);
+                                tmem_st_32x16_start(at + k * 16, x);
+                            }
                         }
+                        tmem_st_wait();
                     }
                     if (up) m = tmax;
-                    shift = m - (float)kWShift;
                 }
-                // P over the upper half of this warp's score columns, whose scores (the second 32) are in registers or used up by then
-                float add[4] = {0.f, 0.f, 0.f, 0.f};
-                const float* lse = s_lse + stage * 128 + ch * 64;
-#pragma unroll 1
-                for (int k = 1; k >= 0; k--) {
-                    if (NEG || k == 0) load(k, v);  // (queries: the second half is still there)
-                    uint32_t w[16];
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        float4 sh = make_float4(shift, shift, shift, shift);
-                        if (NEG) sh = *reinterpret_cast<const float4*>(lse + k * 32 + 4 * q);
-                        const float e0 = exp2f_fast(fmaf(v[4 * q], kLog2e, -sh.x)), e1 = exp2f_fast(fmaf(v[4 * q + 1], kLog2e, -sh.y));
-                        const float e2 = exp2f_fast(fmaf(v[4 * q + 2], kLog2e, -sh.z)), e3 = exp2f_fast(fmaf(v[4 * q + 3], kLog2e, -sh.w));
-                        if (!NEG) add[0] += e0, add[1] += e1, add[2] += e2, add[3] += e3;
-                        w[2 * q] = pack_half2(e0, e1);
-                        w[2 * q + 1] = pack_half2(e2, e3);
-                    }
-                    tmem_st_32x16(tS + 32 + k * 16, w);
+                if (!ok) break;
+                if (!NEG) {
+                    const float2 x = add2(sum[0], sum[1]);
+                    l += x.x + x.y;
                 }
-                l += (add[0] + add[1]) + (add[2] + add[3]);
+                if (h == 1) {
+                    tmem_ld_32x32_start(tS, va);
+                    tmem_ld_32x32_start(tS + 32, vb);
+                }
+                tmem_st_32x16_start(tS + h * 64, wa);
+                tmem_st_32x16_start(tS + h * 64 + 16, wb);
+                tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&bars[kBarPFull + grp]);
-                    mbar_arrive(&bars[kBarInfoEmpty + stage]);
-                }
+                if (lane == 0) mbar_arrive(&bars[kBarPFull + grp * 2 + h]);
             }
-            if (!NEG && (it == n_iter - 1 || un.tile == sc.T - 1)) {  // end of the block (or of this CTA's share of it)
-                const int h = sg & 1;
-                if (!warp_wait(kBarStatFree + h, ((sg >> 1) & 1) ^ 1)) break;
-                s_stat[(h * 4 + grp * 2 + ch) * 128 + my_row] = make_float2(m, l);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars[kBarStat + h]);
-            }
+            if (!ok) break;
+            if ((NEG || fs.masks) && lane == 0) mbar_arrive(&bars[kBarInfoEmpty + stage]);
         }
+        if (!NEG && ok && n_iter > 0) leave(decode_a(ue - 1, sc).item + 1);
     } else if (warp < kTmaWarp) {
-        // ================================ drain warps (16-19) ================================
+        regs_inc<kDrainRegs>();
+        // ================================ drain warps (8-11) ================================
         const int wq = warp & 3;
         if (NEG) {
             // dQ of the blocks the first launch split between CTAs, from the parts they left: boundary j of that launch is looked after
@@ -452,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         const int drain_slabs = full_slabs + (tail > 0 ? 1 : 0);
         unsigned char* scr = smem + LY::kDrain + wq * 4096;
-        int sg = 0;
+        int sg = 0, filled[2] = {0, 0};  // blocks so far, of them with a tile of either group
 #pragma unroll 1
         for (int u = ub; u < ue; sg++) {
             const UnitA un = decode_a(u, sc);
@@ -460,30 +452,73 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool whole = un.tile == 0 && seg_end == (un.item + 1) * sc.T;
             const int row0 = un.rb * BM + wq * 32;
             const bool live = row0 + lane < x_rows;
-            float w0 = 1.f, w1 = 0.f;
+            // Iterations u - ub ... seg_end - ub - 1 alternate between the groups and their accumulators; the one that the next block's first tile
+            // wants is read first.
+            const int acc0 = (seg_end - ub) & 1;
+            const bool two = seg_end - u > 1, have0 = two || ((u - ub) & 1) == acc0, have1 = two || !have0;
+            int& n0 = acc0 == 0 ? filled[0] : filled[1];
+            int& n1 = acc0 == 0 ? filled[1] : filled[0];
+            float pos2 = 0.f;
+            if (!NEG && live) pos2 = __ldg(&L.pos[(int64_t)un.zc * L.npc + row0 + lane]) * kLog2e;
+            // the whole of O into registers, so that the accumulators are free before anything is stored; the first of them as it is, before the
+            // other group is done
+            float v[DP];
+            if (have0) {
+                if (!warp_wait(kBarOFull + acc0, n0++ & 1)) break;
+                tc_fence_after();
+            }
+#pragma unroll
+            for (int q = 0; q < DP / 32; q++) {
+                float o[32];
+                if (have0) tmem_ld_32x32(tmem + 256 + acc0 * 128 + lane_sel + q * 32, o);
+#pragma unroll
+                for (int j = 0; j < 32; j++) v[q * 32 + j] = have0 ? o[j] : 0.f;
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (have0 && lane == 0) mbar_arrive(&bars[kBarOEmpty + acc0]);
+            float w1 = 1.f, m = 0.f, l = 0.f, lse2 = 0.f;
             if (!NEG) {
                 const int h = sg & 1, r = wq * 32 + lane;
-                const int64_t grow = (int64_t)un.zc * L.npc + row0 + lane;
-                const float pos2 = live ? __ldg(&L.pos[grow]) * kLog2e : 0.f;
                 if (!warp_wait(kBarStat + h, (sg >> 1) & 1)) break;
-                const float2 a0 = s_stat[(h * 4 + 0) * 128 + r], a1 = s_stat[(h * 4 + 1) * 128 + r];
-                const float2 b0 = s_stat[(h * 4 + 2) * 128 + r], b1 = s_stat[(h * 4 + 3) * 128 + r];
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars[kBarStatFree + h]);
-                const float m = fmaxf(a0.x, b0.x);  // (a group without a tile in this share: -inf, weight 0)
-                w0 = exp2f_fast(a0.x - m), w1 = exp2f_fast(b0.x - m);
-                const float l = ((a0.y + a1.y) * w0 + (b0.y + b1.y) * w1) * (1.f / (1 << kWShift));
+                const float2 a0 = s_stat[(h * 2 + acc0) * 128 + r], b0 = s_stat[(h * 2 + (acc0 ^ 1)) * 128 + r];
+                m = fmaxf(a0.x, b0.x);  // (a group without a tile in this share: weight 0)
+                float w0 = exp2f_fast(a0.x - m);
+                w1 = exp2f_fast(b0.x - m);
+                l = (a0.y * w0 + b0.y * w1) * (1.f / (1 << kWShift));
                 if (whole) {
                     const float nm = fmaxf(m, pos2);
-                    const float lse2 = nm + __log2f(l * exp2f_fast(m - nm) + exp2f_fast(pos2 - nm));
+                    lse2 = nm + __log2f(l * exp2f_fast(m - nm) + exp2f_fast(pos2 - nm));
                     const float f = exp2f_fast(m - lse2);
                     w0 *= f, w1 *= f;
+                }
+#pragma unroll
+                for (int j = 0; j < DP; j++) v[j] *= w0;
+            }
+            if (have1) {
+                if (!warp_wait(kBarOFull + (acc0 ^ 1), n1++ & 1)) break;
+                tc_fence_after();
+#pragma unroll
+                for (int q = 0; q < DP / 32; q++) {
+                    float o[32];
+                    tmem_ld_32x32(tmem + 256 + (acc0 ^ 1) * 128 + lane_sel + q * 32, o);
+#pragma unroll
+                    for (int j = 0; j < 32; j++) v[q * 32 + j] = NEG ? v[q * 32 + j] + o[j] : fmaf(o[j], w1, v[q * 32 + j]);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (have1 && lane == 0) mbar_arrive(&bars[kBarOEmpty + (acc0 ^ 1)]);
+            if (!NEG) {
+                if (lane == 0) mbar_arrive(&bars[kBarStatFree + (sg & 1)]);
+                const int64_t grow = (int64_t)un.zc * L.npc + row0 + lane;
+                if (whole) {
                     float loss = 0.f;
                     if (live) {
                         L.lse[grow] = lse2 * kLn2;
                         loss = (lse2 - pos2) * kLn2;
                     }
-                    L.lse2s[(int64_t)un.item * BM + r] = live ? lse2 - (float)kWShift : kDeadRow;
+                    L.lse2s[(int64_t)un.item * BM + wq * 32 + lane] = live ? lse2 - (float)kWShift : kDeadRow;
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
                     if (lane == 0) atomicAdd(L.loss_acc, (double)loss);
@@ -492,42 +527,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (part < kMaxParts) reinterpret_cast<float2*>(L.part)[grow * kMaxParts + part] = make_float2(m, l);
                 }
             }
-            // which groups had a tile: iterations u - ub ... seg_end - ub - 1 alternate between them
-            const bool two = !NEG && seg_end - u > 1;
-            const int only = !NEG && !two ? (u - ub) & 1 : 0;
-            if (only == 1) w0 = w1;
-            if (!warp_wait(kBarOFull, sg & 1)) break;
-            tc_fence_after();
             float* part_rows = L.o_part + (((int64_t)blockIdx.x * 2 + (un.tile == 0 ? 1 : 0)) * BM + wq * 32 + lane) * DP;
             int y = row0, z = un.zc;
             // The coordinates are pinned in ordinary registers here, where the whole warp is active: taken straight from the
             // index arithmetic into the one-lane section below, the third coordinate was seen to reach the store as 0.
             asm volatile("" : "+r"(y), "+r"(z));
-#pragma unroll 1
-            for (int cb = 0; cb < drain_slabs; cb++) {
-                float v[32];
-                tmem_ld_32x32(tmem + 256 + only * 128 + lane_sel + cb * 32, v);
-                if (!NEG) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] *= w0;
-                    if (two) {
-#pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            float o[16];
-                            tmem_ld_32x16(tmem + 384 + lane_sel + cb * 32 + q * 16, o);
-#pragma unroll
-                            for (int j = 0; j < 16; j++) v[q * 16 + j] = fmaf(o[j], w1, v[q * 16 + j]);
-                        }
-                    }
-                }
-                if (cb == drain_slabs - 1) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars[kBarOEmpty]);
-                }
+            for (int cb = 0; cb < DP / 32; cb++) {
+                if (cb >= drain_slabs) break;
                 if (!NEG && !whole) {
 #pragma unroll
-                    for (int q = 0; q < 8; q++) *reinterpret_cast<float4*>(part_rows + cb * 32 + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    for (int q = 0; q < 8; q++)
+                        *reinterpret_cast<float4*>(part_rows + cb * 32 + 4 * q) =
+                            make_float4(v[cb * 32 + 4 * q], v[cb * 32 + 4 * q + 1], v[cb * 32 + 4 * q + 2], v[cb * 32 + 4 * q + 3]);
                     continue;
                 }
                 if (lane == 0) bulk_wait_group_read<0>();  // the operation that last used the slab has read it
@@ -536,12 +548,14 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!narrow) {
 #pragma unroll
                     for (int q = 0; q < 8; q++)
-                        *reinterpret_cast<float4*>(scr + lane * 128 + ((q ^ (lane & 7)) << 4)) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                        *reinterpret_cast<float4*>(scr + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                            make_float4(v[cb * 32 + 4 * q], v[cb * 32 + 4 * q + 1], v[cb * 32 + 4 * q + 2], v[cb * 32 + 4 * q + 3]);
                 } else {
 #pragma unroll
                     for (int q = 0; q < 8; q++)
                         if (q * 4 < tail)
-                            *reinterpret_cast<float4*>(scr + lane * (tail * 4) + q * 16) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                            *reinterpret_cast<float4*>(scr + lane * (tail * 4) + q * 16) =
+                                make_float4(v[cb * 32 + 4 * q], v[cb * 32 + 4 * q + 1], v[cb * 32 + 4 * q + 2], v[cb * 32 + 4 * q + 3]);
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
@@ -557,89 +571,190 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) bulk_wait_group<0>();  // all of this warp's stores have landed before the CTA can exit
         __syncwarp();
     } else {
-        // ================================ warps 22-23 ================================
-        const int grp = warp - kHelpWarp;
-        if (!NEG) {
-            // clear the dK rows the second launch reduces into: those of every block whose stream it cuts at a CTA boundary (boundary j
-            // is looked after by CTA (j - 1) % gridDim.x)
-#pragma unroll 1
-            for (int j = 1 + (int)blockIdx.x; j < fs.n.gridA; j += (int)gridDim.x) {
-                const UnitA un = decode_a(range_begin(j, fs.n.unitsA, fs.n.gridA), fs.n);
-                if (un.tile == 0) continue;  // the boundary falls between two blocks: nothing is split
-                float4* p4 = reinterpret_cast<float4*>(L.dK + ((int64_t)un.zc * d.N + (int64_t)un.rb * BM) * DP);
-                const int n4 = min(BM, d.N - un.rb * BM) * (DP / 4);
-#pragma unroll 4
-                for (int k = grp * 32 + lane; k < n4; k += 64) p4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        }
-        const float per_unit = NEG ? (float)fs.q.gridA / (float)fs.q.unitsA : 0.f;
-        IterA un(ub, sc);
-        if (grp == 1) un.next(sc);
-#pragma unroll 1
-        for (int it = grp; it < n_iter; it += 2, un.next(sc), un.next(sc)) {
-            const int stage = it & (kInfoStages - 1);
-            // filter words: one per negative, naming a batch row in the padded numbering
-            int w[4];
-            const int n0 = (NEG ? un.rb : un.tile) * 128;
-            const int r0 = (un.zc >= d.C ? un.zc - d.C : un.zc) * L.npc + (NEG ? un.tile : un.rb) * 128;
+        regs_dec<kServiceRegs>();
+        if (warp == kTmaWarp) {
+            int sg = -1, users[2] = {0, 0}, uses[4] = {0, 0, 0, 0};  // of the X buffers: groups with a tile of the block there, uses so far [buffer][group]
+            bool ok = true;
+            IterA un(ub, sc);
+            for (int it = 0; it < n_iter; it++, un.next(sc)) {
+                if (it == 0 || un.tile == 0) {  // a new block
+                    sg++;
+                    const int xs = sg & 1;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int j = n0 + q * 32 + lane;
-                w[q] = j < d.N ? __ldg(&L.mask[(int64_t)un.zc * d.N + j]) : -1;
-            }
-            float v[4];
-            if (NEG) {
-                const int item = un.zc * fs.q.RB + un.tile;  // the query block these columns are
-                const int u0 = item * fs.q.T, u1 = u0 + fs.q.T;
-                int p = min((int)((float)u0 * per_unit), fs.q.gridA - 1), nparts = 1;
-                while (s_range[p] > u0) p--;
-                while (s_range[p + 1] <= u0) p++;
-                while (s_range[p + nparts] < u1) nparts++;
-                const int64_t grow0 = (int64_t)un.zc * L.npc + un.tile * BN;
-                if (nparts == 1) {
-#pragma unroll
-                    for (int q = 0; q < 4; q++) v[q] = __ldg(&L.lse2s[(int64_t)item * BM + q * 32 + lane]);
-                } else {
-                    float4 pk[4];  // (m, sum) of the first two parts
-                    float pos2[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int r = min(q * 32 + lane, L.npc - 1 - un.tile * BN);
-                        pk[q] = __ldg(reinterpret_cast<const float4*>(L.part + (grow0 + r) * kMaxParts * 2));
-                        pos2[q] = __ldg(&L.pos[grow0 + r]) * kLog2e;
+                    for (int g = 0; g < 2; g++) {
+                        int& n = xs == 0 ? uses[g] : uses[2 + g];
+                        if (((xs == 0 ? users[0] : users[1]) >> g) & 1) ok = ok && warp_wait(kBarXEmpty + 2 * xs + g, n & 1), n++;
                     }
+                    if (!ok) break;
+                    (xs == 0 ? users[0] : users[1]) = min(sc.T - un.tile, n_iter - it) > 1 ? 3 : 1 << (it & 1);
+                    mbar_expect_tx_warp(&bars[kBarXFull + xs], LY::kTileBytes);
+#pragma unroll
+                    for (int b = 0; b < NB; b++) tma_load_3d_warp(sX + xs * LY::kTileBytes + b * kBlockBytes, &tmX, b * 64, un.rb * BM, un.zc, &bars[kBarXFull + xs]);
+                }
+                const int st = it % kStages;
+                if (!warp_wait(kBarYEmpty + st, ((it / kStages) & 1) ^ 1)) break;
+                mbar_expect_tx_warp(&bars[kBarYFull + st], LY::kTileBytes);
+#pragma unroll
+                for (int b = 0; b < NB; b++)
+                    tma_load_3d_warp(sY + st * LY::kTileBytes + b * kBlockBytes, &tmY, b * 64, un.tile * BN, un.zc, &bars[kBarYFull + st]);
+            }
+        } else if (warp < kHelpWarp) {
+            // ================================ contractions ================================
+            // One warp a group, so that one's waits do not keep the tensor pipe from the other's contractions.  S of the group's next tile follows O
+            // of this one, so the score accumulator is overwritten only behind the contraction that reads the P in it, and "S complete"
+            // also says that the O contraction is.
+            const int g = warp - kMmaWarp;
+            const int D16 = ((d.D + kMmaK - 1) / kMmaK) * kMmaK;  // the embedding dimension rounded up to the MMA k step
+            constexpr uint32_t kIdescS = idesc_f16(BM, BN, 0, 0);
+            const uint32_t idesc_o = idesc_f16(BM, D16, 0, 1);
+            const uint32_t dXk = desc_lo_sw128(smem_u32(sX), 16), dYk = desc_lo_sw128(smem_u32(sY), 16), dYm = desc_lo_sw128(smem_u32(sY), kBlockBytes);
+            const uint32_t s = tmem + g * 128, o = tmem + 256 + g * 128;
+            const int T = sc.T;
+            int ts = decode_a(ub, sc).tile + g, bs = 0;  // the tile whose S is next: number within its block, block within this share
+            while (ts >= T) ts -= T, bs++;
+            int to = 0, bo = -1, used = -1, filled = 0;  // the one whose O is next; the block o holds something of; blocks it has held
+            uint32_t par = 0;                            // of this group's tiles
+            // The groups take turns at O of a tile and S of the next one: if both were given to the pipe at once, both would be done
+            // late, and the groups would wait and exponentiate at the same time ever after.
 #pragma unroll 1
-                    for (int q = 0; q < 4; q++) {
-                        const float4 a4 = q == 0 ? pk[0] : q == 1 ? pk[1] : q == 2 ? pk[2] : pk[3];
-                        const float ps = q == 0 ? pos2[0] : q == 1 ? pos2[1] : q == 2 ? pos2[2] : pos2[3];
-                        float x;
-                        if (nparts == 2) {
-                            const float mm = fmaxf(ps, fmaxf(a4.x, a4.z));
-                            x = mm + __log2f(exp2f_fast(ps - mm) + a4.y * exp2f_fast(a4.x - mm) + a4.w * exp2f_fast(a4.z - mm));
-                        } else {
-                            x = combine_parts(reinterpret_cast<const float2*>(L.part) + (grow0 + min(q * 32 + lane, L.npc - 1 - un.tile * BN)) * kMaxParts, nparts, ps);
+            for (int k = g; k < n_iter + 2; k += 2) {
+                const bool do_s = k < n_iter, do_o = k >= 2;
+                const int xs = bs & 1, st = k % kStages, ko = k - 2;
+                // whatever S needs besides its place is there before O is issued: nothing comes between the two in the pipe
+                if (do_s) {
+                    if (bs != bo && !warp_wait(kBarXFull + xs, (bs >> 1) & 1)) break;
+                    if (!warp_wait(kBarYFull + st, (k / kStages) & 1)) break;
+                }
+                bool ok = true;
+                if (do_o) {
+                    uint32_t more = 1u;
+                    if (used != bo) {  // a new block: the drain has read what is there
+                        if (!warp_wait(kBarOEmpty + g, (filled & 1) ^ 1)) break;
+                        filled++;
+                        used = bo;
+                        more = 0u;
+                    }
+                    const uint32_t y0 = dYm + (ko % kStages) * (LY::kTileBytes >> 4);
+#pragma unroll
+                    for (int h = 1; h >= 0; h--) {  // P of columns 64 h ... + 63 of the tile sits in columns 64 h ... + 31 of the score accumulator
+                        if (!(ok = warp_wait(kBarPFull + g * 2 + h, par) && (h == 0 || warp_wait(kBarTurn + g, g == 0 ? par : par ^ 1u)))) break;
+                        tc_fence_after();
+#pragma unroll
+                        for (int ks = 4 * h; ks < 4 * h + 4; ks++) {
+                            mma_f16_ts_warp(o, s + h * 64 + (ks & 3) * 8, y0 + (uint32_t)koff_mnmajor(ks), idesc_o, more);
+                            more = 1u;
                         }
-                        x = un.tile * BN + q * 32 + lane < L.npc ? x - (float)kWShift : kDeadRow;
-                        v[0] = q == 0 ? x : v[0], v[1] = q == 1 ? x : v[1], v[2] = q == 2 ? x : v[2], v[3] = q == 3 ? x : v[3];
+                        if (!NEG && h == 1) mma_commit_warp(&bars[kBarHalf + g]);
                     }
+                } else if (g == 1) {
+                    ok = warp_wait(kBarTurn + 1, 0);
+                }
+                if (!ok) break;
+                if (do_s) {
+                    const uint32_t x0 = dXk + xs * (LY::kTileBytes >> 4), y0 = dYk + st * (LY::kTileBytes >> 4);
+                    if (!do_o) tc_fence_after();
+#pragma unroll
+                    for (int ks = 0; ks < DP / kMmaK; ks++) mma_f16_ss_warp(s, x0 + (uint32_t)koff_kmajor(ks), y0 + (uint32_t)koff_kmajor(ks), kIdescS, ks > 0);
+                    mma_commit_warp(&bars[kBarSFull + g]);
+                    if (ts + 2 >= T || k + 2 >= n_iter) mma_commit_warp(&bars[kBarXEmpty + 2 * xs + g]);
+                }
+                if (lane == 0) mbar_arrive(&bars[kBarTurn + (g ^ 1)]);
+                __syncwarp();
+                if (do_o) {
+                    mma_commit_warp(&bars[kBarYEmpty + ko % kStages]);
+                    if (to + 2 >= T || !do_s) mma_commit_warp(&bars[kBarOFull + g]);  // the group's last tile of the block
+                    par ^= 1u;
+                }
+                to = ts, bo = bs;
+                ts += 2;
+                while (ts >= T) ts -= T, bs++;
+            }
+        } else {
+            // ================================ warp 15 ================================
+            if (!NEG) {
+                // clear the dK rows the second launch reduces into: those of every block whose stream it cuts at a CTA boundary (boundary j
+                // is looked after by CTA (j - 1) % gridDim.x)
+#pragma unroll 1
+                for (int j = 1 + (int)blockIdx.x; j < fs.n.gridA; j += (int)gridDim.x) {
+                    const UnitA un = decode_a(range_begin(j, fs.n.unitsA, fs.n.gridA), fs.n);
+                    if (un.tile == 0) continue;  // the boundary falls between two blocks: nothing is split
+                    float4* p4 = reinterpret_cast<float4*>(L.dK + ((int64_t)un.zc * d.N + (int64_t)un.rb * BM) * DP);
+                    const int n4 = min(BM, d.N - un.rb * BM) * (DP / 4);
+#pragma unroll 8
+                    for (int k = lane; k < n4; k += 32) p4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             }
-            bool any = false;
+            const int n_info = NEG || fs.masks ? n_iter : 0;
+            const float per_unit = NEG ? (float)fs.q.gridA / (float)fs.q.unitsA : 0.f;
+            int w[4] = {-1, -1, -1, -1};  // of a tile: filter words (one per negative, naming a batch row in the padded numbering)
+            float v[4];                   // ... negatives: the columns' lse
+            auto read = [&](const IterA& un) {
+                if (fs.masks) {
+                    const int n0 = (NEG ? un.rb : un.tile) * 128;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                w[q] = w[q] >= r0 && w[q] < r0 + 128 ? w[q] - r0 : -1;
-                any |= w[q] >= 0;
-            }
-            any = __any_sync(0xffffffffu, any);
-            if (!warp_wait(kBarInfoEmpty + stage, ((it / kInfoStages) & 1) ^ 1)) break;
+                    for (int q = 0; q < 4; q++) {
+                        const int j = n0 + q * 32 + lane;
+                        w[q] = j < d.N ? __ldg(&L.mask[(int64_t)un.zc * d.N + j]) : -1;
+                    }
+                }
+                if (NEG) {
+                    const int item = un.zc * fs.q.RB + un.tile;  // the query block these columns are
+                    const int u0 = item * fs.q.T, u1 = u0 + fs.q.T;
+                    int p = min((int)((float)u0 * per_unit), fs.q.gridA - 1), nparts = 1;
+                    while (s_range[p] > u0) p--;
+                    while (s_range[p + 1] <= u0) p++;
+                    while (s_range[p + nparts] < u1) nparts++;
+                    if (nparts == 1) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                if (any) s_mask[stage * 128 + q * 32 + lane] = w[q];
-                if (NEG) s_lse[stage * 128 + q * 32 + lane] = v[q];
+                        for (int q = 0; q < 4; q++) v[q] = __ldg(&L.lse2s[(int64_t)item * BM + q * 32 + lane]);
+                    } else {  // a block that the first launch split between CTAs
+                        const int64_t grow0 = (int64_t)un.zc * L.npc + un.tile * BN;
+                        float4 pk[4];  // (m, sum) of the first two parts
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const int64_t r = grow0 + min(q * 32 + lane, L.npc - 1 - un.tile * BN);
+                            pk[q] = __ldg(reinterpret_cast<const float4*>(L.part + r * kMaxParts * 2));
+                            v[q] = __ldg(&L.pos[r]) * kLog2e;
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const int r = min(q * 32 + lane, L.npc - 1 - un.tile * BN);
+                            const float mm = fmaxf(v[q], fmaxf(pk[q].x, pk[q].z));
+                            float x = mm + __log2f(exp2f_fast(v[q] - mm) + pk[q].y * exp2f_fast(pk[q].x - mm) + pk[q].w * exp2f_fast(pk[q].z - mm));
+                            if (nparts > 2) x = combine_parts(reinterpret_cast<const float2*>(L.part) + (grow0 + r) * kMaxParts, nparts, v[q]);
+                            v[q] = r == q * 32 + lane ? x - (float)kWShift : kDeadRow;
+                        }
+                    }
+                }
+            };
+            IterA un(ub, sc);
+            if (n_info > 0) read(un);
+#pragma unroll 1
+            for (int it = 0; it < n_info; it++) {
+                const int stage = it & (kInfoStages - 1);
+                const int r0 = (un.zc >= d.C ? un.zc - d.C : un.zc) * L.npc + (NEG ? un.tile : un.rb) * 128;
+                int cw[4];
+                float cv[4];
+                bool any = false;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    cw[q] = w[q] >= r0 && w[q] < r0 + 128 ? w[q] - r0 : -1;
+                    any |= cw[q] >= 0;
+                    if (NEG) cv[q] = v[q];
+                }
+                un.next(sc);
+                if (it + 1 < n_info) read(un);  // (on their way while this tile's are written)
+                any = __any_sync(0xffffffffu, any);
+                if (!warp_wait(kBarInfoEmpty + stage, ((it / kInfoStages) & 1) ^ 1)) break;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (any) s_mask[stage * 128 + q * 32 + lane] = cw[q];
+                    if (NEG) s_lse[stage * 128 + q * 32 + lane] = -cv[q];
+                }
+                if (lane == 0) s_any[stage] = any;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars[kBarInfoFull + stage]);
             }
-            if (lane == 0) s_any[stage] = any;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars[kBarInfoFull + stage]);
         }
     }
     // ---- common exit: every role ends here, normally or after an abort; then tensor memory is released ----------
@@ -651,7 +766,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // tensor memory are handed to the next CTA
             for (int k = 0; k < kStages; k++) settle_bar(&bars[kBarYFull + k]);
             for (int k = 0; k < 2; k++) settle_bar(&bars[kBarSFull + k]);
-            settle_bar(&bars[kBarOFull]);
+            for (int k = 0; k < 2; k++) settle_bar(&bars[kBarOFull + k]);
         }
         __syncwarp();
         tc_fence_after();
@@ -681,6 +796,7 @@ int launch(const LpKernelArgs& a, cudaStream_t stream) {
     if (2 * units > 0x3fffffff) return GE2_ERR_UNSUPPORTED;
     fs.q.RB = qb, fs.q.T = nb, fs.n.RB = nb, fs.n.T = qb;
     fs.q.ZC = fs.n.ZC = ZC;
+    fs.masks = a.d.deg_sample_rows != nullptr || a.d.dst_filter_n > 0 || a.d.src_filter_n > 0;
     fs.q.unitsA = fs.n.unitsA = fs.q.unitsB = fs.n.unitsB = (int)units;
     // every CTA's range is at least ceil(T / 7) units long, so a row block is shared by at most kMaxParts CTAs
     fs.q.gridA = fs.q.gridB = std::max(1, std::min(kNumSMs, (int)units / ceil_div(nb, kMaxParts - 1)));

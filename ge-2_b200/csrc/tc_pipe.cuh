@@ -72,6 +72,18 @@ __device__ __forceinline__ bool warp_pipe_wait(uint64_t* bar, uint32_t parity, v
     return __all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0) || warp_pipe_wait_slow(bar, parity, abort_flag, status);
 }
 
+// The same without a call: a kernel that shares its registers out among its warps (setmaxnreg) cannot have any.
+__device__ __forceinline__ bool warp_wait_inline(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < (1u << 20); i++) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity) ? 1 : 0)) return true;
+        if ((i & 15u) == 15u && __any_sync(0xffffffffu, *abort_flag)) return false;
+    }
+    *abort_flag = 1;
+    or_status(status, GE2_STATUS_PIPE_TIMEOUT);
+    return false;
+}
+
 // What may still be on its way when the roles of a kernel have left their loops after a wait that ran out -- a copy into shared memory, a
 // contraction -- gets a bounded chance to land before that memory goes to the next CTA.  The barrier it arrives on is in either phase: one that
 // has completed its phase 0 is in its phase 1.

@@ -272,6 +272,28 @@ def test_streaming_softmax_where_it_is_taken(capi, cuda_device, kind, B, C, N, D
             assert rel_err(got[key], getattr(o, key)) <= 1e-2, key
 
 
+@pytest.mark.parametrize("kind,B,C,N,D", [("DISTMULT", 330, 110, 1000, 128), ("DISTMULT", 1400, 700, 100, 128), ("COMPLEX", 660, 220, 1100, 64)])
+@pytest.mark.parametrize("rising", [True, False])
+def test_streaming_softmax_reference_moves(capi, cuda_device, kind, B, C, N, D, rising):
+    """Scores that grow along a chunk's negatives by dozens of octaves: the reference of a row has to follow in either half of nearly every tile;
+    falling ones leave it where the first scores put it.  The second shape has one tile a block."""
+    case = workloads.make_case(kind, B, C, N, D, 5, 150, min(N, 50), 21)
+    case.emb *= np.linspace(0.1, 4.0, len(case.emb), dtype=np.float32)[:, None]
+    for negs in (case.dst_negs, case.src_negs):
+        negs.sort(axis=1)
+        if not rising:
+            negs[:] = negs[:, ::-1].copy()
+    case = workloads.BatchCase(case.kind, case.edges, case.emb, case.state, case.rel, case.inv_rel, case.dst_negs, case.src_negs, None, case.filt[:0])
+    o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
+    got = run_lp_step(capi, case, cuda_device, "f16", "pairs", dump_scores=False)
+    assert got["status"] == 0
+    # |q| |k| of up to 190 over 128 terms with operands of 11 bits: 190 / sqrt(128) * 2^-11 = 0.01 in a score, so in a probability
+    assert abs(got["loss"] - o.loss) <= 1e-2 * abs(o.loss)
+    for key in ("node_grad", "rel_grad", "inv_rel_grad"):
+        assert np.isfinite(got[key]).all(), key
+        assert np.linalg.norm(got[key] - getattr(o, key)) <= 2e-2 * np.linalg.norm(getattr(o, key)), key
+
+
 @pytest.mark.parametrize("kind,B,C,N,D", [("COMPLEX", 600, 3, 300, 50), ("COMPLEX", 500, 2, 7001, 100), ("DISTMULT", 300, 2, 3000, 128), ("DISTMULT", 257, 2, 640, 3)])
 def test_one_node_in_most_edges_and_negatives(capi, cuda_device, kind, B, C, N, D):
     """Rows of a node that most edges and degree negatives have are added up where they meet, and leave as sums."""
