@@ -1,4 +1,4 @@
-// Scores kernels of the link-prediction step's tensor path (kind::f16) for batches whose dK does not stay in the L2: the streaming
+// Scores kernels of the link-prediction step's tensor path (kind::f16) for large batches (lp_uses_flash): the streaming
 // softmax, in which every gradient row is written once.  The other kernels of this path (lp_scores_f16.cu) contract a logsumexp pass
 // first and then make dQ and dK from one P; every row block of a chunk adds its part into global dK there, which is the faster way
 // while those reductions hit the L2 and 1.6 GB of HBM traffic when they do not.
@@ -27,12 +27,12 @@
 // exponentiated.
 // Bound by the chain scores -> exponentials -> O -> scores of a group, about 4200 cycles for its tile: 2300 ... 2800 of exponentials (2048 if
 // the unit for them were never idle, for both groups' tiles), 768 of contractions behind the last of them, the hand-overs.  The tensor pipe,
-// 1024 cycles a tile, is half busy.  B = 100 000, N = 2000, D = 128, two sides: 225 + 220 us on fresh tables, 230 + 224 inside training steps.
-// Measured before and on the way there (fresh tables; on one GPU the last of these forms took 229 + 227): two warps a row with a pass over the
-// scores for the maximum and an exchange of it, 258 + 230 (285 + 234 in training); one issuing warp for both groups, 261 + 235; an issuing warp a
+// 1024 cycles a tile, is half busy.  B = 100 000, N = 2000, D = 128, two sides: 226 + 212 us (two warps a row, with a pass over the
+// scores for the maximum and an exchange of it: 259 + 231).
+// Measured on the way there, in turn with a form that took 229 + 227: one issuing warp for both groups, 261 + 235; an issuing warp a
 // group without turns, 246 + 244; with turns at the second half of O only, 229 + 227; halves of a tile as score tiles of their own (the
 // tensor pipe then has 1280 cycles a tile, and every hand-over twice), 264 + 278; an L2 prefetch of tiles to come, 227 + 224; five stages and
-// one X, 221 + 230; three stages, 325 + 287.
+// one X, 221 + 230; three stages, 325 + 287; the maximum of every 64 scores before their exponentials instead of sums of those, 253 + 209 (226 + 212).
 // P carries a factor 2^14, so that probabilities down to 2^-38 keep their full significand instead of falling into fp16's subnormal
 // range; dQ and dK leave this kernel with that factor still on them and the scatter kernel, their only reader, takes it off
 // (LpLayout::grad_unscale).
@@ -69,8 +69,8 @@ constexpr uint32_t kTmemCols = 512;
 constexpr float kMasked = -1e9f;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr int kWShift = 14;             // P is scaled by 2^14; undone by the reader of dQ / dK (kLpF16GradUnscale)
-constexpr float kHeadStart = 3.f;       // queries: log2 of how far the reference is set above the maximum it is taken from
-constexpr float kNoReference = -1e30f;  // queries: no score of the block has been seen by this group yet
+constexpr float kHeadStart = 6.f;       // queries: log2 of how far the reference is set above the maximum it is taken from
+constexpr float kNoReference = -1e30f;  // queries: of a group without a tile of the block
 constexpr float kDeadRow = 1e30f;       // "lse" of a row past the end of its chunk: exp2(anything - 1e30) = 0
 
 enum Bar { kBarXFull = 0, kBarXEmpty = 2, kBarYFull = 6, kBarYEmpty = kBarYFull + kStages, kBarSFull = kBarYEmpty + kStages, kBarPFull = kBarSFull + 2,
@@ -107,6 +107,11 @@ __device__ __forceinline__ float exp2f_fast(float x) {  // one MUFU.EX2; 2^-inf 
     return y;
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {  // one instruction
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
 // two at a time: one instruction, the same roundings
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 r;
@@ -227,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         float m = kNoReference, l = 0.f;  // queries: reference and sum (scaled by 2^14) of this group's tiles of the block
         if (grp == 1) un.next(sc);
         int item = decode_a(ub, sc).item, sg = 0;  // the block at hand, and how many came before it
-        float pos2 = 0.f;  // positive score of my row in the block at hand
+        bool begun = false;  // has this group made a P of the block at hand?
         auto leave = [&](int next) -> bool {  // queries: what this group knows about the blocks before `next`
             for (; item < next; item++, sg++) {
                 const int h = sg & 1;
@@ -246,7 +251,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!NEG && !(ok = leave(un.item))) break;
             if (!NEG && (it == grp || un.tile < 2)) {  // (a block's first tile for this group)
                 const int r = un.rb * BM + my_row;
-                pos2 = r < x_rows ? __ldg(&L.pos[(int64_t)un.zc * L.npc + r]) * kLog2e : kNoReference;
+                m = r < x_rows ? fmaxf(__ldg(&L.pos[(int64_t)un.zc * L.npc + r]) * kLog2e, kNoReference) : 0.f;
+                begun = false;
             }
             const int nth = it >> 1, stage = it & (kInfoStages - 1);
             const int nv = y_rows - un.tile * BN;  // columns of the tile that exist (negatives: the others' lse leaves nothing of them)
@@ -297,52 +303,59 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll 1
             for (int h = 1; h >= 0; h--) {
                 uint32_t wa[16], wb[16];
-                float2 sum[2];  // of this half
-                bool settled = false;
+                float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
                 tmem_ld_wait(va, vb);
+                auto largest = [&](const float (&a)[32]) {
+                    float mx[4] = {max3(a[0], a[1], a[2]), max3(a[3], a[4], a[5]), max3(a[6], a[7], a[8]), max3(a[9], a[10], a[11])};
+#pragma unroll
+                    for (int j = 12; j < 28; j += 2) mx[(j >> 1) & 3] = max3(mx[(j >> 1) & 3], a[j], a[j + 1]);
+                    return max3(max3(mx[0], a[28], a[29]), max3(mx[1], a[30], a[31]), fmaxf(mx[2], mx[3])) * kLog2e;
+                };
+                // Queries: the reference starts at the positive score (that is in the lse, so P is never smaller than the probability) or 2^6 above
+                // the maximum of the group's first tile, whichever is more.  It follows only when a P might leave fp16's range: O and the
+                // sum have to be rescaled then, for 32 rows at a time, so it should be rare (without the head start some row of a warp
+                // did in nearly every tile).  That is looked for in sums of the exponentials (of 16 of them: none is larger), not in a
+                // pass over the scores, which was a tenth of the launch.
+                if (!NEG && !begun && h == 1) {
+                    float tmax = fmaxf(largest(va), largest(vb));
 #pragma unroll 1
-                for (;;) {
-                    // Queries: the reference starts 2^3 above the larger of the positive score (which is in the lse, so nothing is lost below
-                    // it) and the maximum of the group's first scores, and follows only when a P might leave fp16's range: O and the sum have to
-                    // be rescaled when that happens, for 32 rows at a time, so it should be rare (without the head start some row of a warp did
-                    // in nearly every tile, with the first scores alone in many while the positive ones are being learned).  It is
-                    // looked for in sums of the exponentials (of 16 of them: none is larger), not in a pass over the scores.
-                    if (NEG || settled || !__any_sync(0xffffffffu, m == kNoReference)) {
-                        const float neg_shift = (float)kWShift - m;
-                        sum[0] = sum[1] = make_float2(0.f, 0.f);
-#pragma unroll
-                        for (int k = 0; k < 2; k++) {
-                            float (&v)[32] = k == 0 ? va : vb;
-                            uint32_t (&w)[16] = k == 0 ? wa : wb;
-#pragma unroll
-                            for (int q = 0; q < 8; q++) {
-                                float4 sh = make_float4(neg_shift, neg_shift, neg_shift, neg_shift);
-                                if (NEG) sh = *reinterpret_cast<const float4*>(neg_lse + h * 64 + k * 32 + 4 * q);
-                                float2 a = fma2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(kLog2e, kLog2e), make_float2(sh.x, sh.y));
-                                float2 b = fma2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(kLog2e, kLog2e), make_float2(sh.z, sh.w));
-                                a.x = exp2f_fast(a.x), a.y = exp2f_fast(a.y), b.x = exp2f_fast(b.x), b.y = exp2f_fast(b.y);
-                                if (!NEG) sum[0] = add2(sum[0], a), sum[1] = add2(sum[1], b);
-                                w[2 * q] = pack_half2(a.x, a.y);
-                                w[2 * q + 1] = pack_half2(b.x, b.y);
-                                asm volatile("" : "+r"(w[2 * q]), "+r"(w[2 * q + 1]));  // (packed before anything else is looked at)
-                            }
-                        }
-                        if (NEG || settled) break;
-                        if (__builtin_expect(!__any_sync(0xffffffffu, fmaxf(fmaxf(sum[0].x, sum[0].y), fmaxf(sum[1].x, sum[1].y)) > 65504.f), 1)) break;
+                    for (int k = 0; k < 2; k++) {
+                        float x[32];
+                        tmem_ld_32x32(tS + k * 32, x);
+                        tmax = fmaxf(tmax, largest(x));
                     }
-                    settled = true;  // (whatever is found, everything is done again: nothing has to be kept meanwhile)
-                    float tmax = -INFINITY;
+                    m = fmaxf(m, tmax + kHeadStart);
+                }
+#pragma unroll 1
+                for (bool settled = false;; settled = true) {
+                    const float neg_shift = (float)kWShift - m;
+                    sum[0] = sum[1] = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int j = 0; j < 32; j++) tmax = fmaxf(tmax, fmaxf(va[j], vb[j]));
-                    tmax *= kLog2e;
-                    if (m == kNoReference) tmax = fmaxf(tmax, pos2);
-                    const bool up = tmax > m - 2.f;  // (by at least a factor 2)
-                    tmax += kHeadStart;
-                    if (__any_sync(0xffffffffu, up && m != kNoReference)) {
+                    for (int k = 0; k < 2; k++) {
+                        float (&v)[32] = k == 0 ? va : vb;
+                        uint32_t (&w)[16] = k == 0 ? wa : wb;
+#pragma unroll
+                        for (int q = 0; q < 8; q++) {
+                            float4 sh = make_float4(neg_shift, neg_shift, neg_shift, neg_shift);
+                            if (NEG) sh = *reinterpret_cast<const float4*>(neg_lse + h * 64 + k * 32 + 4 * q);
+                            float2 a = fma2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(kLog2e, kLog2e), make_float2(sh.x, sh.y));
+                            float2 b = fma2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(kLog2e, kLog2e), make_float2(sh.z, sh.w));
+                            a.x = exp2f_fast(a.x), a.y = exp2f_fast(a.y), b.x = exp2f_fast(b.x), b.y = exp2f_fast(b.y);
+                            if (!NEG) sum[0] = add2(sum[0], a), sum[1] = add2(sum[1], b);
+                            w[2 * q] = pack_half2(a.x, a.y);
+                            w[2 * q + 1] = pack_half2(b.x, b.y);
+                            asm volatile("" : "+r"(w[2 * q]), "+r"(w[2 * q + 1]));  // (packed before anything else is looked at)
+                        }
+                    }
+                    if (NEG || settled) break;
+                    if (__builtin_expect(!__any_sync(0xffffffffu, fmaxf(fmaxf(sum[0].x, sum[0].y), fmaxf(sum[1].x, sum[1].y)) > 65504.f), 1)) break;
+                    const float tmax = fmaxf(largest(va), largest(vb));
+                    const bool up = tmax > m + 1.f - kHeadStart;  // (by at least a factor 2)
+                    if (begun && __any_sync(0xffffffffu, up)) {
                         // (the contraction of this tile's first half may be adding to O)
                         if (h == 0 && !(ok = warp_wait(kBarHalf + grp, nth & 1))) break;
                         tc_fence_after();
-                        const float f = up ? exp2f_fast(m - tmax) : 1.f;
+                        const float f = up ? exp2f_fast(m - tmax - kHeadStart) : 1.f;
                         l *= f;
 #pragma unroll 1
                         for (int q = 0; q * 32 < d.D; q++) {
@@ -359,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                         tmem_st_wait();
                     }
-                    if (up) m = tmax;
+                    if (up) m = tmax + kHeadStart;
                 }
                 if (!ok) break;
                 if (!NEG) {
@@ -376,6 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars[kBarPFull + grp * 2 + h]);
+                begun = true;
             }
             if (!ok) break;
             if ((NEG || fs.masks) && lane == 0) mbar_arrive(&bars[kBarInfoEmpty + stage]);
@@ -399,12 +413,14 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int r0 = un.rb * BM + wq * 32, rows = min(32, L.npc - r0);
                 if (rows <= 0) continue;
                 const int64_t grow0 = (int64_t)un.zc * L.npc + r0;  // ([S][Bp] = [zc][npc])
-                float lse2 = 0.f, loss = 0.f;
+                float lse2 = 0.f, loss = 0.f, w0 = 0.f, w1 = 0.f;  // (the last two: weights of the first two parts of row `lane`)
                 if (lane < rows) {
                     const float pos2 = __ldg(&L.pos[grow0 + lane]) * kLog2e;
                     lse2 = combine_parts(reinterpret_cast<const float2*>(L.part) + (grow0 + lane) * kMaxParts, nparts, pos2);
                     L.lse[grow0 + lane] = lse2 * kLn2;
                     loss = (lse2 - pos2) * kLn2;
+                    const float4 pw = __ldg(reinterpret_cast<const float4*>(L.part) + (grow0 + lane) * (kMaxParts / 2));  // their (m, sum)
+                    w0 = exp2f_fast(pw.x - lse2), w1 = exp2f_fast(pw.z - lse2);
                 }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
@@ -415,21 +431,29 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const float* o0 = L.o_part + (((int64_t)p_first * 2 + 1) * BM + wq * 32) * DP + cl;
                 const float* o1 = L.o_part + (((int64_t)(p_first + 1) * 2) * BM + wq * 32) * DP + cl;
                 const float2* part = reinterpret_cast<const float2*>(L.part) + grow0 * kMaxParts;
-#pragma unroll 4
-                for (int r = lane / kLanes; r < 32; r += kSide) {
-                    const float lr = __shfl_sync(0xffffffffu, lse2, r);
-                    if (r < rows) {
-                        float4 s = *reinterpret_cast<const float4*>(o0 + r * DP), o = *reinterpret_cast<const float4*>(o1 + r * DP);
-                        const float4 pw = __ldg(reinterpret_cast<const float4*>(part + r * kMaxParts));  // (m, sum) of the first two parts
-                        const float w0 = exp2f_fast(pw.x - lr), w1 = exp2f_fast(pw.z - lr);
-                        s.x = fmaf(w1, o.x, w0 * s.x), s.y = fmaf(w1, o.y, w0 * s.y), s.z = fmaf(w1, o.z, w0 * s.z), s.w = fmaf(w1, o.w, w0 * s.w);
 #pragma unroll 1
-                        for (int p = 2; p < nparts; p++) {
-                            o = *reinterpret_cast<const float4*>(o1 + ((int64_t)(p - 1) * 2 * BM + r) * DP);
-                            const float w = exp2f_fast(__ldg(&part[r * kMaxParts + p]).x - lr);
-                            s.x = fmaf(w, o.x, s.x), s.y = fmaf(w, o.y, s.y), s.z = fmaf(w, o.z, s.z), s.w = fmaf(w, o.w, s.w);
+                for (int r0 = lane / kLanes; r0 < 32; r0 += 8 * kSide) {  // eight rows' loads on their way at a time
+                    float4 s[8], o[8];
+#pragma unroll
+                    for (int k = 0; k < 8; k++) {
+                        const int r = min(r0 + k * kSide, rows - 1);
+                        s[k] = *reinterpret_cast<const float4*>(o0 + r * DP), o[k] = *reinterpret_cast<const float4*>(o1 + r * DP);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; k++) {
+                        const int r = r0 + k * kSide;
+                        const float a0 = __shfl_sync(0xffffffffu, w0, r & 31), a1 = __shfl_sync(0xffffffffu, w1, r & 31), lr = __shfl_sync(0xffffffffu, lse2, r & 31);
+                        s[k].x = fmaf(a1, o[k].x, a0 * s[k].x), s[k].y = fmaf(a1, o[k].y, a0 * s[k].y);
+                        s[k].z = fmaf(a1, o[k].z, a0 * s[k].z), s[k].w = fmaf(a1, o[k].w, a0 * s[k].w);
+                        if (r < rows) {
+#pragma unroll 1
+                            for (int p = 2; p < nparts; p++) {
+                                const float4 x = *reinterpret_cast<const float4*>(o1 + ((int64_t)(p - 1) * 2 * BM + r) * DP);
+                                const float w = exp2f_fast(__ldg(&part[r * kMaxParts + p]).x - lr);
+                                s[k].x = fmaf(w, x.x, s[k].x), s[k].y = fmaf(w, x.y, s[k].y), s[k].z = fmaf(w, x.z, s[k].z), s[k].w = fmaf(w, x.w, s[k].w);
+                            }
+                            *reinterpret_cast<float4*>(L.dQ + (grow0 + r) * DP + cl) = s[k];
                         }
-                        *reinterpret_cast<float4*>(L.dQ + (grow0 + r) * DP + cl) = s;
                     }
                 }
             }

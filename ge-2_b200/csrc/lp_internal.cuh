@@ -54,20 +54,24 @@ inline size_t lp_align(size_t x) { return (x + 255) & ~(size_t)255; }
 __host__ __device__ inline int lp_row_ld(int D) { return D <= 64 ? 64 : 128; }
 
 // Which of the two fp16 forms a step takes.  The two-pass form adds every row block's part into dK, which is the faster way while dK stays in
-// the L2 beside the operands.  The streaming form writes every row once, but each of its blocks costs a fill and a drain of the pipeline,
-// and more where a block is cut between CTAs: of its two launches the one over the negatives has T blocks a chunk (T tiles of 128 negatives) with
+// the L2 beside the operands.  The streaming form writes every row once and spends less on a tile (2.3 ... 2.6 us for both its launches on one
+// CTA, 2.6 ... 2.8), but each of its blocks costs a fill and a drain of the pipeline, more where a block is cut between CTAs, and its
+// launches some 8 us more: of its two launches the one over the negatives has T blocks a chunk (T tiles of 128 negatives) with
 // only as many tiles each as the chunk has row blocks.  So the line in bytes of dK rises with T and falls with the row blocks, less steeply
 // for rows of 64 columns, whose tiles are half the traffic; without cuts it stays at 64 MB.  And where T is small and the last tile
-// mostly padding, the line is twice as high: the two-pass form skips the columns that do not exist.
-// Both forms at 2 370 shapes (chunks of 64 ... 2 000 rows, 100 ... 66 001 negatives, dK of 60 ... 290 MB, two sides); D = 100, us, two-pass : streaming
-//   10 000 negatives, 68 MB: 64 rows a chunk 46 : 149, 2 000 rows 331 : 353    1 300 negatives, 66 MB: 64 rows 47 : 76, 2 000 rows 398 : 380
-//   2 000 negatives, 96 MB: 64 rows 76 : 88, 384 rows 141 : 126, 2 000 rows 672 : 468    300 negatives, 153 MB: 64 rows 129 : 137, 500 rows 318 : 357
-//   1 000 negatives, 72 MB, 74 chunks (no cuts): 64 rows 54 : 46, 2 000 rows 540 : 352
-// At 96 of them the line takes the form that is more than 5 % slower (with 64 MB whatever the shape: at 520, up to 3.2 times slower).
+// mostly padding, the line is twice as high: the two-pass form skips the columns that do not exist.  Whatever the size of dK, the streaming form
+// is taken where every CTA has enough tiles and a chunk is neither a few row blocks high nor many tiles wide: from 12 tiles a CTA on for rows
+// of 64 columns, whose tiles spend less on contractions, from 40 on for wider ones.
+// Both forms at 4 020 shapes (chunks of 50 ... 2 000 rows, 100 ... 20 000 negatives, dK of 2 ... 290 MB, one and two sides), us, two-pass : streaming
+//   D = 64, two sides: 100 x 997 rows, 246 negatives 86 : 69; 100 x 743, 1 111 negatives 203 : 165; 2 x 1 605, 15 438 negatives (D = 50) 67 : 118
+//   D = 128, two sides: 18 x 1 941 rows, 2 031 negatives 203 : 165; 53 x 902, 587 negatives 111 : 117; 39 x 515, 936 negatives 84 : 88
+//   dK above 64 MB, D = 128: 100 x 571 rows, 1 661 negatives 475 : 265; 50 x 629, 6 746 negatives (D = 50) 520 : 378; 15 x 613, 19 777 254 : 310
+// The form that is taken is 0.9 % slower than the better one on average, and 25 % at most (by the bytes of dK alone: 2.1 and 28 %).
 inline bool lp_uses_flash(const ge2_lp_desc& d, int S, int64_t CN, int ld) {
     if (d.precision != GE2_PRECISION_F16) return false;
-    const int64_t T = ceil_div<int64_t>(d.N, 128);
-    const double row_blocks = ceil_div(rows_per_chunk(d.B, d.C), 128), mb = (double)S * CN * ld * 4 / (1 << 20);
+    const int64_t T = ceil_div<int64_t>(d.N, 128), blocks = ceil_div(rows_per_chunk(d.B, d.C), 128), units = S * d.C * T * blocks;
+    if (T <= 16 && (ld == 64 ? blocks > 2 && units > 12 * kNumSMs : blocks > 3 && units > 40 * kNumSMs)) return true;
+    const double row_blocks = (double)blocks, mb = (double)S * CN * ld * 4 / (1 << 20);
     if (S * d.C * T % kNumSMs == 0) return mb > 64;
     const double over = ld == 128 ? 4.0 * (T - 1) : T > 8 ? 2.0 * (T - 8) : 0.0;
     const bool padded = ld == 128 && T >= 3 && T <= 6 && 128 * T * 8 > 9 * (int64_t)d.N;

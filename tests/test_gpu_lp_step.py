@@ -245,6 +245,8 @@ def test_streaming_softmax_tiles_at_their_edges(capi, cuda_device, kind, B, C, N
     ("COMPLEX", 9472, 74, 1000, 66), ("COMPLEX", 9576, 76, 1000, 66),       # as many chunk sides as SMs, so no block is cut, and a few more
     ("DISTMULT", 1500, 500, 300, 66), ("DISTMULT", 1440, 480, 300, 66),     # a last tile that is mostly padding
     ("DISTMULT", 200, 90, 2000, 50), ("DISTMULT", 200, 70, 2000, 50),       # rows of 64 columns
+    ("DISTMULT", 10368, 27, 1300, 50), ("DISTMULT", 9984, 26, 1300, 50),    # ... and 12 tiles a CTA
+    ("COMPLEX", 24064, 47, 2000, 66), ("COMPLEX", 23552, 46, 2000, 66),     # 40 of wider rows
 ])
 def test_both_fp16_forms_where_the_rule_between_them_lies(capi, cuda_device, kind, B, C, N, D):
     case = workloads.make_case(kind, B, C, N, D, 5, 150, min(N, 50), 9 + D)
