@@ -27,6 +27,7 @@ EXPORTS = [
     "ge2_eval_workspace_bytes", "ge2_eval_ranks", "ge2_selected_neg_scores", "ge2_selected_neg_scores_backward",
     "ge2_tournament_select", "ge2_unique_bitmap_shared", "ge2_adagrad_scatter_shared", "ge2_train_step",
     "ge2_selected_neg_backward_workspace_bytes", "ge2_selected_neg_scores_backward_ws",
+    "ge2_sample_unique", "ge2_lp_idle_sms",
 ]
 
 
@@ -75,6 +76,14 @@ class TrainDesc(C.Structure):
                 ("dense_state", C.c_void_p * 2), ("dense_grad", C.c_void_p * 2), ("dense_numel", C.c_int64)]
 
 
+class FrontDesc(C.Structure):
+    _fields_ = [("edges", C.c_void_p), ("cols", C.c_int32), ("sms", C.c_int32), ("num_batches", C.c_int64), ("num_batches_dev", C.c_void_p),
+                ("step_dev", C.c_void_p), ("seed", C.c_uint64), ("batch_index", C.c_uint64), ("B", C.c_int32), ("C", C.c_int32), ("N", C.c_int32),
+                ("n_deg", C.c_int32), ("domain", C.c_int64), ("mapped", C.c_int64), ("want_src_negs", C.c_int32), ("num_counters", C.c_int32),
+                ("packed", C.c_void_p), ("deg_rows", C.c_void_p), ("rel_ids", C.c_void_p), ("unique_ws", C.c_void_p), ("unique_ws_bytes", C.c_size_t),
+                ("unique", C.c_void_p), ("inverse", C.c_void_p), ("count", C.c_void_p), ("shared", C.c_void_p), ("counters", C.c_void_p)]
+
+
 class SwapDesc(C.Structure):
     _fields_ = [("world", C.c_int32), ("rank", C.c_int32), ("flag_rows", C.POINTER(C.c_void_p)), ("epoch", C.c_uint64),
                 ("wait_budget_us", C.c_uint32), ("num_pulls", C.c_int32), ("pull_src", C.POINTER(C.c_void_p)), ("pull_dst", C.POINTER(C.c_void_p)),
@@ -118,6 +127,8 @@ def load_library():
     lib.ge2_dense_adagrad.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_float, C.c_float, C.c_int32, C.c_void_p]
     lib.ge2_dense_adagrad_peers.argtypes = [C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p), C.c_int32, C.c_int32, C.c_int64, C.c_void_p, C.c_float,
                                             C.c_float, C.c_float, C.c_uint32, C.c_void_p, C.c_void_p]
+    lib.ge2_lp_idle_sms.argtypes = [C.POINTER(LpDesc), C.POINTER(C.c_int32)]
+    lib.ge2_sample_unique.argtypes = [C.POINTER(FrontDesc), C.c_void_p]
     lib.ge2_enable_peer_access.argtypes = [C.c_int32]
     lib.ge2_sample_negatives.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int64, C.c_int32,
                                          C.c_uint64, C.c_uint64, C.c_void_p, C.c_void_p, C.c_void_p]
@@ -256,6 +267,17 @@ def lp_workspace_bytes(desc: LpDesc) -> int:
 
 def lp_step(desc: LpDesc):
     check(load_library().ge2_lp_step(C.byref(desc), cur_stream()), "ge2_lp_step")
+
+
+def lp_idle_sms(desc: LpDesc) -> int:
+    """SMs that the scores kernels of a step with this descriptor leave to others"""
+    n = C.c_int32(0)
+    check(load_library().ge2_lp_idle_sms(C.byref(desc), C.byref(n)), "ge2_lp_idle_sms")
+    return n.value
+
+
+def sample_unique(desc: FrontDesc):
+    check(load_library().ge2_sample_unique(C.byref(desc), cur_stream()), "ge2_sample_unique")
 
 
 def train_step(desc: TrainDesc):

@@ -5,7 +5,7 @@ namespace ge2 {
 thread_local int g_last_cuda_error = 0;
 }
 
-extern "C" const char* ge2_version(void) { return "ge2_b200 0.2 (sm_100a)"; }
+extern "C" const char* ge2_version(void) { return "ge2_b200 0.3 (sm_100a)"; }
 
 extern "C" int ge2_last_cuda_error(void) { return ge2::g_last_cuda_error; }
 

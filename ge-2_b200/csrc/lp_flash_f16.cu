@@ -823,8 +823,8 @@ int launch(const LpKernelArgs& a, cudaStream_t stream) {
     fs.masks = a.d.deg_sample_rows != nullptr || a.d.dst_filter_n > 0 || a.d.src_filter_n > 0;
     fs.q.unitsA = fs.n.unitsA = fs.q.unitsB = fs.n.unitsB = (int)units;
     // every CTA's range is at least ceil(T / 7) units long, so a row block is shared by at most kMaxParts CTAs
-    fs.q.gridA = fs.q.gridB = std::max(1, std::min(kNumSMs, (int)units / ceil_div(nb, kMaxParts - 1)));
-    fs.n.gridA = fs.n.gridB = std::max(1, std::min(kNumSMs, (int)units));
+    fs.q.gridA = fs.q.gridB = std::max(1, std::min(scores_ctas(units), (int)units / ceil_div(nb, kMaxParts - 1)));
+    fs.n.gridA = fs.n.gridB = scores_ctas(units);
     GE2_CUDA_TRY(cudaFuncSetAttribute(lp_flash_kernel<DP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<DP>::kDynamic));
     GE2_CUDA_TRY(cudaFuncSetAttribute(lp_flash_kernel<DP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<DP>::kDynamic));
     GE2_CUDA_TRY(launch_after(lp_flash_kernel<DP, false>, dim3((unsigned)fs.q.gridA), dim3(kThreads), Layout<DP>::kDynamic, stream, tmQ, tmK, tmO[0], tmOt[0], a, fs));

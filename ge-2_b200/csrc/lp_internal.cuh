@@ -125,6 +125,20 @@ inline LpLayout lp_make_layout(const ge2_lp_desc& d, void* base) {
     return L;
 }
 
+// CTAs of a persistent scores launch over `units` tiles, one a CTA at a time and one CTA an SM: no more than it takes for the longest share to be
+// as short as it is with one on every SM, but at most eight SMs are left to others (what runs on them meanwhile: the next batch's sampler and
+// unique-map in a pipelined step).
+inline int scores_ctas(long long units) {
+    if (units <= kNumSMs) return (int)(units < 1 ? 1 : units);
+    const long long share = ceil_div<long long>(units, kNumSMs), ctas = ceil_div(units, share);
+    return (int)(ctas < kNumSMs - 8 ? kNumSMs - 8 : ctas);
+}
+constexpr int kLp32Rows = 128, kLp32Cols = 64;  // a tile of the fp32 path
+inline long long scores_units(const ge2_lp_desc& d, int S) {
+    const int cols = d.precision == GE2_PRECISION_F16 ? 128 : kLp32Cols;
+    return (long long)S * d.C * ceil_div(rows_per_chunk(d.B, d.C), 128) * ceil_div(d.N, cols);
+}
+
 // scores kernels (one per precision); both fill lse, dQ, dK (+ optional score dumps) from Q, K, pos, mask
 int lp_scores_fp32(const LpKernelArgs& a, cudaStream_t stream);
 int lp_scores_f16(const LpKernelArgs& a, cudaStream_t stream);

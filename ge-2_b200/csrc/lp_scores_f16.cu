@@ -884,10 +884,10 @@ int launch(const LpKernelArgs& a, cudaStream_t stream) {
     if (2 * unitsA > 0x3fffffff) return GE2_ERR_UNSUPPORTED;
     sc.unitsA = (int)unitsA;
     sc.unitsB = sc.unitsA;
-    const int sms = std::max(1, std::min(kNumSMs, env_int("GE2_F16_CTAS", kNumSMs)));  // development switch: fewer CTAs than SMs
+    const int ctas = scores_ctas(unitsA), sms = std::max(1, std::min(ctas, env_int("GE2_F16_CTAS", ctas)));  // development switch: fewer CTAs
     // every CTA's range is at least ceil(T / 7) units long, so a row block is shared by at most kMaxParts CTAs
     sc.gridA = std::max(1, std::min(sms, sc.unitsA / ceil_div(sc.T, kMaxParts - 1)));
-    sc.gridB = std::max(1, std::min(sms, sc.unitsB));
+    sc.gridB = sms;
     GE2_CUDA_TRY(cudaFuncSetAttribute(lp_lse_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<DP>::kDynamicA));
     GE2_CUDA_TRY(cudaFuncSetAttribute(lp_grad_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<DP>::kDynamicB));
     const int only = env_int("GE2_F16_ONLY", 0);  // development switch: 1 = logsumexp pass alone, 2 = gradient pass alone (on a workspace a full step left behind)

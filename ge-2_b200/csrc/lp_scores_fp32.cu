@@ -613,8 +613,8 @@ int launch(const LpKernelArgs& a, cudaStream_t stream) {
     if (units > 0x3fffffff) return GE2_ERR_UNSUPPORTED;
     sc.unitsA = sc.unitsB = (int)units;
     // every CTA's range is at least ceil(T / 7) units long, so a row block is shared by at most kMaxParts CTAs
-    sc.gridA = std::max(1, std::min(kNumSMs, sc.unitsA / ceil_div(sc.T, kMaxParts - 1)));
-    sc.gridB = std::max(1, std::min(kNumSMs, sc.unitsB));
+    sc.gridA = std::max(1, std::min(scores_ctas(units), sc.unitsA / ceil_div(sc.T, kMaxParts - 1)));
+    sc.gridB = scores_ctas(units);
     // per-device function attributes; setting them on every launch keeps multi-device processes correct and is not a stream operation
     GE2_CUDA_TRY(cudaFuncSetAttribute(lp_lse32_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::kBytesA));
     GE2_CUDA_TRY(cudaFuncSetAttribute(lp_grad32_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::kBytesB));

@@ -673,6 +673,14 @@ extern "C" int ge2_lp_workspace_bytes(const ge2_lp_desc* desc, size_t* bytes) {
     return GE2_OK;
 }
 
+extern "C" int ge2_lp_idle_sms(const ge2_lp_desc* desc, int32_t* sms) {
+    if (sms == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+    const int rc = validate(desc);
+    if (rc != GE2_OK) return rc;
+    *sms = kNumSMs - scores_ctas(scores_units(*desc, desc->has_relations && desc->use_inverse ? 2 : 1));
+    return GE2_OK;
+}
+
 extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     int rc = validate(desc);
     if (rc != GE2_OK) return rc;

@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "adagrad.cuh"
+#include "unique_map.cuh"
 
 namespace ge2 {
 namespace {
@@ -349,12 +350,27 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 // (out of line: a 64-bit division is 1 KB of code, and kernels this short are bound by fetching theirs)
 __device__ __noinline__ uint64_t div_u64(uint64_t a, uint64_t b) { return a / b; }
 
+// What the sampler marks in the unique-map's bitsets on the way (words == null: nothing).  A marking kernel of its own reads every id again, one
+// launch later: steps issued launch by launch, 1 000 edges, 69.2 us with it, 65.4 without.
+struct SampleMarks {
+    unsigned long long *words, *dup;
+    int64_t domain;  // ids below it get a local id
+    int32_t* status;
+};
+
 __global__ void __launch_bounds__(256) sample_negatives_kernel(const int64_t* __restrict__ src_ids, const int64_t* __restrict__ dst_ids,
                                                                int64_t edge_stride, int B, int C, int N, int n_deg, int64_t domain,
                                                                int want_src, uint64_t key, int64_t* __restrict__ packed,
                                                                int64_t* __restrict__ deg_rows, const uint64_t* __restrict__ step_dev,
                                                                int64_t num_batches, const int64_t* __restrict__ rel_ids,
-                                                               int64_t* __restrict__ out_rel, const int64_t* __restrict__ num_batches_dev) {
+                                                               int64_t* __restrict__ out_rel, const int64_t* __restrict__ num_batches_dev,
+                                                               SampleMarks mk) {
+    bool bad = false;
+    auto mark = [&](int64_t id) {
+        if (mk.words == nullptr) return;
+        if ((uint64_t)id < (uint64_t)mk.domain) mark_id(mk.words, mk.dup, id);
+        else bad = true;
+    };
     // graph-replay form: the batch index lives on the device, so the same launch serves every batch of the epoch
     if (step_dev != nullptr) {
         const uint64_t step = *step_dev;
@@ -376,10 +392,14 @@ __global__ void __launch_bounds__(256) sample_negatives_kernel(const int64_t* __
 #pragma unroll 1
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         if (i < B) {
-            packed[i] = src_ids[i * edge_stride];
+            const int64_t id = src_ids[i * edge_stride];
+            packed[i] = id;
+            mark(id);
             if (out_rel != nullptr) out_rel[i] = rel_ids[i * edge_stride];
         } else if (i < 2 * (int64_t)B) {
-            packed[i] = dst_ids[(i - B) * edge_stride];
+            const int64_t id = dst_ids[(i - B) * edge_stride];
+            packed[i] = id;
+            mark(id);
         } else {
             const int64_t e = i - 2 * (int64_t)B;
             const int c = e >> 32 ? (int)div_u64((uint64_t)e, (uint64_t)N) : (int)((uint32_t)e / (uint32_t)N);
@@ -388,15 +408,20 @@ __global__ void __launch_bounds__(256) sample_negatives_kernel(const int64_t* __
             if (j < n_deg) {
                 const int64_t row = (int64_t)__umul64hi(r, (uint64_t)B);
                 if (deg_rows != nullptr) deg_rows[(int64_t)c * n_deg + j] = row;
-                out_dst_neg[e] = dst_ids[row * edge_stride];
-                if (want_src) out_src_neg[e] = src_ids[row * edge_stride];
+                const int64_t id = dst_ids[row * edge_stride], other = want_src ? src_ids[row * edge_stride] : id;
+                out_dst_neg[e] = id;
+                if (want_src) out_src_neg[e] = other;
+                mark(id);
+                if (other != id) mark(other);  // (equal ones, a negative of both sides, count as one occurrence)
             } else {
                 const int64_t id = (int64_t)__umul64hi(r, (uint64_t)domain);
                 out_dst_neg[e] = id;
                 if (want_src) out_src_neg[e] = id;
+                mark(id);
             }
         }
     }
+    if (bad) atomicOr(mk.status, GE2_STATUS_ID_OUT_OF_RANGE);
 }
 
 inline int vec_width(int D, const void* a, const void* b = nullptr, const void* c = nullptr, const void* d = nullptr) {
@@ -538,7 +563,7 @@ extern "C" int ge2_sample_negatives(const int64_t* src_ids, const int64_t* dst_i
     const uint64_t key = seed * 0xD1342543DE82EF95ull + batch_index * 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull;
     sample_negatives_kernel<<<stream_grid(total, 256), 256, 0, as_stream(stream_)>>>(src_ids, dst_ids, edge_stride, B, C, N, n_deg, domain,
                                                                                    want_src_negs, key, out_packed_ids, out_deg_rows, nullptr, 1,
-                                                                                   nullptr, nullptr, nullptr);
+                                                                                   nullptr, nullptr, nullptr, SampleMarks{});
     GE2_LAUNCH_CHECK();
     return GE2_OK;
 }
@@ -554,7 +579,7 @@ static int sample_batch_impl(const int64_t* edges, int32_t cols, int64_t num_bat
     const uint64_t key = seed * 0xD1342543DE82EF95ull + 0x632BE59BD9B4E019ull;
     sample_negatives_kernel<<<stream_grid(total, 256), 256, 0, as_stream(stream_)>>>(
         edges, edges + cols - 1, cols, B, C, N, n_deg, domain, want_src_negs, key, out_packed_ids, out_deg_rows, step_dev, num_batches,
-        cols == 3 ? edges + 1 : nullptr, cols == 3 ? out_rel_ids : nullptr, num_batches_dev);
+        cols == 3 ? edges + 1 : nullptr, cols == 3 ? out_rel_ids : nullptr, num_batches_dev, SampleMarks{});
     GE2_LAUNCH_CHECK();
     return GE2_OK;
 }
@@ -583,6 +608,42 @@ extern "C" int ge2_advance_step(uint64_t* step_dev, int32_t n, ge2_stream_t stre
     advance_step_kernel<<<1, 32, 0, as_stream(stream_)>>>(step_dev, n);
     GE2_LAUNCH_CHECK();
     return GE2_OK;
+}
+
+static int front_check(const ge2_front_desc* f) {
+    if (f == nullptr || f->B <= 0 || f->C <= 0 || f->N <= 0 || f->n_deg < 0 || f->n_deg > f->N || f->domain <= 0 || f->mapped <= 0 ||
+        (f->cols != 2 && f->cols != 3))
+        return GE2_ERR_INVALID_ARGUMENT;
+    if (f->step_dev != nullptr && f->num_batches <= 0 && f->num_batches_dev == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+    if (f->edges == nullptr || f->packed == nullptr || f->unique == nullptr || f->inverse == nullptr || f->count == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+    if (f->n_deg > 0 && f->deg_rows == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+    if (f->sms < 0 || f->sms > kNumSMs) return GE2_ERR_INVALID_ARGUMENT;
+    if (f->num_counters < 0 || f->num_counters > 32 || (f->num_counters > 0 && f->counters == nullptr)) return GE2_ERR_INVALID_ARGUMENT;
+    const int64_t n = 2 * (int64_t)f->B + (f->want_src_negs ? 2 : 1) * (int64_t)f->C * f->N;
+    if (n > kUniqueMaxIds || num_words_of(f->mapped) > kUniqueMaxIds) return GE2_ERR_UNSUPPORTED;
+    if (f->unique_ws == nullptr || ((uintptr_t)f->unique_ws & 255) != 0 || f->unique_ws_bytes < unique_ws_bytes(f->mapped, f->shared != nullptr ? 2 : 1))
+        return GE2_ERR_WORKSPACE;
+    return GE2_OK;
+}
+
+extern "C" int ge2_sample_unique(const ge2_front_desc* f, ge2_stream_t stream_) {
+    const int rc = front_check(f);
+    if (rc != GE2_OK) return rc;
+    cudaStream_t stream = as_stream(stream_);
+    const int sms = f->sms == 0 ? kNumSMs : f->sms;
+    const UniqueWorkspace ws = unique_carve(f->unique_ws, f->mapped, f->shared != nullptr);
+    const int64_t CN = (int64_t)f->C * f->N, total = 2 * (int64_t)f->B + CN;
+    GE2_CUDA_TRY(cudaMemsetAsync(ws.tile_state, 0, ws.clear_bytes, stream));
+    uint64_t key = f->seed * 0xD1342543DE82EF95ull + 0x632BE59BD9B4E019ull;
+    if (f->step_dev == nullptr) key += f->batch_index * 0x9E3779B97F4A7C15ull;
+    const bool rel = f->cols == 3 && f->rel_ids != nullptr;
+    sample_negatives_kernel<<<std::min(stream_grid(total, 256), sms * 6), 256, 0, stream>>>(
+        f->edges, f->edges + f->cols - 1, f->cols, f->B, f->C, f->N, f->n_deg, f->domain, f->want_src_negs, key, f->packed, f->deg_rows, f->step_dev,
+        f->num_batches, rel ? f->edges + 1 : nullptr, rel ? f->rel_ids : nullptr, f->num_batches_dev,
+        SampleMarks{ws.words, ws.dup, f->mapped, ws.status});
+    GE2_LAUNCH_CHECK();
+    return unique_emit(ws, f->packed, total + (f->want_src_negs ? CN : 0), f->mapped, f->unique, f->inverse, f->count, f->shared, f->counters,
+                           f->num_counters, sms, stream);
 }
 
 extern "C" int ge2_remap_edges_to_slots(const int64_t* edges, int64_t n, int32_t cols, const int64_t* partition_to_slot,
@@ -644,11 +705,23 @@ extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
     const int64_t mapped = std::min(t->domain, t->table_rows);  // ids past the table get no local id: they are flagged, and no later kernel meets them
     if (t->unique_ws == nullptr || ((uintptr_t)t->unique_ws & 255) != 0 || t->unique_ws_bytes < ge2_unique_workspace_bytes(mapped)) return GE2_ERR_WORKSPACE;
 
-    rc = ge2_sample_negatives(t->edges, t->edges + t->cols - 1, t->cols, d.B, d.C, d.N, t->n_deg, t->domain, d.use_inverse, t->seed, t->batch_index,
-                              t->packed, t->deg_rows, stream);
-    if (rc != GE2_OK) return rc;
-    rc = ge2_unique_bitmap_shared(t->packed, t->n_ids, mapped, t->unique_ws, t->unique_ws_bytes, t->unique, t->inverse, t->count, t->shared,
-                                  t->twin_begin, t->twin_len, stream);
+    ge2_front_desc f = {};
+    f.edges = t->edges, f.cols = t->cols, f.seed = t->seed, f.batch_index = t->batch_index;
+    f.B = d.B, f.C = d.C, f.N = d.N, f.n_deg = t->n_deg, f.domain = t->domain, f.want_src_negs = d.use_inverse;
+    f.packed = t->packed, f.deg_rows = t->deg_rows, f.mapped = mapped;
+    f.unique_ws = t->unique_ws, f.unique_ws_bytes = t->unique_ws_bytes;
+    f.unique = t->unique, f.inverse = t->inverse, f.count = t->count, f.shared = t->shared;
+    // the sampler's own marking counts a negative that both sides share once
+    const bool twins = t->shared == nullptr || (d.use_inverse ? t->twin_begin == 2 * (int64_t)d.B && t->twin_len == (int64_t)d.C * d.N : t->twin_len == 0);
+    if (twins && (t->cols == 2 || t->cols == 3)) {
+        rc = ge2_sample_unique(&f, stream);
+    } else {
+        rc = ge2_sample_negatives(t->edges, t->edges + t->cols - 1, t->cols, d.B, d.C, d.N, t->n_deg, t->domain, d.use_inverse, t->seed, t->batch_index,
+                                  t->packed, t->deg_rows, stream);
+        if (rc == GE2_OK)
+            rc = ge2_unique_bitmap_shared(t->packed, t->n_ids, mapped, t->unique_ws, t->unique_ws_bytes, t->unique, t->inverse, t->count, t->shared,
+                                          t->twin_begin, t->twin_len, stream);
+    }
     if (rc != GE2_OK) return rc;
     rc = ge2_lp_step(&d, stream);
     if (rc != GE2_OK) return rc;

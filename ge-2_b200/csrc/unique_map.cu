@@ -16,27 +16,17 @@
 //
 // It can also say which ids occur more than once (out_shared): a second bitset collects the bits that were set already when they were
 // marked.  The rows of the other ids have one contribution to their gradient, so the training step can finish them on the spot.
-#include "common.cuh"
+#include <algorithm>
+
+#include "unique_map.cuh"
 
 namespace ge2 {
 namespace {
 
-constexpr int kScanThreads = 128;
-constexpr int kWordsPerThread = 1;
-constexpr int kTileWords = kScanThreads * kWordsPerThread;  // 128 words = 8192 ids per tile: a small domain still spreads over CTAs
 constexpr uint32_t kFlagAggregate = 1u << 30;               // tile state: local sum published
 constexpr uint32_t kFlagPrefix = 2u << 30;                  // tile state: inclusive prefix published
-constexpr uint32_t kValueMask = (1u << 30) - 1;
+constexpr uint32_t kValueMask = (uint32_t)kUniqueMaxIds;
 constexpr int kSpinLimit = 1 << 20;                          // look-back poll budget before giving up
-
-struct UniqueWorkspace {
-    uint32_t* tile_state;       // [num_tiles]   } control words: cleared together with the bitset by one memset
-    uint32_t* ticket;           // [1]           }
-    int32_t* status;            // [1]           } GE2_STATUS_* bits of this call
-    unsigned long long* words;  // [num_words]  one bit per id that occurs   } cleared by the same memset
-    unsigned long long* dup;    // [num_words]  ... that occurs again        } (null without out_shared)
-    int32_t* word_offsets;      // [num_words]
-};
 
 // ids[begin + k] and ids[begin + len + k] count as one occurrence when they are equal (len == 0: no such pairs)
 struct Twins {
@@ -46,16 +36,6 @@ __device__ __forceinline__ bool is_second_twin(const int64_t* ids, int64_t i, in
     const int64_t k = i - tw.begin - tw.len;
     return k >= 0 && k < tw.len && ids[i - tw.len] == key;
 }
-
-constexpr size_t align256c(size_t x) { return (x + 255) & ~(size_t)255; }
-// control words (tile states, ticket, status, one spare), one bitset or (for out_shared) two, per-word offsets
-constexpr size_t unique_ws_bytes(int64_t domain, int bitsets) {
-    const int64_t nw = (domain + 63) >> 6;
-    const int64_t tiles = (nw + kTileWords - 1) / kTileWords;
-    return align256c((size_t)(tiles + 4) * 4) + bitsets * align256c((size_t)nw * 8) + align256c((size_t)nw * 4);
-}
-
-__host__ __device__ inline int64_t num_words_of(int64_t domain) { return (domain + 63) >> 6; }
 
 __global__ void __launch_bounds__(256) mark_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t domain,
                                                    unsigned long long* __restrict__ words, unsigned long long* __restrict__ dup, Twins tw,
@@ -69,12 +49,7 @@ __global__ void __launch_bounds__(256) mark_kernel(const int64_t* __restrict__ i
             bad = true;
             continue;
         }
-        const unsigned long long bit = 1ull << (key & 63);
-        if (dup == nullptr) {
-            atomicOr(&words[key >> 6], bit);
-        } else if (!is_second_twin(ids, i, key, tw)) {
-            if ((atomicOr(&words[key >> 6], bit) & bit) != 0ull) atomicOr(&dup[key >> 6], bit);
-        }
+        if (dup == nullptr || !is_second_twin(ids, i, key, tw)) mark_id(words, dup, key);
     }
     if (bad) atomicOr(status, GE2_STATUS_ID_OUT_OF_RANGE);
 }
@@ -211,9 +186,11 @@ __global__ void __launch_bounds__(kScanThreads) scan_extract_kernel(const unsign
 __global__ void __launch_bounds__(256) inverse_kernel(const int64_t* __restrict__ ids, int64_t n, int64_t domain,
                                                       const unsigned long long* __restrict__ words,
                                                       const int32_t* __restrict__ word_offsets, int64_t* __restrict__ inverse,
-                                                      const int32_t* __restrict__ status, int32_t* __restrict__ out_status) {
+                                                      const int32_t* __restrict__ status, int32_t* __restrict__ out_status, uint64_t* counters,
+                                                      int num_counters) {
     griddep_wait();  // offsets and the count come from the scan kernel
     if (blockIdx.x == 0 && threadIdx.x == 0) *out_status = *status;  // the marking and scan kernels are over: the word is final
+    if (blockIdx.x == 0 && (int)threadIdx.x < num_counters) counters[threadIdx.x] += 1;
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
 #pragma unroll 1
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -247,6 +224,20 @@ __global__ void pack_ids_kernel(const int64_t* p0, const int64_t* p1, const int6
 }  // namespace
 }  // namespace ge2
 
+namespace ge2 {
+int unique_emit(const UniqueWorkspace& ws, const int64_t* ids, int64_t n, int64_t domain, int64_t* out_unique, int64_t* out_inverse, int32_t* out_count,
+                uint8_t* out_shared, uint64_t* counters, int num_counters, int sms, cudaStream_t stream) {
+    const int64_t nw = num_words_of(domain), tiles = ceil_div<int64_t>(nw, kTileWords), cap = n < domain ? n : domain;
+    const int64_t scan_grid = std::min<int64_t>(tiles, (int64_t)sms * (sms < kNumSMs ? 16 : 8));
+    GE2_CUDA_TRY(launch_after(scan_extract_kernel, dim3((unsigned)scan_grid), dim3(kScanThreads), 0, stream, (const unsigned long long*)ws.words, nw,
+                              ws.word_offsets, ws.tile_state, ws.ticket, (int)tiles, out_unique, cap, out_count, (const unsigned long long*)ws.dup, out_shared, ws.status));
+    GE2_CUDA_TRY(launch_after(inverse_kernel, dim3((unsigned)std::min(stream_grid(n, 256), sms * 8)), dim3(256), 0, stream, ids, n, domain,
+                              (const unsigned long long*)ws.words, (const int32_t*)ws.word_offsets, out_inverse, (const int32_t*)ws.status,
+                              out_count + 1, counters, num_counters));
+    return GE2_OK;
+}
+}  // namespace ge2
+
 using namespace ge2;
 
 extern "C" size_t ge2_unique_workspace_bytes(int64_t domain) {
@@ -273,42 +264,17 @@ extern "C" int ge2_unique_bitmap_shared(const int64_t* ids, int64_t n, int64_t d
     }
     const int64_t nw = num_words_of(domain);
     if (nw > (int64_t)kValueMask) return GE2_ERR_UNSUPPORTED;
-    const int64_t tiles = ceil_div<int64_t>(nw, kTileWords);
     if (workspace == nullptr || ((uintptr_t)workspace & 255) != 0 || workspace_bytes < unique_ws_bytes(domain, out_shared != nullptr ? 2 : 1))
         return GE2_ERR_WORKSPACE;
 
-    const int64_t cap = n < domain ? n : domain;
     const Twins tw = {twin_begin, twin_len};
-
-    char* p = (char*)workspace;
-    UniqueWorkspace ws;
-    ws.tile_state = (uint32_t*)p;
-    ws.ticket = ws.tile_state + tiles;
-    ws.status = (int32_t*)(ws.tile_state + tiles + 1);
-    const size_t ctl_bytes = align256c((size_t)(tiles + 4) * 4);
-    p += ctl_bytes;
-    ws.words = (unsigned long long*)p;
-    p += align256c((size_t)nw * 8);
-    ws.dup = nullptr;
-    if (out_shared != nullptr) {
-        ws.dup = (unsigned long long*)p;
-        p += align256c((size_t)nw * 8);
-    }
-    ws.word_offsets = (int32_t*)p;
-
+    const UniqueWorkspace ws = unique_carve(workspace, domain, out_shared != nullptr);
     // control words and bitsets are adjacent: one memset; out_count needs none (the scan's last tile writes the count, the
     // inverse kernel the status)
-    GE2_CUDA_TRY(cudaMemsetAsync(ws.tile_state, 0, ctl_bytes + (out_shared != nullptr ? align256c((size_t)nw * 8) : 0) + (size_t)nw * 8, stream));
-
+    GE2_CUDA_TRY(cudaMemsetAsync(ws.tile_state, 0, ws.clear_bytes, stream));
     mark_kernel<<<stream_grid(n, 256), 256, 0, stream>>>(ids, n, domain, ws.words, ws.dup, tw, ws.status);
     GE2_LAUNCH_CHECK();
-    const int scan_grid = (int)(tiles < (int64_t)kNumSMs * 8 ? tiles : (int64_t)kNumSMs * 8);
-    GE2_CUDA_TRY(launch_after(scan_extract_kernel, dim3((unsigned)scan_grid), dim3(kScanThreads), 0, stream, (const unsigned long long*)ws.words, nw,
-                              ws.word_offsets, ws.tile_state, ws.ticket, (int)tiles, out_unique, cap, out_count, (const unsigned long long*)ws.dup, out_shared, ws.status));
-    GE2_CUDA_TRY(launch_after(inverse_kernel, dim3((unsigned)stream_grid(n, 256)), dim3(256), 0, stream, ids, n, domain,
-                              (const unsigned long long*)ws.words, (const int32_t*)ws.word_offsets, out_inverse, (const int32_t*)ws.status,
-                              out_count + 1));
-    return GE2_OK;
+    return unique_emit(ws, ids, n, domain, out_unique, out_inverse, out_count, out_shared, nullptr, 0, kNumSMs, stream);
 }
 
 extern "C" int ge2_pack_ids(const int64_t* const parts[4], const int64_t lens[4], const int64_t strides[4], int64_t* out,

@@ -119,6 +119,10 @@ class PeerGradients:
 class BatchPipeline:
     """Owns the per-batch scratch (ids, unique map, gradients, workspaces); tables are owned by the caller."""
 
+    # Ids of a batch for every SM that the scores kernels leave over, up to which the next batch's sampler and unique-map run there: a thousand
+    # ids an SM take them about 5 us, and they have the time of the scores (8 000: 38 of 42 us)
+    IDS_PER_IDLE_SM = 16384
+
     def __init__(self, cfg: PipelineConfig, table, state, rel=None, rel_state=None, inv_rel=None, inv_rel_state=None):
         capi.load_library()
         self.cfg = cfg
@@ -174,15 +178,6 @@ class BatchPipeline:
         if self.nb_dev is None:
             self.nb_dev = torch.zeros(1, dtype=torch.int64, device=self.device)
         self.nb_dev.fill_(max(1, int(num_batches)))
-
-    def _sample(self, ids: "_IdSet", edges_all, num_batches: int, counter):
-        cfg = self.cfg
-        args = (cfg.B, cfg.C, cfg.N, cfg.n_deg, cfg.domain, cfg.sides == 2, cfg.seed, ids.packed, ids.deg_rows if cfg.n_deg > 0 else None,
-                ids.rel_ids if cfg.has_relations else None)
-        if self.nb_dev is not None:
-            capi.sample_batch_dev(edges_all, self.nb_dev, counter, *args)
-        else:
-            capi.sample_batch(edges_all, num_batches, counter, *args)
 
     def _unique(self, ids: "_IdSet"):
         capi.unique_bitmap(ids.packed, self._mapped_domain(), workspace=ids.uws, out_unique=ids.unique, out_inverse=ids.inverse, out_count=ids.count,
@@ -368,10 +363,10 @@ class BatchPipeline:
         advances the device-side counter at the end.  No argument changes from step to step, so the launch list can be
         captured once into a CUDA graph (capture_resident) and replayed."""
         cfg = self.cfg
-        self._sample(self.ids[0], edges_all, num_batches, self.step_dev)
-        self._unique(self.ids[0])
+        self._front(self.ids[0], edges_all, num_batches, self.step_dev, advance=True)
         self._backward_and_update(self._make_desc(edges_all, self.rel_ids, 1), scores_events, rel_hook)
-        capi.advance_step(self.step_dev, 2)
+        if self.peer is not None:
+            capi.advance_step(self.step_dev, 2)
         self._t_host += 1
         self._ids_parity = self._t_host & 1  # (a pipelined runner used after this needs refill(): nothing is drawn ahead)
 
@@ -397,13 +392,10 @@ class BatchPipeline:
         cfg = self.cfg
         ga, gb = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
         with torch.cuda.graph(ga):
-            capi.sample_batch(edges_all, num_batches, self.step_dev, cfg.B, cfg.C, cfg.N, cfg.n_deg, cfg.domain, cfg.sides == 2, cfg.seed,
-                              self.packed, self.deg_rows if cfg.n_deg > 0 else None, self.rel_ids if cfg.has_relations else None)
-            self._unique(self.ids[0])
+            self._front(self.ids[0], edges_all, num_batches, self.step_dev, advance=True)
             self._backward(self._make_desc(edges_all, self.rel_ids, 1))
         with torch.cuda.graph(gb):
             self._update()
-            capi.advance_step(self.step_dev, 2)
 
         class _Split:
             def replay(_self):
@@ -415,11 +407,22 @@ class BatchPipeline:
         return _Split()
 
     # ---- pipelined form: batch t+1 is sampled and deduplicated on a side stream while batch t trains -----------------
-    def _front(self, ids: _IdSet, edges_all, num_batches: int, counter):
-        """sampler + unique-map into one id set; `counter` is the device counter holding the batch number to use"""
+    def _front(self, ids: _IdSet, edges_all, num_batches: int, counter, advance: bool = False, sms: int = 0):
+        """sampler + unique-map into one id set; `counter` is the device counter holding the batch number to use.  advance: both
+        device counters go up by one at the end, unless the step's own exchange between ranks still reads them.  sms: SMs to keep to (0: all)."""
         cfg = self.cfg
-        self._sample(ids, edges_all, num_batches, counter)
-        self._unique(ids)
+        assert edges_all.dtype == torch.int64 and edges_all.is_contiguous() and edges_all.shape[1] in (2, 3)
+        f = capi.FrontDesc()
+        f.edges, f.cols, f.num_batches, f.sms = edges_all.data_ptr(), edges_all.shape[1], num_batches, sms
+        f.num_batches_dev = None if self.nb_dev is None else self.nb_dev.data_ptr()
+        f.step_dev, f.seed = counter.data_ptr(), cfg.seed
+        f.B, f.C, f.N, f.n_deg, f.domain, f.mapped, f.want_src_negs = cfg.B, cfg.C, cfg.N, cfg.n_deg, cfg.domain, self._mapped_domain(), cfg.sides == 2
+        f.packed, f.deg_rows, f.rel_ids = ids.packed.data_ptr(), ids.deg_rows.data_ptr(), ids.rel_ids.data_ptr() if cfg.has_relations else None
+        f.unique_ws, f.unique_ws_bytes = ids.uws.data_ptr(), ids.uws.numel()
+        f.unique, f.inverse, f.count, f.shared = (a.data_ptr() for a in (ids.unique, ids.inverse, ids.count, ids.shared))
+        if advance and self.peer is None:
+            f.counters, f.num_counters = self.step_dev.data_ptr(), 2
+        capi.sample_unique(f)
 
     def idle_step(self):
         """A step of a lane that has no batch (lanes of a superstep have unequal batch counts): the relation-gradient
@@ -437,8 +440,8 @@ class BatchPipeline:
         step (they share the id sets, the counters and the rule "the step whose counter is t uses id set t & 1").
         warm = False skips the host-issued warm-up step (a later capture of a pipeline that has run already).
 
-        Software-pipelined steps: while the decoder step of batch t runs (its scores kernel leaves most SMs idle in its
-        second round), the ids of batch t+1 are drawn and deduplicated on a side stream into the other id set; the optimizer
+        Software-pipelined steps: while the decoder step of batch t runs, the ids of batch t+1 are drawn and deduplicated on a side stream into
+        the other id set (on SMs that the scores kernels leave, or beside the finish kernel); the optimizer
         updates of batch t follow the join, so batch t+1 gathers the updated rows.  Two graphs alternate (one per id set);
         with rel_hook (the multi-GPU all-reduce, host-issued) each step is two graph launches around the hook.
         Returns an object with replay().  The same batches, negatives and arithmetic as the plain resident form."""
@@ -477,21 +480,28 @@ class BatchPipeline:
                     # graph p trains the steps whose counter has parity p: id set p, half p of the peer gradient buffer
                     desc = self._make_desc(edges_all, cur.rel_ids, 1, ids=cur, parity=p)
                     if front_after_scores:
-                        # The scores kernel owns whole SMs (one CTA with all of its shared memory); the small kernels of the next
-                        # batch's sampler and unique-map would delay its CTAs, so they are forked after it and run beside the
-                        # scatter and the optimizer updates, which leave room on every SM.
-                        desc.phases = 3
+                        # The scores kernels own whole SMs (one CTA with all of its shared memory), and small kernels would delay their CTAs.
+                        # Where they leave SMs over, and the batch is small enough for those, the sampler and the unique-map run there; else
+                        # behind the scores, beside finish -- which fills the SMs first, so that what was left of this chain for the
+                        # end of the step was 11 us: 88.0 us a step at configuration 2, 84.6 on the SMs left over.  (Beside prepare, which
+                        # fills the SMs as well, it holds up the scores: 87.7.)
+                        idle = capi.lp_idle_sms(desc)
+                        idle = idle if cfg.n_ids <= self.IDS_PER_IDLE_SM * idle else 0
+                        desc.phases = 1 if idle else 3
                         capi.lp_step(desc)
                         side.wait_stream(main)
                         with torch.cuda.stream(side):
-                            self._front(nxt, edges_all, num_batches, ctr_next)
+                            self._front(nxt, edges_all, num_batches, ctr_next, advance=rel_hook is None, sms=idle)
+                        if idle:
+                            desc.phases = 2
+                            capi.lp_step(desc)
                         desc.phases = 4
                         capi.lp_step(desc)
                         desc.phases = 0
                     else:
                         side.wait_stream(main)
                         with torch.cuda.stream(side):
-                            self._front(nxt, edges_all, num_batches, ctr_next)
+                            self._front(nxt, edges_all, num_batches, ctr_next, advance=rel_hook is None)
                         self._backward(desc)
                         main.wait_stream(side)
                     if rel_hook is None:
@@ -503,7 +513,8 @@ class BatchPipeline:
                         self._update_nodes(cur)
                         main.wait_stream(side2)
                         main.wait_stream(side)
-                        capi.advance_step(self.step_dev, 2)
+                        if self.peer is not None:
+                            capi.advance_step(self.step_dev, 2)
                     if rel_hook is not None and front_after_scores:
                         main.wait_stream(side)
                 gb = None
@@ -548,14 +559,14 @@ class BatchPipeline:
     def launches_per_step(self, resident: bool = True) -> int:
         """Kernels of libge2_b200.so launched per step (memsets not counted)."""
         cfg = self.cfg
-        n = 1 + 3                              # sampler; unique-map: mark, scan, inverse
+        n = 3                                  # sampler, which marks what it draws; unique-map: scan, inverse (and the counters)
         n += 1                                 # prepare (gather + relation operator + positive scores + filter words)
         n += 2                                 # scores: logsumexp pass + gradient pass, or both passes of the streaming form
         n += 1                                 # finish (operator backward + scatter)
         n += 1                                 # sparse Adagrad scatter
         if cfg.has_relations:
             n += 1 if (cfg.sides == 1 or self._rel_tables_adjacent) else 2
-        return n + (1 if resident else 0)      # device-side counter bump of the resident / graph forms
+        return n + (1 if resident and self.peer is not None else 0)  # counters that the exchange between ranks still reads
 
     def check_status(self):
         """Synchronises and raises if any kernel flagged bad data (call between epochs, not per batch)."""

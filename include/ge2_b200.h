@@ -46,7 +46,7 @@ typedef void *ge2_stream_t; /* cudaStream_t */
 
 /* "ge2_b200 <major>.<minor> (...)".  0.2: ge2_lp_desc grew by the members behind GE2_LP_HAS_ROW_UPDATE; ge2_train_step,
  * ge2_unique_bitmap_shared, ge2_adagrad_scatter_shared and the selected-negative backward with scratch are new.  A descriptor laid
- * out as in 0.1 (without that flag) is still understood. */
+ * out as in 0.1 (without that flag) is still understood.  0.3: ge2_sample_unique and ge2_lp_idle_sms are new. */
 GE2_API const char *ge2_version(void);
 GE2_API int ge2_last_cuda_error(void);            /* cudaError_t of the last failing runtime call on this thread */
 GE2_API const char *ge2_status_string(int status);
@@ -196,6 +196,8 @@ typedef struct ge2_lp_desc {
 } ge2_lp_desc;
 
 GE2_API int ge2_lp_workspace_bytes(const ge2_lp_desc *desc, size_t *bytes);
+/* SMs that the scores kernels of a step like this one leave to others */
+GE2_API int ge2_lp_idle_sms(const ge2_lp_desc *desc, int32_t *sms);
 GE2_API int ge2_lp_step(const ge2_lp_desc *desc, ge2_stream_t stream);
 
 /* =====================================================================================================
@@ -280,7 +282,8 @@ GE2_API int ge2_sample_negatives(const int64_t *src_ids, const int64_t *dst_ids,
 GE2_API int ge2_sample_batch(const int64_t *edges, int32_t cols, int64_t num_batches, const uint64_t *step_dev, int32_t B, int32_t C,
                              int32_t N, int32_t n_deg, int64_t domain, int32_t want_src_negs, uint64_t seed, int64_t *out_packed_ids,
                              int64_t *out_deg_rows, int64_t *out_rel_ids, ge2_stream_t stream);
-/* One training step in one call: ge2_sample_negatives, ge2_unique_bitmap_shared, ge2_lp_step, ge2_adagrad_scatter_shared and
+/* One training step in one call: ge2_sample_unique (or, for twins that are not the sampler's, ge2_sample_negatives and
+ * ge2_unique_bitmap_shared), ge2_lp_step, ge2_adagrad_scatter_shared and
  * ge2_dense_adagrad (num_dense <= 2 parameters of dense_numel floats each) with the same arguments, issued from native code.  n_ids is what
  * the sampler packs, 2 B + sides C N; ids in [table_rows, domain) are flagged like ids outside the domain.  With the row update in lp
  * (node_state), the members that name the same thing must agree: shared = row_shared, lr = node_lr, table = node_emb, state = node_state,
@@ -315,6 +318,33 @@ GE2_API int ge2_sample_batch_dev(const int64_t *edges, int32_t cols, const int64
                                  int32_t C, int32_t N, int32_t n_deg, int64_t domain, int32_t want_src_negs, uint64_t seed,
                                  int64_t *out_packed_ids, int64_t *out_deg_rows, int64_t *out_rel_ids, ge2_stream_t stream);
 GE2_API int ge2_advance_step(uint64_t *step_dev, int32_t n, ge2_stream_t stream);
+
+/* Sampler and unique-map of one batch in three launches: what ge2_sample_negatives (step_dev NULL: edges is the batch [B, cols], its number
+ * batch_index) or ge2_sample_batch / _dev (step_dev: batch *step_dev mod the number of batches of a resident list; num_batches_dev, where it is
+ * not NULL, holds that number) and ge2_unique_bitmap_shared (shared NULL: without it) leave, with the negatives that both sides share for
+ * twins, ids in [mapped, domain) flagged and the same workspace.  The sampler marks the ids it draws, so they are not read again for that.
+ * rel_ids is written for cols == 3 where it is not NULL; inverse has one entry per packed id, 2 B + sides C N of them.
+ * counters[0 ... num_counters): device-side counters that are incremented at the end (for a step in which nothing else reads them later). */
+typedef struct ge2_front_desc {
+    const int64_t *edges;
+    int32_t cols;
+    int32_t sms; /* at most as many CTAs as fit on so many SMs (0: all): those that ge2_lp_idle_sms says are free while another batch is scored */
+    int64_t num_batches;
+    const int64_t *num_batches_dev;
+    const uint64_t *step_dev;
+    uint64_t seed, batch_index;
+    int32_t B, C, N, n_deg;
+    int64_t domain, mapped;
+    int32_t want_src_negs, num_counters;
+    int64_t *packed, *deg_rows, *rel_ids;
+    void *unique_ws;
+    size_t unique_ws_bytes;
+    int64_t *unique, *inverse;
+    int32_t *count;
+    uint8_t *shared;
+    uint64_t *counters;
+} ge2_front_desc;
+GE2_API int ge2_sample_unique(const ge2_front_desc *desc, ge2_stream_t stream);
 
 /* GraphModelStorage::mapEdgesWithPartitionSlots_ (cpp/src/storage/graph_storage.cpp:270-303):
  * id -> slot[id / partition_size] * partition_size + id % partition_size on the first and last column of

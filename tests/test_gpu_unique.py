@@ -114,3 +114,63 @@ def test_the_form_without_out_shared_needs_one_bitset(capi, cuda_device, domain)
     assert bool((ws[small:] == 0xCD).all())
     with pytest.raises(capi.Ge2Error, match="workspace"):
         capi.unique_bitmap(ids, domain, workspace=ws[:small], out_shared=torch.empty(5000, dtype=torch.uint8, device=cuda_device))
+
+
+@pytest.mark.parametrize("cols,want_src,n_deg,shared,mapped,sms,resident", [
+    (3, True, 5, True, 300, 0, True), (3, True, 5, True, 300, 2, True), (3, False, 0, True, 300, 1, True), (2, False, 11, False, 300, 0, False),
+    (3, True, 11, True, 300, 3, False), (2, True, 4, True, 250, 0, True), (3, True, 0, False, 300, 148, True)])
+@pytest.mark.parametrize("B,C,N", [(1, 1, 11), (257, 3, 100), (1000, 2, 700)])
+def test_drawing_and_mapping_in_one_go(capi, cuda_device, cols, want_src, n_deg, shared, mapped, sms, resident, B, C, N):
+    """ge2_sample_unique leaves what the sampler and the unique-map leave one after the other, whatever the form, on all SMs or on a few."""
+    domain, batches, dev = 300, 3, cuda_device
+    rng = np.random.default_rng(B + N + n_deg)
+    edges = torch.from_numpy(rng.integers(0, domain, ((batches if resident else 1) * B, cols))).to(dev)
+    step, counters = torch.tensor([4], device=dev), torch.tensor([7, 8, 9], device=dev)
+    nb = torch.tensor([batches], device=dev)
+    n_ids = 2 * B + (2 if want_src else 1) * C * N
+    i64 = dict(dtype=torch.int64, device=dev)
+
+    def outputs():
+        return dict(packed=torch.full((n_ids,), -7, **i64), deg_rows=torch.full((C * max(n_deg, 1),), -7, **i64), rel_ids=torch.full((B,), -7, **i64),
+                    unique=torch.full((min(n_ids, mapped),), -7, **i64), inverse=torch.full((n_ids,), -7, **i64),
+                    count=torch.full((2,), -7, dtype=torch.int32, device=dev), shared=torch.full((min(n_ids, mapped),), 9, dtype=torch.uint8, device=dev))
+
+    want = outputs()
+    deg = want["deg_rows"] if n_deg else None
+    if resident:
+        capi.sample_batch_dev(edges, nb, step, B, C, N, n_deg, domain, want_src, 99, want["packed"], deg, want["rel_ids"] if cols == 3 else None)
+    else:
+        capi.sample_negatives(edges, edges[:, cols - 1], cols, B, C, N, n_deg, domain, want_src, 99, 4, want["packed"], deg)
+    capi.unique_bitmap(want["packed"], mapped, out_unique=want["unique"], out_inverse=want["inverse"], out_count=want["count"],
+                       out_shared=want["shared"] if shared else None, twins=(2 * B, C * N) if want_src and shared else (0, 0))
+    got = outputs()
+    ws = capi.unique_workspace(mapped, dev).fill_(0xAB)
+    f = capi.FrontDesc(edges=edges.data_ptr(), cols=cols, sms=sms, num_batches=batches, num_batches_dev=nb.data_ptr() if sms != 1 else None,
+                       step_dev=step.data_ptr() if resident else None, seed=99, batch_index=4, B=B, C=C, N=N, n_deg=n_deg, domain=domain, mapped=mapped,
+                       want_src_negs=want_src, num_counters=2, unique_ws=ws.data_ptr(), unique_ws_bytes=ws.numel(), counters=counters.data_ptr())
+    for name in ("packed", "deg_rows", "unique", "inverse", "count"):
+        setattr(f, name, got[name].data_ptr())
+    f.rel_ids = got["rel_ids"].data_ptr() if resident else None
+    f.shared = got["shared"].data_ptr() if shared else None
+    capi.sample_unique(f)
+    torch.cuda.synchronize()
+    for name in want:
+        assert torch.equal(want[name], got[name]), name
+    assert counters.tolist() == [8, 9, 9] and (mapped < domain or int(want["count"][1]) == 0)
+
+
+def test_drawing_and_mapping_refuses_what_does_not_fit(capi, cuda_device):
+    import ctypes
+
+    t = torch.zeros(64, dtype=torch.int64, device=cuda_device)
+    ws = capi.unique_workspace(50, cuda_device)
+    p = t.data_ptr()
+
+    def call(**kw):
+        a = dict(edges=p, cols=2, B=2, C=1, N=3, domain=50, mapped=50, packed=p, unique=p, inverse=p, count=p, unique_ws=ws.data_ptr(), unique_ws_bytes=ws.numel())
+        return capi.load_library().ge2_sample_unique(ctypes.byref(capi.FrontDesc(**{**a, **kw})), None)
+
+    for kw in (dict(B=0), dict(cols=4), dict(n_deg=4), dict(n_deg=1), dict(mapped=0), dict(sms=-1), dict(sms=149), dict(edges=None), dict(count=None),
+               dict(step_dev=p), dict(num_counters=1), dict(num_counters=33, counters=p)):
+        assert call(**kw) == 1, kw
+    assert call(unique_ws=None) == 3 and call(unique_ws_bytes=ws.numel() // 4) == 3 and call(unique_ws=ws.data_ptr() + 8) == 3
