@@ -358,11 +358,10 @@ struct FinScalars {
     unsigned char shared[2 * kFinBatch];  // the node occurs elsewhere in the batch
 };
 
-// one row's Adagrad step (called, not inlined: four exact divisions and square roots are 3 KB of code, and this kernel runs too briefly to
-// fetch several copies)
+// one row's Adagrad step
 template <int V, bool CPLX>
-__device__ __noinline__ void adagrad_row(float* emb, float* state, int l, int D, float4 e, float4 s, float4 g, float neg_lr) {
-    // a lane without columns must not divide: 0 / 1e-10 is off the fast path of the division, and the whole warp would wait for it
+__device__ __forceinline__ void adagrad_row(float* emb, float* state, int l, int D, float4 e, float4 s, float4 g, float neg_lr) {
+    // a lane without columns must not divide: 0 / 1e-10 is off the short path, and the whole warp would wait for it
     const int n = lp_row_ld(D) >> 2;
     // values of this lane that exist (at least); ComplEx: pairs of them
     const int cols = CPLX ? (V == 1 ? ((D >> 1) - l + n - 1) / n : (D >> 1) - 2 * l) : V == 1 ? (D - l + n - 1) / n : D - 4 * l;
@@ -371,12 +370,11 @@ __device__ __noinline__ void adagrad_row(float* emb, float* state, int l, int D,
         if (CPLX) s.y = s.w = 1.f;
         else s.w = 1.f, s.z = cols < 3 ? 1.f : s.z, s.y = cols < 2 ? 1.f : s.y;
     }
-    float dl, up;
-    adagrad_elem(g.x, s.x, dl, up, neg_lr), e.x = __fadd_rn(e.x, dl);
-    adagrad_elem(g.y, s.y, dl, up, neg_lr), e.y = __fadd_rn(e.y, dl);
-    adagrad_elem(g.z, s.z, dl, up, neg_lr), e.z = __fadd_rn(e.z, dl);
-    adagrad_elem(g.w, s.w, dl, up, neg_lr), e.w = __fadd_rn(e.w, dl);
-    put_row<V, CPLX, PutStore>(state, l, D, s);
+    const float gr[4] = {g.x, g.y, g.z, g.w};
+    float st[4] = {s.x, s.y, s.z, s.w}, dl[4], up[4];
+    adagrad_elems<4>(gr, st, dl, up, neg_lr);
+    e.x = __fadd_rn(e.x, dl[0]), e.y = __fadd_rn(e.y, dl[1]), e.z = __fadd_rn(e.z, dl[2]), e.w = __fadd_rn(e.w, dl[3]);
+    put_row<V, CPLX, PutStore>(state, l, D, make_float4(st[0], st[1], st[2], st[3]));
     put_row<V, CPLX, PutStore>(emb, l, D, e);
 }
 

@@ -76,8 +76,7 @@ __global__ void __launch_bounds__(256) sparse_adagrad_kernel(const float* __rest
         float g[V], s[V], d[V], u[V];
         to_arr<V>(reinterpret_cast<const VT*>(grad)[i], g);
         to_arr<V>(reinterpret_cast<const VT*>(state)[i], s);
-#pragma unroll
-        for (int k = 0; k < V; k++) adagrad_elem(g[k], s[k], d[k], u[k], neg_lr);
+        adagrad_elems<V>(g, s, d, u, neg_lr);
         reinterpret_cast<VT*>(state)[i] = from_arr<V>(s);
         if (out_upd != nullptr) reinterpret_cast<VT*>(out_upd)[i] = from_arr<V>(u);
         reinterpret_cast<VT*>(out_delta)[i] = from_arr<V>(d);
@@ -161,11 +160,11 @@ __global__ void __launch_bounds__(256) adagrad_scatter_kernel(float* __restrict_
 #pragma unroll
             for (int k = 0; k < kRows; k++) {
                 if (!on[k]) continue;
+                float dl[V], up[V];
+                adagrad_elems<V>(g[k], s[k], dl, up, neg_lr);
 #pragma unroll
                 for (int v = 0; v < V; v++) {
-                    float dl, up;
-                    adagrad_elem(g[k][v], s[k][v], dl, up, neg_lr);
-                    e[k][v] = __fadd_rn(e[k][v], dl);
+                    e[k][v] = __fadd_rn(e[k][v], dl[v]);
                     g[k][v] = 0.f;
                 }
                 reinterpret_cast<VT*>(state)[row[k] * vec_per_row + c] = from_arr<V>(s[k]);

@@ -24,6 +24,36 @@ def test_sparse_adagrad_bit_exact(capi, cuda_device, D):
     assert np.array_equal(ts.cpu().numpy(), st + ou)  # state updated in place, as node_embeddings_state_.add_ does
 
 
+@pytest.mark.parametrize("D", [1, 2, 4])
+def test_adagrad_is_ieee_over_the_whole_range(capi, cuda_device, D):
+    """Square root and division bit for bit, whichever way they are taken: sizes from subnormal to huge, zeros of both signs, denominators whose
+    significand is all ones (and their neighbours), infinities and NaN."""
+    rng = np.random.default_rng(D)
+    n = 400_000
+
+    def wide(lo, hi):
+        return np.ldexp(1.0 + rng.random(n), rng.integers(lo, hi, n)).astype(np.float32)
+
+    g, st = wide(-149, 40) * rng.choice([-1, 1], n).astype(np.float32), wide(-149, 70)
+    g[: n // 2] = (wide(-40, 10) * rng.choice([-1, 1], n).astype(np.float32))[: n // 2]  # the ordinary range, densely
+    st[: n // 4] = wide(-45, 10)[: n // 4]
+    st[n // 4 : n // 2] = 0.0
+    ones = np.ldexp(np.float64(2.0 - 2.0**-23), rng.integers(-18, 20, 40_000))
+    st[-40_000:] = (ones * ones).astype(np.float32).view(np.int32).__add__(rng.integers(-2, 3, 40_000, dtype=np.int32)).view(np.float32)
+    g[-40_000:] = wide(-90, -30)[-40_000:]  # (too small to move the state)
+    g[:64:4], g[1:64:4], g[2:64:8], g[3:64:8], st[40:48] = 0.0, -0.0, np.inf, np.nan, np.inf
+    g, st = g.reshape(-1, D), st.reshape(-1, D)
+    ts = torch.from_numpy(st.copy()).to(cuda_device)
+    delta, upd = capi.sparse_adagrad(torch.from_numpy(g).to(cuda_device), ts, 0.1)
+    with np.errstate(all="ignore"):
+        want_delta, want_upd = O.sparse_adagrad(g, st, 0.1)
+        want_state = st + want_upd
+    for got, want in ((delta, want_delta), (upd, want_upd), (ts, want_state)):
+        got = got.cpu().numpy()
+        same = (got.view(np.int32) == want.view(np.int32)) | (np.isnan(got) & np.isnan(want))
+        assert same.all(), (g[~same][:4], st[~same][:4], got[~same][:4], want[~same][:4])
+
+
 @pytest.mark.parametrize("D", [50, 100, 128])
 def test_index_read_add_and_fused_scatter(capi, cuda_device, D):
     rng = np.random.default_rng(100 + D)
