@@ -32,7 +32,7 @@ constexpr int kTileQ = 128;       // query rows of a score tile
 constexpr int kTileN = 256;       // candidates of a score tile
 constexpr int kGroupTiles = 16;   // most query tiles of a group
 constexpr int kAccs = 2;          // score accumulators in tensor memory
-constexpr int kCountThreads = 896, kTmaWarp = 0, kMmaWarp = 1, kEpiWarp0 = 4, kEpiWarps = 16, kConvWarp0 = 20, kConvWarps = 8;
+constexpr int kCountThreads = 896, kTmaWarp = 0, kMmaWarp = 1, kCopyWarp = 2, kEpiWarp0 = 4, kEpiWarps = 16, kConvWarp0 = 20, kConvWarps = 8;
 constexpr int kConvRows = kTileN / kConvWarps, kConvBatch = 8;
 constexpr int kListCap = 64;      // undecided candidates a warp collects before it hands 32 of them on
 constexpr int kPrepRows = 32, kPrepThreads = 256;
@@ -50,6 +50,7 @@ struct EvalArgs {
     uint2* open_list;             // (query row, candidate column) of comparisons the counting pass left open
     unsigned long long* open_count;  // how many were put there (may exceed open_cap: the rest was evaluated in place)
     int64_t open_cap;
+    unsigned char* stage;         // D > 64: [kNumSMs] split candidate tiles on their way into shared memory
     int64_t Bp;
     int S, ld;
     int vec;                      // floats per access to a candidate row: 4 or 2 (rows aligned and whole), else 1
@@ -79,6 +80,50 @@ __device__ __forceinline__ float score_chain(const float* __restrict__ q, const 
             const float2 a = __ldg(reinterpret_cast<const float2*>(q) + k), b = __ldg(reinterpret_cast<const float2*>(e) + k);
             acc = __fmaf_rn(a.x, b.x, acc);
             acc = __fmaf_rn(a.y, b.y, acc);
+        }
+    } else {
+#pragma unroll 8
+        for (int k = 0; k < D; k++) acc = __fmaf_rn(__ldg(q + k), __ldg(e + k), acc);
+    }
+    return acc;
+}
+
+// the same with more loads on their way (and more registers than a call out of the counting pass can have)
+__device__ __forceinline__ float score_chain_ahead(const float* __restrict__ q, const float* __restrict__ e, int D, int vec) {
+    float acc = 0.f;
+    if (vec == 4) {
+        constexpr int kAhead = 7;
+        const int n = D / 4;
+#pragma unroll 1
+        for (int k0 = 0; k0 < n; k0 += kAhead) {  // loads of a round are on their way together, those of the last one too
+            float4 x[kAhead], y[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; k++)
+                if (k0 + k < n) x[k] = __ldg(reinterpret_cast<const float4*>(q) + k0 + k), y[k] = __ldg(reinterpret_cast<const float4*>(e) + k0 + k);
+#pragma unroll
+            for (int k = 0; k < kAhead; k++)
+                if (k0 + k < n) {
+                    acc = __fmaf_rn(x[k].x, y[k].x, acc);
+                    acc = __fmaf_rn(x[k].y, y[k].y, acc);
+                    acc = __fmaf_rn(x[k].z, y[k].z, acc);
+                    acc = __fmaf_rn(x[k].w, y[k].w, acc);
+                }
+        }
+    } else if (vec == 2) {
+        constexpr int kAhead = 9;
+        const int n = D / 2;
+#pragma unroll 1
+        for (int k0 = 0; k0 < n; k0 += kAhead) {
+            float2 x[kAhead], y[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; k++)
+                if (k0 + k < n) x[k] = __ldg(reinterpret_cast<const float2*>(q) + k0 + k), y[k] = __ldg(reinterpret_cast<const float2*>(e) + k0 + k);
+#pragma unroll
+            for (int k = 0; k < kAhead; k++)
+                if (k0 + k < n) {
+                    acc = __fmaf_rn(x[k].x, y[k].x, acc);
+                    acc = __fmaf_rn(x[k].y, y[k].y, acc);
+                }
         }
     } else {
 #pragma unroll 8
@@ -196,13 +241,15 @@ __device__ __forceinline__ void add_to_rank(const EvalArgs& a, int64_t w, int64_
 }
 
 // an undecided comparison, by the score's definition
+template <bool kAhead>
 __device__ __forceinline__ void settle(const EvalArgs& a, uint2 what) {
     const float* e = node_row(a.d, what.y);
     // a candidate id outside the table scores 0
-    const float s = e != nullptr ? score_chain(a.Q + (int64_t)what.x * a.d.D, e, a.d.D, a.vec) : 0.f;
+    const float* q = a.Q + (int64_t)what.x * a.d.D;
+    const float s = e == nullptr ? 0.f : kAhead ? score_chain_ahead(q, e, a.d.D, a.vec) : score_chain(q, e, a.d.D, a.vec);
     if (s >= a.pos[what.x]) add_to_rank(a, what.x, 1);
 }
-__device__ __noinline__ void settle_in_place(const EvalArgs& a, uint2 what) { settle(a, what); }
+__device__ __noinline__ void settle_in_place(const EvalArgs& a, uint2 what) { settle<false>(a, what); }
 
 // fma(v, scale, shift) clamped to [0, 1]
 __device__ __forceinline__ float saturated(float v, float scale, float shift) {
@@ -237,13 +284,14 @@ __device__ __forceinline__ float sum2(uint64_t a) {
 struct CountSched {
     int q_tiles, groups;
     int64_t cand_tiles, num_cols;
+    int staged;   // do CTAs convert the next candidate tile into EvalArgs::stage while one is contracted? (one CTA an SM)
     float bound;  // |score on the tensor cores - score chain| <= bound * |q| * |e| (+ underflow terms)
 };
 
 template <int NB>
 struct CountSmem {
     static constexpr int kSlots = 5;                                  // ring of query blocks (128 rows x 64 columns of one term)
-    static constexpr int kCandBufs = NB == 2 ? 1 : 2;                 // a candidate tile of D > 64 leaves no room for a second
+    static constexpr int kCandBufs = NB == 2 ? 1 : 2;                 // a candidate tile of D > 64 leaves no room for a second: it waits in global memory
     static constexpr int kCandBlock = kTileN * 128;                   // 64 columns of one term
     static constexpr int kCandBytes = 2 * NB * kCandBlock;            // one candidate tile, both terms
     static constexpr int kCand = 0;
@@ -255,7 +303,7 @@ struct CountSmem {
     static constexpr int kBytes = kEnd + 1024;                        // 1024 bytes of slack to align the base
     static_assert(kBytes <= 227 * 1024, "counting pass exceeds the shared memory of an SM");
 };
-enum CountBar { kQFull = 0, kQEmpty = 8, kCFull = 16, kCEmpty = 18, kAccFull = 20, kAccEmpty = 24, kCountBars = 28 };
+enum CountBar { kQFull = 0, kQEmpty = 8, kCFull = 16, kCEmpty = 18, kAccFull = 20, kAccEmpty = 24, kStaged = 28, kCountBars = 29 };
 
 // #(candidates whose score is >= the positive's) for every query row.
 //
@@ -272,11 +320,13 @@ enum CountBar { kQFull = 0, kQEmpty = 8, kCFull = 16, kCEmpty = 18, kAccFull = 2
 //
 // One CTA per SM, warps by role: TMA producer of query blocks, MMA issuer, 16 epilogue warps (a thread owns one query row and a
 // quarter of the tile's columns: its threshold is a register), 8 warps that read candidate rows (fp32, each once per query group),
-// split them and write them swizzled.  The candidates stay while the group's query tiles stream past: 64 KB of query blocks for
-// 21 contractions of 128 x 256 x 16 (128 candidates instead of 256 left the contractions waiting for query blocks).  2 000 queries x
-// 1 M nodes, D = 100: 1.2 ms (18.5 ms as chains of fp32 multiply-adds), 2 000 queries x 14 951 nodes, D = 50: 27 us (142 us).  What
-// is left above the 0.6 ms of the contractions is the conversion of candidate tiles (D > 64: one buffer, so it is not hidden) and the
-// issue of small contractions.
+// split them and write them swizzled, and one that copies.  The candidates stay while the group's query tiles stream past: 64 KB of query
+// blocks for 21 contractions of 128 x 256 x 16 (128 candidates instead of 256 left the contractions waiting for query blocks).  D <= 64:
+// two candidate tiles fit.  Wider: the next one is split into global memory (128 KB a CTA, which stay in the L2) while this one is
+// contracted, and comes in as four bulk copies: 6 800 cycles without a tile instead of the 15 400 of splitting it there and then, of 67 000 a tile.
+// 2 000 queries x 1 M nodes, D = 100: 1.11 ms (1.17 without the staging, 18.5 as chains of fp32 multiply-adds); 600 x 200 000, D = 128: 188 us in
+// all instead of 226; 2 000 queries x 14 951 nodes, D = 50: 28 us (142).  Of the first, 0.64 ms are the contractions at the clock that
+// power leaves; the rest is waiting for query blocks (13 %), candidate tiles (10 %) and accumulators (9 %).
 template <int NB, int VEC>
 __global__ void __launch_bounds__(kCountThreads, 1)
     eval_count_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ EvalArgs a, CountSched sc) {
@@ -309,6 +359,7 @@ __global__ void __launch_bounds__(kCountThreads, 1)
             mbar_init(&bars[kAccFull + k], 1);
             mbar_init(&bars[kAccEmpty + k], kEpiWarps);
         }
+        mbar_init(&bars[kStaged], kConvWarps);
         *s_abort = 0;
         mbar_init_fence();
         prefetch_tensormap(&tmQ);
@@ -381,6 +432,20 @@ __global__ void __launch_bounds__(kCountThreads, 1)
         }
         // the last arrivals that the tensor pipe makes on barriers of this CTA have landed before it can exit
         if (ok && cc > 0) spin_wait(kCEmpty + (cc - 1) % SM::kCandBufs, ((cc - 1) / SM::kCandBufs) & 1);
+    } else if (warp == kCopyWarp) {
+        // ---- staged candidate tiles: into shared memory as soon as it is free; the arrivals stand for those of the converting warps ----
+        if (NB == 2 && sc.staged) {
+            const unsigned char* stage = a.stage + (int64_t)(blockIdx.y * gridDim.x + blockIdx.x) * SM::kCandBytes;
+            uint32_t cc = 1;
+            for (int64_t t = tb + 1; t < te; t++, cc++) {
+                if (!spin_wait(kStaged, (cc - 1) & 1) || !spin_wait(kCEmpty, (cc & 1) ^ 1)) break;
+                if (lane == 0) mbar_expect_tx(&bars[kCFull], SM::kCandBytes);
+                __syncwarp();
+                if (lane > 0 && lane < kConvWarps) mbar_arrive(&bars[kCFull]);
+                if (lane < 2 * NB) bulk_load_1d(smem + SM::kCand + lane * SM::kCandBlock, stage + lane * SM::kCandBlock, SM::kCandBlock, &bars[kCFull]);
+                __syncwarp();
+            }
+        }
     } else if (warp >= kConvWarp0) {
         // ---- candidate rows: kConvRows per warp and tile, kConvBatch in flight ----
         // Kept small: this code runs once in tens of microseconds and comes out of a cold instruction cache every time; written out
@@ -419,8 +484,10 @@ __global__ void __launch_bounds__(kCountThreads, 1)
         while (true) {  // one turn: the batch in registers (none in the first) goes to shared memory, the next one is fetched
             if (r0 >= 0) {
                 const int cb = cc % SM::kCandBufs;
+                const bool staged = NB == 2 && sc.staged && cc > 0;  // (the first tile goes straight to shared memory)
                 if (r0 == 0) {
-                    if (!warp_wait(kCEmpty + cb, ((cc / SM::kCandBufs) & 1) ^ 1)) break;
+                    // the place it goes to is free: the copy before has been taken, or the tile before has been contracted
+                    if (staged ? !warp_wait(kCFull, (cc & 1) ^ 1) : !warp_wait(kCEmpty + cb, ((cc / SM::kCandBufs) & 1) ^ 1)) break;
                     // a power of two for these 32 rows, from the first eight: the others may be 2^6 times larger before fp16 ends
                     float most = 0.f;
 #pragma unroll
@@ -428,7 +495,8 @@ __global__ void __launch_bounds__(kCountThreads, 1)
                     scale = pow2_near_256(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(most))));
                     norm2 = 0.f;  // largest squared norm that this lane's four columns contribute to a row
                 }
-                unsigned char* at0 = smem + SM::kCand + cb * SM::kCandBytes + (lane >> 4) * SM::kCandBlock + (lane & 1) * 8 + (cw * kConvRows + r0) * 128;
+                unsigned char* at0 = (staged ? a.stage + (int64_t)(blockIdx.y * gridDim.x + blockIdx.x) * SM::kCandBytes : smem + SM::kCand + cb * SM::kCandBytes) +
+                                     (lane >> 4) * SM::kCandBlock + (lane & 1) * 8 + (cw * kConvRows + r0) * 128;
 #pragma unroll
                 for (int k = 0; k < kConvBatch; k++) {
                     const float4 x = make_float4(v[k].x * scale, v[k].y * scale, v[k].z * scale, v[k].w * scale);
@@ -448,10 +516,10 @@ __global__ void __launch_bounds__(kCountThreads, 1)
                     // |e| of no row exceeds the root of the sum over lanes (tighter by a third with a sum per row, and not worth it)
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) norm2 += __shfl_xor_sync(0xffffffffu, norm2, o);
-                    if (lane == 0) s_cand[cb * kConvWarps + cw] = make_float2(sqrtf(norm2) * 1.001f, scale);
-                    fence_proxy_async_smem();  // written with ordinary stores; the MMA reads through the async proxy
+                    if (lane == 0) s_cand[(cc & 1) * kConvWarps + cw] = make_float2(sqrtf(norm2) * 1.001f, scale);
+                    fence_proxy_async();  // written with ordinary stores; the MMA, or the copy, reads through the async proxy
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars[kCFull + cb]);
+                    if (lane == 0) mbar_arrive(&bars[staged ? kStaged : kCFull + cb]);
                     t++;
                     cc++;
                     if (t >= te) break;
@@ -493,7 +561,7 @@ __global__ void __launch_bounds__(kCountThreads, 1)
             float slope[2], cscale[2];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const float2 cand = s_cand[cb * kConvWarps + quarter * 2 + k];
+                const float2 cand = s_cand[(cc & 1) * kConvWarps + quarter * 2 + k];
                 cscale[k] = cand.y;
                 slope[k] = cand.x < 60000.f ? 1.05f * (sc.bound * cand.x + 4e-7f) : INFINITY;  // (at the end of fp16 nothing is decided)
             }
@@ -594,7 +662,7 @@ __global__ void __launch_bounds__(kCountThreads, 1)
     __syncthreads();
     if (warp == kMmaWarp) {
         if (*s_abort && lane == 0)  // copies still in flight get a bounded chance to land
-            for (int k = 0; k < SM::kSlots; k++) settle_bar(&bars[kQFull + k]);
+            for (int k = 0; k < SM::kSlots + SM::kCandBufs; k++) settle_bar(&bars[k < SM::kSlots ? kQFull + k : kCFull + k - SM::kSlots]);
         __syncwarp();
         tc_fence_after();
         tmem_dealloc(tmem, 512);
@@ -621,26 +689,20 @@ __device__ __forceinline__ void apply_filter_pair(const EvalArgs& a, int s, int6
     }
     const int64_t w = (int64_t)s * a.Bp + i;
     const unsigned long long key = ((unsigned long long)s << 62) + (unsigned long long)i * (unsigned long long)num_cols + (unsigned long long)col + 1ull;
-    unsigned long long slot = (key * 0x9E3779B97F4A7C15ull) >> 20;
-    bool first = false, placed = false;
-    for (int64_t probe = 0; probe < a.hash_slots; probe++) {
-        slot &= (unsigned long long)(a.hash_slots - 1);
-        const unsigned long long old = atomicCAS(&a.hash[slot], 0ull, key);
-        if (old == 0ull) {
-            first = placed = true;
-            break;
-        }
-        if (old == key) {
-            placed = true;
-            break;
-        }
-        slot++;
-    }
-    if (!placed) or_status(d.status, GE2_STATUS_FILTER_COLLISION);  // cannot happen: the set has twice as many slots as pairs
-    if (!first) return;
+    unsigned long long slot = (key * 0x9E3779B97F4A7C15ull) >> 20 & (unsigned long long)(a.hash_slots - 1);
+    // (the chain is walked while the answer is on its way: few pairs occur again)
+    unsigned long long old = atomicCAS(&a.hash[slot], 0ull, key);
     const float* e = node_row(d, col);
-    const float acc = e != nullptr ? score_chain(a.Q + w * d.D, e, d.D, a.vec) : 0.f;
     const float pos = a.pos[w];
+    const float acc = e != nullptr ? score_chain_ahead(a.Q + w * d.D, e, d.D, a.vec) : 0.f;
+    for (int64_t probe = 1; old != 0ull && old != key && probe < a.hash_slots; probe++) {
+        slot = (slot + 1) & (unsigned long long)(a.hash_slots - 1);
+        old = atomicCAS(&a.hash[slot], 0ull, key);
+    }
+    if (old != 0ull) {
+        if (old != key) or_status(d.status, GE2_STATUS_FILTER_COLLISION);  // cannot happen: the set has twice as many slots as pairs
+        return;
+    }
     int64_t delta = 0;
     if (acc >= pos) delta -= 1;
     if (-1e9f >= pos) delta += 1;
@@ -649,6 +711,7 @@ __device__ __forceinline__ void apply_filter_pair(const EvalArgs& a, int s, int6
 
 // What the counting pass left open, and the filter: a thread each, blockIdx.x < filter_blocks the filter pairs (both sides), the others
 // the open comparisons.  All of it adds to the ranks, in any order.
+// Bound by the latency of scattered rows; 56 loads of a chain are on their way at a time (10: 98 us at 1 M nodes and 19.8 at 14 951, now 91 and 14.7).
 __global__ void __launch_bounds__(kSettleThreads) eval_settle_kernel(const __grid_constant__ EvalArgs a, int64_t num_cols, int filter_blocks) {
     griddep_wait();
     if ((int)blockIdx.x < filter_blocks) {
@@ -658,7 +721,7 @@ __global__ void __launch_bounds__(kSettleThreads) eval_settle_kernel(const __gri
         return;
     }
     const int64_t n = min((int64_t)*a.open_count, a.open_cap), stride = (int64_t)(gridDim.x - filter_blocks) * kSettleThreads;
-    for (int64_t k = (int64_t)(blockIdx.x - filter_blocks) * kSettleThreads + threadIdx.x; k < n; k += stride) settle(a, a.open_list[k]);
+    for (int64_t k = (int64_t)(blockIdx.x - filter_blocks) * kSettleThreads + threadIdx.x; k < n; k += stride) settle<true>(a, a.open_list[k]);
 }
 
 int64_t hash_slots_for(int64_t pairs) {
@@ -682,7 +745,7 @@ namespace {
 // workspace sections of a call, in order
 struct EvalSections {
     int64_t Bp;
-    size_t q, split, pos, norm, qinv, hash, open_count, open, bytes;
+    size_t q, split, pos, norm, qinv, hash, open_count, open, stage, bytes;
     int64_t open_cap;
     explicit EvalSections(const ge2_eval_desc* d) {
         const int S = sides_of(d);
@@ -705,6 +768,7 @@ struct EvalSections {
         const int64_t num_cols = d->neg_ids != nullptr ? d->num_negs : d->num_nodes;
         open_cap = std::min<int64_t>(std::max<int64_t>(S * Bp * std::max<int64_t>(num_cols, 0) / 1024, 4096), 4 << 20);
         open = take((size_t)open_cap * 8);
+        stage = take(d->D > 64 && num_cols > (int64_t)kTileN ? (size_t)kNumSMs * CountSmem<2>::kCandBytes : 0);
         bytes = off;
     }
 };
@@ -725,6 +789,7 @@ int launch_count(const EvalArgs& a, CountSched sc, const CUtensorMap& tmQ, cudaS
     }
     if (sc.groups > 65535) return GE2_ERR_UNSUPPORTED;
     const dim3 grid((unsigned)std::min<int64_t>(std::max(1, kNumSMs / sc.groups), sc.cand_tiles), (unsigned)sc.groups);
+    sc.staged = NB == 2 && sc.cand_tiles > grid.x && (int64_t)grid.x * grid.y <= kNumSMs;
     GE2_CUDA_TRY(launch_after(kernel, grid, dim3(kCountThreads), CountSmem<NB>::kBytes, stream, tmQ, a, sc));
     return GE2_OK;
 }
@@ -774,6 +839,7 @@ extern "C" int ge2_eval_ranks(const ge2_eval_desc* d, ge2_stream_t stream_) {
     a.open_list = (uint2*)(p + at.open);
     a.open_count = (unsigned long long*)(p + at.open_count);
     a.open_cap = at.open_cap;
+    a.stage = (unsigned char*)(p + at.stage);
     const int64_t rows = (int64_t)S * a.Bp;
     if (rows > 0x7fffffffLL) return GE2_ERR_UNSUPPORTED;
     // the set of filter pairs and the counter behind it

@@ -79,6 +79,7 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
 // generic-proxy writes to shared memory (st.shared) must be fenced before the async proxy (tcgen05.mma) reads them
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }  // (and to global memory before a bulk copy does)
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ---- tensor memory ---------------------------------------------------------------------------------------------

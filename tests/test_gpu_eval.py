@@ -93,6 +93,7 @@ def test_candidate_list_and_bad_ids(capi, cuda_device):
 @pytest.mark.parametrize("nodes,B,D,scale", [
     (255, 127, 64, 1.0), (256, 128, 65, 1e-3), (257, 129, 128, 30.0),   # edges of the score tiles; odd, half and full row widths
     (513, 1, 2, 1.0), (40, 300, 100, 1e-12), (5000, 40, 98, 1e6),       # few candidates, few queries, values far from one
+    (148 * 256 + 1, 3, 100, 1.0), (77_000, 130, 66, 1.0), (115_000, 2, 65, 1.0),  # several wide candidate tiles a CTA, staged ahead
 ])
 def test_ranks_are_exact_at_tile_edges_and_on_ties(capi, cuda_device, nodes, B, D, scale):
     """The counting pass compares scores computed on the tensor cores and evaluates only what those leave open: ranks must still be
