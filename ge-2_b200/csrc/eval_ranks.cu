@@ -399,37 +399,40 @@ __global__ void __launch_bounds__(kCountThreads, 1)
         int slot = 0;
         uint32_t phase = 0, ac = 0, cc = 0;
         bool ok = true;
-        for (int64_t t = tb; ok && t < te; t++, cc++) {
-            const int cb = cc % SM::kCandBufs;
-            if (!spin_wait(kCFull + cb, (cc / SM::kCandBufs) & 1)) break;
-            const uint32_t ch = cand + cb * (2 * NB * kCandStep), cl = ch + NB * kCandStep;
-            for (int qt = q0; ok && qt < q1; qt++, ac++) {
-                const int ab = ac % kAccs;
-                ok = spin_wait(kAccEmpty + ab, ((ac / kAccs) & 1) ^ 1);
-                if (!ok) break;
-                const uint32_t acc = tmem + ab * kTileN;
-                auto product = [&](uint32_t da, uint32_t db, int b, bool first) {  // one 64-column block
-                    mma_kmajor<1, kBlockBytes, SM::kCandBlock>(min(4, KS - 4 * b), acc, da, db + b * kCandStep, kIdesc, first ? 0u : 1u);
-                };
-#pragma unroll
-                for (int k = 0; k < 2 * NB; k++) {
-                    ok = ok && spin_wait(kQFull + slot, phase);
+        with_steps<NB>(KS, [&](auto steps) {
+            for (int64_t t = tb; ok && t < te; t++, cc++) {
+                const int cb = cc % SM::kCandBufs;
+                if (!spin_wait(kCFull + cb, (cc / SM::kCandBufs) & 1)) break;
+                const uint32_t ch = cand + cb * (2 * NB * kCandStep), cl = ch + NB * kCandStep;
+                for (int qt = q0; ok && qt < q1; qt++, ac++) {
+                    const int ab = ac % kAccs;
+                    ok = spin_wait(kAccEmpty + ab, ((ac / kAccs) & 1) ^ 1);
                     if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t da = ring + slot * kSlotStep;
-                    if (k < NB) {
-                        product(da, ch, k, k == 0);
-                    } else {
-                        product(da, cl, k - NB, false);
-                        product(da, ch, k - NB, false);
+                    const uint32_t acc = tmem + ab * kTileN;
+                    auto product = [&](uint32_t da, uint32_t db, int b, bool first) {  // one 64-column block
+                        if (b < NB - 1) mma_kmajor<4, kBlockBytes, SM::kCandBlock>(acc, da, db + b * kCandStep, kIdesc, first ? 0u : 1u);
+                        else mma_kmajor<steps - 4 * (NB - 1), kBlockBytes, SM::kCandBlock>(acc, da, db + b * kCandStep, kIdesc, first ? 0u : 1u);
+                    };
+    #pragma unroll
+                    for (int k = 0; k < 2 * NB; k++) {
+                        ok = ok && spin_wait(kQFull + slot, phase);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t da = ring + slot * kSlotStep;
+                        if (k < NB) {
+                            product(da, ch, k, k == 0);
+                        } else {
+                            product(da, cl, k - NB, false);
+                            product(da, ch, k - NB, false);
+                        }
+                        mma_commit_warp(&bars[kQEmpty + slot]);
+                        if (k == 2 * NB - 1) mma_commit_warp(&bars[kAccFull + ab]);
+                        if (++slot == SM::kSlots) slot = 0, phase ^= 1;
                     }
-                    mma_commit_warp(&bars[kQEmpty + slot]);
-                    if (k == 2 * NB - 1) mma_commit_warp(&bars[kAccFull + ab]);
-                    if (++slot == SM::kSlots) slot = 0, phase ^= 1;
                 }
+                if (ok) mma_commit_warp(&bars[kCEmpty + cb]);
             }
-            if (ok) mma_commit_warp(&bars[kCEmpty + cb]);
-        }
+        });
         // the last arrivals that the tensor pipe makes on barriers of this CTA have landed before it can exit
         if (ok && cc > 0) spin_wait(kCEmpty + (cc - 1) % SM::kCandBufs, ((cc - 1) / SM::kCandBufs) & 1);
     } else if (warp == kCopyWarp) {

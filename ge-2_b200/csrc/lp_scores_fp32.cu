@@ -159,25 +159,27 @@ __global__ void __launch_bounds__(kThreadsA, 1)
         const int KS = (d.D + kMmaK - 1) / kMmaK;
         int sg = -1;
         IterA un(ub, sc);
-        for (int it = 0; it < n_iter; it++, un.next(sc)) {
-            if (it == 0 || un.tile == 0) {
-                sg++;
-                if (!spin_wait(kAXFull, sg & 1)) break;
+        with_steps<LY::NB>(KS, [&](auto steps) {
+            for (int it = 0; it < n_iter; it++, un.next(sc)) {
+                if (it == 0 || un.tile == 0) {
+                    sg++;
+                    if (!spin_wait(kAXFull, sg & 1)) break;
+                }
+                const int st = it % kLseStages, use = it / kLseStages, sb = it & 1, su = it >> 1;
+                if (!spin_wait(kAYFull + st, use & 1)) break;
+                if (!spin_wait(kASEmpty + sb, (su & 1) ^ 1)) break;
+                tc_fence_after();
+                const uint32_t dY = dY0 + st * (kPlanes * LY::kYPlane >> 4);
+    #pragma unroll 1
+                for (int p = 0; p < 6; p++) {
+                    const uint32_t da = dX + ((kFirst >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY + ((kSecond >> (2 * p)) & 3) * (LY::kYPlane >> 4);
+                    mma_kmajor<steps, LY::kXBlock, LY::kYBlock>(tmem + sb * BN, da, db, kIdesc, p > 0 ? 1u : 0u);
+                }
+                mma_commit_warp(&bars[kAYEmpty + st]);
+                if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit_warp(&bars[kAXEmpty]);
+                mma_commit_warp(&bars[kASFull + sb]);  // last: whoever waits for it has seen the others' arrivals land before the CTA exits
             }
-            const int st = it % kLseStages, use = it / kLseStages, sb = it & 1, su = it >> 1;
-            if (!spin_wait(kAYFull + st, use & 1)) break;
-            if (!spin_wait(kASEmpty + sb, (su & 1) ^ 1)) break;
-            tc_fence_after();
-            const uint32_t dY = dY0 + st * (kPlanes * LY::kYPlane >> 4);
-#pragma unroll 1
-            for (int p = 0; p < 6; p++) {
-                const uint32_t da = dX + ((kFirst >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY + ((kSecond >> (2 * p)) & 3) * (LY::kYPlane >> 4);
-                mma_kmajor<LY::NB, LY::kXBlock, LY::kYBlock>(KS, tmem + sb * BN, da, db, kIdesc, p > 0 ? 1u : 0u);
-            }
-            mma_commit_warp(&bars[kAYEmpty + st]);
-            if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit_warp(&bars[kAXEmpty]);
-            mma_commit_warp(&bars[kASFull + sb]);  // last: whoever waits for it has seen the others' arrivals land before the CTA exits
-        }
+        });
     } else if (warp >= kClearWarpA) {
         // clear what the gradient pass will add to: dK, and the dQ rows of every block whose stream that pass cuts at a CTA boundary
         const int wz = (warp - kClearWarpA) * 32 + lane;
@@ -376,32 +378,34 @@ __global__ void __launch_bounds__(kThreadsB, 1)
         uint32_t ph0 = 0;
         bool ok = true;
         IterA un(ub, sc);
-        for (int it = 0; ok && it < n_iter; it++, un.next(sc)) {
-            if (it == 0 || un.tile == 0) {
-                sg++;
-                if (!spin_wait(kBXFull, sg & 1)) break;
-            }
-            const int sb = it & 1, su = it >> 1;
-            if (!spin_wait(kBSEmpty + sb, (su & 1) ^ 1)) break;
-            int seen = 0;  // planes of this tile known to have arrived, in the order m, h, l
-#pragma unroll 1
-            for (int p = 0; p < 6; p++) {
-                const int k = slot_of_plane((kSecondS >> (2 * p)) & 3);
-                const int slot = slot0 + k >= kYSlots ? slot0 + k - kYSlots : slot0 + k;
-                if (k >= seen) {
-                    ok = spin_wait(kBYFull + slot, slot0 + k >= kYSlots ? ph0 ^ 1 : ph0);
-                    if (!ok) break;
-                    seen = k + 1;
-                    tc_fence_after();
+        with_steps<LY::NB>(KS, [&](auto steps) {
+            for (int it = 0; ok && it < n_iter; it++, un.next(sc)) {
+                if (it == 0 || un.tile == 0) {
+                    sg++;
+                    if (!spin_wait(kBXFull, sg & 1)) break;
                 }
-                const uint32_t da = dX + ((kFirstS >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY0 + slot * (LY::kYPlane >> 4);
-                mma_kmajor<LY::NB, LY::kXBlock, LY::kYBlock>(KS, tmem + kTmS + sb * BN, da, db, kIdesc, p > 0 ? 1u : 0u);
+                const int sb = it & 1, su = it >> 1;
+                if (!spin_wait(kBSEmpty + sb, (su & 1) ^ 1)) break;
+                int seen = 0;  // planes of this tile known to have arrived, in the order m, h, l
+    #pragma unroll 1
+                for (int p = 0; p < 6; p++) {
+                    const int k = slot_of_plane((kSecondS >> (2 * p)) & 3);
+                    const int slot = slot0 + k >= kYSlots ? slot0 + k - kYSlots : slot0 + k;
+                    if (k >= seen) {
+                        ok = spin_wait(kBYFull + slot, slot0 + k >= kYSlots ? ph0 ^ 1 : ph0);
+                        if (!ok) break;
+                        seen = k + 1;
+                        tc_fence_after();
+                    }
+                    const uint32_t da = dX + ((kFirstS >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY0 + slot * (LY::kYPlane >> 4);
+                    mma_kmajor<steps, LY::kXBlock, LY::kYBlock>(tmem + kTmS + sb * BN, da, db, kIdesc, p > 0 ? 1u : 0u);
+                }
+                if (!ok) break;
+                mma_commit_warp(&bars[kBSFull + sb]);
+                slot0 += kPlanes;
+                if (slot0 >= kYSlots) slot0 -= kYSlots, ph0 ^= 1;
             }
-            if (!ok) break;
-            mma_commit_warp(&bars[kBSFull + sb]);
-            slot0 += kPlanes;
-            if (slot0 >= kYSlots) slot0 -= kYSlots, ph0 ^= 1;
-        }
+        });
     } else if (warp == kGradWarpB) {
         // ---- dK^T [d x 64] = X^T W, then dQ [128 x D] of the tile = W Y ----
         const uint32_t kIdescDk = idesc_bf16(128, BN, 1, 1), kIdescDq = idesc_bf16(BM, KS * kMmaK, 0, 1);

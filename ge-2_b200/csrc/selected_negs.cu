@@ -742,26 +742,28 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
         uint32_t items = 0, tiles = 0;
         TourSegment sg;
         bool ok = true;
-        for (int64_t at = begin, next = 0; ok && tour_segment(a, at, end, sg, next); at = next, items++) {
-            ok = spin_wait(kTQFull, items & 1);
-            if (!ok) break;
-            for (int64_t n0 = sg.col; n0 < sg.col_end; n0 += kTourCols, tiles++) {
-                const int b = tiles & 1;
-                const uint32_t use = (tiles >> 1) & 1;
-                ok = spin_wait(kTYFull + b, use) && spin_wait(kTSEmpty + b, use ^ 1);
+        with_steps<NB>(KS, [&](auto steps) {
+            for (int64_t at = begin, next = 0; ok && tour_segment(a, at, end, sg, next); at = next, items++) {
+                ok = spin_wait(kTQFull, items & 1);
                 if (!ok) break;
-                tc_fence_after();
-#pragma unroll 1
-                for (int p = 0; p < 6; p++) {
-                    const uint32_t da = dQ + ((kFirst >> (2 * p)) & 3) * (SM::kQPlane >> 4),
-                                   db = dY0 + (b * kTourPlanes + ((kSecond >> (2 * p)) & 3)) * (SM::kYPlane >> 4);
-                    mma_kmajor<NB, SM::kQBlock, SM::kYBlock>(KS, tmem + b * kTourCols, da, db, kIdesc, p > 0 ? 1u : 0u);
+                for (int64_t n0 = sg.col; n0 < sg.col_end; n0 += kTourCols, tiles++) {
+                    const int b = tiles & 1;
+                    const uint32_t use = (tiles >> 1) & 1;
+                    ok = spin_wait(kTYFull + b, use) && spin_wait(kTSEmpty + b, use ^ 1);
+                    if (!ok) break;
+                    tc_fence_after();
+    #pragma unroll 1
+                    for (int p = 0; p < 6; p++) {
+                        const uint32_t da = dQ + ((kFirst >> (2 * p)) & 3) * (SM::kQPlane >> 4),
+                                       db = dY0 + (b * kTourPlanes + ((kSecond >> (2 * p)) & 3)) * (SM::kYPlane >> 4);
+                        mma_kmajor<steps, SM::kQBlock, SM::kYBlock>(tmem + b * kTourCols, da, db, kIdesc, p > 0 ? 1u : 0u);
+                    }
+                    mma_commit_warp(&bars[kTYEmpty + b]);
+                    if (n0 + kTourCols >= sg.col_end) mma_commit_warp(&bars[kTQEmpty]);
+                    mma_commit_warp(&bars[kTSFull + b]);  // last: whoever waits for it has seen the others' arrivals land before the CTA exits
                 }
-                mma_commit_warp(&bars[kTYEmpty + b]);
-                if (n0 + kTourCols >= sg.col_end) mma_commit_warp(&bars[kTQEmpty]);
-                mma_commit_warp(&bars[kTSFull + b]);  // last: whoever waits for it has seen the others' arrivals land before the CTA exits
             }
-        }
+        });
     } else if (warp < kTourEpi0 + 4) {
         // ---- winners: thread = row; columns in order, the running winner of the group in registers ----
         const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;

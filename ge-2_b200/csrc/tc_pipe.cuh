@@ -5,6 +5,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -90,26 +92,26 @@ __device__ __forceinline__ bool warp_wait_inline(uint64_t* bar, uint32_t parity,
 __device__ __forceinline__ void settle_bar(uint64_t* bar) { mbar_wait(bar, mbar_try_wait(bar, 0) ? 1u : 0u, 1u << 14); }
 
 // ---- contractions ---------------------------------------------------------------------------------------------------------
-// D (+)= A B^T over the first `steps` k-steps (1 ... 4 NB) of operands of NB 64-column blocks, both K-major.  The number of steps is made a
-// constant of straight-line code: with a test per step a contraction of N = 64 took 71 cycles to issue instead of 48.
+// D (+)= A B^T over the first STEPS k-steps (1 ... 4 NB) of operands of 64-column blocks, both K-major, in straight-line code.
 template <int STEPS, int A_BLOCK, int B_BLOCK>
-__device__ __forceinline__ void mma_kmajor_fixed(uint32_t acc, uint32_t da, uint32_t db, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_kmajor(uint32_t acc, uint32_t da, uint32_t db, uint32_t idesc, uint32_t accumulate) {
 #pragma unroll
     for (int ks = 0; ks < STEPS; ks++)
         mma_f16_ss_warp(acc, da + (((ks >> 2) * A_BLOCK + (ks & 3) * 32) >> 4), db + (((ks >> 2) * B_BLOCK + (ks & 3) * 32) >> 4), idesc,
                         ks > 0 ? 1u : accumulate);
 }
-template <int NB, int A_BLOCK, int B_BLOCK>
-__device__ __forceinline__ void mma_kmajor(int steps, uint32_t acc, uint32_t da, uint32_t db, uint32_t idesc, uint32_t accumulate) {
-    switch (steps) {
-        case 1: mma_kmajor_fixed<1, A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
-        case 2: mma_kmajor_fixed<2, A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
-        case 3: mma_kmajor_fixed<3, A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
-        case 4: mma_kmajor_fixed<4, A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
-        case 5: if (NB > 1) mma_kmajor_fixed<(NB > 1 ? 5 : 1), A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
-        case 6: if (NB > 1) mma_kmajor_fixed<(NB > 1 ? 6 : 1), A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
-        case 7: if (NB > 1) mma_kmajor_fixed<(NB > 1 ? 7 : 1), A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
-        default: if (NB > 1) mma_kmajor_fixed<(NB > 1 ? 8 : 1), A_BLOCK, B_BLOCK>(acc, da, db, idesc, accumulate); break;
+// Makes the number of k-steps of rows of NB 64-column blocks, 4 NB - 3 ... 4 NB, a constant of the body given, which holds the issuing warp's
+// whole loop.  The issue must not stop between contractions, for the tensor pipe has next to no queue: the six contractions of a three-plane
+// product (7 steps of N = 64 each) take 2016 cycles this way, the rate of the pipe, 2829 with a branch on the number of steps before each,
+// and 3600 where the other warps of the SM are busy too.
+template <int NB, class Body>
+__device__ __forceinline__ void with_steps(int steps, Body&& body) {
+    constexpr int kFull = 4 * (NB - 1);
+    switch (steps - kFull) {
+        case 1: body(std::integral_constant<int, kFull + 1>()); break;
+        case 2: body(std::integral_constant<int, kFull + 2>()); break;
+        case 3: body(std::integral_constant<int, kFull + 3>()); break;
+        default: body(std::integral_constant<int, kFull + 4>()); break;
     }
 }
 
