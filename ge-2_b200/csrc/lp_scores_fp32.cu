@@ -20,7 +20,7 @@
 // block is a K-major operand, along columns an MN-major one, so each serves both of its contractions.
 //
 // Bound by the contractions: 6 products a multiply-add, 4 contractions' worth of them (S twice, dQ, dK) = 24 x S B N D x 2 flops of bf16.
-// B = 10 000, 1 000 negatives, D = 100, two sides: 53 + 101 us (one kernel of fp32 multiply-adds: 776 us); 1 000 edges, D = 50: 13 + 21 us
+// B = 10 000, 1 000 negatives, D = 100, two sides: 36 + 86 us (one kernel of fp32 multiply-adds: 776 us); 1 000 edges, D = 50: 9.5 + 17.4 us
 // (202 us).  Relative 2-norm error against float64 at B = 4 000, N = 1 000, D = 100 (and that of the multiply-adds): node gradient 5.3e-7
 // (4.2e-7), scores 1.5e-7 (1.6e-7).
 #include <math.h>
@@ -202,7 +202,12 @@ __global__ void __launch_bounds__(kThreadsA, 1)
         const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
         float run_m = -INFINITY, run_l = 0.f;
         int sg = -1;
-        IterA un(ub, sc);
+        IterA un(ub, sc), ahead(ub, sc);
+        auto mask_word = [&](const IterA& u) {
+            const int n0 = u.tile * BN + half * 32;
+            return lane < d.N - n0 ? __ldg(&L.mask[(int64_t)u.zc * d.N + n0 + lane]) : -1;
+        };
+        int32_t word = n_iter > 0 ? mask_word(ahead) : -1;
         for (int it = 0; it < n_iter; it++, un.next(sc)) {
             const int s = un.zc / d.C, c = un.zc - s * d.C, row0 = un.rb * BM, valid_rows = min(BM, L.npc - row0);
             if (it == 0 || un.tile == 0) {
@@ -212,8 +217,9 @@ __global__ void __launch_bounds__(kThreadsA, 1)
             }
             const int n0 = un.tile * BN + half * 32, nv = min(32, d.N - n0);  // live columns among this warp's (may be <= 0)
             const int brow = c * L.npc + row0 + my_row;  // batch row in the padded numbering the filter uses
-            const int32_t word = lane < nv ? __ldg(&L.mask[(int64_t)un.zc * d.N + n0 + lane]) : -1;
             const uint32_t mb = mask_bits(word, brow - lane, brow);
+            ahead.next(sc);
+            word = it + 1 < n_iter ? mask_word(ahead) : -1;  // the next tile's, a trip to memory ahead of its use
             const int sb = it & 1;
             if (!warp_wait(kASFull + sb, (it >> 1) & 1)) break;
             tc_fence_after();
@@ -224,15 +230,23 @@ __global__ void __launch_bounds__(kThreadsA, 1)
             if (lane == 0) mbar_arrive(&bars[kASEmpty + sb]);
             if (nv > 0) {
                 float* dump = s == 0 ? d.neg_scores : d.inv_neg_scores;
-                float mx = -INFINITY;
+                if (__any_sync(0xffffffffu, mb != 0u)) {
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    v[j] = ((mb >> j) & 1u) ? kMasked : v[j];
-                    if (dump != nullptr && my_row < valid_rows && j < nv) dump[(int64_t)brow * d.N + n0 + j] = v[j];
-                    v[j] = j < nv ? v[j] : -INFINITY;
-                    mx = fmaxf(mx, v[j]);
+                    for (int j = 0; j < 32; j++) v[j] = ((mb >> j) & 1u) ? kMasked : v[j];
                 }
-                const float nm = fmaxf(run_m, mx);
+                if (dump != nullptr && my_row < valid_rows) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (j < nv) dump[(int64_t)brow * d.N + n0 + j] = v[j];
+                }
+                if (nv < 32) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) v[j] = j < nv ? v[j] : -INFINITY;
+                }
+                float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int j = 0; j < 32; j++) mx[j & 3] = fmaxf(mx[j & 3], v[j]);
+                const float nm = fmaxf(run_m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
                 float add[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int j = 0; j < 32; j++) add[j & 3] += expf(v[j] - nm);  // exp(-inf) = 0 for absent columns
@@ -407,7 +421,8 @@ __global__ void __launch_bounds__(kThreadsB, 1)
             }
         });
     } else if (warp == kGradWarpB) {
-        // ---- dK^T [d x 64] = X^T W, then dQ [128 x D] of the tile = W Y ----
+        // ---- dQ [128 x D] of the tile = W Y, then dK^T [d x 64] = X^T W ----
+        // dQ first: it gives the planes of Y back, and the one of the next tile that had no room in the ring arrives while dK^T is summed
         const uint32_t kIdescDk = idesc_bf16(128, BN, 1, 1), kIdescDq = idesc_bf16(BM, KS * kMmaK, 0, 1);
         // X along its columns: the second 64 of them lie a block further (for D <= 64 there are none, and what is read there ends up in
         // accumulator rows that nobody reads)
@@ -423,13 +438,6 @@ __global__ void __launch_bounds__(kThreadsB, 1)
             tc_fence_after();
 #pragma unroll 1
             for (int p = 0; p < 6; p++) {
-                const uint32_t da = dXm + ((kFirst >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dWm + ((kSecond >> (2 * p)) & 3) * (LY::kWPlane >> 4);
-#pragma unroll
-                for (int ks = 0; ks < BM / kMmaK; ks++)
-                    mma_f16_ss_warp(tmem + kTmDk + pb * BN, da + ks * (2048 >> 4), db + ks * (2048 >> 4), kIdescDk, (p > 0 || ks > 0) ? 1u : 0u);
-            }
-#pragma unroll 1
-            for (int p = 0; p < 6; p++) {
                 const int k = slot_of_plane((kSecondDq >> (2 * p)) & 3);
                 const int slot = slot0 + k >= kYSlots ? slot0 + k - kYSlots : slot0 + k;
                 const uint32_t da = dWk + ((kFirstDq >> (2 * p)) & 3) * (LY::kWPlane >> 4), db = dYm0 + slot * (LY::kYPlane >> 4);
@@ -437,6 +445,13 @@ __global__ void __launch_bounds__(kThreadsB, 1)
                 for (int ks = 0; ks < BN / kMmaK; ks++)
                     mma_f16_ss_warp(tmem + kTmDq + pb * 128, da + ks * (32 >> 4), db + ks * (2048 >> 4), kIdescDq, (p > 0 || ks > 0) ? 1u : 0u);
                 if (p == 1 || p == 2 || p == 5) mma_commit_warp(&bars[kBYEmpty + slot]);  // the last product with this plane of Y
+            }
+#pragma unroll 1
+            for (int p = 0; p < 6; p++) {
+                const uint32_t da = dXm + ((kFirst >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dWm + ((kSecond >> (2 * p)) & 3) * (LY::kWPlane >> 4);
+#pragma unroll
+                for (int ks = 0; ks < BM / kMmaK; ks++)
+                    mma_f16_ss_warp(tmem + kTmDk + pb * BN, da + ks * (2048 >> 4), db + ks * (2048 >> 4), kIdescDk, (p > 0 || ks > 0) ? 1u : 0u);
             }
             mma_commit_warp(&bars[kBWEmpty]);
             if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit_warp(&bars[kBXEmpty]);
@@ -449,7 +464,12 @@ __global__ void __launch_bounds__(kThreadsB, 1)
         const int half = warp >> 2, my_row = tid & 127;
         const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
         float lrow = kDeadRow;
-        IterA un(ub, sc);
+        IterA un(ub, sc), ahead(ub, sc);
+        auto mask_word = [&](const IterA& u) {
+            const int n0 = u.tile * BN + half * 32;
+            return lane < d.N - n0 ? __ldg(&L.mask[(int64_t)u.zc * d.N + n0 + lane]) : -1;
+        };
+        int32_t word = n_iter > 0 ? mask_word(ahead) : -1;
         for (int it = 0; it < n_iter; it++, un.next(sc)) {
             const int s = un.zc / d.C, c = un.zc - s * d.C, row0 = un.rb * BM;
             const int brow = c * L.npc + row0 + my_row;
@@ -491,9 +511,10 @@ __global__ void __launch_bounds__(kThreadsB, 1)
                     }
                 }
             }
-            const int n0 = un.tile * BN + half * 32, nv = min(32, d.N - n0);  // live columns among this warp's (may be <= 0)
-            const int32_t word = lane < nv ? __ldg(&L.mask[(int64_t)un.zc * d.N + n0 + lane]) : -1;
+            const int nv = min(32, d.N - un.tile * BN - half * 32);  // live columns among this warp's (may be <= 0)
             const uint32_t mb = mask_bits(word, brow - lane, brow);
+            ahead.next(sc);
+            word = it + 1 < n_iter ? mask_word(ahead) : -1;
             const int sb = it & 1;
             if (!warp_wait(kBSFull + sb, (it >> 1) & 1)) break;
             tc_fence_after();
@@ -503,10 +524,11 @@ __global__ void __launch_bounds__(kThreadsB, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars[kBSEmpty + sb]);
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                const float p = expf(v[j] - lrow);
-                // masked entries were overwritten in place by the reference: no gradient reaches them; columns past the chunk have none
-                v[j] = j < nv && !((mb >> j) & 1u) ? p : 0.f;
+            for (int j = 0; j < 32; j++) v[j] = expf(v[j] - lrow);
+            // masked entries were overwritten in place by the reference: no gradient reaches them; columns past the chunk have none
+            if (nv < 32 || __any_sync(0xffffffffu, mb != 0u)) {
+#pragma unroll
+                for (int j = 0; j < 32; j++) v[j] = j < nv && !((mb >> j) & 1u) ? v[j] : 0.f;
             }
             if (!warp_wait(kBWEmpty, (it & 1) ^ 1)) break;
             unsigned char* w0 = smem + LY::kW + my_row * 128;
