@@ -12,17 +12,24 @@
 // Exponentials and logarithms are CUDA's expf / logf.  Errors against float64 are about those of a kernel of fp32 multiply-adds: gradients a
 // quarter above, scores a little below (figures further down).
 //
-// Two persistent launches, as on the f16 path (lp_scores_f16.cu): a block X of 128 query rows stays in shared memory and tiles Y of 64
+// Two persistent launches, as on the f16 path (lp_scores_f16.cu): a block X of 128 query rows stays on the SM and tiles Y of 64
 // negatives stream past it,
 //   lp_lse32_kernel    S = X Y^T tile by tile, running (max, sum) per row                                             -> lse, loss
 //   lp_grad32_kernel   S again, P = exp(S - lse) split into W (three planes in shared memory), dQ += W Y, dK^T = X^T W
-// All operands sit in shared memory as planes of 64-column blocks in the 128-byte-swizzled layout that TMA writes; read along rows a
+// Operands sit in shared memory (X of the logsumexp pass: in tensor memory) as planes of 64-column blocks in the 128-byte-swizzled layout that TMA writes; read along rows a
 // block is a K-major operand, along columns an MN-major one, so each serves both of its contractions.
 //
-// Bound by the contractions: 6 products a multiply-add, 4 contractions' worth of them (S twice, dQ, dK) = 24 x S B N D x 2 flops of bf16.
-// B = 10 000, 1 000 negatives, D = 100, two sides: 36 + 86 us (one kernel of fp32 multiply-adds: 776 us); 1 000 edges, D = 50: 9.5 + 17.4 us
+// Bound by the contractions: 6 products a multiply-add, 4 contractions' worth of them (S twice, dQ, dK) = 24 x S B N D x 2 flops of bf16, at
+// N = 64 with both operands in shared memory limited by its bandwidth (48 cycles a k-step; A in tensor memory: 32).
+// B = 10 000, 1 000 negatives, D = 100, two sides: 31 + 86 us (one kernel of fp32 multiply-adds: 776 us); 1 000 edges, D = 50: 9.7 + 17.5 us
 // (202 us).  Relative 2-norm error against float64 at B = 4 000, N = 1 000, D = 100 (and that of the multiply-adds): node gradient 5.3e-7
 // (4.2e-7), scores 1.5e-7 (1.6e-7).
+// The logsumexp pass keeps X in tensor memory, and two warps issue a tile in turns: 31.0 us instead of 35.4 with X in shared memory and one warp (2950
+// cycles a tile, 2470 of them contractions, the rest that warp's waits and commits).  X straight from global memory into tensor memory: 38.3 us, a
+// row a lane reads 32 lines an instruction.
+// The gradient pass takes 7200 cycles a tile, 5760 of them contractions: S, softmax and W of the next tile wait for the last plane of Y, for which
+// the ring has no room before dQ.  Tried: one issuing warp and planes of Y loaded twice, so that S runs two tiles ahead (108 us); two warps and two
+// rings for the same (98 ... 100 us); W split before the wait for its buffer (90 us).
 #include <math.h>
 
 #include <algorithm>
@@ -39,7 +46,7 @@ constexpr int BM = 128, BN = 64;
 constexpr int kPlanes = 3;
 constexpr float kMasked = -1e9f;
 constexpr float kDeadRow = 1e30f;  // "lse" of a row past the end of its chunk: exp(anything - 1e30) = 0
-constexpr int kLseStages = 2;
+constexpr int kLseStages = 3;      // logsumexp pass: tiles of Y under way (its two issuing warps rely on there being no more)
 constexpr int kYSlots = 5;         // gradient pass: ring of Y planes; three belong to a tile, two are ahead
 
 // the six products, small ones first: plane of the first / second operand, two bits each
@@ -56,8 +63,11 @@ struct Layout32 {
     static constexpr int kXBlock = BM * 128, kYBlock = BN * 128;
     static constexpr int kXPlane = NB * kXBlock, kYPlane = NB * kYBlock, kWPlane = BM * 128;
     static constexpr int kX = 0, kY = kPlanes * kXPlane;
-    // logsumexp pass
-    static constexpr int kXch = kY + kLseStages * kPlanes * kYPlane;  // [2][128] (max, sum) of the right half of the columns
+    // logsumexp pass: X is in tensor memory
+    static constexpr int kXCols = NB * 32;                            // tensor-memory columns of a plane of X
+    static constexpr int kXHalves = NB == 1 ? 2 : 1;                  // buffers for the halves of X on their way there, each like a tile of Y
+    static constexpr int kXHalf = kLseStages * kPlanes * kYPlane;
+    static constexpr int kXch = kXHalf + kXHalves * kPlanes * kYPlane;  // [2][128] (max, sum) of the right half of the columns
     static constexpr int kMiscA = kXch + 2 * BM * 8;
     static constexpr int kBytesA = (kMiscA + 512 + 1024) > 120 * 1024 ? (kMiscA + 512 + 1024) : 120 * 1024;  // one CTA an SM
     // gradient pass
@@ -79,13 +89,36 @@ __device__ __forceinline__ uint32_t mask_bits(int32_t word, int wrow0, int brow)
     return mb;
 }
 
+// Three planes of 64 rows of X, staged like a tile of Y -> tensor memory, for one warp: lane = row, two consecutive elements a column
+template <int DP>
+__device__ __forceinline__ void x_to_tmem(uint32_t taddr, const unsigned char* stage, int row) {
+    using LY = Layout32<DP>;
+#pragma unroll 1
+    for (int p = 0; p < kPlanes; p++) {
+#pragma unroll
+        for (int c = 0; c < LY::kXCols; c += 16) {
+            const unsigned char* src = stage + p * LY::kYPlane + (c / 32) * LY::kYBlock + row * 128;
+            uint32_t r[16];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint4 q = *reinterpret_cast<const uint4*>(src + ((((c % 32) / 4 + k) ^ (row & 7)) << 4));
+                r[4 * k] = q.x, r[4 * k + 1] = q.y, r[4 * k + 2] = q.z, r[4 * k + 3] = q.w;
+            }
+            tmem_st_32x16_start(taddr + p * LY::kXCols + c, r);
+        }
+    }
+    tmem_st_wait();
+}
+
 // =====================================================================================================================
 // launch 1: row logsumexp
 // =====================================================================================================================
 constexpr int kSoftWarps = 8;                                    // 4 row quarters x 2 halves of 32 columns
-constexpr int kTmaWarpA = 8, kMmaWarpA = 9, kClearWarpA = 10, kClearWarps = 3, kThreadsA = 416;
-enum BarA { kAXFull = 0, kAXEmpty, kAYFull, kAYEmpty = kAYFull + kLseStages, kASFull = kAYEmpty + kLseStages, kASEmpty = kASFull + 2, kAXch = kASEmpty + 2,
+constexpr int kTmaWarpA = 8, kMmaWarpA = 9, kLoadWarpA = 11, kLoadWarps = 4, kThreadsA = 480;  // two MMA warps
+enum BarA { kAXIn = 0, kAXOut = kAXIn + 2, kAXFull = kAXOut + 2, kAXEmpty = kAXFull + 2, kAYFull = kAXEmpty + 2, kAYEmpty = kAYFull + kLseStages, kASFull = kAYEmpty + kLseStages, kASEmpty = kASFull + 2, kAXch = kASEmpty + 2,
             kAXchFree = kAXch + 2, kNumBarsA = kAXchFree + 2 };
+// tensor memory: scores at 0 and 64, X of two blocks
+constexpr uint32_t kTmXa = 128;
 
 template <int DP>
 __global__ void __launch_bounds__(kThreadsA, 1)
@@ -106,13 +139,15 @@ __global__ void __launch_bounds__(kThreadsA, 1)
     auto warp_wait = [&](int bar, uint32_t parity) { return warp_pipe_wait(&bars[bar], parity, s_abort, d.status); };
 
     if (warp == kTmaWarpA && lane == 0) {
-        mbar_init(&bars[kAXFull], 1);
-        mbar_init(&bars[kAXEmpty], 1);
         for (int k = 0; k < kLseStages; k++) {
             mbar_init(&bars[kAYFull + k], 1);
             mbar_init(&bars[kAYEmpty + k], 1);
         }
         for (int k = 0; k < 2; k++) {
+            mbar_init(&bars[kAXIn + k], 1);
+            mbar_init(&bars[kAXOut + k], kLoadWarps / 2);
+            mbar_init(&bars[kAXFull + k], kLoadWarps);
+            mbar_init(&bars[kAXEmpty + k], 2);
             mbar_init(&bars[kASFull + k], 1);
             mbar_init(&bars[kASEmpty + k], kSoftWarps);
             mbar_init(&bars[kAXch + k], kSoftWarps / 2);
@@ -124,7 +159,7 @@ __global__ void __launch_bounds__(kThreadsA, 1)
         prefetch_tensormap(&tmK);
     }
     if (warp == kMmaWarpA) {
-        tmem_alloc(s_tmem, 128);
+        tmem_alloc(s_tmem, 512);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -134,67 +169,100 @@ __global__ void __launch_bounds__(kThreadsA, 1)
     const uint32_t tmem = *s_tmem;
 
     if (warp == kTmaWarpA) {
+        bool ok = true;
         int sg = -1;
-        IterA un(ub, sc);
-        for (int it = 0; it < n_iter; it++, un.next(sc)) {
-            if (it == 0 || un.tile == 0) {
-                sg++;
-                if (!spin_wait(kAXEmpty, (sg & 1) ^ 1)) break;
-                mbar_expect_tx_warp(&bars[kAXFull], kPlanes * LY::kXPlane);
-                for (int p = 0; p < kPlanes; p++)
-                    for (int b = 0; b < LY::NB; b++)
-                        tma_load_3d_warp(smem + LY::kX + p * LY::kXPlane + b * LY::kXBlock, &tmQ, b * 64, un.rb * BM, p * sc.ZC + un.zc, &bars[kAXFull]);
-            }
-            const int st = it % kLseStages, use = it / kLseStages;
-            if (!spin_wait(kAYEmpty + st, (use & 1) ^ 1)) break;
-            mbar_expect_tx_warp(&bars[kAYFull + st], kPlanes * LY::kYPlane);
+        auto load = [&](const CUtensorMap& map, int row, int zc, int at, int full) {
+            mbar_expect_tx_warp(&bars[full], kPlanes * LY::kYPlane);
             for (int p = 0; p < kPlanes; p++)
-                for (int b = 0; b < LY::NB; b++)
-                    tma_load_3d_warp(smem + LY::kY + (st * kPlanes + p) * LY::kYPlane + b * LY::kYBlock, &tmK, b * 64, un.tile * BN, p * sc.ZC + un.zc,
-                                     &bars[kAYFull + st]);
+                for (int b = 0; b < LY::NB; b++) tma_load_3d_warp(smem + at + p * LY::kYPlane + b * LY::kYBlock, &map, b * 64, row, p * sc.ZC + zc, &bars[full]);
+        };
+        IterA un(ub, sc);
+        for (int it = 0; ok && it < n_iter; it++, un.next(sc)) {
+            const bool fresh = it == 0 || un.tile == 0;
+            auto second_half = [&] { load(tmQ, un.rb * BM + BM / 2, un.zc, LY::kXHalf + (LY::kXHalves - 1) * kPlanes * LY::kYPlane, kAXIn + 1); };
+            if (fresh) {
+                sg++;
+                ok = spin_wait(kAXOut, (sg & 1) ^ 1) && spin_wait(kAXOut + 1, (sg & 1) ^ 1);
+                if (!ok) break;
+                load(tmQ, un.rb * BM, un.zc, LY::kXHalf, kAXIn);
+                if (LY::kXHalves == 2) second_half();
+            }
+            const int st = it % kLseStages;
+            ok = spin_wait(kAYEmpty + st, ((it / kLseStages) & 1) ^ 1);
+            if (!ok) break;
+            load(tmK, un.tile * BN, un.zc, st * kPlanes * LY::kYPlane, kAYFull + st);
+            if (fresh && LY::kXHalves == 1) {
+                ok = spin_wait(kAXOut, sg & 1);
+                if (!ok) break;
+                second_half();
+            }
         }
-    } else if (warp == kMmaWarpA) {
+    } else if (warp < kLoadWarpA && warp >= kMmaWarpA) {
+        // two warps, a tile in turns: the pipe has the other's contractions while one waits
         constexpr uint32_t kIdesc = idesc_bf16(BM, BN, 0, 0);
-        const uint32_t dX = desc_lo_sw128(smem_u32(smem + LY::kX), 16), dY0 = desc_lo_sw128(smem_u32(smem + LY::kY), 16);
-        const int KS = (d.D + kMmaK - 1) / kMmaK;
+        const uint32_t dY0 = desc_lo_sw128(smem_u32(smem), 16);
+        const int KS = (d.D + kMmaK - 1) / kMmaK, sb = warp - kMmaWarpA;
         int sg = -1;
         IterA un(ub, sc);
         with_steps<LY::NB>(KS, [&](auto steps) {
             for (int it = 0; it < n_iter; it++, un.next(sc)) {
                 if (it == 0 || un.tile == 0) {
+                    if (sg >= 0) mma_commit_warp(&bars[kAXEmpty + (sg & 1)]);
                     sg++;
-                    if (!spin_wait(kAXFull, sg & 1)) break;
+                    // by both warps, also by one that has no tile in the block: it then gives back no X that has not come
+                    if (!spin_wait(kAXFull + (sg & 1), (sg >> 1) & 1)) break;
                 }
-                const int st = it % kLseStages, use = it / kLseStages, sb = it & 1, su = it >> 1;
-                if (!spin_wait(kAYFull + st, use & 1)) break;
-                if (!spin_wait(kASEmpty + sb, (su & 1) ^ 1)) break;
+                if ((it & 1) != sb) continue;
+                const int st = it % kLseStages, xb = sg & 1;
+                // The scores first: with those of tile it - 2 read, those of it - 3 are, so that the last use of this stage, the other warp's, lies
+                // behind, and the phase waited for is the next one of its barrier.
+                if (!spin_wait(kASEmpty + sb, ((it >> 1) & 1) ^ 1)) break;
+                if (!spin_wait(kAYFull + st, (it / kLseStages) & 1)) break;
                 tc_fence_after();
-                const uint32_t dY = dY0 + st * (kPlanes * LY::kYPlane >> 4);
-    #pragma unroll 1
-                for (int p = 0; p < 6; p++) {
-                    const uint32_t da = dX + ((kFirst >> (2 * p)) & 3) * (LY::kXPlane >> 4), db = dY + ((kSecond >> (2 * p)) & 3) * (LY::kYPlane >> 4);
-                    mma_kmajor<steps, LY::kXBlock, LY::kYBlock>(tmem + sb * BN, da, db, kIdesc, p > 0 ? 1u : 0u);
-                }
+                const uint32_t dY = dY0 + st * (kPlanes * LY::kYPlane >> 4), tX = tmem + kTmXa + xb * (kPlanes * LY::kXCols);
+#pragma unroll 1
+                for (int p = 0; p < 6; p++)
+                    mma_ts_kmajor<steps, LY::kYBlock>(tmem + sb * BN, tX + ((kFirst >> (2 * p)) & 3) * LY::kXCols,
+                                                      dY + ((kSecond >> (2 * p)) & 3) * (LY::kYPlane >> 4), kIdesc, p > 0 ? 1u : 0u);
                 mma_commit_warp(&bars[kAYEmpty + st]);
-                if (it == n_iter - 1 || un.tile == sc.T - 1) mma_commit_warp(&bars[kAXEmpty]);
-                mma_commit_warp(&bars[kASFull + sb]);  // last: whoever waits for it has seen the others' arrivals land before the CTA exits
+                mma_commit_warp(&bars[kASFull + sb]);
             }
         });
-    } else if (warp >= kClearWarpA) {
-        // clear what the gradient pass will add to: dK, and the dQ rows of every block whose stream that pass cuts at a CTA boundary
-        const int wz = (warp - kClearWarpA) * 32 + lane;
-        const int64_t n4 = (int64_t)sc.ZC * d.N * (DP / 4);
-        const int64_t z0 = n4 * blockIdx.x / gridDim.x, z1 = n4 * (blockIdx.x + 1) / gridDim.x;
-        float4* p4 = reinterpret_cast<float4*>(L.dK);
-        for (int64_t k = z0 + wz; k < z1; k += kClearWarps * 32) p4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int j = 1 + (int)blockIdx.x; j < sc.gridB; j += (int)gridDim.x) {
-            const int u = range_begin(j, sc.unitsB, sc.gridB);
-            if (u <= 0 || u >= sc.unitsB) continue;
-            const UnitA un = decode_a(u, sc);
-            if (un.tile == 0) continue;  // the boundary falls between two blocks: nothing is split
-            float4* q4 = reinterpret_cast<float4*>(L.dQ + ((int64_t)un.zc * L.npc + (int64_t)un.rb * BM) * DP);
-            const int n = min(BM, L.npc - un.rb * BM) * (DP / 4);
-            for (int k = wz; k < n; k += kClearWarps * 32) q4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        // the last arrivals of the pipe on a block's barrier land before the CTA exits; those on the others come before scores that are waited for
+        if (sg > 0) spin_wait(kAXEmpty + ((sg - 1) & 1), ((sg - 1) >> 1) & 1);
+    } else if (warp >= kLoadWarpA) {
+        // X of every block, a block ahead of the contractions: each pair of warps moves the half that holds its quarters of the lanes
+        const int quarter = warp & 3, half = quarter >> 1;
+        const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
+        for (int sg = 0, at = ub; at < ue; sg++) {
+            const int xb = sg & 1;
+            if (!warp_wait(kAXEmpty + xb, ((sg >> 1) & 1) ^ 1)) break;
+            if (!warp_wait(kAXIn + half, sg & 1)) break;
+            tc_fence_after();
+            x_to_tmem<DP>(tmem + kTmXa + xb * (kPlanes * LY::kXCols) + lane_sel, smem + LY::kXHalf + half * (LY::kXHalves - 1) * kPlanes * LY::kYPlane, (quarter & 1) * 32 + lane);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&bars[kAXFull + xb]);
+                mbar_arrive(&bars[kAXOut + half]);
+            }
+            at += sc.T - at % sc.T;
+            if (sg > 0) continue;
+            // clear what the gradient pass will add to: dK, and the dQ rows of every block whose stream that pass cuts at a CTA boundary
+            const int wz = (warp - kLoadWarpA) * 32 + lane;
+            const int64_t n4 = (int64_t)sc.ZC * d.N * (DP / 4);
+            const int64_t z0 = n4 * blockIdx.x / gridDim.x, z1 = n4 * (blockIdx.x + 1) / gridDim.x;
+            float4* p4 = reinterpret_cast<float4*>(L.dK);
+            for (int64_t k = z0 + wz; k < z1; k += kLoadWarps * 32) p4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j = 1 + (int)blockIdx.x; j < sc.gridB; j += (int)gridDim.x) {
+                const int u = range_begin(j, sc.unitsB, sc.gridB);
+                if (u <= 0 || u >= sc.unitsB) continue;
+                const UnitA un = decode_a(u, sc);
+                if (un.tile == 0) continue;  // the boundary falls between two blocks: nothing is split
+                float4* q4 = reinterpret_cast<float4*>(L.dQ + ((int64_t)un.zc * L.npc + (int64_t)un.rb * BM) * DP);
+                const int n = min(BM, L.npc - un.rb * BM) * (DP / 4);
+                for (int k = wz; k < n; k += kLoadWarps * 32) q4[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
     } else {
         // ---- softmax warps: warp w takes rows 32 (w & 3) ... + 31 and columns 32 (w >> 2) ... + 31 of every tile ----
@@ -295,11 +363,13 @@ __global__ void __launch_bounds__(kThreadsA, 1)
     tc_fence_before();
     __syncthreads();
     if (warp == kMmaWarpA) {
-        if (*s_abort && lane == 0)  // copies still in flight get a bounded chance to land
+        if (*s_abort && lane == 0) {  // copies still in flight get a bounded chance to land
+            for (int k = 0; k < 2; k++) settle_bar(&bars[kAXIn + k]);
             for (int k = 0; k < kLseStages; k++) settle_bar(&bars[kAYFull + k]);
+        }
         __syncwarp();
         tc_fence_after();
-        tmem_dealloc(tmem, 128);
+        tmem_dealloc(tmem, 512);
     }
 }
 
@@ -626,8 +696,10 @@ template <int DP>
 int launch(const LpKernelArgs& a, cudaStream_t stream) {
     using LY = Layout32<DP>;
     const int ZC = a.L.S * a.d.C;
-    CUtensorMap tmQ, tmK;
+    CUtensorMap tmQ, tmQHalf, tmK;
     int rc = make_operand_map(&tmQ, a.L.Qs, true, DP, a.L.npc, (int64_t)kPlanes * ZC, BM);
+    if (rc != GE2_OK) return rc;
+    rc = make_operand_map(&tmQHalf, a.L.Qs, true, DP, a.L.npc, (int64_t)kPlanes * ZC, BM / 2);
     if (rc != GE2_OK) return rc;
     rc = make_operand_map(&tmK, a.L.Ks, true, DP, a.d.N, (int64_t)kPlanes * ZC, BN);
     if (rc != GE2_OK) return rc;
@@ -644,7 +716,7 @@ int launch(const LpKernelArgs& a, cudaStream_t stream) {
     // per-device function attributes; setting them on every launch keeps multi-device processes correct and is not a stream operation
     GE2_CUDA_TRY(cudaFuncSetAttribute(lp_lse32_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::kBytesA));
     GE2_CUDA_TRY(cudaFuncSetAttribute(lp_grad32_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::kBytesB));
-    GE2_CUDA_TRY(launch_after(lp_lse32_kernel<DP>, dim3((unsigned)sc.gridA), dim3(kThreadsA), LY::kBytesA, stream, tmQ, tmK, a, sc));
+    GE2_CUDA_TRY(launch_after(lp_lse32_kernel<DP>, dim3((unsigned)sc.gridA), dim3(kThreadsA), LY::kBytesA, stream, tmQHalf, tmK, a, sc));
     GE2_CUDA_TRY(launch_after(lp_grad32_kernel<DP>, dim3((unsigned)sc.gridB), dim3(kThreadsB), LY::kBytesB, stream, tmQ, tmK, a, sc));
     return GE2_OK;
 }

@@ -100,6 +100,14 @@ __device__ __forceinline__ void mma_kmajor(uint32_t acc, uint32_t da, uint32_t d
         mma_f16_ss_warp(acc, da + (((ks >> 2) * A_BLOCK + (ks & 3) * 32) >> 4), db + (((ks >> 2) * B_BLOCK + (ks & 3) * 32) >> 4), idesc,
                         ks > 0 ? 1u : accumulate);
 }
+// The same with A in tensor memory: two elements a column, 8 columns a k-step.  A is not read from shared memory then, which is what bounds a
+// contraction of N = 64 (48 cycles a k-step with A there, 32 this way).
+template <int STEPS, int B_BLOCK>
+__device__ __forceinline__ void mma_ts_kmajor(uint32_t acc, uint32_t ta, uint32_t db, uint32_t idesc, uint32_t accumulate) {
+#pragma unroll
+    for (int ks = 0; ks < STEPS; ks++)
+        mma_f16_ts_warp(acc, ta + ks * 8, db + (((ks >> 2) * B_BLOCK + (ks & 3) * 32) >> 4), idesc, ks > 0 ? 1u : accumulate);
+}
 // Makes the number of k-steps of rows of NB 64-column blocks, 4 NB - 3 ... 4 NB, a constant of the body given, which holds the issuing warp's
 // whole loop.  The issue must not stop between contractions, for the tensor pipe has next to no queue: the six contractions of a three-plane
 // product (7 steps of N = 64 each) take 2016 cycles this way, the rate of the pipe, 2829 with a branch on the number of steps before each,

@@ -224,6 +224,21 @@ def test_split_operand_tiles_at_their_edges(capi, cuda_device, kind, B, C, N, D)
         assert rel_err(got[key], exp[key]) <= 5e-6, key
 
 
+@pytest.mark.parametrize("kind,B,C,N,D", [
+    ("DISTMULT", 38400, 300, 40, 50),    # a tile a block, four blocks a CTA: every block brings its own rows, and one issuing warp has none of some
+    ("COMPLEX", 38400, 300, 40, 100),    # the same with two 64-column blocks a row, the halves of the rows through one buffer
+    ("DISTMULT", 51300, 300, 100, 128),  # two tiles a block, blocks of 128 and of 43 rows
+    ("COMPLEX", 25000, 125, 150, 66),    # three tiles a block: as many as are under way
+])
+def test_short_blocks_of_the_split_operand_scores(capi, cuda_device, kind, B, C, N, D):
+    """Many short blocks a CTA, so that rows, tiles and scores of several are under way at once; twice, for what one pass leaves to the next."""
+    case = workloads.make_case(kind, B, C, N, D, 20, 5000, 0, seed=B + N + D, relations=True, inverse=True, alpha=1.1)
+    o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
+    for _ in range(2):
+        res = run_lp_step(capi, case, cuda_device, "fp32", "pairs", dump_scores=False)
+        check_against(res, dict(loss=o.loss, node_grad=o.node_grad, rel_grad=o.rel_grad, inv_rel_grad=o.inv_rel_grad), TOL["fp32"], 2)
+
+
 @pytest.mark.parametrize("kind,B,C,N,D", [("DISTMULT", 130, 1, 66001, 128), ("COMPLEX", 210, 70, 1000, 66), ("DISTMULT", 300, 2, 70001, 50), ("COMPLEX", 1290, 10, 7003, 100)])
 def test_streaming_softmax_tiles_at_their_edges(capi, cuda_device, kind, B, C, N, D):
     """The fp16 path with a dK that does not stay in the L2 (which of its forms a shape gets: lp_uses_flash; the streaming one at sizes of its
