@@ -587,15 +587,20 @@ int launch_pair_columns(const PairArgs& a, const PairCut& p, bool vec, const flo
 //
 // A CTA keeps a tile of query rows and takes a contiguous share of all (chunk, row tile, group) triples, so every SM is busy to the end and a
 // share begins and ends on a group boundary.  Warps by role: 8 warps convert rows (fp32, read along the row) into one of two tile
-// buffers, one issues the contractions, 4 epilogue warps walk the scores: a thread owns a row, keeps the running winner of the group
-// in registers and writes it where the group ends.  Groups of less than eight end so often that their winners are put aside first, and 17 ... 32
-// of the warp's 32 rows leave together, a row at a time (groups of one, 33 000 x 1000 winners: 591 us written one by one, each to a sector
-// of its own, 178 us together; groups of ten are faster one by one).  Groups need not fit tiles.
-// Bound by the contractions (6 ceil(D / 16) steps of 48 cycles a tile at best, 92 beside the conversion's shared-memory stores) and the
-// one epilogue warp a scheduler.  50 000 rows x 1 000 negatives, D = 100, 100 kept: 122 us (405 us as fp32 multiply-adds).
+// buffers, one issues the contractions, 8 epilogue warps in two sets walk the scores: a thread owns a row, keeps the running winner of a
+// group in registers and writes it where the group ends.  The sets take the groups in turns and read a part of one at a time, at most 16 columns
+// from wherever it begins, so that a column costs a compare, a select and a maximum (50 000 rows x 1 000 negatives, D = 100: groups of 10 in 102 us, of
+// 1 000 in 86; 118 and
+// 121 with one set that walked all columns and asked at each whether a group ends there; one set taking all groups by parts: 110 for groups of 10).
+// Groups of less than five end so often that a part each, and a write of each winner to a sector of its own, costs more than that walk:
+// there one set asks at every column, winners are put aside, and 17 ... 32 of the warp's 32 rows leave together, a row at a time (us, this way
+// and by parts: groups of two 205 and 448, of three 176 and 299, of four 162 and 199, of five 152 and 141, of seven 136 and 117).
+// Groups need not fit tiles.
+// Bound by the contractions (6 ceil(D / 16) steps of 48 cycles a tile at best, 78 beside the conversion's shared-memory stores) and, with short groups, the
+// writes of the winners.  As fp32 multiply-adds: 405 us.
 using namespace tc;
 constexpr int kTourRows = 128, kTourCols = 64, kTourPlanes = 3;
-constexpr int kTourThreads = 512, kTourEpi0 = 0, kTourMma = 4, kTourConv0 = 8, kTourConvWarps = 8;
+constexpr int kTourEpiWarps = 8, kTourMma = kTourEpiWarps, kTourConv0 = kTourMma + 1, kTourConvWarps = 8, kTourThreads = (kTourConv0 + kTourConvWarps) * 32;
 
 struct TourArgs {
     const float* chunked;    // [chunks, R, D]
@@ -676,7 +681,7 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
             mbar_init(&bars[kTYFull + k], kTourConvWarps);
             mbar_init(&bars[kTYEmpty + k], 1);
             mbar_init(&bars[kTSFull + k], 1);
-            mbar_init(&bars[kTSEmpty + k], 4);
+            mbar_init(&bars[kTSEmpty + k], STAGED ? 4 : kTourEpiWarps);
         }
         *s_abort = 0;
         mbar_init_fence();
@@ -764,19 +769,73 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
                 }
             }
         });
-    } else if (warp < kTourEpi0 + 4) {
+    } else if (warp < (STAGED ? 4 : kTourEpiWarps)) {
         // ---- winners: thread = row; columns in order, the running winner of the group in registers ----
-        const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;
-        float* const st_s = reinterpret_cast<float*>(smem + SM::kStage) + warp * (32 * 33 * 2);
-        int* const st_c = reinterpret_cast<int*>(st_s) + 32 * 33;
+        const int quarter = warp & 3, set = warp >> 2;
+        const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
         uint32_t tiles = 0;
         TourSegment sg;
         bool ok = true;
         for (int64_t at = begin, next = 0; ok && tour_segment(a, at, end, sg, next); at = next) {
-            const int rows = (int)(a.R - sg.row0 - warp * 32 < 32 ? a.R - sg.row0 - warp * 32 : 32);  // of this warp
-            const int64_t first = (sg.chunk * a.R + sg.row0 + warp * 32) * a.K + sg.group;
-            float* out_s = a.out_scores + first + lane * a.K;
-            int64_t* out_i = a.out_idx + first + lane * a.K;
+            const int rows = (int)(a.R - sg.row0 - quarter * 32 < 32 ? a.R - sg.row0 - quarter * 32 : 32);  // of this warp
+            const int64_t first = (sg.chunk * a.R + sg.row0 + quarter * 32) * a.K + sg.group;
+            const int T = (int)a.T;
+            int todo = (int)((sg.col_end - sg.col) / a.T);  // groups of this segment still to be written; columns are counted from its first
+            float best = -CUDART_INF_F;
+            int best_c = 0;
+            if (!STAGED) {
+                // Two sets of four warps take the groups in turns, a part of one at a time, 16 columns at most; a part that ends the tile is read
+                // with the columns before it, which lie in the tile.
+                float* out_s = a.out_scores + first + lane * a.K + set;
+                int64_t* out_i = a.out_idx + first + lane * a.K + set;
+                int g_begin = set < todo ? set * T : INT_MAX, g_end = set < todo ? g_begin + T : INT_MAX;
+                best_c = g_begin;
+                todo -= set;
+                for (int64_t n0 = sg.col; n0 < sg.col_end; n0 += kTourCols, tiles++) {
+                    const int b = tiles & 1, rel = (int)(n0 - sg.col), cols = (int)(sg.col_end - n0 < kTourCols ? sg.col_end - n0 : kTourCols);
+                    ok = warp_wait(kTSFull + b, (tiles >> 1) & 1);
+                    if (!ok) break;
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = max(g_begin - rel, 0); c < cols;) {
+                        const int c0 = min(c, kTourCols - 16), stop = min(min(cols, g_end - rel), c0 + 16);
+                        float v[16];
+                        tmem_ld_32x16(tmem + b * kTourCols + c0 + lane_sel, v);
+                        if (stop - c < 16) {
+#pragma unroll
+                            for (int j = 0; j < 16; j++) v[j] = j >= c - c0 && j < stop - c0 ? v[j] : -CUDART_INF_F;
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; j++) {
+                            best_c = v[j] > best ? rel + c0 + j : best_c;  // the first of equal scores wins, a NaN never
+                            best = fmaxf(best, v[j]);
+                        }
+                        c = stop;
+                        if (rel + c == g_end) {
+                            if (lane < rows) {
+                                *out_s = best;
+                                *out_i = sg.col + best_c;
+                            }
+                            out_s += 2;
+                            out_i += 2;
+                            todo -= 2;
+                            g_begin = todo > 0 ? g_end + T : INT_MAX;
+                            g_end = todo > 0 ? g_begin + T : INT_MAX;
+                            best = -CUDART_INF_F;
+                            best_c = g_begin;
+                            c = g_begin - rel;
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars[kTSEmpty + b]);
+                }
+                continue;
+            }
+            // groups of a few columns: straight-line and predicated, since with one warp a scheduler a branch per column leaves it waiting for
+            // latencies (81 cycles a column)
+            float* const st_s = reinterpret_cast<float*>(smem + SM::kStage) + warp * (32 * 33 * 2);
+            int* const st_c = reinterpret_cast<int*>(st_s) + 32 * 33;
             int cnt = 0, done = 0;  // winners put aside, and written
             auto flush = [&]() {
                 __syncwarp();
@@ -791,10 +850,7 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
                 done += cnt;
                 cnt = 0;
             };
-            const int T = (int)a.T;
-            int todo = (int)((sg.col_end - sg.col) / a.T);  // groups of this segment still to be written; columns are counted from its first
-            float best = -CUDART_INF_F;
-            int best_c = 0, left = T;  // left: columns from the current position to the end of the group
+            int left = T;  // columns from the current position to the end of the group
             for (int64_t n0 = sg.col; n0 < sg.col_end; n0 += kTourCols, tiles++) {
                 const int b = tiles & 1;
                 ok = warp_wait(kTSFull + b, (tiles >> 1) & 1);
@@ -810,38 +866,27 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
                         if (lane == 0) mbar_arrive(&bars[kTSEmpty + b]);
                     }
                     const int col0 = (int)(n0 - sg.col) + k;
-                    // straight-line and predicated: with one warp a scheduler a branch per column, or a winner that is updated through a
-                    // compare, leaves it waiting for latencies (81 cycles a column)
 #pragma unroll
                     for (int j = 0; j < 16; j++) {
-                        best_c = v[j] > best ? col0 + j : best_c;  // the first of equal scores wins, a NaN never
+                        best_c = v[j] > best ? col0 + j : best_c;
                         best = fmaxf(best, v[j]);
-                        const bool end = left == j + 1;            // the same for all threads
+                        const bool end = left == j + 1;  // the same for all threads
                         const bool put = end && todo > 0;
-                        if (STAGED) {
-                            if (put) {
-                                st_s[lane * 33 + cnt] = best;
-                                st_c[lane * 33 + cnt] = best_c;
-                            }
-                            cnt += put ? 1 : 0;
-                        } else {
-                            if (put && lane < rows) {
-                                *out_s = best;
-                                *out_i = sg.col + best_c;
-                            }
-                            out_s += end ? 1 : 0;
-                            out_i += end ? 1 : 0;
+                        if (put) {
+                            st_s[lane * 33 + cnt] = best;
+                            st_c[lane * 33 + cnt] = best_c;
                         }
+                        cnt += put ? 1 : 0;
                         todo -= end ? 1 : 0;
                         best = end ? -CUDART_INF_F : best;
                         best_c = end ? col0 + j + 1 : best_c;
                         left += end ? T : 0;
                     }
                     left -= 16;
-                    if (STAGED && cnt > 16) flush();
+                    if (cnt > 16) flush();
                 }
             }
-            if (STAGED && ok) flush();
+            if (ok) flush();
         }
     }
     // ---- common exit ----
@@ -856,7 +901,7 @@ __global__ void __launch_bounds__(kTourThreads, 1) tournament_kernel(const __gri
 template <int NB, int VEC>
 int launch_tournament(const TourArgs& a, cudaStream_t stream) {
     // per-device function attribute; setting it on every call keeps multi-device processes correct and is not a stream operation
-    auto kernel = a.T < 8 ? tournament_kernel<NB, VEC, true> : tournament_kernel<NB, VEC, false>;
+    auto kernel = a.T < 5 ? tournament_kernel<NB, VEC, true> : tournament_kernel<NB, VEC, false>;
     GE2_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TourSmem<NB>::kBytes));
     kernel<<<(unsigned)std::min<int64_t>(kNumSMs, a.shares_total), kTourThreads, TourSmem<NB>::kBytes, stream>>>(a);
     GE2_LAUNCH_CHECK();

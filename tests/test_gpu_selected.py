@@ -206,3 +206,28 @@ def test_tournament_at_tile_edges_and_on_ties(capi, cuda_device, C, R, N, D, K):
     _check_tournament(scores, idx, q, n, K)
     if K == 1 and N > 1:
         assert int(idx.max()) < N // 2
+
+
+@pytest.mark.parametrize("T,K", [(5, 31), (8, 33), (9, 1), (15, 40), (16, 12), (17, 9), (48, 3), (49, 7), (63, 2), (64, 5), (65, 4), (127, 3), (500, 1)])
+def test_tournament_groups_read_in_parts(capi, cuda_device, T, K):
+    """Groups whose parts begin and end at every place of a tile, one or an odd number of them in a share; scores that are NaN never win, and a
+    group without any other has the value of nothing at its first column, on the path of the short groups (a group of four here) as well."""
+    C, R, D = 3, 140, 20
+    for T, K in ((T, K), (4, T)):
+        N = T * K
+        rng = np.random.default_rng(T * 1000 + K)
+        q = rng.standard_normal((C, R, D)).astype(np.float32)
+        n = rng.standard_normal((C, N, D)).astype(np.float32)
+        n[:, N // 2:] = n[:, :N - N // 2]
+        scores, idx = capi.tournament_select(torch.from_numpy(q).to(cuda_device), torch.from_numpy(n).to(cuda_device), K)
+        _check_tournament(scores, idx, q, n, K)
+        n[:, ::3] = np.nan
+        n[1, :T] = np.nan
+        scores, idx = (x.cpu().numpy().reshape(C, R, K) for x in capi.tournament_select(torch.from_numpy(q).to(cuda_device), torch.from_numpy(n).to(cuda_device), K))
+        assert np.isneginf(scores[1, :, 0]).all() and (idx[1, :, 0] == 0).all()
+        exact = np.einsum("crd,cnd->crn", q.astype(np.float64), n.astype(np.float64)).reshape(C, R, K, T)
+        live = ~np.isnan(exact).all(-1)
+        at = np.take_along_axis(exact.reshape(C, R, N), idx, 2)
+        best = np.fmax.reduce(exact, -1)
+        assert (idx // T == np.arange(K)).all() and np.abs(at - best)[live].max() < 1e-5 * np.abs(best[live]).max()  # fp32 sums of 20 products
+        assert np.abs(scores - at)[live].max() < 1e-5 * np.abs(best[live]).max()
