@@ -123,17 +123,16 @@ __global__ void __launch_bounds__(256) index_rows_kernel(float* __restrict__ tab
 // row_shared only the rows it names are touched (the others were finished where their gradient arose), and those that
 // are not cost one load.
 template <int V>
-__global__ void __launch_bounds__(256) adagrad_scatter_kernel(float* __restrict__ table, float* __restrict__ state, int64_t table_rows,
-                                                              const int64_t* __restrict__ unique_ids, int64_t U, const int32_t* U_dev,
-                                                              float* __restrict__ node_grad, int vec_per_row, int lg, float neg_lr, int clear_grad,
-                                                              const uint8_t* __restrict__ row_shared, int32_t* status) {
+__device__ __forceinline__ void adagrad_rows(int64_t block, int64_t blocks, float* __restrict__ table, float* __restrict__ state, int64_t table_rows,
+                                             const int64_t* __restrict__ unique_ids, int64_t U, const int32_t* U_dev, float* __restrict__ node_grad,
+                                             int vec_per_row, int lg, float neg_lr, int clear_grad, const uint8_t* __restrict__ row_shared,
+                                             int32_t* status) {
     using VT = typename Vec<V>::type;
     constexpr int kRows = 2;
-    griddep_wait();  // the gradient rows come from the kernel before this one
     const int64_t rows = live_rows(U, U_dev);
-    const int64_t groups = ((int64_t)gridDim.x * blockDim.x) >> lg;
+    const int64_t groups = (blocks * blockDim.x) >> lg;
     const int l = threadIdx.x & ((1 << lg) - 1);
-    for (int64_t r0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> lg) * kRows; r0 < rows; r0 += groups * kRows) {
+    for (int64_t r0 = ((block * blockDim.x + threadIdx.x) >> lg) * kRows; r0 < rows; r0 += groups * kRows) {
         int64_t row[kRows];
         bool on[kRows];
 #pragma unroll
@@ -176,13 +175,21 @@ __global__ void __launch_bounds__(256) adagrad_scatter_kernel(float* __restrict_
 }
 
 template <int V>
-__global__ void __launch_bounds__(256) dense_adagrad_kernel(float* __restrict__ param, float* __restrict__ sum, float* __restrict__ grad,
-                                                            int64_t vecs, float neg_lr, float eps, float grad_scale, int clear_grad) {
+__global__ void __launch_bounds__(256) adagrad_scatter_kernel(float* __restrict__ table, float* __restrict__ state, int64_t table_rows,
+                                                              const int64_t* __restrict__ unique_ids, int64_t U, const int32_t* U_dev,
+                                                              float* __restrict__ node_grad, int vec_per_row, int lg, float neg_lr, int clear_grad,
+                                                              const uint8_t* __restrict__ row_shared, int32_t* status) {
+    griddep_wait();  // the gradient rows come from the kernel before this one
+    adagrad_rows<V>(blockIdx.x, gridDim.x, table, state, table_rows, unique_ids, U, U_dev, node_grad, vec_per_row, lg, neg_lr, clear_grad, row_shared, status);
+}
+
+template <int V>
+__device__ __forceinline__ void adagrad_dense(int64_t block, int64_t blocks, float* __restrict__ param, float* __restrict__ sum, float* __restrict__ grad,
+                                              int64_t vecs, float neg_lr, float eps, float grad_scale, int clear_grad) {
     using VT = typename Vec<V>::type;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    griddep_wait();
+    const int64_t stride = blocks * blockDim.x;
 #pragma unroll 1
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += stride) {
+    for (int64_t i = block * blockDim.x + threadIdx.x; i < vecs; i += stride) {
         float g[V], s[V], p[V];
         to_arr<V>(reinterpret_cast<const VT*>(grad)[i], g);
         to_arr<V>(reinterpret_cast<const VT*>(sum)[i], s);
@@ -198,6 +205,35 @@ __global__ void __launch_bounds__(256) dense_adagrad_kernel(float* __restrict__ 
         reinterpret_cast<VT*>(sum)[i] = from_arr<V>(s);
         reinterpret_cast<VT*>(param)[i] = from_arr<V>(p);
         if (clear_grad) reinterpret_cast<VT*>(grad)[i] = from_arr<V>(g);
+    }
+}
+
+template <int V>
+__global__ void __launch_bounds__(256) dense_adagrad_kernel(float* __restrict__ param, float* __restrict__ sum, float* __restrict__ grad,
+                                                            int64_t vecs, float neg_lr, float eps, float grad_scale, int clear_grad) {
+    griddep_wait();
+    adagrad_dense<V>(blockIdx.x, gridDim.x, param, sum, grad, vecs, neg_lr, eps, grad_scale, clear_grad);
+}
+
+// Both in one launch, for a step whose launches follow one another: the first blocks take the dense tables, the others the rows.  Two launches
+// fewer of 3 us each, side by side on most SMs, where the tables are two (steps of 1 000 and 7 919 edges: 59.3 -> 57.7 and 68.9 -> 67.2 us).
+struct DenseTables {
+    float *param[2], *sum[2], *grad[2];
+};
+template <int V, int VD>
+__global__ void __launch_bounds__(256) adagrad_step_kernel(float* __restrict__ table, float* __restrict__ state, int64_t table_rows,
+                                                           const int64_t* __restrict__ unique_ids, int64_t U, const int32_t* U_dev,
+                                                           float* __restrict__ node_grad, int vec_per_row, int lg, float neg_lr,
+                                                           const uint8_t* __restrict__ row_shared, int32_t* status, const DenseTables dense, int blocks_each,
+                                                           int num_dense, int64_t vecs, float neg_dense_lr, float eps, float grad_scale) {
+    griddep_wait();  // the gradients come from the kernel before this one
+    const int first = blocks_each * num_dense, b = blockIdx.x;
+    if (b < first) {
+        const int k = b >= blocks_each ? 1 : 0;
+        adagrad_dense<VD>(b - k * blocks_each, blocks_each, k ? dense.param[1] : dense.param[0], k ? dense.sum[1] : dense.sum[0], k ? dense.grad[1] : dense.grad[0],
+                          vecs, neg_dense_lr, eps, grad_scale, 1);
+    } else {
+        adagrad_rows<V>(b - first, (int)gridDim.x - first, table, state, table_rows, unique_ids, U, U_dev, node_grad, vec_per_row, lg, neg_lr, 1, row_shared, status);
     }
 }
 
@@ -677,6 +713,21 @@ extern "C" int ge2_copy_slabs(const float* src, float* dst, const int32_t* moves
     return GE2_OK;
 }
 
+namespace {
+template <int V, int VD>
+int launch_adagrad_step(const ge2_train_desc& t, const DenseTables& dense, cudaStream_t stream) {
+    const ge2_lp_desc& d = *t.lp;
+    const int vpr = d.D / V;
+    int lg = 0;
+    while (lg < 5 && (1 << lg) < vpr) lg++;
+    const int64_t vecs = t.dense_numel / VD;
+    const int each = stream_grid(vecs, 256), rows = stream_grid(ceil_div<int64_t>(d.U, 2) << lg, 256);
+    GE2_CUDA_TRY(launch_after(adagrad_step_kernel<V, VD>, dim3((unsigned)(each * t.num_dense + rows)), dim3(256), 0, stream, t.table, t.state, t.table_rows, t.unique,
+                              d.U, t.count, d.node_grad, vpr, lg, -t.lr, t.shared, d.status, dense, each, t.num_dense, vecs, -t.dense_lr, 1e-10f, t.grad_scale));
+    return GE2_OK;
+}
+}  // namespace
+
 extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
     // everything is looked at before the first launch: a call that is refused has changed nothing
     if (t == nullptr || t->lp == nullptr) return GE2_ERR_INVALID_ARGUMENT;
@@ -724,6 +775,19 @@ extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
     if (rc != GE2_OK) return rc;
     rc = ge2_lp_step(&d, stream);
     if (rc != GE2_OK) return rc;
+    if (t->num_dense > 0 && t->dense_numel > 0 && d.U > 0 && t->unique != nullptr && d.node_grad != nullptr) {
+        const int V = vec_width(d.D, t->table, t->state, d.node_grad);
+        DenseTables dense = {};
+        uintptr_t bits = (uintptr_t)(t->dense_numel % 4) * 4;
+        for (int k = 0; k < t->num_dense; k++) {
+            dense.param[k] = t->dense_param[k], dense.sum[k] = t->dense_state[k], dense.grad[k] = t->dense_grad[k];
+            bits |= (uintptr_t)t->dense_param[k] | (uintptr_t)t->dense_state[k] | (uintptr_t)t->dense_grad[k];
+        }
+        const bool wide = (bits & 15) == 0;
+        return V == 4 ? wide ? launch_adagrad_step<4, 4>(*t, dense, as_stream(stream)) : launch_adagrad_step<4, 1>(*t, dense, as_stream(stream))
+               : V == 2 ? wide ? launch_adagrad_step<2, 4>(*t, dense, as_stream(stream)) : launch_adagrad_step<2, 1>(*t, dense, as_stream(stream))
+                        : wide ? launch_adagrad_step<1, 4>(*t, dense, as_stream(stream)) : launch_adagrad_step<1, 1>(*t, dense, as_stream(stream));
+    }
     rc = ge2_adagrad_scatter_shared(t->table, t->state, t->table_rows, t->unique, d.U, t->count, d.node_grad, d.D, t->lr, 1, t->shared, d.status, stream);
     for (int k = 0; rc == GE2_OK && k < t->num_dense; k++)
         rc = ge2_dense_adagrad(t->dense_param[k], t->dense_state[k], t->dense_grad[k], t->dense_numel, t->dense_lr, 1e-10f, t->grad_scale, 1, stream);

@@ -283,8 +283,8 @@ GE2_API int ge2_sample_batch(const int64_t *edges, int32_t cols, int64_t num_bat
                              int32_t N, int32_t n_deg, int64_t domain, int32_t want_src_negs, uint64_t seed, int64_t *out_packed_ids,
                              int64_t *out_deg_rows, int64_t *out_rel_ids, ge2_stream_t stream);
 /* One training step in one call: ge2_sample_unique (or, for twins that are not the sampler's, ge2_sample_negatives and
- * ge2_unique_bitmap_shared), ge2_lp_step, ge2_adagrad_scatter_shared and
- * ge2_dense_adagrad (num_dense <= 2 parameters of dense_numel floats each) with the same arguments, issued from native code.  n_ids is what
+ * ge2_unique_bitmap_shared), ge2_lp_step, and what ge2_adagrad_scatter_shared and
+ * ge2_dense_adagrad do (num_dense <= 2 parameters of dense_numel floats each; in one launch) with the same arguments, issued from native code.  n_ids is what
  * the sampler packs, 2 B + sides C N; ids in [table_rows, domain) are flagged like ids outside the domain.  With the row update in lp
  * (node_state), the members that name the same thing must agree: shared = row_shared, lr = node_lr, table = node_emb, state = node_state,
  * table_rows, unique = row_index, and rows are dense (emb_stride = D); without it shared is NULL.  Anything else is
