@@ -27,7 +27,7 @@ EXPORTS = [
     "ge2_eval_workspace_bytes", "ge2_eval_ranks", "ge2_selected_neg_scores", "ge2_selected_neg_scores_backward",
     "ge2_tournament_select", "ge2_unique_bitmap_shared", "ge2_adagrad_scatter_shared", "ge2_train_step",
     "ge2_selected_neg_backward_workspace_bytes", "ge2_selected_neg_scores_backward_ws",
-    "ge2_sample_unique", "ge2_lp_idle_sms",
+    "ge2_sample_unique", "ge2_lp_idle_sms", "ge2_adagrad_step",
 ]
 
 
@@ -127,6 +127,8 @@ def load_library():
     lib.ge2_dense_adagrad.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_float, C.c_float, C.c_int32, C.c_void_p]
     lib.ge2_dense_adagrad_peers.argtypes = [C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p), C.c_int32, C.c_int32, C.c_int64, C.c_void_p, C.c_float,
                                             C.c_float, C.c_float, C.c_uint32, C.c_void_p, C.c_void_p]
+    lib.ge2_adagrad_step.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int32, C.c_float, C.c_void_p,
+                                     C.c_void_p, C.c_int32] + [C.POINTER(C.c_void_p)] * 3 + [C.c_int64, C.c_float, C.c_float, C.c_float, C.c_void_p]
     lib.ge2_lp_idle_sms.argtypes = [C.POINTER(LpDesc), C.POINTER(C.c_int32)]
     lib.ge2_sample_unique.argtypes = [C.POINTER(FrontDesc), C.c_void_p]
     lib.ge2_enable_peer_access.argtypes = [C.c_int32]
@@ -319,6 +321,16 @@ def adagrad_scatter(table, state, unique_ids, node_grad, lr: float, U=None, U_de
     U = unique_ids.numel() if U is None else U
     check(load_library().ge2_adagrad_scatter_shared(ptr(table), ptr(state), table.shape[0], ptr(unique_ids), U, ptr(U_dev), ptr(node_grad), D, lr,
                                                     1 if clear_grad else 0, ptr(row_shared), ptr(status), cur_stream()), "ge2_adagrad_scatter")
+
+
+def adagrad_step(table, state, unique_ids, node_grad, lr: float, dense, dense_lr: float, U=None, U_dev=None, status=None, row_shared=None, eps: float = 1e-10,
+                 grad_scale: float = 1.0):
+    """adagrad_scatter and dense_adagrad of the (parameter, state, gradient) triples in `dense`, at most two of one size, in one launch; every
+    gradient is cleared."""
+    U = unique_ids.numel() if U is None else U
+    columns = [(C.c_void_p * 2)(*(ptr(x) for x in col)) for col in zip(*dense)]
+    check(load_library().ge2_adagrad_step(ptr(table), ptr(state), table.shape[0], ptr(unique_ids), U, ptr(U_dev), ptr(node_grad), table.shape[1], lr, ptr(row_shared),
+                                          ptr(status), len(dense), *columns, dense[0][0].numel(), dense_lr, eps, grad_scale, cur_stream()), "ge2_adagrad_step")
 
 
 def dense_adagrad(param, sum_state, grad, lr: float, eps: float = 1e-10, grad_scale: float = 1.0, clear_grad=False):

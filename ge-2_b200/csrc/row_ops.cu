@@ -216,7 +216,8 @@ __global__ void __launch_bounds__(256) dense_adagrad_kernel(float* __restrict__ 
 }
 
 // Both in one launch, for a step whose launches follow one another: the first blocks take the dense tables, the others the rows.  Two launches
-// fewer of 3 us each, side by side on most SMs, where the tables are two (steps of 1 000 and 7 919 edges: 59.3 -> 57.7 and 68.9 -> 67.2 us).
+// fewer of 3 us each, where the tables are two (steps of 1 000 and 7 919 edges issued launch by launch: 59.3 -> 57.7 and 68.9 -> 67.2 us; in a graph, without the fork
+// that put them beside each other, 10 000 edges: 82.6 -> 81.9).
 struct DenseTables {
     float *param[2], *sum[2], *grad[2];
 };
@@ -714,19 +715,58 @@ extern "C" int ge2_copy_slabs(const float* src, float* dst, const int32_t* moves
 }
 
 namespace {
+struct RowUpdate {
+    float *table, *state;
+    int64_t table_rows;
+    const int64_t* unique;
+    int64_t U;
+    const int32_t* U_dev;
+    float* grad;
+    int D;
+    float lr;
+    const uint8_t* shared;
+    int32_t* status;
+};
 template <int V, int VD>
-int launch_adagrad_step(const ge2_train_desc& t, const DenseTables& dense, cudaStream_t stream) {
-    const ge2_lp_desc& d = *t.lp;
-    const int vpr = d.D / V;
+int launch_adagrad_step(const RowUpdate& r, const DenseTables& dense, int num_dense, int64_t numel, float dense_lr, float eps, float grad_scale, cudaStream_t stream) {
+    const int vpr = r.D / V;
     int lg = 0;
     while (lg < 5 && (1 << lg) < vpr) lg++;
-    const int64_t vecs = t.dense_numel / VD;
-    const int each = stream_grid(vecs, 256), rows = stream_grid(ceil_div<int64_t>(d.U, 2) << lg, 256);
-    GE2_CUDA_TRY(launch_after(adagrad_step_kernel<V, VD>, dim3((unsigned)(each * t.num_dense + rows)), dim3(256), 0, stream, t.table, t.state, t.table_rows, t.unique,
-                              d.U, t.count, d.node_grad, vpr, lg, -t.lr, t.shared, d.status, dense, each, t.num_dense, vecs, -t.dense_lr, 1e-10f, t.grad_scale));
+    const int64_t vecs = numel / VD;
+    const int each = stream_grid(vecs, 256), rows = stream_grid(ceil_div<int64_t>(r.U, 2) << lg, 256);
+    GE2_CUDA_TRY(launch_after(adagrad_step_kernel<V, VD>, dim3((unsigned)(each * num_dense + rows)), dim3(256), 0, stream, r.table, r.state, r.table_rows, r.unique, r.U,
+                              r.U_dev, r.grad, vpr, lg, -r.lr, r.shared, r.status, dense, each, num_dense, vecs, -dense_lr, eps, grad_scale));
     return GE2_OK;
 }
 }  // namespace
+
+extern "C" int ge2_adagrad_step(float* table, float* state, int64_t table_rows, const int64_t* unique_ids, int64_t U, const int32_t* U_dev, float* node_grad,
+                                int32_t D, float lr, const uint8_t* row_shared, int32_t* status, int32_t num_dense, float* const* dense_param,
+                                float* const* dense_state, float* const* dense_grad, int64_t dense_numel, float dense_lr, float eps, float grad_scale,
+                                ge2_stream_t stream) {
+    if (U < 0 || D <= 0 || table_rows < 0 || num_dense < 0 || num_dense > 2 || dense_numel < 0) return GE2_ERR_INVALID_ARGUMENT;
+    if (U > 0 && (table == nullptr || state == nullptr || unique_ids == nullptr || node_grad == nullptr)) return GE2_ERR_INVALID_ARGUMENT;
+    if (dense_numel == 0) num_dense = 0;
+    DenseTables dense = {};
+    uintptr_t bits = (uintptr_t)(dense_numel % 4) * 4;
+    for (int k = 0; k < num_dense; k++) {
+        if (dense_param == nullptr || dense_state == nullptr || dense_grad == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+        dense.param[k] = dense_param[k], dense.sum[k] = dense_state[k], dense.grad[k] = dense_grad[k];
+        if (dense.param[k] == nullptr || dense.sum[k] == nullptr || dense.grad[k] == nullptr) return GE2_ERR_INVALID_ARGUMENT;
+        bits |= (uintptr_t)dense_param[k] | (uintptr_t)dense_state[k] | (uintptr_t)dense_grad[k];
+    }
+    if (num_dense > 0 && U > 0) {
+        const RowUpdate r = {table, state, table_rows, unique_ids, U, U_dev, node_grad, D, lr, row_shared, status};
+        const int V = vec_width(D, table, state, node_grad);
+        auto go = [&](auto kernel) { return kernel(r, dense, num_dense, dense_numel, dense_lr, eps, grad_scale, as_stream(stream)); };
+        if ((bits & 15) == 0) return V == 4 ? go(launch_adagrad_step<4, 4>) : V == 2 ? go(launch_adagrad_step<2, 4>) : go(launch_adagrad_step<1, 4>);
+        return V == 4 ? go(launch_adagrad_step<4, 1>) : V == 2 ? go(launch_adagrad_step<2, 1>) : go(launch_adagrad_step<1, 1>);
+    }
+    int rc = ge2_adagrad_scatter_shared(table, state, table_rows, unique_ids, U, U_dev, node_grad, D, lr, 1, row_shared, status, stream);
+    for (int k = 0; rc == GE2_OK && k < num_dense; k++)
+        rc = ge2_dense_adagrad(dense.param[k], dense.sum[k], dense.grad[k], dense_numel, dense_lr, eps, grad_scale, 1, stream);
+    return rc;
+}
 
 extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
     // everything is looked at before the first launch: a call that is refused has changed nothing
@@ -775,21 +815,6 @@ extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
     if (rc != GE2_OK) return rc;
     rc = ge2_lp_step(&d, stream);
     if (rc != GE2_OK) return rc;
-    if (t->num_dense > 0 && t->dense_numel > 0 && d.U > 0 && t->unique != nullptr && d.node_grad != nullptr) {
-        const int V = vec_width(d.D, t->table, t->state, d.node_grad);
-        DenseTables dense = {};
-        uintptr_t bits = (uintptr_t)(t->dense_numel % 4) * 4;
-        for (int k = 0; k < t->num_dense; k++) {
-            dense.param[k] = t->dense_param[k], dense.sum[k] = t->dense_state[k], dense.grad[k] = t->dense_grad[k];
-            bits |= (uintptr_t)t->dense_param[k] | (uintptr_t)t->dense_state[k] | (uintptr_t)t->dense_grad[k];
-        }
-        const bool wide = (bits & 15) == 0;
-        return V == 4 ? wide ? launch_adagrad_step<4, 4>(*t, dense, as_stream(stream)) : launch_adagrad_step<4, 1>(*t, dense, as_stream(stream))
-               : V == 2 ? wide ? launch_adagrad_step<2, 4>(*t, dense, as_stream(stream)) : launch_adagrad_step<2, 1>(*t, dense, as_stream(stream))
-                        : wide ? launch_adagrad_step<1, 4>(*t, dense, as_stream(stream)) : launch_adagrad_step<1, 1>(*t, dense, as_stream(stream));
-    }
-    rc = ge2_adagrad_scatter_shared(t->table, t->state, t->table_rows, t->unique, d.U, t->count, d.node_grad, d.D, t->lr, 1, t->shared, d.status, stream);
-    for (int k = 0; rc == GE2_OK && k < t->num_dense; k++)
-        rc = ge2_dense_adagrad(t->dense_param[k], t->dense_state[k], t->dense_grad[k], t->dense_numel, t->dense_lr, 1e-10f, t->grad_scale, 1, stream);
-    return rc;
+    return ge2_adagrad_step(t->table, t->state, t->table_rows, t->unique, d.U, t->count, d.node_grad, d.D, t->lr, t->shared, d.status, t->num_dense, t->dense_param,
+                            t->dense_state, t->dense_grad, t->dense_numel, t->dense_lr, 1e-10f, t->grad_scale, stream);
 }

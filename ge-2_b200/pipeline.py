@@ -328,8 +328,19 @@ class BatchPipeline:
         return a.elapsed_time(b) / reps
 
     def _update(self, ids: Optional[_IdSet] = None):
-        self._update_nodes(ids)
-        self._update_relations()
+        cfg = self.cfg
+        if not cfg.has_relations or self.peer is not None:
+            self._update_nodes(ids)
+            self._update_relations()
+            return
+        ids = ids or self.ids[0]
+        if cfg.sides == 2 and self._rel_tables_adjacent:
+            # relation and inverse-relation tables (and their states) sit back to back, as the gradients do: one table
+            dense = [(self._rel_both, self._rel_state_both, self.rel_grads)]
+        else:
+            dense = [(self.rel, self.rel_state, self.rel_grad)] + ([(self.inv_rel, self.inv_rel_state, self.inv_rel_grad)] if cfg.sides == 2 else [])
+        capi.adagrad_step(self.table, self.state, ids.unique, self.node_grad, cfg.lr, dense, cfg.lr if cfg.dense_lr is None else cfg.dense_lr, U=self.cap,
+                          U_dev=ids.count, status=self.status, row_shared=ids.shared, grad_scale=self.grad_scale)
 
     def _update_nodes(self, ids: Optional[_IdSet] = None):
         cfg = self.cfg
@@ -505,13 +516,16 @@ class BatchPipeline:
                         self._backward(desc)
                         main.wait_stream(side)
                     if rel_hook is None:
-                        # the two optimizer updates touch different tables: the dense one (with its wait for the other ranks'
-                        # gradients in the multi-GPU form) runs beside the sparse scatter
-                        side2.wait_stream(main)
-                        with torch.cuda.stream(side2):
-                            self._update_relations()
-                        self._update_nodes(cur)
-                        main.wait_stream(side2)
+                        if self.peer is None:
+                            self._update(cur)
+                        else:
+                            # the two optimizer updates touch different tables: the dense one, with its wait for the other ranks' gradients,
+                            # runs beside the sparse scatter
+                            side2.wait_stream(main)
+                            with torch.cuda.stream(side2):
+                                self._update_relations()
+                            self._update_nodes(cur)
+                            main.wait_stream(side2)
                         main.wait_stream(side)
                         if self.peer is not None:
                             capi.advance_step(self.step_dev, 2)
@@ -563,8 +577,8 @@ class BatchPipeline:
         n += 1                                 # prepare (gather + relation operator + positive scores + filter words)
         n += 2                                 # scores: logsumexp pass + gradient pass, or both passes of the streaming form
         n += 1                                 # finish (operator backward + scatter)
-        n += 1                                 # sparse Adagrad scatter
-        if cfg.has_relations:
+        n += 1                                 # Adagrad: the rows, and without peers the relation tables
+        if cfg.has_relations and self.peer is not None:
             n += 1 if (cfg.sides == 1 or self._rel_tables_adjacent) else 2
         return n + (1 if resident and self.peer is not None else 0)  # counters that the exchange between ranks still reads
 

@@ -46,7 +46,7 @@ typedef void *ge2_stream_t; /* cudaStream_t */
 
 /* "ge2_b200 <major>.<minor> (...)".  0.2: ge2_lp_desc grew by the members behind GE2_LP_HAS_ROW_UPDATE; ge2_train_step,
  * ge2_unique_bitmap_shared, ge2_adagrad_scatter_shared and the selected-negative backward with scratch are new.  A descriptor laid
- * out as in 0.1 (without that flag) is still understood.  0.3: ge2_sample_unique and ge2_lp_idle_sms are new. */
+ * out as in 0.1 (without that flag) is still understood.  0.3: ge2_sample_unique, ge2_lp_idle_sms and ge2_adagrad_step are new. */
 GE2_API const char *ge2_version(void);
 GE2_API int ge2_last_cuda_error(void);            /* cudaError_t of the last failing runtime call on this thread */
 GE2_API const char *ge2_status_string(int status);
@@ -282,9 +282,15 @@ GE2_API int ge2_sample_negatives(const int64_t *src_ids, const int64_t *dst_ids,
 GE2_API int ge2_sample_batch(const int64_t *edges, int32_t cols, int64_t num_batches, const uint64_t *step_dev, int32_t B, int32_t C,
                              int32_t N, int32_t n_deg, int64_t domain, int32_t want_src_negs, uint64_t seed, int64_t *out_packed_ids,
                              int64_t *out_deg_rows, int64_t *out_rel_ids, ge2_stream_t stream);
+/* ge2_adagrad_scatter_shared and ge2_dense_adagrad of num_dense <= 2 tables (dense_numel floats each), both with clear_grad, in one launch. */
+GE2_API int ge2_adagrad_step(float *table, float *state, int64_t table_rows, const int64_t *unique_ids, int64_t U, const int32_t *U_dev, float *node_grad,
+                             int32_t D, float lr, const uint8_t *row_shared, int32_t *status, int32_t num_dense, float *const *dense_param,
+                             float *const *dense_state, float *const *dense_grad, int64_t dense_numel, float dense_lr, float eps, float grad_scale,
+                             ge2_stream_t stream);
+
 /* One training step in one call: ge2_sample_unique (or, for twins that are not the sampler's, ge2_sample_negatives and
- * ge2_unique_bitmap_shared), ge2_lp_step, and what ge2_adagrad_scatter_shared and
- * ge2_dense_adagrad do (num_dense <= 2 parameters of dense_numel floats each; in one launch) with the same arguments, issued from native code.  n_ids is what
+ * ge2_unique_bitmap_shared), ge2_lp_step and
+ * ge2_adagrad_step with the same arguments, issued from native code.  n_ids is what
  * the sampler packs, 2 B + sides C N; ids in [table_rows, domain) are flagged like ids outside the domain.  With the row update in lp
  * (node_state), the members that name the same thing must agree: shared = row_shared, lr = node_lr, table = node_emb, state = node_state,
  * table_rows, unique = row_index, and rows are dense (emb_stride = D); without it shared is NULL.  Anything else is

@@ -259,32 +259,3 @@ def test_timing_a_phase_trains_nothing(ge2, cuda_device):
     for t, old in zip(kept, before):
         assert torch.equal(t, old)
     pipe.check_status()
-
-
-@pytest.mark.parametrize("decoder,D,R,adjacent", [("DISTMULT", 25, 3, False), ("DISTMULT", 50, 7, True), ("COMPLEX", 50, 8, False), ("DISTMULT", 64, 2, True), ("COMPLEX", 100, 900, False),
-                                                  ("DISTMULT", 128, 40_000, True)])
-def test_one_optimizer_launch_does_what_several_do(ge2, cuda_device, decoder, D, R, adjacent):
-    """A step in one call updates rows and relation tables in one launch, a step with a hook between backward pass and optimizer in several: from
-    the same state, on widths of every access and tables of one block and of many, they leave the same tables (up to the order in which the
-    gradients were added)."""
-    from importlib import import_module
-
-    pl, B, C, N, nodes = import_module("ge-2_b200.pipeline"), 300, 3, 40, 2000
-    g = torch.Generator(device=cuda_device)
-    left = []
-    for hook in (None, lambda *a: None):
-        g.manual_seed(D + R)
-        new = lambda *s: torch.randn(s, device=cuda_device, generator=g) * 0.3  # noqa: E731
-        table, state = new(nodes, D), new(nodes, D).abs() + 0.01
-        both, both_s = new(2, R, D), new(2, R, D).abs() + 0.01
-        cut = (lambda x: (x[0], x[1])) if adjacent else (lambda x: (x[0].clone(), x[1].clone()))
-        (rel, inv), (rel_s, inv_s) = cut(both), cut(both_s)
-        pipe = pl.BatchPipeline(pl.PipelineConfig(decoder, B, C, N, 0.5, D, R, nodes, precision="fp32"), table, state, rel, rel_s, inv, inv_s)
-        col = lambda hi: torch.randint(0, hi, (B,), device=cuda_device, generator=g)  # noqa: E731
-        for t in range(2):
-            pipe.step(torch.stack([col(nodes), col(R), col(nodes)], 1).contiguous(), t, rel_hook=hook)
-        pipe.check_status()
-        left.append([x.double() for x in (table, state, rel, rel_s, inv, inv_s)])
-    for a, b in zip(*left):
-        # fp32 sums of at most 300 terms in another order; a step of Adagrad passes a relative error of its gradient on
-        assert float((a - b).abs().max()) <= 300 * 2 ** -23 * max(1.0, float(b.abs().max()))

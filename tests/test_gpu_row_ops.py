@@ -246,3 +246,50 @@ def test_peer_wait_runs_out_and_leaves_everything_untouched(capi, cuda_device):
     capi.dense_adagrad_peers(t_p, t_s, [b.data_ptr() for b in bufs], 0, numel, step, 0.1, status, grad_scale=0.5, wait_budget_us=5000)
     torch.cuda.synchronize()
     assert int(status) == 0 and not np.array_equal(t_p.cpu().numpy(), p)
+
+
+@pytest.mark.parametrize("D,numel,tables,offset", [(25, 75, 2, 0), (50, 350, 2, 0), (50, 352, 2, 0), (6, 1, 1, 0), (64, 128, 1, 1), (100, 90_000, 2, 0), (128, 5_120_000, 1, 0), (100, 0, 2, 0),
+                                                   (100, 400, 0, 0)])
+@pytest.mark.parametrize("U", [0, 1, 777, 60_001])
+def test_rows_and_dense_tables_in_one_launch(capi, cuda_device, D, numel, tables, offset, U):
+    """The same bits as the two operators one after the other: every width of access, tables of one block and of many, tables that do not lie on
+    16 bytes, neither rows nor tables, and the count in device memory below U."""
+    g = torch.Generator(device=cuda_device)
+    left = []
+    for one in (True, False):
+        g.manual_seed(D + numel + U)
+        rnd = lambda *s: torch.randn(s, device=cuda_device, generator=g)  # noqa: E731
+        table, state, grad = rnd(70_000, D), rnd(70_000, D).abs(), rnd(max(U, 1), D)
+        ids = torch.randperm(70_000, device=cuda_device, generator=g)[:max(U, 1)].contiguous()
+        shared = (rnd(max(U, 1)) > 0).to(torch.uint8)
+        live, status = torch.tensor([U - U // 5, 0], dtype=torch.int32, device=cuda_device), torch.zeros(1, dtype=torch.int32, device=cuda_device)
+        dense = [tuple(x[offset:] for x in (rnd(numel + offset), rnd(numel + offset).abs(), rnd(numel + offset))) for _ in range(tables)]
+        if one and tables:
+            capi.adagrad_step(table, state, ids, grad, 0.1, dense, 0.05, U=U, U_dev=live, status=status, row_shared=shared, grad_scale=0.5)
+        else:
+            capi.adagrad_scatter(table, state, ids, grad, 0.1, U=U, U_dev=live, clear_grad=True, status=status, row_shared=shared)
+            for d in dense:
+                capi.dense_adagrad(*d, 0.05, grad_scale=0.5, clear_grad=True)
+        torch.cuda.synchronize()
+        assert int(status) == 0
+        left.append([table, state, grad, *(x for d in dense for x in d)])
+    assert all(torch.equal(a, b) for a, b in zip(*left))
+    if U > 1000 and tables and numel:
+        assert not bool(left[0][3 + 2].any()) and bool(left[0][2].any())  # the tables' gradients are cleared, those of rows not named are not
+
+
+def test_rows_and_dense_tables_refuse_what_does_not_fit(capi, cuda_device):
+    import ctypes
+
+    t = torch.ones(64, device=cuda_device)
+    i = torch.zeros(4, dtype=torch.int64, device=cuda_device)
+    p = t.data_ptr()
+    two = lambda a, b: (ctypes.c_void_p * 2)(a, b)  # noqa: E731
+
+    def call(table=p, rows=4, ids=i.data_ptr(), U=1, D=4, n=1, param=two(p, p), grad=two(p, p), numel=4):
+        return capi.load_library().ge2_adagrad_step(table, p, rows, ids, U, None, p, D, 0.1, None, None, n, param, two(p, p), grad, numel, 0.1, 1e-10, 1.0, None)
+
+    for kw in (dict(table=None), dict(rows=-1), dict(ids=None), dict(U=-1), dict(D=0), dict(n=3), dict(n=-1), dict(param=two(None, p)), dict(n=2, grad=two(p, None)), dict(param=None), dict(numel=-1)):
+        assert call(**kw) == 1, kw
+    torch.cuda.synchronize()
+    assert bool((t == 1).all())
