@@ -14,12 +14,13 @@ __device__ __forceinline__ void adagrad_elem(float g, float& state, float& delta
     delta = __fmul_rn(neg_lr, __fdiv_rn(g, den));
 }
 
-// -g / (sqrt(s) + eps) with both operations rounded correctly, for s in [2^-40, 2^60], g zero or at least 2^-100 in size, and a denominator d
+// -g / (sqrt(s) + eps) with both operations rounded correctly, for s in [2^-40, 2^60], g zero or at least 2^-94 in size, and a denominator d
 // (an output) whose significand is not all ones.
 // Square root and quotient by the iterations of P. Markstein (IA-64 and Elementary Functions, 2000): from y ~ 1 / sqrt(s), the pair
 // (r, h) = (s y, y / 2) is refined once together, and the last correction r + (s - r r) h, whose remainder is exact, rounds correctly.  2 h then
 // is 1 / (r + eps) to 2^-13 or better (that is what the lower bound on s is for); two Newton steps round the reciprocal correctly, unless
-// the significand is all ones, and q + (g - q d) / d does the quotient.  Compared with the IEEE operations on 64 quotients for every
+// the significand is all ones, and q + (g - q d) / d does the quotient, provided that it is a normal number (the last sum would break a tie
+// between two subnormal ones the wrong way; that is what the bound on g is for: d is at most 2^30) and the remainder a multiple of 2^-149.  Compared with the IEEE operations on 64 quotients for every
 // significand of s at both parities of the exponent and on 2^34 random pairs.
 __device__ __forceinline__ float2 neg_step2(float2 g, float2 s, float2& d) {
     float2 y;
@@ -68,7 +69,7 @@ __device__ __forceinline__ void adagrad_elems(const float (&g)[N], float (&state
             most = max(most, max(__float_as_uint(d.x) << 9, __float_as_uint(d.y) << 9));
             upd[2 * k] = up.x, upd[2 * k + 1] = up.y, delta[2 * k] = __fmul_rn(-neg_lr, nq.x), delta[2 * k + 1] = __fmul_rn(-neg_lr, nq.y);
         }
-        fine = fine && least >= 2u * 0x0D800000u - 1u && most < 0xFFFFFE00u;  // 2^-100; all ones
+        fine = fine && least >= 2u * 0x10800000u - 1u && most < 0xFFFFFE00u;  // 2^-94; all ones
         if (__builtin_expect(!fine, 0)) {
 #pragma unroll
             for (int k = 0; k < N; k++) {

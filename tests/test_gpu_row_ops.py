@@ -54,6 +54,30 @@ def test_adagrad_is_ieee_over_the_whole_range(capi, cuda_device, D):
         assert same.all(), (g[~same][:4], st[~same][:4], got[~same][:4], want[~same][:4])
 
 
+@pytest.mark.parametrize("D", [1, 2, 4])
+def test_adagrad_quotients_around_the_smallest_normal_one(capi, cuda_device, D):
+    """Quotients from 2^-140 to 2^-120, ties between two subnormal numbers among them (random operands meet none): g is an odd number of halves of
+    the spacing, times a denominator of few bits that is no power of two."""
+    rng = np.random.default_rng(D)
+    n = 200_000
+    den = np.ldexp(rng.choice([3, 5, 7, 9, 11, 13, 15], n).astype(np.float64), rng.integers(20, 27, n))
+    st = (den * den).astype(np.float32)  # exact, and so is its root; epsilon is lost beside it
+    g = np.ldexp(1.0 + rng.random(n), rng.integers(-140, -120, n)) * den
+    few = n // 2
+    den[:few] = rng.choice([3 * 2.0**28, 5 * 2.0**27, 7 * 2.0**27, 3 * 2.0**27], few)  # up to 2^30, so that g of 21 bits more is not below 2^-100
+    st[:few] = (den * den)[:few]
+    g[:few] = (2 * rng.integers(1 << 19, 1 << 20, few) + 1) * 2.0**-150 * den[:few]
+    assert (g[:few].astype(np.float32) == g[:few]).all()
+    g = (g * rng.choice([-1, 1], n)).astype(np.float32)
+    g[0], st[0] = 1.0911102193146107e-30, 6.485183463413514e17
+    g, st = g.reshape(-1, D), st.reshape(-1, D)
+    delta, _ = capi.sparse_adagrad(torch.from_numpy(g).to(cuda_device), torch.from_numpy(st.copy()).to(cuda_device), 1.0)
+    want, _ = O.sparse_adagrad(g, st, 1.0)
+    got = delta.cpu().numpy()
+    same = got.view(np.int32) == want.view(np.int32)
+    assert same.all(), ((~same).sum(), g[~same][:4], st[~same][:4], got[~same][:4], want[~same][:4])
+
+
 @pytest.mark.parametrize("D", [50, 100, 128])
 def test_index_read_add_and_fused_scatter(capi, cuda_device, D):
     rng = np.random.default_rng(100 + D)
