@@ -33,9 +33,10 @@
 // group without turns, 246 + 244; with turns at the second half of O only, 229 + 227; halves of a tile as score tiles of their own (the
 // tensor pipe then has 1280 cycles a tile, and every hand-over twice), 264 + 278; an L2 prefetch of tiles to come, 227 + 224; five stages and
 // one X, 221 + 230; three stages, 325 + 287; the maximum of every 64 scores before their exponentials instead of sums of those, 253 + 209 (226 + 212).
-// P carries a factor 2^14, so that probabilities down to 2^-38 keep their full significand instead of falling into fp16's subnormal
-// range; dQ and dK leave this kernel with that factor still on them and the scatter kernel, their only reader, takes it off
-// (LpLayout::grad_unscale).
+// P carries a factor 2^14, for fp16's subnormal range: against its reference a P of the queries keeps its full significand down to 2^-28
+// and its last bit down to 2^-38; the same holds for a probability in the negatives' launch, whose reference is the row's lse (a row whose
+// positive leads by 2^38 and more adds nothing to dK).  dQ and dK leave this kernel with that factor still on them and the finish
+// kernel, their only reader, takes it off (LpLayout::grad_unscale).
 //
 // Warp roles, connected by mbarrier pipelines (no block-wide barrier inside the loops):
 //   warps 0-7   softmax: warp w takes rows 32 (w & 3) ... + 31 (its quarter of the tensor-memory lanes) of its group's (w >> 2) tiles
@@ -69,7 +70,9 @@ constexpr uint32_t kTmemCols = 512;
 constexpr float kMasked = -1e9f;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr int kWShift = 14;             // P is scaled by 2^14; undone by the reader of dQ / dK (kLpF16GradUnscale)
-constexpr float kHeadStart = 6.f;       // queries: log2 of how far the reference is set above the maximum it is taken from
+constexpr float kHeadStart = 6.f;       // queries: log2 of how far the reference is set above the maximum it is taken from ...
+constexpr float kFarthest = 14.f;       // ... and, for a positive that leads it, at most (the largest P of the tile then is 1)
+constexpr float kNothing = 128.f;       // log2 of how much smaller than the positive's a term of the row's sum is nothing, in fp32 too
 constexpr float kNoReference = -1e30f;  // queries: of a group without a tile of the block
 constexpr float kDeadRow = 1e30f;       // "lse" of a row past the end of its chunk: exp2(anything - 1e30) = 0
 
@@ -295,11 +298,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                     for (int j = 12; j < 28; j += 2) mx[(j >> 1) & 3] = max3(mx[(j >> 1) & 3], a[j], a[j + 1]);
                     return max3(max3(mx[0], a[28], a[29]), max3(mx[1], a[30], a[31]), fmaxf(mx[2], mx[3])) * kLog2e;
                 };
-                // Queries: the reference starts at the positive score (that is in the lse, so P is never smaller than the probability) or 2^6 above
-                // the maximum of the group's first tile, whichever is more.  It follows only when a P might leave fp16's range: O and the
-                // sum have to be rescaled then, for 32 rows at a time, so it should be rare (without the head start some row of a warp
-                // did in nearly every tile).  That is looked for in sums of the exponentials (of 16 of them: none is larger), not in a
-                // pass over the scores, which was a tenth of the launch.
+                // Queries: the reference starts at the positive score, but from 2^6 to 2^14 above the maximum of the group's first tile: a P of 1 or more then
+                // belongs to that maximum, 14 octaves above fp16's subnormal numbers.  (A reference at the positive alone took P's bits where the positive
+                // leads by more: dQ of such a row was off by 1 % at 20 nats, and zero at 28.)  Later tiles have 2^8 to 2^16 of room, less what
+                // a sum of 16 takes.  The reference follows only when a P might leave fp16's range: O and the sum have to be rescaled then, for 32
+                // rows at a time, so it should be rare: that is why it starts no lower where the positive leads.  Scores on trained tables (positives ahead
+                // by 0 to 11 octaves), B = 100 000, N = 2000, Dot 64 and 128: 200 and 248 us; with at most 2^10 above the maximum, 213 and 259;
+                // 2^8, 220 and 269 (a reference that moved towards the positive again: 1 us more).  It is looked for in sums of the exponentials (none of the 16 is larger), not in a pass over the
+                // scores, which was a tenth of the launch.  A first tile that is masked for the row as a whole says nothing about its scores: the
+                // reference is 2^-128 of the positive then.
                 if (!NEG && !begun && h == 1) {
                     float tmax = fmaxf(largest(va), largest(vb));
 #pragma unroll 1
@@ -308,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         tmem_ld_32x32(tS + k * 32, x);
                         tmax = fmaxf(tmax, largest(x));
                     }
-                    m = fmaxf(m, tmax + kHeadStart);
+                    m = fmaxf(fmaxf(tmax + kHeadStart, m - kNothing), fminf(m, tmax + kFarthest));
                 }
 #pragma unroll 1
                 for (bool settled = false;; settled = true) {

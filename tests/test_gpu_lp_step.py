@@ -311,6 +311,47 @@ def test_streaming_softmax_reference_moves(capi, cuda_device, kind, B, C, N, D, 
         assert np.linalg.norm(got[key] - getattr(o, key)) <= 2e-2 * np.linalg.norm(getattr(o, key)), key
 
 
+@pytest.mark.parametrize("B,C,N,D", [(600, 200, 1000, 128), (1400, 1400, 100, 128), (990, 330, 1100, 64), (1400, 350, 1100, 50)])
+@pytest.mark.parametrize("order", ["drawn", "rising", "masked"])
+def test_streaming_softmax_row_by_row(capi, cuda_device, B, C, N, D, order):
+    """dQ of every row against float64, relative to that row, however far its positive leads the largest negative: 0 to 70 nats (beyond 80 a
+    probability leaves fp32).  Sources and destinations use other coordinates than the negatives, so the gradient of a source in the negatives'
+    coordinates is dQ alone; operands are multiples of 2^-6 and at most 4, so fp16 holds them and fp32 their products.  "masked": the first 128
+    negatives are masked for every row that has a chunk to itself (those the filter words can mask).
+    Bound: P is rounded to 11 bits, and where it is small to a multiple of at most 2^-25 of a row's largest (N of them); four arguments of exp2 and the
+    lse, of up to 2^8, are rounded to 24 bits; N / 16 sums in tensor memory are cut off after 23; nothing cancels, since the negatives' rows are positive."""
+    rng = np.random.default_rng(B + D)
+    npc, h = -(-B // C), D // 2
+    U = 2 * B + C * N
+    grid = lambda a: np.round(a * 64) / 64  # noqa: E731
+    emb = np.zeros((U, D), np.float32)
+    src, dst, negs = np.arange(B), B + np.arange(B), (2 * B + np.arange(C * N)).reshape(C, N)
+    emb[src, :h] = grid(rng.uniform(-0.5, 0.5, (B, h)))
+    emb[negs.ravel(), :h] = grid(rng.uniform(0.5, 2.0, (C * N, h)))
+    chunk = np.arange(B) // npc
+    scores = np.einsum("bd,bnd->bn", emb[src, :h].astype(np.float64), emb[negs[chunk], :h].astype(np.float64))
+    if order == "rising":
+        by = np.argsort(scores[np.arange(C) * npc], axis=1)  # for the first row of every chunk
+        negs = np.take_along_axis(negs, by, axis=1)
+        scores = np.take_along_axis(scores, by[chunk], axis=1)
+    filt = np.empty((0, 2), np.int64)
+    if order == "masked":
+        rows = np.arange(0, B, npc)
+        filt = np.stack([np.repeat(rows, min(N - 1, 128)), np.tile(np.arange(min(N - 1, 128)), len(rows))], 1)
+        scores[filt[:, 0], filt[:, 1]] = -np.inf
+    lead = rng.choice([0.0, 4.0, 9.0, 14.0, 20.0, 28.0, 45.0, 70.0], B)
+    emb[src, h:h + 8], emb[dst, h:h + 8] = 4.0, grid((lead + scores.max(1)) / 32)[:, None]  # eight products of 4 and a multiple of 2^-6
+    pos = 32 * emb[dst, h].astype(np.float64)
+    lse = np.logaddexp(pos, np.logaddexp.reduce(scores, axis=1))
+    want = np.einsum("bn,bnd->bd", np.exp(scores - lse[:, None]), emb[negs[chunk], :h].astype(np.float64))
+    case = workloads.BatchCase("DISTMULT", np.stack([src, dst], 1).astype(np.int64), emb, np.zeros_like(emb), None, None, negs.astype(np.int64), None, None, filt)
+    got = run_lp_step(capi, case, cuda_device, "f16", "pairs", dump_scores=False)
+    assert got["status"] == 0
+    err = np.abs(got["node_grad"][src, :h] - want).max(1) / want.max(1)
+    bound = 2.0**-11 + N * 2.0**-25 + 4 * 2.0**-17 + N / 16 * 2.0**-23
+    assert err.max() <= bound, [(x, float(err[lead == x].max())) for x in np.unique(lead)]
+
+
 @pytest.mark.parametrize("kind,B,C,N,D", [("COMPLEX", 600, 3, 300, 50), ("COMPLEX", 500, 2, 7001, 100), ("DISTMULT", 300, 2, 3000, 128), ("DISTMULT", 257, 2, 640, 3)])
 def test_one_node_in_most_edges_and_negatives(capi, cuda_device, kind, B, C, N, D):
     """Rows of a node that most edges and degree negatives have are added up where they meet, and leave as sums."""
