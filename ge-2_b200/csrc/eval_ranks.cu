@@ -50,7 +50,7 @@ struct EvalArgs {
     uint2* open_list;             // (query row, candidate column) of comparisons the counting pass left open
     unsigned long long* open_count;  // how many were put there (may exceed open_cap: the rest was evaluated in place)
     int64_t open_cap;
-    unsigned char* stage;         // D > 64: [kNumSMs] split candidate tiles on their way into shared memory
+    unsigned char* stage;         // D > 64: [kNumSMs] split candidate tiles on their way into shared memory; null: no room for them
     int64_t Bp;
     int S, ld;
     int vec;                      // floats per access to a candidate row: 4 or 2 (rows aligned and whole), else 1
@@ -792,7 +792,7 @@ int launch_count(const EvalArgs& a, CountSched sc, const CUtensorMap& tmQ, cudaS
     }
     if (sc.groups > 65535) return GE2_ERR_UNSUPPORTED;
     const dim3 grid((unsigned)std::min<int64_t>(std::max(1, kNumSMs / sc.groups), sc.cand_tiles), (unsigned)sc.groups);
-    sc.staged = NB == 2 && sc.cand_tiles > grid.x && (int64_t)grid.x * grid.y <= kNumSMs;
+    sc.staged = NB == 2 && a.stage != nullptr && sc.cand_tiles > grid.x && (int64_t)grid.x * grid.y <= kNumSMs;
     GE2_CUDA_TRY(launch_after(kernel, grid, dim3(kCountThreads), CountSmem<NB>::kBytes, stream, tmQ, a, sc));
     return GE2_OK;
 }
@@ -820,10 +820,11 @@ extern "C" int ge2_eval_ranks(const ge2_eval_desc* d, ge2_stream_t stream_) {
         return GE2_ERR_INVALID_ARGUMENT;
     const int64_t num_cols = d->neg_ids != nullptr ? d->num_negs : d->num_nodes;
     if (num_cols <= 0) return GE2_ERR_INVALID_ARGUMENT;
-    if (d->workspace == nullptr || ((uintptr_t)d->workspace & 255) != 0 || d->workspace_bytes < ge2_eval_workspace_bytes(d)) return GE2_ERR_WORKSPACE;
+    const EvalSections at(d);
+    // the last section can be missing: a candidate tile then is split only when the one before it is done with
+    if (d->workspace == nullptr || ((uintptr_t)d->workspace & 255) != 0 || d->workspace_bytes < at.stage) return GE2_ERR_WORKSPACE;
 
     cudaStream_t stream = as_stream(stream_);
-    const EvalSections at(d);
     char* p = (char*)d->workspace;
     EvalArgs a;
     a.d = *d;
@@ -842,7 +843,7 @@ extern "C" int ge2_eval_ranks(const ge2_eval_desc* d, ge2_stream_t stream_) {
     a.open_list = (uint2*)(p + at.open);
     a.open_count = (unsigned long long*)(p + at.open_count);
     a.open_cap = at.open_cap;
-    a.stage = (unsigned char*)(p + at.stage);
+    a.stage = d->workspace_bytes < at.bytes ? nullptr : (unsigned char*)(p + at.stage);
     const int64_t rows = (int64_t)S * a.Bp;
     if (rows > 0x7fffffffLL) return GE2_ERR_UNSUPPORTED;
     // the set of filter pairs and the counter behind it

@@ -452,7 +452,8 @@ typedef struct ge2_eval_desc {
     float *pos_scores;     /* [B] out, optional */
     float *inv_pos_scores; /* [B] out, optional */
     int32_t *status;       /* device int32, GE2_STATUS_* bits OR-ed in; may be NULL */
-    void *workspace;       /* 256-byte aligned, ge2_eval_workspace_bytes(desc) bytes */
+    void *workspace;       /* 256-byte aligned, ge2_eval_workspace_bytes(desc) bytes.  For D > 64 and more than 256 candidates the last
+                              148 * 131072 of them are optional: ranks are the same without, wide tables take 5 % longer */
     size_t workspace_bytes;
 } ge2_eval_desc;
 GE2_API size_t ge2_eval_workspace_bytes(const ge2_eval_desc *desc);

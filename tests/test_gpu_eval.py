@@ -131,3 +131,32 @@ def test_ranks_are_exact_for_query_rows_of_any_size(capi, cuda_device, D, size):
     t = lambda a: torch.from_numpy(a).to(cuda_device)  # noqa: E731
     got_d, got_s = capi.eval_ranks("DISTMULT", t(table), t(edges), t(rel), t(rel), dst_filter=t(filt), src_filter=t(filt))
     assert np.array_equal(got_d.cpu().numpy(), exp_d) and np.array_equal(got_s.cpu().numpy(), exp_s)
+
+
+@pytest.mark.parametrize("nodes,D", [(148 * 256 + 1, 100), (77_000, 66), (300, 128)])
+def test_a_workspace_without_the_optional_part_will_do(capi, cuda_device, monkeypatch, nodes, D):
+    """the last 148 x 128 KB, in which wide candidate tiles are split ahead; one byte less than that is refused"""
+    lib = capi.load_library()
+
+    class Less:
+        def __init__(self, less):
+            self.less = less
+
+        def __getattr__(self, name):
+            return getattr(lib, name)
+
+        def ge2_eval_workspace_bytes(self, d):
+            return lib.ge2_eval_workspace_bytes(d) - self.less
+
+    rng = np.random.default_rng(nodes)
+    table = rng.standard_normal((nodes, D)).astype(np.float32)
+    edges = rng.integers(0, nodes, (130, 2)).astype(np.int64)
+    exp, _ = O.eval_ranks("DISTMULT", table, None, None, edges, np.empty((0, 2), np.int64), None)
+    t_table, t_edges = torch.from_numpy(table).to(cuda_device), torch.from_numpy(edges).to(cuda_device)
+    for less in (1, 148 * 131072):
+        monkeypatch.setattr(capi, "load_library", lambda less=less: Less(less))
+        got, _ = capi.eval_ranks("DISTMULT", t_table, t_edges)
+        assert np.array_equal(got.cpu().numpy(), exp)
+    monkeypatch.setattr(capi, "load_library", lambda: Less(148 * 131072 + 1))
+    with pytest.raises(capi.Ge2Error):
+        capi.eval_ranks("DISTMULT", t_table, t_edges)
