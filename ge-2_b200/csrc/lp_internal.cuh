@@ -78,7 +78,8 @@ inline bool lp_uses_flash(const ge2_lp_desc& d, int S, int64_t CN, int ld) {
     return mb > (64 + over / (row_blocks * sqrt(row_blocks))) * (padded ? 2 : 1);
 }
 
-inline LpLayout lp_make_layout(const ge2_lp_desc& d, void* base) {
+// streaming: false = the two-pass form whatever lp_uses_flash says (its layout is the other's without the last section)
+inline LpLayout lp_make_layout(const ge2_lp_desc& d, void* base, bool streaming = true) {
     LpLayout L;
     L.S = (d.has_relations && d.use_inverse) ? 2 : 1;
     L.npc = rows_per_chunk(d.B, d.C);
@@ -106,8 +107,9 @@ inline LpLayout lp_make_layout(const ge2_lp_desc& d, void* base) {
     const int row_blocks = (L.npc + 127) / 128;
     L.n_items = L.S * d.C * row_blocks;
     size_t olse2 = take((size_t)L.n_items * 128 * 4);
-    size_t oopart = take(lp_uses_flash(d, L.S, L.CN, L.ld) ? (size_t)kNumSMs * 2 * 128 * L.ld * 4 : 0);
-    L.o_part = lp_uses_flash(d, L.S, L.CN, L.ld) ? (float*)(p + oopart) : nullptr;
+    streaming = streaming && lp_uses_flash(d, L.S, L.CN, L.ld);
+    size_t oopart = take(streaming ? (size_t)kNumSMs * 2 * 128 * L.ld * 4 : 0);
+    L.o_part = streaming ? (float*)(p + oopart) : nullptr;
     L.dQ = (float*)(p + odQ);
     L.dK = (float*)(p + odK);
     L.pos = (float*)(p + opos);

@@ -686,6 +686,8 @@ extern "C" int ge2_lp_step(const ge2_lp_desc* desc, ge2_stream_t stream_) {
     a.d = whole_desc(desc);
     if (desc->workspace == nullptr || ((uintptr_t)desc->workspace & 255) != 0) return GE2_ERR_WORKSPACE;
     a.L = lp_make_layout(*desc, desc->workspace);
+    // no room for the streaming form's parts (a workspace for a larger batch that takes the other form, or of an earlier version's size)
+    if (desc->workspace_bytes < a.L.bytes) a.L = lp_make_layout(*desc, desc->workspace, false);
     if (desc->workspace_bytes < a.L.bytes) return GE2_ERR_WORKSPACE;
     const LpLayout& L = a.L;
     cudaStream_t stream = as_stream(stream_);

@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "adagrad.cuh"
+#include "lp_internal.cuh"
 #include "unique_map.cuh"
 
 namespace ge2 {
@@ -775,6 +776,7 @@ extern "C" int ge2_train_step(const ge2_train_desc* t, ge2_stream_t stream) {
     size_t need = 0;
     int rc = ge2_lp_workspace_bytes(&d, &need);  // also: is the descriptor a valid one?
     if (rc != GE2_OK) return rc;
+    need = lp_make_layout(d, nullptr, false).bytes;  // what ge2_lp_step can do with
     if (d.workspace == nullptr || ((uintptr_t)d.workspace & 255) != 0 || d.workspace_bytes < need) return GE2_ERR_WORKSPACE;
     if (t->edges == nullptr || t->cols <= 0 || t->n_deg < 0 || t->n_deg > d.N || t->domain <= 0 || t->table_rows <= 0) return GE2_ERR_INVALID_ARGUMENT;
     if (t->packed == nullptr || t->unique == nullptr || t->inverse == nullptr || t->count == nullptr || (t->n_deg > 0 && t->deg_rows == nullptr))

@@ -178,7 +178,8 @@ typedef struct ge2_lp_desc {
     float *inv_neg_scores;
 
     int32_t *status;      /* device int32, GE2_STATUS_* bits are OR-ed in; may be NULL             */
-    void *workspace;      /* ge2_lp_workspace_bytes() bytes, 256-byte aligned                      */
+    void *workspace;      /* ge2_lp_workspace_bytes() bytes, 256-byte aligned.  Where that is more than the same step would need in the other of
+                             its two fp16 forms (by 37888 * 64 or 128 floats, D up to 64 or above), so much less will do: the other form is taken */
     size_t workspace_bytes;
 
     /* read when flags has GE2_LP_HAS_ROW_UPDATE; optional (both pointers or neither): the optimizer step of the rows that need no sum over occurrences, inside the scatter.  row_shared[U]

@@ -20,9 +20,9 @@ def dev(a, device, dtype=None):
     return t.to(device)
 
 
-def run_lp_step(capi, case, device, precision="fp32", filter_mode="pairs", indirect=False, dump_scores=True):
+def run_lp_step(capi, case, device, precision="fp32", filter_mode="pairs", indirect=False, dump_scores=True, less_workspace=0):
     """Returns a dict of numpy outputs.  filter_mode: 'pairs' | 'deg_rows' | 'none'.  indirect: node_emb is a larger table
-    addressed through row_index (the fused pipeline's way)."""
+    addressed through row_index (the fused pipeline's way).  less_workspace: bytes by which the workspace falls short of what is asked for."""
     B, C, N, D, R, U = case.dims
     has_rel = case.rel is not None
     S = 2 if (has_rel and case.inv_rel is not None and case.src_negs is not None) else 1
@@ -66,7 +66,7 @@ def run_lp_step(capi, case, device, precision="fp32", filter_mode="pairs", indir
         node_grad=out["node_grad"], rel_grad=rel_grad, inv_rel_grad=inv_rel_grad, loss=out["loss"],
         pos_scores=out.get("pos_scores"), neg_scores=out.get("neg_scores"), inv_pos_scores=out.get("inv_pos_scores"),
         inv_neg_scores=out.get("inv_neg_scores"), status=out["status"])
-    ws = torch.empty(capi.lp_workspace_bytes(d), dtype=torch.uint8, device=device)
+    ws = torch.empty(capi.lp_workspace_bytes(d) - less_workspace, dtype=torch.uint8, device=device)
     d.workspace, d.workspace_bytes = ws.data_ptr(), ws.numel()
     capi.lp_step(d)
     torch.cuda.synchronize()

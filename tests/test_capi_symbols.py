@@ -197,6 +197,20 @@ def test_whole_step_refuses_what_does_not_fit_together(ge2):
     assert call(t) == 3
 
 
+def test_whole_step_takes_a_workspace_without_the_streaming_forms_parts(ge2):
+    """the smaller of the two sizes that an fp16 step can do with; what is refused next is the missing edge list"""
+    lib, capi = ge2.load_library(), ge2.capi
+    t, lp = _train_desc(capi)
+    lp.precision, lp.B, lp.C, lp.N, lp.D, lp.emb_stride, lp.n_deg, lp.deg_sample_rows = 1, 10368, 27, 1300, 50, 50, 0, None
+    need = ctypes.c_size_t()
+    assert lib.ge2_lp_workspace_bytes(ctypes.byref(lp), ctypes.byref(need)) == 0
+    t.edges = None
+    parts = 148 * 2 * 128 * 64 * 4
+    for size, rc in ((need.value, 1), (need.value - parts, 1), (need.value - parts - 1, 3)):
+        lp.workspace_bytes = size
+        assert lib.ge2_train_step(ctypes.byref(t), None) == rc
+
+
 def test_train_struct_matches_header(ge2):
     import subprocess
     import tempfile

@@ -352,6 +352,21 @@ def test_streaming_softmax_row_by_row(capi, cuda_device, B, C, N, D, order):
     assert err.max() <= bound, [(x, float(err[lead == x].max())) for x in np.unique(lead)]
 
 
+@pytest.mark.parametrize("kind,B,C,N,D", [("DISTMULT", 10368, 27, 1300, 50), ("COMPLEX", 330, 110, 1000, 66)])
+def test_streaming_softmax_gives_way_where_its_parts_have_no_room(capi, cuda_device, kind, B, C, N, D):
+    """shapes of the streaming form with a workspace of the two-pass form's size, and a byte less than that"""
+    case = workloads.make_case(kind, B, C, N, D, 5, 150, min(N, 50), 9 + D)
+    o = O.lp_train_forward_backward(case.kind, case.edges, case.emb, case.rel, case.inv_rel, case.dst_negs, case.src_negs, case.filt, case.filt)
+    parts = 148 * 2 * 128 * (64 if D <= 64 else 128) * 4
+    got = run_lp_step(capi, case, cuda_device, "f16", "pairs", dump_scores=False, less_workspace=parts)
+    assert got["status"] == 0
+    assert abs(got["loss"] - o.loss) <= 1e-2 * abs(o.loss)
+    for key in ("node_grad", "rel_grad", "inv_rel_grad"):
+        assert rel_err(got[key], getattr(o, key)) <= 1e-2, key
+    with pytest.raises(capi.Ge2Error):
+        run_lp_step(capi, case, cuda_device, "f16", "pairs", dump_scores=False, less_workspace=parts + 1)
+
+
 @pytest.mark.parametrize("kind,B,C,N,D", [("COMPLEX", 600, 3, 300, 50), ("COMPLEX", 500, 2, 7001, 100), ("DISTMULT", 300, 2, 3000, 128), ("DISTMULT", 257, 2, 640, 3)])
 def test_one_node_in_most_edges_and_negatives(capi, cuda_device, kind, B, C, N, D):
     """Rows of a node that most edges and degree negatives have are added up where they meet, and leave as sums."""
