@@ -119,8 +119,14 @@ class PeerGradients:
 class BatchPipeline:
     """Owns the per-batch scratch (ids, unique map, gradients, workspaces); tables are owned by the caller."""
 
-    # Ids of a batch for every SM that the scores kernels leave over, up to which the next batch's sampler and unique-map run there: a thousand
-    # ids an SM take them about 5 us, and they have the time of the scores (8 000: 38 of 42 us)
+    # Ids of a batch for every SM that the scores kernels leave over, up to which the next batch's sampler and unique-map run there.  They take
+    # about 11 us and 0.7 us for every thousand ids an SM, beside scores of 13 us and more.  The pipelined step at 320 shapes (1 000 ... 60 000
+    # edges, 60 ... 2 000 negatives, both precisions), on those SMs : behind the scores, mean ratio by ids an SM: up to 6 000 0.92;
+    # 6 000 ... 16 384 0.98; to 20 000 0.99; to 26 000 1.01; to 40 000 1.06; to 70 000 1.10; above 1.35.  In us: fp16, 3 061 edges, Dot 64,
+    # 5 700 ids an SM 35.4 : 42.9; fp32, 47 126, Dot 64, 13 400 121.1 : 132.2; fp16, 10 751, Dot 100, 14 700 127.0 : 118.6 (finish is long there);
+    # fp32, 7 144, ComplEx 50, 17 200 150.3 : 155.8; fp16, 12 413, ComplEx 50, 30 200 138.0 : 138.5; 14 711, ComplEx 64, 39 200 122.3 : 109.9.
+    # The way that is taken is 0.7 % slower than the better one on average (never there: 6.4 %, always: 4.7); measured times of these kernels,
+    # the scores and finish in place of the ids would leave 0.5.
     IDS_PER_IDLE_SM = 16384
 
     def __init__(self, cfg: PipelineConfig, table, state, rel=None, rel_state=None, inv_rel=None, inv_rel_state=None):
