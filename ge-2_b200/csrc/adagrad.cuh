@@ -19,9 +19,9 @@ __device__ __forceinline__ void adagrad_elem(float g, float& state, float& delta
 // Square root and quotient by the iterations of P. Markstein (IA-64 and Elementary Functions, 2000): from y ~ 1 / sqrt(s), the pair
 // (r, h) = (s y, y / 2) is refined once together, and the last correction r + (s - r r) h, whose remainder is exact, rounds correctly.  2 h then
 // is 1 / (r + eps) to 2^-13 or better (that is what the lower bound on s is for); two Newton steps round the reciprocal correctly, unless
-// the significand is all ones, and q + (g - q d) / d does the quotient, provided that it is a normal number (the last sum would break a tie
-// between two subnormal ones the wrong way; that is what the bound on g is for: d is at most 2^30) and the remainder a multiple of 2^-149.  Compared with the IEEE operations on 64 quotients for every
-// significand of s at both parities of the exponent and on 2^34 random pairs.
+// the significand is all ones, and q + (g - q d) / d does the quotient, provided that it is a normal number: the last sum would break a tie
+// between two subnormal ones the wrong way.  That is what the bound on g is for (d is at most 2^30); the remainder is a multiple of 2^-141 then.
+// Compared with the IEEE operations on 64 quotients for every significand of s at both parities of the exponent and on 2^34 random pairs.
 __device__ __forceinline__ float2 neg_step2(float2 g, float2 s, float2& d) {
     float2 y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(s.x));

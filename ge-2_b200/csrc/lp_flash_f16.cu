@@ -38,6 +38,15 @@
 // positive leads by 2^38 and more adds nothing to dK).  dQ and dK leave this kernel with that factor still on them and the finish
 // kernel, their only reader, takes it off (LpLayout::grad_unscale).
 //
+// A row's reference starts at its positive score, but from 2^6 to 2^14 above the maximum of the group's first tile: a P of 1 or more then belongs
+// to that maximum, 14 octaves above the subnormal numbers, and later tiles have 2^8 to 2^16 of room, less what a sum of 16 takes, before the
+// reference has to follow.  The positive alone, as a reference, takes P's bits where it leads by more: dQ of a row was off by 1 % at
+// 20 nats and zero at 28.  It starts no lower than that because following costs: B = 100 000, N = 2000, tables trained for 400 steps (positives
+// ahead by up to 2^11), Dot 64 and 128, both launches: 200 and 248 us; with at most 2^10 above the maximum 213 and 259, with 2^8 220
+// and 269.  Where one batch of DistMult 128 is trained 650 times over, positives are ahead by 2^10 to 2^50 and later tiles' maxima
+// ahead of the first's by as much: 271 us for the queries' launch, 227 with the positive alone.  (Moving towards the positive again: 267 there, 1 us
+// more elsewhere.)
+//
 // Warp roles, connected by mbarrier pipelines (no block-wide barrier inside the loops):
 //   warps 0-7   softmax: warp w takes rows 32 (w & 3) ... + 31 (its quarter of the tensor-memory lanes) of its group's (w >> 2) tiles
 //   warps 8-11  drain: O -> registers (-> weighted sum of the two groups) -> staging slab -> TMA store / reduce-add
@@ -65,7 +74,7 @@ constexpr int kThreads = 512;           // 128 registers each at the launch; the
 constexpr int kLaunchRegs = 128, kDrainRegs = 184, kServiceRegs = 2 * kLaunchRegs - kDrainRegs;
 constexpr int kDrainWarps = 4, kTmaWarp = 12, kMmaWarp = 13, kHelpWarp = 15;  // (an issuing warp a group)
 constexpr int kStages = 4;              // Y ring: two tiles wait for their O contraction, two are on their way
-constexpr int kInfoStages = 4;          // ring of what warps 22-23 find out about tiles
+constexpr int kInfoStages = 4;          // ring of what warp 15 finds out about tiles
 constexpr uint32_t kTmemCols = 512;
 constexpr float kMasked = -1e9f;
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
@@ -298,15 +307,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                     for (int j = 12; j < 28; j += 2) mx[(j >> 1) & 3] = max3(mx[(j >> 1) & 3], a[j], a[j + 1]);
                     return max3(max3(mx[0], a[28], a[29]), max3(mx[1], a[30], a[31]), fmaxf(mx[2], mx[3])) * kLog2e;
                 };
-                // Queries: the reference starts at the positive score, but from 2^6 to 2^14 above the maximum of the group's first tile: a P of 1 or more then
-                // belongs to that maximum, 14 octaves above fp16's subnormal numbers.  (A reference at the positive alone took P's bits where the positive
-                // leads by more: dQ of such a row was off by 1 % at 20 nats, and zero at 28.)  Later tiles have 2^8 to 2^16 of room, less what
-                // a sum of 16 takes.  The reference follows only when a P might leave fp16's range: O and the sum have to be rescaled then, for 32
-                // rows at a time, so it should be rare: that is why it starts no lower where the positive leads.  Scores on trained tables (positives ahead
-                // by 0 to 11 octaves), B = 100 000, N = 2000, Dot 64 and 128: 200 and 248 us; with at most 2^10 above the maximum, 213 and 259;
-                // 2^8, 220 and 269 (a reference that moved towards the positive again: 1 us more).  It is looked for in sums of the exponentials (none of the 16 is larger), not in a pass over the
-                // scores, which was a tenth of the launch.  A first tile that is masked for the row as a whole says nothing about its scores: the
-                // reference is 2^-128 of the positive then.
+                // Queries: the first reference (see above).  It follows only when a P might leave fp16's range: O and the sum have to be rescaled then, for
+                // 32 rows at a time.  That is looked for in sums of the exponentials (of 16 of them: none is larger), not in a pass over
+                // the scores, which was a tenth of the launch.  A first tile that is masked for the row as a whole says nothing about its scores:
+                // the reference is 2^-128 of the positive then.
                 if (!NEG && !begun && h == 1) {
                     float tmax = fmaxf(largest(va), largest(vb));
 #pragma unroll 1

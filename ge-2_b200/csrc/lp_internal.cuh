@@ -40,7 +40,7 @@ struct LpLayout {
     float* lse2s;     // [S*C][row_blocks*128] row logsumexp in base-2 units minus the probability scale exponent; 1e30 for rows past the chunk
     float* o_part;    // f16: [CTAs][2][128][ld] parts of dQ of the (at most two) row blocks a CTA of the query launch shares with others
     int n_items;        // S * C * row_blocks
-    float grad_unscale; // factor the scatter kernel applies to what it reads from dQ / dK: 1, or 2^-14 on the tensor path
+    float grad_unscale; // factor the finish kernel applies to what it reads from dQ / dK: 1, or 2^-14 on the tensor path
     size_t bytes;
 };
 

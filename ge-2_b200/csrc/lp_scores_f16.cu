@@ -33,9 +33,10 @@
 // tile to tile, so the contraction of one tile runs while the other's result is drained.  Logsumexp pass: two score
 // accumulators at 0 and 128.
 // (32-bit tf32 operands cannot do this: the hardware transposes them only from a different, 32-byte-atom swizzle.)
-// W is scaled by 2^14 before it is packed to fp16, so that probabilities down to 2^-38 keep their full significand instead
-// of falling into fp16's subnormal range; dQ and dK leave this kernel with that factor still on them and the scatter
-// kernel, their only reader, takes it off (LpLayout::grad_unscale).
+// W is scaled by 2^14 before it is packed to fp16, so that probabilities down to 2^-28 keep their full significand, and those
+// down to 2^-38 their last bit, instead of falling into fp16's subnormal range: a row whose positive leads its negatives by
+// more has no gradient from them.  dQ and dK leave this kernel with that factor still on them and the finish kernel, their
+// only reader, takes it off (LpLayout::grad_unscale).
 //
 // Warp roles, connected by mbarrier pipelines (no block-wide barrier inside the loops):
 //   warps 0-15  softmax: thread = accumulator row (tensor-memory lane).  lse pass: two groups of 8 warps take alternate
@@ -660,7 +661,7 @@ __global__ void __launch_bounds__(kThreadsB, 1)
                     lrow = __ldg(&L.lse2s[(int64_t)un.item * BM + my_row]);
                 } else {
                     // A block that the lse pass split between CTAs: combine the partial (max, sum) pairs its sharers left;
-                    // the CTA of this launch that starts the block also writes the lse for the scatter kernel and adds the
+                    // the CTA of this launch that starts the block also writes the lse for the finish kernel and adds the
                     // rows' loss terms.
                     const int64_t grow = (int64_t)s * L.Bp + row_base + my_row;
                     const bool live = my_row < min(BM, L.npc - un.rb * BM);

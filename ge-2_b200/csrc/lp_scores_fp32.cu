@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(kThreadsB, 1)
                     lrow = __ldg(&L.lse2s[(int64_t)un.item * BM + my_row]);
                 } else {
                     // combine the partial (max, sum) pairs its sharers left; the CTA that starts the block here also writes the lse for
-                    // the scatter kernel and adds the rows' loss terms
+                    // the finish kernel and adds the rows' loss terms
                     const int64_t grow = (int64_t)s * L.Bp + brow;
                     const bool writer = un.tile == 0 && half == 0;
                     float loss = 0.f;
