@@ -125,8 +125,9 @@ class BatchPipeline:
     # 6 000 ... 16 384 0.98; to 20 000 0.99; to 26 000 1.01; to 40 000 1.06; to 70 000 1.10; above 1.35.  In us: fp16, 3 061 edges, Dot 64,
     # 5 700 ids an SM 35.4 : 42.9; fp32, 47 126, Dot 64, 13 400 121.1 : 132.2; fp16, 10 751, Dot 100, 14 700 127.0 : 118.6 (finish is long there);
     # fp32, 7 144, ComplEx 50, 17 200 150.3 : 155.8; fp16, 12 413, ComplEx 50, 30 200 138.0 : 138.5; 14 711, ComplEx 64, 39 200 122.3 : 109.9.
-    # The way that is taken is 0.7 % slower than the better one on average (never there: 6.4 %, always: 4.7); measured times of these kernels,
-    # the scores and finish in place of the ids would leave 0.5.
+    # The way that is taken is 0.7 % slower than the better one on average (never there: 6.4 %, always: 4.7), at worst 9.5 % on those SMs (5 642
+    # edges, DistMult 50, 2.9 M nodes: 63.4 : 57.9) and 22 % behind the scores (4 060, DistMult 64, 19 300 ids an SM: 62.5 : 76.2).  A linear
+    # rule on the measured times of these kernels, the scores and finish in place of the ids: 0.5 % on average, 11 % at worst.
     IDS_PER_IDLE_SM = 16384
 
     def __init__(self, cfg: PipelineConfig, table, state, rel=None, rel_state=None, inv_rel=None, inv_rel_state=None):
