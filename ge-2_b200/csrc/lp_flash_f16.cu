@@ -44,8 +44,8 @@
 // 20 nats and zero at 28.  It starts no lower than that because following costs: B = 100 000, N = 2000, tables trained for 400 steps (positives
 // ahead by up to 2^11), Dot 64 and 128, both launches: 200 and 248 us; with at most 2^10 above the maximum 213 and 259, with 2^8 220
 // and 269.  Where one batch of DistMult 128 is trained 650 times over, positives are ahead by 2^10 to 2^50 and later tiles' maxima
-// ahead of the first's by as much: 271 us for the queries' launch, 227 with the positive alone.  (Moving towards the positive again: 267 there, 1 us
-// more elsewhere.)
+// ahead of the first's by as much: 271 us for the queries' launch, 227 with the positive alone.  (Moving as far towards the positive again, and all
+// rows of the warp at once: 257 there, 1 to 2 us more on the tables before.)
 //
 // Warp roles, connected by mbarrier pipelines (no block-wide barrier inside the loops):
 //   warps 0-7   softmax: warp w takes rows 32 (w & 3) ... + 31 (its quarter of the tensor-memory lanes) of its group's (w >> 2) tiles
